@@ -142,6 +142,28 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 columns of this thread's row, asked for and not waited for; tmem_wait32 waits for every load asked for so far and
+// hands the registers on (they are operands of the wait, so nothing that reads them is moved ahead of it).
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.wait::ld.sync.aligned;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+          "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+          "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+        :: "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 bf16) with the
 // 128-byte swizzle: 8-row groups 1024 bytes apart, version 1, layout type SWIZZLE_128B.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
@@ -154,14 +176,15 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return d;
 }
 
-__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + __expf(-g)) * u; }
+// __fdividef: the quotient to 2 ulp; where 1 + e^-g overflows it gives the 0 that the division gives.
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 // The gated unit of the epilogue.  limit == 0: SwiGLU, silu(g) * u.  limit > 0: the clamped unit,
 // g' = min(g, limit), u' = clamp(u, -limit, limit), g' * sigmoid(slope * g') * (u' + 1).
 __device__ __forceinline__ float gated_unit(float limit, float slope, float g, float u) {
     if (limit > 0.0f) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + __expf(-slope * g)) * (u + 1.0f);
+        return __fdividef(g, 1.0f + __expf(-slope * g)) * (u + 1.0f);
     }
     return silu_mul(g, u);
 }
@@ -212,15 +235,29 @@ struct SmemLayout {
 //   m = 0: relu(z)^2   1: z * sigmoid(z)   2: 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))   3: relu(z)
 //       4: 0.5 z (1 + erf(z / sqrt(2)))
 __device__ __forceinline__ void epilogue_act(float* v, int m) {
+    if (m == 0) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float z = v[i];
-        if (m == 0) { const float r = fmaxf(z, 0.0f); v[i] = r * r; }
-        else if (m == 1) v[i] = z / (1.0f + __expf(-z));
-        else if (m == 2) v[i] = 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-        else if (m == 4) v[i] = 0.5f * z * (1.0f + erff(z * 0.7071067811865476f));
-        else v[i] = fmaxf(z, 0.0f);
+        for (int i = 0; i < 16; ++i) { const float r = fmaxf(v[i], 0.0f); v[i] = r * r; }
+    } else if (m == 1) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __fdividef(v[i], 1.0f + __expf(-v[i]));
+    } else if (m == 2) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
+    } else if (m == 4) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + erff(v[i] * 0.7071067811865476f));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
     }
+}
+
+// 32 bytes in one store.  The lanes of a warp write to 32 rows, so a store costs a line a lane whatever its width: half as
+// many stores are half the time of an epilogue that is bound by them.
+__device__ __forceinline__ void store_32b(void* p, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                 "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
 }
 
 // Epilogue for 16 consecutive accumulator columns [c0, c0+16) of this thread's row.
@@ -232,7 +269,15 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float* v,
         const int n0 = b0 + c0;
         if (EPI == EPI_F32) {
             float* o = (float*)p.out + (size_t)a_row * p.ldc + n0;
-            if (n0 + 16 <= p.b_rows && (((size_t)o) & 15) == 0) {
+            if (n0 + 16 <= p.b_rows && (((size_t)o) & 31) == 0) {
+#pragma unroll
+                for (int i = 0; i < 16; i += 8) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) w[k] = __float_as_uint(v[i + k]);
+                    store_32b(o + i, w);
+                }
+            } else if (n0 + 16 <= p.b_rows && (((size_t)o) & 15) == 0) {
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
             } else {
@@ -248,8 +293,12 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float* v,
                     __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
                     w[i] = *reinterpret_cast<uint32_t*>(&h);
                 }
-                *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                if ((((size_t)o) & 31) == 0) {
+                    store_32b(o, w);
+                } else {
+                    *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                }
             } else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) if (n0 + i < p.b_rows) o[i] = __float2bfloat16_rn(v[i]);
@@ -281,8 +330,12 @@ __device__ __forceinline__ void store_swiglu_normal(const GemmParams& p, const f
                                                       gated_unit(p.glu_limit, p.glu_slope, g[2 * i + 1], u[2 * i + 1]));
             w[i] = *reinterpret_cast<uint32_t*>(&h);
         }
-        *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+        if ((((size_t)o) & 31) == 0) {
+            store_32b(o, w);
+        } else {
+            *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
         return;
     }
 #pragma unroll
@@ -668,11 +721,13 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
 // columns meets zeros there: beyond K the tensor map of B has nothing.
 #define PBN 256
 #define PSTAGES 4
+#define P_EPI_WARPS 8                         // two per quadrant of tensor-memory lanes, half of the columns each
+#define P_THREADS (64 + 32 * P_EPI_WARPS)
 #define GROUP_MAX_TILES 1024
 #define GROUP_MAX_SEGS 1024
 enum { FORM_PLAIN = 0, FORM_GROUPED = 1, FORM_BATCHED = 2 };
 template <int EPI, int FORM>
-__global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kernel(
+__global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p,
     int m_tiles, int n_tiles) {
     constexpr bool GROUPED = FORM == FORM_GROUPED, BATCHED = FORM == FORM_BATCHED;
@@ -690,7 +745,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kerne
     const uint32_t accf0 = smem_u32(bars + 2 * PSTAGES), acce0 = smem_u32(bars + 2 * PSTAGES + 2);
     if (threadIdx.x == 0) {
         for (int s = 0; s < PSTAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(accf0 + 8 * b, 1); mbar_init(acce0 + 8 * b, 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(accf0 + 8 * b, 1); mbar_init(acce0 + 8 * b, P_EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -713,7 +768,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kerne
     }
     pdl_wait();
     if (GROUPED) {
-        for (int e = threadIdx.x; e < p.n_seg; e += GEMM_THREADS) s_first[e + 1] = (p.seg[e + 1] - p.seg[e] + BM - 1) / BM;
+        for (int e = threadIdx.x; e < p.n_seg; e += P_THREADS) s_first[e + 1] = (p.seg[e + 1] - p.seg[e] + BM - 1) / BM;
         __syncthreads();
         if (threadIdx.x == 0) {
             int at = 0;
@@ -721,7 +776,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kerne
             s_first[p.n_seg] = at;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < p.n_seg; e += GEMM_THREADS) {
+        for (int e = threadIdx.x; e < p.n_seg; e += P_THREADS) {
             const int lo = p.seg[e], hi = p.seg[e + 1];
             int j = s_first[e];
             for (int r = lo; r < hi && j < GROUP_MAX_TILES; r += BM, ++j) { s_tab[3 * j] = r; s_tab[3 * j + 1] = hi; s_tab[3 * j + 2] = e; }
@@ -780,7 +835,11 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kerne
             }
         }
     } else {
-        const int quad = warp & 3;
+        // Eight warps: two share a quadrant of lanes and take 128 columns each.  With four, a tile of K = 2048 was bound
+        // by its epilogue and not by its products (one warp a scheduler hides neither the tensor memory's nor its own
+        // latencies): 2,048 tokens x [12288, 2048] with the gated unit 107 -> 80 us, x [6144, 4096] 87 -> 80 us.  (The residual epilogue adds up a row's squares, so there one warp keeps all columns of its rows.)
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        constexpr int COLS = EPI == EPI_RESID ? PBN : PBN / 2;
         GemmParams q = p;                                    // BATCHED: with this product's part of the output
         int n = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++n) {
@@ -796,28 +855,59 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_persistent_kerne
             if (!mbar_wait(accf0 + 8 * buf, (n >> 1) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
             tc_fence_after();
             const uint32_t lane_addr = tmem_base + buf * PBN + ((uint32_t)(quad * 32) << 16);
-            constexpr int STEP = EPI == EPI_SWIGLU ? 32 : 16;
-#pragma unroll 2
-            for (int c = 0; c < PBN; c += STEP) {
-                float v[16], u[16];
-                tmem_ld16(lane_addr + c, v);
-                if (STEP == 32) tmem_ld16(lane_addr + c + 16, u);
-                if (c + STEP >= PBN) {                      // the last columns are in registers: hand the buffer back
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf) : "memory");
-                }
-                if (AIRUN_FOLD_NORM && p.ssq_in) {
+            const int c_first = half * COLS;
+            // the last columns are in registers: hand the buffer back
+            auto hand_back = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf) : "memory");
+            };
+            if constexpr (EPI == EPI_SWIGLU) {
+                // the next 32 columns are on their way while these are combined
+                uint32_t r[2][32];
+                tmem_ld32_async(lane_addr + c_first, r[0]);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) { v[i] *= row_scale; if (STEP == 32) u[i] *= row_scale; }
+                for (int j = 0; j < COLS / 32; ++j) {
+                    const int c = c_first + 32 * j;
+                    __syncwarp();
+                    tmem_wait32(r[j & 1]);
+                    if (j + 1 < COLS / 32) tmem_ld32_async(lane_addr + c + 32, r[(j + 1) & 1]);
+                    else hand_back();
+                    float v[16], u[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        v[i] = __uint_as_float(r[j & 1][i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
+                        u[i] = __uint_as_float(r[j & 1][16 + i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
+                    }
+                    if (row_on) store_swiglu_normal(p, v, u, a_row, b0, c);
                 }
-                if (!row_on) continue;
-                if (EPI == EPI_SWIGLU) store_swiglu_normal(p, v, u, a_row, b0, c);
-                else if (EPI == EPI_RESID) ssq_acc += store_resid_normal(p, v, a_row, b0 + c);
-                else {
-                    if (p.act) epilogue_act(v, p.act - 1);
-                    store_chunk<EPI, false>(BATCHED ? q : p, v, a_row, b0, c);
+            } else {
+                // one body for all columns: unrolled, the activations' code would not stay in the instruction cache
+#pragma unroll 1
+                for (int c = c_first; c < c_first + COLS && c < PBN; c += 32) {
+                    uint32_t r[32];
+                    __syncwarp();
+                    tmem_ld32_async(lane_addr + c, r);
+                    tmem_wait32(r);
+                    if (c + 32 >= c_first + COLS) hand_back();
+#pragma unroll
+                    for (int h = 0; h < 32; h += 16) {
+                        float v[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h + i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
+                        if (EPI == EPI_RESID) {
+                            if (row_on) ssq_acc += store_resid_normal(p, v, a_row, b0 + c + h);
+                        } else if (row_on) {
+                            if (p.act) epilogue_act(v, p.act - 1);
+                            store_chunk<EPI, false>(BATCHED ? q : p, v, a_row, b0, c + h);
+                        }
+                    }
                 }
+            }
+            if (c_first >= PBN) {                            // nothing of this buffer is this warp's
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf) : "memory");
+                continue;
             }
             if (EPI == EPI_RESID && a_row < p.a_rows) p.ssq_out[(size_t)(tile / m_tiles) * p.ssq_out_ld + a_row] = ssq_acc;
         }
@@ -947,7 +1037,7 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmPa
     const long long total = (long long)m_tiles * n_tiles * (FORM == FORM_BATCHED ? p.n_seg : 1);
     if (total > 0x3fffffff) return AIRUN_ERR_ARG;
     const int grid = total < n_sm ? total : n_sm;
-    airun_launch(kern, dim3(grid), dim3(GEMM_THREADS), SMEM, stream, ma, mb, p, m_tiles, n_tiles);
+    airun_launch(kern, dim3(grid), dim3(P_THREADS), SMEM, stream, ma, mb, p, m_tiles, n_tiles);
     return airun_launch_status();
 }
 

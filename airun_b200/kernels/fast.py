@@ -66,7 +66,7 @@ DISABLED = set(filter(None, os.environ.get("AIRUN_DISABLE_FAST", "").split(","))
 
 
 def all_libraries():
-    return [("gemm_tcgen05", None), ("gemm_tcgen05", {"AIRUN_FOLD_NORM": 1}), ("attention_plan", None), ("attention_mma", {"HD": 128}), ("attention_mma", {"HD": 64}),
+    return [("gemm_tcgen05", None), ("gemm_tcgen05", {"AIRUN_FOLD_NORM": 1}), ("gemm_rows", None), ("attention_plan", None), ("attention_mma", {"HD": 128}), ("attention_mma", {"HD": 64}),
             ("attention_tcgen05", {"HD": 128}), ("attention_tcgen05", {"HD": 64}), ("diff_attention_mma", None),
             ("latent_attention_mma", None), ("sigmoid_attention_mma", None), ("softmax_attention_mma", None)]
 
@@ -203,11 +203,46 @@ def _normed_args(normed) -> dict:
     return {} if normed is None else dict(ssq_in=normed.ssq, eps_in=normed.eps, norm_size=normed.size)
 
 
+ROWS_MAX = 16                          # tokens up to which a product's weights go straight to registers (csrc/gemm_rows.cu)
+
+
+def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, glu: Tuple[float, float] = (0.0, 0.0),
+              act: Optional[int] = None) -> None:
+    """out = x @ w^T for few rows of x (csrc/gemm_rows.cu): the epilogues of ``gemm_tcgen05`` and the clamped gated unit."""
+    _cuda(x, w, out)
+    M, K = x.shape
+    N = w.shape[0]
+    _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
+          and out.stride(1) == 1, "operands must be row-major bfloat16")
+    _need(tuple(out.shape) == (M, N // 2 if epi == EPI_SWIGLU else N), "output must be [M, N], of a gated unit [M, N/2]")
+    _need(out.dtype == (torch.float32 if epi == EPI_F32 else torch.bfloat16), "output type does not match the epilogue")
+    f = _fn("gemm_rows", "airun_gemm_rows", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
+                                             c_int, c_float, c_float, c_int, c_void_p])
+    _check(f(_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), epi, float(glu[0]), float(glu[1]),
+             0 if act is None else 1 + int(act), _stream()), "gemm_rows")
+
+
+def _few_rows(M: int, N: int, K: int) -> bool:
+    """Whether a product of M tokens with an [N, K] weight goes to csrc/gemm_rows.cu.  Both kernels timed in graphs, B200, us
+    (tcgen05, rows).  Up to 8 tokens, as long as its blocks of 32 weight rows run in one wave of two an SM: 8 tokens x
+    [2048, 2048] 7.2, 4.3; [4096, 12288] 21.7, 19.0; [6144, 4096] 12.2, 11.5; a second wave costs more than the ring of
+    the tcgen05 kernel: [12288, 2048] 11.5, 12.4; [151936, 4096] 186, 203.  From 9 tokens a block reads twice the
+    tokens and both kernels are equal at 16 M weights ([4096, 4096] 9.9, 10.0; [2048, 2048] 7.5, 5.1; [6144, 4096] 12.3,
+    14.6)."""
+    if M > ROWS_MAX or "gemm_rows" in DISABLED:
+        return False
+    one_wave = (N + 31) // 32 <= 2 * machine().sms
+    return one_wave and (M <= 8 or N * K <= 16 << 20)
+
+
 def linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, normed=None) -> bool:
     """``normed``: x is the un-normalised activation of a NormedActivations; its token scales are
     applied in the epilogue."""
     if not _usable(x, w) or out.dtype not in (torch.float32, torch.bfloat16):
         return False
+    if normed is None and _few_rows(x.shape[0], w.shape[0], x.shape[1]):
+        gemm_rows(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16)
+        return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])
     gemm_tcgen05(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16, swap, bn, ksplit, ctx.err,
                  **_normed_args(normed))
@@ -217,12 +252,18 @@ def linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, normed
 def linear_swiglu_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch.Tensor, group: int, normed=None) -> bool:
     if group != 16 or not _usable(x, w_gu) or w_gu.shape[0] % 32 != 0:
         return False
+    if normed is None and _few_rows(x.shape[0], w_gu.shape[0], x.shape[1]):
+        gemm_rows(x, w_gu, out, EPI_SWIGLU)
+        return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w_gu.shape[0], x.shape[1])
     gemm_tcgen05(x, w_gu, out, EPI_SWIGLU, swap, bn, ksplit, ctx.err, **_normed_args(normed))
     return True
 
 
 GROUPED_MAX_TILES = 1024
+# rows a segment on average up to which the product goes to csrc/gemm_rows.cu: 16 matrices of 3072 x 2048, tcgen05 and rows,
+# 32 rows 43.2 and 33.8 us, 128 rows 43.4 and 42.0, 256 rows 43.2 and 51.1 (29, 31 and 31 us of weights)
+GROUPED_ROWS_MAX = 8
 
 
 def grouped_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor, swiglu_group: int = 0,
@@ -248,6 +289,13 @@ def grouped_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor
     _cuda(x, w, out, seg)
     _need(out.stride(1) == 1 and seg.dtype == torch.int32 and seg.numel() >= E + 1 and seg.is_contiguous(),
           "out must be row-major and seg int32 [E + 1]")
+    if M <= GROUPED_ROWS_MAX * E and "gemm_rows" not in DISABLED:
+        f = _fn("gemm_rows", "airun_gemm_rows_grouped", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int,
+                                                         c_void_p, c_int, c_float, c_float, c_int, c_void_p])
+        lim, slope = glu if glu is not None else (0.0, 0.0)
+        _check(f(_p(x), _p(w), _p(out), M, N, K, x.stride(0), out.stride(0), epi, _p(seg), E, float(lim), float(slope),
+                 0 if act is None or swiglu_group else 1 + int(act), _stream()), "gemm_rows_grouped")
+        return True
     if act is not None and not swiglu_group:
         f = _fn("gemm_tcgen05", "airun_gemm_tcgen05_grouped_act",
                 [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_int, c_int, c_void_p,
@@ -284,6 +332,12 @@ def head_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -
         return False
     _cuda(x, w, out)
     _need(tuple(w.shape) == (heads, N, K) and tuple(out.shape) == (T, heads, N), "per-head product shapes do not agree")
+    if _few_rows(T, N, K):
+        f = _fn("gemm_rows", "airun_gemm_rows_batched", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong,
+                                                         c_longlong, c_longlong, c_void_p])
+        _check(f(_p(x), _p(w), _p(out), T, N, K, heads, x.stride(0), x.stride(1) if heads > 1 else 0, out.stride(0),
+                 out.stride(1) if heads > 1 else 0, _stream()), "gemm_rows_batched")
+        return True
     f = _fn("gemm_tcgen05", "airun_gemm_tcgen05_batched",
             [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p])
     sx, so = (x.stride(1), out.stride(1)) if heads > 1 else (K, N)
@@ -612,6 +666,9 @@ def linear_glu_clamped_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch
     N = w_gu.shape[0]
     _cuda(x, w_gu, out, ctx.err)
     _need(tuple(out.shape) == (M, N // 2), "the gated unit's epilogue writes bfloat16 [M, N/2]")
+    if _few_rows(M, N, K):
+        gemm_rows(x, w_gu, out, EPI_SWIGLU, glu=(limit, slope))
+        return True
     swap, bn, ksplit = plan_gemm(M, N, K)
     scratch = counters = None
     if ksplit > 1:
@@ -736,6 +793,9 @@ def linear_act_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mo
     runs the product and the activation apart."""
     if "linear_act" in DISABLED or not _usable(x, w) or out.dtype != torch.bfloat16 or tuple(out.shape) != (x.shape[0], w.shape[0]):
         return False
+    if _few_rows(x.shape[0], w.shape[0], x.shape[1]):
+        gemm_rows(x, w, out, EPI_BF16, act=mode)
+        return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])
     gemm_tcgen05(x, w, out, EPI_BF16, swap, bn, ksplit, ctx.err, act=mode)
     return True

@@ -113,27 +113,53 @@ __device__ __forceinline__ void gla_cp16(float* smem, const float* gmem) {
 }
 // With CONST the decay is one number per head (`head_decay`), the same for every token and key channel, and nothing is
 // staged for it; `in_silu` applies z * sigmoid(z) to the staged q, k and v (projections that carry their activation).
-template <int NS, bool CONST>
+//
+// SEG: a request's tokens are cut into segments of GLA_SEG that run side by side (blockIdx.x counts the segments of all
+// requests in turn): the first starts from the request's state, the others from zero, and each leaves its last state and, per
+// key channel, the product of its decays; gla_segment_kernel then adds what the state in front of a segment gives to its
+// tokens.  One request's prompt is otherwise a chain of its tokens on heads x Dv / 32 blocks: 2,048 tokens at 16 heads took
+// 250 us on 64 blocks and take 123 us in 16 segments (76 us here, 47 in gla_segment_kernel), at 8 heads with one decay a
+// head 330 and 85.
+#define GLA_SEG 128
+struct GlaSegments {
+    float* ends;                  // [segments][heads][D][Dv]: a segment's last state, begun from zero but for a request's first
+    float* prods;                 // [segments][heads][D]: products of a segment's decays
+};
+// The request and the place within it of segment g; false: there are not so many segments.
+__device__ __forceinline__ bool gla_find_segment(const int32_t* cu_tokens, int num_reqs, int g, int& r, int& s, int& count) {
+    for (r = 0; r < num_reqs; ++r) {
+        count = (cu_tokens[r + 1] - cu_tokens[r] + GLA_SEG - 1) / GLA_SEG;
+        if (g < count) { s = g; return true; }
+        g -= max(count, 0);
+    }
+    return false;
+}
+template <int NS, bool CONST, bool SEG>
 __global__ __launch_bounds__(256) void gla_recurrent_kernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long row_stride,
     const float* __restrict__ decay, float* __restrict__ state, long long slot_stride,
     const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int max_slots,
     float* __restrict__ out, int heads, int D, int Dv, float q_scale, int* __restrict__ err,
-    const float* __restrict__ head_decay, int in_silu) {
+    const float* __restrict__ head_decay, int in_silu, int num_reqs, GlaSegments segs) {
     pdl_trigger();
     pdl_wait();
     constexpr int DP = NS * GLA_WARPS;
     constexpr int GLA_TT = NS >= 32 ? 4 : NS >= 16 ? 8 : 16;     // tokens of a stage (static shared memory stays under 48 KB)
     __shared__ __align__(16) float s_q[2][GLA_TT][DP], s_k[2][GLA_TT][DP], s_a[2][GLA_TT][DP], s_v[2][GLA_TT][GLA_COLS];
     __shared__ float s_p[GLA_WARPS][GLA_TT][GLA_COLS];
-    const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * GLA_COLS;
-    const int t0 = cu_tokens[r], n = cu_tokens[r + 1] - t0;
+    int r = blockIdx.x, part = 0, parts = 1;
+    const int head = blockIdx.y, col0 = blockIdx.z * GLA_COLS;
+    if (SEG && !gla_find_segment(cu_tokens, num_reqs, blockIdx.x, r, part, parts)) return;
+    int t0 = cu_tokens[r], n = cu_tokens[r + 1] - t0;
     if (n <= 0) return;
+    if (SEG) { t0 += part * GLA_SEG; n = min(GLA_SEG, n - part * GLA_SEG); }
     const int slot = state_slots[r];
     if (slot < 0 || slot >= max_slots) {
         if (threadIdx.x == 0) atomicOr(err, AIRUN_DEV_BAD_REQ);
         return;
     }
+    const bool from_state = !SEG || part == 0, to_state = !SEG || parts == 1;
+    float prod = 1.0f;                                     // SEG: of key channel threadIdx.x, by the blocks of the first columns
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = col0 + lane, d0 = warp * NS;
     const bool col_ok = col < Dv;
@@ -183,7 +209,7 @@ __global__ __launch_bounds__(256) void gla_recurrent_kernel(
     float* sbase = state + (size_t)slot * slot_stride + (size_t)head * D * Dv + (col_ok ? col : 0);
     float S[NS];
 #pragma unroll
-    for (int i = 0; i < NS; ++i) S[i] = (col_ok && d0 + i < D) ? sbase[(size_t)(d0 + i) * Dv] : 0.0f;
+    for (int i = 0; i < NS; ++i) S[i] = (from_state && col_ok && d0 + i < D) ? sbase[(size_t)(d0 + i) * Dv] : 0.0f;
     int it = 0;
     for (int base = 0; base < n; base += GLA_TT, ++it) {
         const int buf = it & 1, nt = min(GLA_TT, n - base);
@@ -206,6 +232,8 @@ __global__ __launch_bounds__(256) void gla_recurrent_kernel(
             }
             __syncthreads();
         }
+        if (SEG && !CONST && blockIdx.z == 0 && threadIdx.x < D)
+            for (int tt = 0; tt < nt; ++tt) prod *= s_a[buf][tt][threadIdx.x];
 #pragma unroll 4
         for (int tt = 0; tt < nt; ++tt) {
             const float vj = s_v[buf][tt][lane];
@@ -232,28 +260,154 @@ __global__ __launch_bounds__(256) void gla_recurrent_kernel(
         }
         __syncthreads();
     }
+    float* const end = to_state ? sbase : segs.ends + ((size_t)blockIdx.x * heads + head) * D * Dv + (col_ok ? col : 0);
     if (col_ok) {
 #pragma unroll
         for (int i = 0; i < NS; ++i)
-            if (d0 + i < D) sbase[(size_t)(d0 + i) * Dv] = S[i];
+            if (d0 + i < D) end[(size_t)(d0 + i) * Dv] = S[i];
+    }
+    if (SEG && !CONST && blockIdx.z == 0 && threadIdx.x < D) segs.prods[((size_t)blockIdx.x * heads + head) * D + threadIdx.x] = prod;
+}
+
+// What the state in front of a segment gives to the segment's tokens, o_t += (q_t * a_first * .. * a_t) . S_in, and the
+// request's last state.  One block per (segment, head, 64 value columns): the states the earlier segments of the request
+// ended with are brought together in their order (S <- product of a segment's decays * S + its end), the decayed queries are
+// formed in shared memory (four runs of 32 tokens a channel side by side), and the product of the two is added to the
+// output, 8 tokens x 4 columns a thread.  Only products of decays occur, never quotients, so a decay near zero only wipes.
+template <bool CONST>
+__global__ __launch_bounds__(256) void gla_segment_kernel(
+    const float* __restrict__ q, long long row_stride, const float* __restrict__ decay, float* __restrict__ state, long long slot_stride,
+    const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int max_slots, float* __restrict__ out, int heads,
+    int D, int Dv, float q_scale, const float* __restrict__ head_decay, int in_silu, int num_reqs, GlaSegments segs) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float s_seg[];
+    const int QS = D + 4;
+    float* const s_qt = s_seg;                             // [GLA_SEG][D + 4]
+    float* const s_S = s_seg + GLA_SEG * QS;               // [D][64]
+    __shared__ float s_run[4][128];
+    int r, part, parts;
+    if (!gla_find_segment(cu_tokens, num_reqs, blockIdx.x, r, part, parts) || part == 0) return;
+    const int slot = state_slots[r];
+    if (slot < 0 || slot >= max_slots) return;             // the kernel in front has said so
+    const int head = blockIdx.y, c0 = blockIdx.z * 64, tid = threadIdx.x;
+    const int t0 = cu_tokens[r] + part * GLA_SEG, n = min(GLA_SEG, cu_tokens[r + 1] - t0);
+    const size_t first = (size_t)blockIdx.x - part;        // the request's first segment
+    const float dec = CONST ? head_decay[head] : 0.0f, dec_seg = CONST ? powf(dec, (float)GLA_SEG) : 0.0f;
+    float* const srow = state + (size_t)slot * slot_stride + (size_t)head * D * Dv;
+    for (int e = tid * 4; e < D * 64; e += 1024) {
+        const int d = e / 64, c = c0 + e % 64;
+        float4 S = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (c < Dv) {
+#pragma unroll 4
+            for (int j = 0; j <= part; ++j) {
+                const size_t at = (first + j) * heads + head;
+                const float4 E = *reinterpret_cast<const float4*>(segs.ends + at * D * Dv + (size_t)d * Dv + c);
+                const int len = j < part ? GLA_SEG : n;
+                const float a = CONST ? (j < part ? dec_seg : powf(dec, (float)len)) : segs.prods[at * D + d];
+                if (j == part) {
+                    *reinterpret_cast<float4*>(&s_S[d * 64 + e % 64]) = S;
+                    if (part != parts - 1) break;
+                }
+                S.x = fmaf(a, S.x, E.x); S.y = fmaf(a, S.y, E.y); S.z = fmaf(a, S.z, E.z); S.w = fmaf(a, S.w, E.w);
+            }
+            if (part == parts - 1) *reinterpret_cast<float4*>(srow + (size_t)d * Dv + c) = S;
+        } else {
+            *reinterpret_cast<float4*>(&s_S[d * 64 + e % 64]) = S;
+        }
+    }
+    // the decayed queries: run k of a channel has tokens 32 k .. 32 k + 31
+    for (int e = tid; e < 4 * D; e += 256) {
+        const int run = e / D, d = e - run * D;
+        const float* a = decay + (size_t)t0 * heads * D + (size_t)head * D + d;
+        float p = 1.0f;
+        for (int t = 32 * run; t < min(32 * run + 32, n); ++t) {
+            p *= CONST ? dec : a[(size_t)t * heads * D];
+            float qv = q[(size_t)(t0 + t) * row_stride + (size_t)head * D + d];
+            if (in_silu) qv = qv / (1.0f + expf(-qv));
+            s_qt[t * QS + d] = qv * p;
+        }
+        s_run[run][d] = p;
+    }
+    __syncthreads();
+    for (int e = tid; e < 3 * D; e += 256) {
+        const int run = 1 + e / D, d = e % D;
+        float p = s_run[0][d];
+        for (int k = 1; k < run; ++k) p *= s_run[k][d];
+        for (int t = 32 * run; t < min(32 * run + 32, n); ++t) s_qt[t * QS + d] *= p;
+    }
+    __syncthreads();
+    const int cg = (tid & 15) * 4, tg = (tid >> 4) * 8;
+    if (tg >= n || c0 + cg >= Dv) return;
+    float4 acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int d = 0; d < D; d += 4) {
+        float4 S4[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) S4[k] = *reinterpret_cast<const float4*>(&s_S[(d + k) * 64 + cg]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(&s_qt[(tg + i) * QS + d]);       // rows from n on are not stored
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc[i].x = fmaf(xs[k], S4[k].x, acc[i].x); acc[i].y = fmaf(xs[k], S4[k].y, acc[i].y);
+                acc[i].z = fmaf(xs[k], S4[k].z, acc[i].z); acc[i].w = fmaf(xs[k], S4[k].w, acc[i].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (tg + i >= n) break;
+        float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + tg + i) * ((size_t)heads * Dv) + (size_t)head * Dv + c0 + cg);
+        float4 v = *o;
+        v.x = fmaf(q_scale, acc[i].x, v.x); v.y = fmaf(q_scale, acc[i].y, v.y);
+        v.z = fmaf(q_scale, acc[i].z, v.z); v.w = fmaf(q_scale, acc[i].w, v.w);
+        *o = v;
     }
 }
 
 static int gla_recurrent_launch(const float* q, const float* k, const float* v, long long row_stride,
                                 const float* decay, const float* head_decay, int in_silu, float* state, long long slot_stride,
                                 int max_slots, const int32_t* cu_tokens, const int32_t* state_slots, int num_reqs,
-                                float* out, int heads, int D, int Dv, float q_scale, int* err, cudaStream_t stream) {
+                                float* out, int heads, int D, int Dv, float q_scale, float* work, int max_segments, int* err,
+                                cudaStream_t stream) {
     if (num_reqs < 0 || heads <= 0 || D <= 0 || D > 256 || Dv <= 0 || !state || !cu_tokens || !state_slots || !err ||
         slot_stride < (long long)heads * D * Dv || heads > 65535 || (!decay && !head_decay))
         return AIRUN_ERR_ARG;
     if (num_reqs == 0) return AIRUN_OK;
     const int tiles = ceil_div_i(Dv, GLA_COLS);
     if (tiles > 65535) return AIRUN_ERR_ARG;
-    dim3 grid(num_reqs, heads, tiles);
-#define GLA_LAUNCH(NS, C) airun_launch(gla_recurrent_kernel<NS, C>, grid, dim3(256), 0, stream, q, k, v, row_stride, decay, state, \
-        slot_stride, cu_tokens, state_slots, max_slots, out, heads, D, Dv, q_scale, err, head_decay, in_silu)
-#define GLA_PICK(C) do { if (D <= 32) GLA_LAUNCH(4, C); else if (D <= 64) GLA_LAUNCH(8, C); else if (D <= 128) GLA_LAUNCH(16, C); \
-        else GLA_LAUNCH(32, C); } while (0)
+    GlaSegments segs = {};
+#define GLA_LAUNCH(NS, C, SEG) airun_launch(gla_recurrent_kernel<NS, C, SEG>, grid, dim3(256), 0, stream, q, k, v, row_stride, decay, state, \
+        slot_stride, cu_tokens, state_slots, max_slots, out, heads, D, Dv, q_scale, err, head_decay, in_silu, num_reqs, segs)
+    if (work) {
+        if (max_segments <= 0 || D > 128 || D % 4 || Dv % 4 || slot_stride % 4 || (((uintptr_t)state | (uintptr_t)out | (uintptr_t)work) & 15))
+            return AIRUN_ERR_ARG;
+        segs.ends = work;
+        segs.prods = work + (size_t)max_segments * heads * D * Dv;
+        const dim3 grid(max_segments, heads, tiles);
+#define GLA_PICK(C) do { if (D <= 32) GLA_LAUNCH(4, C, true); else if (D <= 64) GLA_LAUNCH(8, C, true); else GLA_LAUNCH(16, C, true); } while (0)
+        if (head_decay) GLA_PICK(true);
+        else GLA_PICK(false);
+#undef GLA_PICK
+        const int smem = (GLA_SEG * (D + 4) + D * 64) * (int)sizeof(float);
+        static unsigned long long configured[2];
+        auto add = [&](auto kern, int i) -> int {
+            if (first_on_device(configured[i])) {
+                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (GLA_SEG * 132 + 128 * 64) * (int)sizeof(float));
+                if (e != cudaSuccess) return (int)e;
+            }
+            airun_launch(kern, dim3(max_segments, heads, ceil_div_i(Dv, 64)), dim3(256), smem, stream, q, row_stride, decay, state, slot_stride,
+                         cu_tokens, state_slots, max_slots, out, heads, D, Dv, q_scale, head_decay, in_silu, num_reqs, segs);
+            return airun_launch_status();
+        };
+        return head_decay ? add(gla_segment_kernel<true>, 0) : add(gla_segment_kernel<false>, 1);
+    }
+    const dim3 grid(num_reqs, heads, tiles);
+#define GLA_PICK(C) do { if (D <= 32) GLA_LAUNCH(4, C, false); else if (D <= 64) GLA_LAUNCH(8, C, false); \
+        else if (D <= 128) GLA_LAUNCH(16, C, false); else GLA_LAUNCH(32, C, false); } while (0)
     if (head_decay) GLA_PICK(true);
     else GLA_PICK(false);
 #undef GLA_PICK
@@ -261,13 +415,18 @@ static int gla_recurrent_launch(const float* q, const float* k, const float* v, 
     return airun_launch_status();
 }
 
+// `work`: null, or max_segments * heads * (D * Dv + D) floats for the segments (D up to 128, D and Dv in multiples of 4);
+// max_segments: at least the sum over the requests of ceil(tokens / GLA_SEG).
+AIRUN_EXPORT int airun_gla_segment_tokens() { return GLA_SEG; }
+
 AIRUN_EXPORT int airun_gla_recurrent(const float* q, const float* k, const float* v, long long row_stride,
                                      const float* decay, float* state, long long slot_stride, int max_slots,
                                      const int32_t* cu_tokens, const int32_t* state_slots, int num_reqs,
-                                     float* out, int heads, int D, int Dv, float q_scale, int* err, cudaStream_t stream) {
+                                     float* out, int heads, int D, int Dv, float q_scale, float* work, int max_segments, int* err,
+                                     cudaStream_t stream) {
     if (!decay) return AIRUN_ERR_ARG;
     return gla_recurrent_launch(q, k, v, row_stride, decay, nullptr, 0, state, slot_stride, max_slots, cu_tokens, state_slots,
-                                num_reqs, out, heads, D, Dv, q_scale, err, stream);
+                                num_reqs, out, heads, D, Dv, q_scale, work, max_segments, err, stream);
 }
 
 // The same recurrence with ONE decay per head, S <- d_h S + k v^T, o = S^T q (times q_scale); `in_silu`: q, k and v
@@ -275,10 +434,11 @@ AIRUN_EXPORT int airun_gla_recurrent(const float* q, const float* k, const float
 AIRUN_EXPORT int airun_decay_recurrent(const float* q, const float* k, const float* v, long long row_stride,
                                        const float* head_decay, int in_silu, float* state, long long slot_stride, int max_slots,
                                        const int32_t* cu_tokens, const int32_t* state_slots, int num_reqs,
-                                       float* out, int heads, int D, int Dv, float q_scale, int* err, cudaStream_t stream) {
+                                       float* out, int heads, int D, int Dv, float q_scale, float* work, int max_segments, int* err,
+                                       cudaStream_t stream) {
     if (!head_decay) return AIRUN_ERR_ARG;
     return gla_recurrent_launch(q, k, v, row_stride, nullptr, head_decay, in_silu, state, slot_stride, max_slots, cu_tokens,
-                                state_slots, num_reqs, out, heads, D, Dv, q_scale, err, stream);
+                                state_slots, num_reqs, out, heads, D, Dv, q_scale, work, max_segments, err, stream);
 }
 
 // out[t][c] = scale * o[t][c] / sqrt(mean_c o[t]^2 + eps) * w[c] * sigmoid(gate[t][c]) over a token's whole row of n

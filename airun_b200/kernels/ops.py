@@ -397,9 +397,23 @@ def gla_decay(low: torch.Tensor, w2: torch.Tensor, bias: Optional[torch.Tensor],
              _stream()), "gla_decay")
 
 
+SEGMENT_TOKENS = 128                   # csrc/linear_attention.cu: GLA_SEG
+SEGMENT_MIN_TOKENS = 256               # tokens of a step from which a request's tokens run in segments side by side
+
+
+def _gla_work(ws, T: int, num_reqs: int, heads: int, D: int, Dv: int, state: torch.Tensor):
+    """(buffer for the segments of a step of T tokens, their largest number), or (None, 0): the step is short, the sizes
+    are not the segments', or no workspace is given.  The cut costs a second kernel and 1 / SEGMENT_TOKENS of a state per
+    token, so it pays once a request brings two segments."""
+    if ws is None or T < SEGMENT_MIN_TOKENS or D > 128 or D % 4 or Dv % 4 or state.stride(0) % 4 or state.data_ptr() % 16:
+        return None, 0
+    n = T // SEGMENT_TOKENS + int(num_reqs)
+    return ws.alloc((n * heads * (D * Dv + D),), torch.float32), n
+
+
 def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                   cu_tokens: torch.Tensor, state_slots: torch.Tensor, num_reqs: int, out: torch.Tensor,
-                  heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor) -> None:
+                  heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None) -> None:
     """The recurrence S <- diag(a) S + k v^T, o = S^T q * q_scale for the tokens of every request in order.
     ``q``, ``k`` [T, heads*D] and ``v`` [T, heads*Dv] are float32 column slices of ONE buffer (equal row strides);
     ``state`` is [slots, heads, D, Dv] float32 and is updated in place; ``out`` float32 [T, heads*Dv]."""
@@ -419,16 +433,17 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torc
           and state_slots.numel() >= num_reqs, "cu_tokens / state_slots must be int32 [R + 1] / [R]")
     _need(D <= 256, f"{D} key channels a head are above the kernel's limit of 256")
     stride = q.stride(0) if T > 1 else max(q.stride(0), k.stride(0), v.stride(0))
+    work, segments = _gla_work(ws, T, num_reqs, heads, D, Dv, state)
     f = _fn("linear_attention", "airun_gla_recurrent",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int,
-             c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p])
+             c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p])
     _check(f(_p(q), _p(k), _p(v), stride, _p(decay), _p(state), state.stride(0), state.shape[0], _p(cu_tokens),
-             _p(state_slots), int(num_reqs), _p(out), heads, D, Dv, float(q_scale), _p(err), _stream()), "gla_recurrent")
+             _p(state_slots), int(num_reqs), _p(out), heads, D, Dv, float(q_scale), _p(work), segments, _p(err), _stream()), "gla_recurrent")
 
 
 def decay_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, head_decay: torch.Tensor, in_silu: bool,
                     state: torch.Tensor, cu_tokens: torch.Tensor, state_slots: torch.Tensor, num_reqs: int, out: torch.Tensor,
-                    heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor) -> None:
+                    heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None) -> None:
     """The recurrence with one decay per head, S <- d_h S + k v^T, o = S^T q * q_scale, for the tokens of every request in
     order.  ``q``, ``k`` [T, heads*D] and ``v`` [T, heads*Dv] are float32 column slices of ONE buffer; with ``in_silu``
     they arrive without their activation z sigmoid(z), which the kernel applies.  ``head_decay`` float32 [heads];
@@ -448,12 +463,13 @@ def decay_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, head_deca
           and state_slots.numel() >= num_reqs, "cu_tokens / state_slots must be int32 [R + 1] / [R]")
     _need(D <= 256, f"{D} key channels a head are above the kernel's limit of 256")
     stride = q.stride(0) if T > 1 else max(q.stride(0), k.stride(0), v.stride(0))
+    work, segments = _gla_work(ws, T, num_reqs, heads, D, Dv, state)
     f = _fn("linear_attention", "airun_decay_recurrent",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int,
-             c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p])
+             c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p])
     _check(f(_p(q), _p(k), _p(v), stride, _p(head_decay), 1 if in_silu else 0, _p(state), state.stride(0), state.shape[0],
-             _p(cu_tokens), _p(state_slots), int(num_reqs), _p(out), heads, D, Dv, float(q_scale), _p(err), _stream()),
-           "decay_recurrent")
+             _p(cu_tokens), _p(state_slots), int(num_reqs), _p(out), heads, D, Dv, float(q_scale), _p(work), segments, _p(err),
+             _stream()), "decay_recurrent")
 
 
 def rownorm_gate(o: torch.Tensor, gate: Optional[torch.Tensor], weight: Optional[torch.Tensor], eps: float, out: torch.Tensor,

@@ -1,0 +1,71 @@
+"""Recurrences that do not run token by token.
+
+The linear attentions' recurrence with a request's tokens cut into segments that run side by side (csrc/linear_attention.cu)
+against the recurrence token by token in float64: requests that end on, before and behind a segment's border, two steps
+with the state carried over, decays from nearly nothing to a hair below one.
+
+Tolerance: an output sums up to D * (tokens the decays let live) float32 products, in either order; 2e-5 of the row's
+largest possible sum (the same recurrence over absolute values) holds at these sizes with room for 170 roundings."""
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+CASES = [  # heads, D, Dv, decay per head, tokens of the requests in the first and in the second step
+    (2, 64, 128, False, (256,), (300,)), (3, 32, 96, False, (128, 129, 1), (257, 1, 127)), (1, 128, 64, False, (1, 700), (383, 1)),
+    (2, 4, 4, True, (640, 0, 5), (0, 255, 130)), (4, 64, 128, True, (1000, 300), (128, 256)), (1, 100, 36, True, (511,), (513,)),
+    (2, 96, 200, False, (300, 2), (0, 401)),
+]
+
+
+def plain(q, k, v, a, S):
+    o = torch.zeros(q.shape[0], q.shape[1], v.shape[-1], dtype=torch.float64)
+    for t in range(q.shape[0]):
+        S = a[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+        o[t] = (S * q[t][:, :, None]).sum(1)
+    return o, S
+
+
+@gpu
+@pytest.mark.parametrize("heads,D,Dv,per_head,first,second", CASES)
+def test_segments_against_token_by_token(heads, D, Dv, per_head, first, second):
+    from airun_b200.engine.batch import Workspace
+    from airun_b200.kernels import ops
+    g = torch.Generator().manual_seed(heads * 1000 + D)
+    slots = list(range(len(first) + 1))[::-1][:len(first)]
+    state = torch.zeros(len(first) + 1, heads, D, Dv, device="cuda")
+    want_state = [torch.zeros(heads, D, Dv, dtype=torch.float64) for _ in first]
+    bound_state = [s.clone() for s in want_state]
+    head_decay = torch.tensor([1.0 - 2.0 ** -(1 + 5 * h % 11) for h in range(heads)]).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws = Workspace(torch.device("cuda"), 8 << 20)
+    for lens in (first, second):
+        T = sum(lens)
+        row = 2 * heads * D + heads * Dv
+        proj = torch.randn(T, row + 8, generator=g)
+        decay = torch.rand(T, heads * D, generator=g) ** (0.02 + torch.rand(heads * D, generator=g) ** 4 * 3)
+        decay[:, ::7] = 1e-20 ** torch.rand(T, (heads * D + 6) // 7, generator=g)
+        pd = proj.cuda()
+        q, k, v = pd[:, :heads * D], pd[:, heads * D:2 * heads * D], pd[:, 2 * heads * D:row]
+        out = torch.empty(T, heads * Dv, device="cuda")
+        cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device="cuda")
+        sl = torch.tensor(slots, dtype=torch.int32, device="cuda")
+        assert ops._gla_work(ws, T, len(lens), heads, D, Dv, state)[1] > 0            # this is the cut form
+        if per_head:
+            ops.decay_recurrent(q, k, v, head_decay, True, state, cu, sl, len(lens), out, heads, D, Dv, 0.5, err, ws=ws)
+        else:
+            ops.gla_recurrent(q, k, v, decay.cuda(), state, cu, sl, len(lens), out, heads, D, Dv, 0.5, err, ws=ws)
+        assert int(err.item()) == 0
+        x = torch.nn.functional.silu(proj.double()) if per_head else proj.double()
+        at = 0
+        for r, n in enumerate(lens):
+            rows = x[at:at + n]
+            qq, kk, vv = (t.reshape(n, heads, w) for t, w in ((rows[:, :heads * D], D), (rows[:, heads * D:2 * heads * D], D), (rows[:, 2 * heads * D:row], Dv)))
+            aa = head_decay.cpu().double()[None, :, None].expand(n, heads, D) if per_head else decay[at:at + n].double().reshape(n, heads, D)
+            o, want_state[r] = plain(qq, kk, vv, aa, want_state[r])
+            most, bound_state[r] = plain(qq.abs(), kk.abs(), vv.abs(), aa, bound_state[r])
+            if n:
+                got = out[at:at + n].cpu().double().reshape(n, heads, Dv)
+                assert bool(((got - 0.5 * o).abs() <= 2e-5 * 0.5 * most + 1e-30).all())
+            assert bool(((state[slots[r]].cpu().double() - want_state[r]).abs() <= 2e-5 * bound_state[r] + 1e-30).all())
+            at += n
+    assert float(state[[s for s in range(len(first) + 1) if s not in slots]].abs().max()) == 0

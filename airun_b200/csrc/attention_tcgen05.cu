@@ -624,12 +624,59 @@ constexpr int W_OFF_K = 2 * Q_BYTES;                    // 2 stages
 constexpr int W_OFF_V = W_OFF_K + 2 * KV_BYTES;         // 2 stages
 constexpr int W_OFF_BAR = W_OFF_V + 2 * KV_BYTES;
 constexpr int W_N_BARS = 15;
-constexpr int W_SMEM_TOTAL = W_OFF_BAR + W_N_BARS * 8 + 64 + 1024;
+constexpr int W_OFF_TAB = W_OFF_BAR + W_N_BARS * 8 + 64;      // distance terms: [2 key tiles][2 Q tiles][G][stride]
+constexpr int W_SMEM_TOTAL = W_OFF_TAB + 1024;
+// What a key weighs and what becomes of a row, for the attentions that share this kernel (head size 128):
+//   W_PLAIN    the softmax of the reference's models
+//   W_OPTIONS  softmax with a sink, a factor and a gate per element on the result, rows of a wider output, and keys that are
+//              values as well (one cached row: the value begins `tail` elements into the key's row)
+//   W_TABLE    the same with a number per head and distance added to the scaled score
+//   W_SIGMOID  no softmax: a key weighs sigmoid(scale * qk - a_h ln(1 + b_h * distance) + c_h)
+//   W_DIFF     differential attention, two maps of 64 dimensions over one value of 128: the two Q tiles are the two maps of the
+//              SAME 128 packed rows, map x reads the x-th half of a key's row; soft-capped scores, keys of the query's
+//              chunk only; the two results meet in shared memory, are subtracted and normed
+// The formulas are those of softmax_attention.cu, sigmoid_attention.cu and diff_attention.cu, the plain twins.  What bounds
+// each, and one 2,048-token prompt of 16 heads over 8 KV heads (tiles of mma.sync before, us):
+//   W_OPTIONS  as W_PLAIN, window 1,024: 109 -> 56;   W_TABLE  a table entry read from shared memory per score, twice: 139 -> 77
+//   W_SIGMOID  an ex2 and half a reciprocal per score in one pass: 120 -> 96;   W_DIFF  two and a half of them: 232 -> 123
+enum { W_PLAIN = 0, W_OPTIONS = 1, W_TABLE = 2, W_SIGMOID = 3, W_DIFF = 4 };
+struct WideExtra {
+    long long out_stride;          // elements from one token's row of `out` to the next
+    const float* table;            // W_TABLE: [nh][table_len], by distance min(i - j, table_len - 1)
+    int table_len;
+    const float* sink;             // [nh]: exp(sink) joins the denominator; null: none
+    const float* gate;             // [T][gate_stride] float32, columns head * 128 + d: the result is times its sigmoid; null: none
+    long long gate_stride;
+    float out_scale;
+    const float *dist_a, *dist_b, *head_c;      // W_SIGMOID: [nh] each, or null
+    int tail;                      // >= 0: one cached row for key and value
+    int tab_toks, tab_stride;      // tokens a Q tile can touch, and floats per head of a table slice
+    float cap_c, cap_k;            // W_DIFF: cap * log2(e) and 2 * scale * log2(e) / cap: log2 of a weight is c - 2 c / (1 + 2^(k qk))
+    float lambda, eps;
+    int chunk;                     // W_DIFF: keys of the query's own run of `chunk` positions; 0: all
+};
+__device__ __forceinline__ float w_log2(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// 1 / (1 + 2^x) of two scores with one reciprocal: 1/a = b / (ab).  x is kept at most 60 (a NaN stays one), so that the
+// product stays finite; such a weight is below 1e-18 either way.
+__device__ __forceinline__ float2 w_sigmoid2(float x, float y) {
+    asm("min.NaN.f32 %0, %0, 0f42700000;" : "+f"(x));
+    asm("min.NaN.f32 %0, %0, 0f42700000;" : "+f"(y));
+    const float a = 1.0f + ex2(x), b = 1.0f + ex2(y);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
+    return make_float2(b * r, a * r);
+}
 enum { W_KFULL = 0, W_KEMPTY = 2, W_VFULL = 4, W_VEMPTY = 6, W_SFULL = 8, W_PFULL = 10, W_FINAL = 12, W_PHALF = 13 };
 
+template <int KIND>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     const TcParams p, const int4* __restrict__ tiles, const __grid_constant__ CUtensorMap kv_map,
-    const int* __restrict__ n_tiles_dev) {
+    const int* __restrict__ n_tiles_dev, const WideExtra ex) {
+    constexpr bool TABLE = KIND == W_TABLE || KIND == W_SIGMOID, DIFF = KIND == W_DIFF;
     pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -672,10 +719,11 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     const int req = t4.x, tok0 = t4.y, n_tok = t4.z;
     const int kvh = lin % (int)gridDim.y;
     const int n_rows = n_tok * G;
-    const bool two = n_rows > QM;                       // is there a Q tile B?
+    const bool two = DIFF || n_rows > QM;               // is there a Q tile B?
     const int32_t* bt = p.block_table + (size_t)req * p.max_blocks;
     const int pos_lo = p.positions[tok0], pos_hi = p.positions[tok0 + n_tok - 1];
-    const int k_first = p.window > 0 ? max(0, pos_lo - p.window + 1) : 0;
+    int k_first = p.window > 0 ? max(0, pos_lo - p.window + 1) : 0;
+    if (DIFF && ex.chunk > 0) k_first = max(k_first, pos_lo / ex.chunk * ex.chunk);
     const int tile_first = k_first / KN;
     const int n_tiles = pos_hi >= 0 ? pos_hi / KN - tile_first + 1 : 0;
 
@@ -699,7 +747,8 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                         if (j >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                         page = 0;
                     }
-                    rows[gkey] = (((page * 2) * p.nkv + kvh) << p.page_shift) + (j & (p.page_size - 1));
+                    const int parts = KIND != W_PLAIN && ex.tail >= 0 ? 1 : 2;       // key rows, then value rows; or rows that are both
+                    rows[gkey] = (((page * parts) * p.nkv + kvh) << p.page_shift) + (j & (p.page_size - 1));
                 }
 #pragma unroll
                 for (int gkey = 0; gkey < KN / 16; ++gkey)
@@ -709,12 +758,13 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 if (!mbar_wait(BAR(W_VEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 mbar_expect_tx(BAR(W_VFULL + s), KV_BYTES);
                 const uint32_t vdst = smem_u32(smem + W_OFF_V + s * KV_BYTES);
-                const int vskip = p.nkv << p.page_shift;
+                const bool one_row = KIND != W_PLAIN && ex.tail >= 0;
+                const int vskip = one_row ? 0 : p.nkv << p.page_shift, v_x = one_row ? ex.tail : 0;
 #pragma unroll
                 for (int gkey = 0; gkey < KN / 16; ++gkey)
 #pragma unroll
                     for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_VFULL + s), h * 64, rows[gkey] + vskip);
+                        tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_VFULL + s), v_x + h * 64, rows[gkey] + vskip);
             }
         }
     } else if (warp == 1) {
@@ -738,9 +788,9 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 }
                 const uint32_t qx = q_lo + x * (Q_BYTES >> 4), ks = k_lo + s * (KV_BYTES >> 4), d = tmem_base + x * KN;
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
+                for (int k = 0; k < (DIFF ? 4 : HD / 16); ++k) {
                     const uint32_t off = ((k >> 2) * ROWBLK + (k & 3) * 32) >> 4;
-                    umma_bf16_lh(d, qx + off, q_hi, ks + off, k_hi, idesc_s, k > 0 ? 1u : 0u);
+                    umma_bf16_lh(d, qx + off, q_hi, ks + off + (DIFF ? x * (ROWBLK >> 4) : 0), k_hi, idesc_s, k > 0 ? 1u : 0u);
                 }
                 if (x == last_x) umma_commit(BAR(W_KEMPTY + s));
                 umma_commit(BAR(W_SFULL + x));
@@ -784,7 +834,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
         const int x = (warp - 2) >> 2;                    // this warpgroup's Q tile
         const int quad = warp & 3;
         const int r = quad * 32 + lane;                   // the thread's lane of tensor memory
-        const int row = x * QM + r;
+        const int row = DIFF ? r : x * QM + r;
         const bool row_ok = row < n_rows;
         const int tok = tok0 + (row_ok ? row / G : 0);
         const int head = kvh * G + (row_ok ? row % G : 0);
@@ -794,9 +844,9 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 
         // the Q row -> shared memory in the K-major swizzled layout
         {
-            const uint4* src = reinterpret_cast<const uint4*>(p.q + ((size_t)tok * p.nh + head) * HD);
+            const uint4* src = reinterpret_cast<const uint4*>(p.q + ((size_t)tok * p.nh + head) * HD) + (DIFF ? x * 8 : 0);
 #pragma unroll
-            for (int c = 0; c < HD / 8; ++c) {
+            for (int c = 0; c < (DIFF ? 8 : HD / 8); ++c) {
                 const uint4 v = row_ok ? src[c] : make_uint4(0, 0, 0, 0);
                 *reinterpret_cast<uint4*>(smem + W_OFF_Q + x * Q_BYTES + (c >> 3) * ROWBLK + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
             }
@@ -808,24 +858,93 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
         float m = NEG_BIG, l = 0.0f;
         bool ok = true;
         const float sc = p.scale_log2;
-        for (int it = 0; it < n_tiles && ok; ++it) {
+        // W_DIFF: the first key this row sees, and the first that all rows see
+        int vis_lo = 0, all_lo = 0;
+        if constexpr (DIFF) {
+            if (ex.chunk > 0) { vis_lo = max(pos, 0) / ex.chunk * ex.chunk; all_lo = pos_hi / ex.chunk * ex.chunk; }
+            if (p.window > 0) { vis_lo = max(vis_lo, pos - p.window + 1); all_lo = max(all_lo, pos_hi - p.window + 1); }
+        }
+        // the distance terms a key tile can need, per head of the group, worked out once by this warpgroup: entry e of a
+        // head is the distance e - 127 of the tile's first token, so this row reads entry (its token) + 127 - (key of the tile)
+        const int tab_tok0 = x * QM / G;                     // first token of this Q tile, counted from the CTA's
+        const int tab_len = ex.tab_toks + 127;
+        float* const tab_mine = reinterpret_cast<float*>(smem + W_OFF_TAB) + (size_t)x * (TABLE ? G * ex.tab_stride : 0);
+        const int tab_row = TABLE && row_ok ? (row % G) * ex.tab_stride + (row / G - tab_tok0) + 127 : 127;
+        // (with a table the warps of a warpgroup meet at a barrier for every tile, so a warp that has given up goes on meeting them)
+        for (int it = 0; it < n_tiles && (TABLE || ok); ++it) {
+            const float* tb = nullptr;
+            if constexpr (TABLE) {
+                // two slices in turn: a slice is written again after the barrier that follows its last reading
+                float* tab = tab_mine + (size_t)(it & 1) * 2 * G * ex.tab_stride;
+                const int d0 = p.positions[tok0] + tab_tok0 - 127 - (tile_first + it) * KN;
+                for (int h = 0; h < G; ++h) {
+                    const int hd = kvh * G + h;
+                    if (KIND == W_TABLE) {
+                        const float* src = ex.table + (size_t)hd * ex.table_len;
+                        for (int e = r; e < tab_len; e += 128)
+                            tab[h * ex.tab_stride + e] = LOG2E * __ldg(src + min(max(d0 + e, 0), ex.table_len - 1));
+                    } else {
+                        const float a = ex.dist_a ? __ldg(ex.dist_a + hd) : 0.0f, bb = ex.dist_a ? __ldg(ex.dist_b + hd) : 0.0f;
+                        const float c = ex.head_c ? -LOG2E * __ldg(ex.head_c + hd) : 0.0f;
+                        for (int e = r; e < tab_len; e += 128)
+                            tab[h * ex.tab_stride + e] = fmaf(a, w_log2(fmaf(bb, (float)max(d0 + e, 0), 1.0f)), c);
+                    }
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + x) : "memory");
+                tb = tab + tab_row;
+                if (!ok) continue;
+            }
             // S of this key tile has landed, and with it the product of the tile before
-            if (!mbar_wait(BAR(W_SFULL + x), it & 1)) { ok = false; break; }
+            if (!mbar_wait(BAR(W_SFULL + x), it & 1)) {
+                ok = false;
+                if (TABLE) continue;
+                break;
+            }
             tc_fence_after();
             const int j0 = (tile_first + it) * KN;
-            const bool full = p.window == 0 && j0 + KN - 1 <= pos_lo;       // every key visible to every row: no masks
+            // every key visible to every row: no masks
+            const bool full = DIFF ? j0 >= all_lo && j0 + KN - 1 <= pos_lo : p.window == 0 && j0 + KN - 1 <= pos_lo;
             float v[64];
+            if constexpr (KIND == W_SIGMOID) {
+                // nothing is normalised over the keys: no maximum, no sum, no rescaling, one pass over the scores
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    tmem_ld64(s_addr + c * 64, v);
+                    uint32_t pw[32];
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        float2 w = w_sigmoid2(fmaf(v[2 * i], -sc, tb[-(c * 64 + 2 * i)]), fmaf(v[2 * i + 1], -sc, tb[-(c * 64 + 2 * i + 1)]));
+                        if (!full) {
+                            const int j = j0 + c * 64 + 2 * i;
+                            if (!(j <= pos && (p.window == 0 || pos - j < p.window))) w.x = 0.0f;
+                            if (!(j + 1 <= pos && (p.window == 0 || pos - j - 1 < p.window))) w.y = 0.0f;
+                        }
+                        __nv_bfloat162 h2 = __floats2bfloat162_rn(w.x, w.y);
+                        pw[i] = *reinterpret_cast<uint32_t*>(&h2);
+                    }
+                    tmem_st32u(s_addr + c * 32, pw);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(BAR((c == 0 ? W_PHALF : W_PFULL) + x));
+                }
+                continue;
+            }
             // the row's maximum, as four chains that the scheduler can interleave: keys 64-127, then keys 0-63,
             // which stay in registers
             float r0 = NEG_BIG, r1 = NEG_BIG, r2 = NEG_BIG, r3 = NEG_BIG;
 #pragma unroll
             for (int c = 1; c >= 0; --c) {
                 tmem_ld64(s_addr + c * 64, v);
+                if constexpr (TABLE) {
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) v[i] = fmaf(v[i], sc, tb[-(c * 64 + i)]);
+                }
                 if (!full) {
 #pragma unroll
                     for (int i = 0; i < 64; ++i) {
                         const int j = j0 + c * 64 + i;
-                        const bool vis = j <= pos && (p.window == 0 || pos - j < p.window);
+                        const bool vis = DIFF ? j <= pos && j >= vis_lo : j <= pos && (p.window == 0 || pos - j < p.window);
                         v[i] = vis ? v[i] : NEG_BIG;
                     }
                 }
@@ -835,7 +954,9 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 }
             }
             const float raw = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
-            const float mx = raw > 0.5f * NEG_BIG ? raw * sc : NEG_BIG;
+            // (with a table the scores are scaled already; a cap keeps their order, so the largest is capped alone)
+            const float capped = TABLE ? raw : DIFF ? ex.cap_c - 2.0f * ex.cap_c * w_sigmoid2(ex.cap_k * raw, 0.0f).x : raw * sc;
+            const float mx = raw > 0.5f * NEG_BIG ? capped : NEG_BIG;
             const bool raise = mx > m + 8.0f;
             if (it == 0) {
                 m = mx;                                              // nothing accumulated yet
@@ -864,11 +985,15 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             for (int c = 0; c < 2; ++c) {
                 if (c == 1) {                                        // keys 64-127 again (their columns are untouched)
                     tmem_ld64(s_addr + 64, v);
+                    if constexpr (TABLE) {
+#pragma unroll
+                        for (int i = 0; i < 64; ++i) v[i] = fmaf(v[i], sc, tb[-(64 + i)]);
+                    }
                     if (!full) {
 #pragma unroll
                         for (int i = 0; i < 64; ++i) {
                             const int j = j0 + 64 + i;
-                            const bool vis = j <= pos && (p.window == 0 || pos - j < p.window);
+                            const bool vis = DIFF ? j <= pos && j >= vis_lo : j <= pos && (p.window == 0 || pos - j < p.window);
                             v[i] = vis ? v[i] : NEG_BIG;
                         }
                     }
@@ -876,8 +1001,18 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 uint32_t pw[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
-                    const float2 e = __ffma2_rn(make_float2(v[2 * i], v[2 * i + 1]), sc2, nm2);
-                    const float2 pp = make_float2(ex2(e.x), ex2(e.y));
+                    float2 e;
+                    if constexpr (DIFF) {
+                        const float2 w = w_sigmoid2(ex.cap_k * v[2 * i], ex.cap_k * v[2 * i + 1]);
+                        e = __ffma2_rn(w, make_float2(-2.0f * ex.cap_c, -2.0f * ex.cap_c), make_float2(ex.cap_c + nm, ex.cap_c + nm));
+                    } else {
+                        e = TABLE ? __fadd2_rn(make_float2(v[2 * i], v[2 * i + 1]), nm2) : __ffma2_rn(make_float2(v[2 * i], v[2 * i + 1]), sc2, nm2);
+                    }
+                    float2 pp = make_float2(ex2(e.x), ex2(e.y));
+                    if (DIFF && !full) {                             // a hidden key's score is capped as well: it weighs nothing
+                        if (v[2 * i] <= 0.5f * NEG_BIG) pp.x = 0.0f;
+                        if (v[2 * i + 1] <= 0.5f * NEG_BIG) pp.y = 0.0f;
+                    }
                     rs2 = __fadd2_rn(rs2, pp);
                     __nv_bfloat162 h2 = __floats2bfloat162_rn(pp.x, pp.y);
                     pw[i] = *reinterpret_cast<uint32_t*>(&h2);
@@ -901,8 +1036,74 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
         if (ok && n_tiles > 0 && !mbar_wait(BAR(W_FINAL), 0)) ok = false;
         if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
         tc_fence_after();
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-        uint4* dst = reinterpret_cast<uint4*>(p.out + ((size_t)tok * p.nh + head) * HD);
+        float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        if constexpr (DIFF) {
+            // every product is complete: map 2's rows go through the stages of K and V to the threads of map 1
+            constexpr int XS = HD + 4;
+            float* const xrow = reinterpret_cast<float*>(smem + W_OFF_K) + (size_t)r * XS;
+            const bool on = ok && n_tiles > 0;
+            if (x == 1) {
+#pragma unroll
+                for (int c = 0; c < HD; c += 32) {
+                    float o[32];
+                    if (on) tmem_ld32(o_addr + c, o);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4*>(xrow + c + i) = on ? make_float4(o[i] * inv * ex.lambda, o[i + 1] * inv * ex.lambda, o[i + 2] * inv * ex.lambda, o[i + 3] * inv * ex.lambda)
+                                                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            }
+            asm volatile("bar.sync 3, 256;" ::: "memory");
+            if (x == 0) {
+                float ss = 0.0f, norm = 0.0f;
+                __nv_bfloat16* orow = p.out + (size_t)tok * ex.out_stride + (size_t)head * HD;
+#pragma unroll 1
+                for (int pass = 0; pass < 2; ++pass) {               // the sum of squares, then the row itself
+#pragma unroll
+                    for (int c = 0; c < HD; c += 32) {
+                        float o[32];
+                        if (on) tmem_ld32(o_addr + c, o);
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 t = *reinterpret_cast<const float4*>(xrow + c + i);
+                            o[i] = on ? fmaf(o[i], inv, -t.x) : 0.0f; o[i + 1] = on ? fmaf(o[i + 1], inv, -t.y) : 0.0f;
+                            o[i + 2] = on ? fmaf(o[i + 2], inv, -t.z) : 0.0f; o[i + 3] = on ? fmaf(o[i + 3], inv, -t.w) : 0.0f;
+                            if (pass == 0) ss = fmaf(o[i], o[i], fmaf(o[i + 1], o[i + 1], fmaf(o[i + 2], o[i + 2], fmaf(o[i + 3], o[i + 3], ss))));
+                        }
+                        if (pass == 1 && row_ok && ok) {
+#pragma unroll
+                            for (int q8 = 0; q8 < 4; ++q8) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    __nv_bfloat162 h2 = __floats2bfloat162_rn(o[q8 * 8 + 2 * i] * norm, o[q8 * 8 + 2 * i + 1] * norm);
+                                    w[i] = *reinterpret_cast<uint32_t*>(&h2);
+                                }
+                                reinterpret_cast<uint4*>(orow)[c / 8 + q8] = make_uint4(w[0], w[1], w[2], w[3]);
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    norm = ex.out_scale / sqrtf(ss / (float)HD + ex.eps);
+                }
+            }
+        } else {
+        const float* gate = nullptr;
+        __nv_bfloat16* orow = p.out + ((size_t)tok * p.nh + head) * HD;
+        if constexpr (KIND != W_PLAIN) {
+            orow = p.out + (size_t)tok * ex.out_stride + (size_t)head * HD;
+            if (KIND == W_SIGMOID) {
+                inv = 1.0f;
+            } else {
+                // the sink joins the denominator; if it is above every score the sums are scaled down to it
+                const float sink2 = ex.sink ? __ldg(ex.sink + head) * LOG2E : NEG_BIG;
+                const float top = fmaxf(m, sink2), f = m > 0.5f * NEG_BIG ? ex2(m - top) : 0.0f;
+                const float den = l * f + (ex.sink ? ex2(sink2 - top) : 0.0f);
+                inv = den > 0.0f ? ex.out_scale * f / den : 0.0f;
+                if (ex.gate) gate = ex.gate + (size_t)tok * ex.gate_stride + (size_t)head * HD;
+            }
+        }
+        uint4* dst = reinterpret_cast<uint4*>(orow);
 #pragma unroll
         for (int c = 0; c < HD; c += 32) {
             float o[32];
@@ -916,6 +1117,16 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 #pragma unroll
                 for (int q8 = 0; q8 < 4; ++q8) {
                     uint32_t w[4];
+                    if (KIND != W_PLAIN && gate) {
+#pragma unroll
+                        for (int i = 0; i < 8; i += 4) {
+                            const float4 g4 = *reinterpret_cast<const float4*>(gate + c + q8 * 8 + i);
+                            o[q8 * 8 + i] = __fdividef(o[q8 * 8 + i], 1.0f + __expf(-g4.x));
+                            o[q8 * 8 + i + 1] = __fdividef(o[q8 * 8 + i + 1], 1.0f + __expf(-g4.y));
+                            o[q8 * 8 + i + 2] = __fdividef(o[q8 * 8 + i + 2], 1.0f + __expf(-g4.z));
+                            o[q8 * 8 + i + 3] = __fdividef(o[q8 * 8 + i + 3], 1.0f + __expf(-g4.w));
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         __nv_bfloat162 h2 = __floats2bfloat162_rn(o[q8 * 8 + 2 * i] * inv, o[q8 * 8 + 2 * i + 1] * inv);
@@ -924,6 +1135,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     dst[c / 8 + q8] = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
+        }
         }
     }
     tc_fence_before();
@@ -950,17 +1162,18 @@ EncodeTiledFn encode_fn() {
     });
     return fn;
 }
-// One layer's pages seen as [rows][HD] bfloat16, boxes of 16 rows x 64 values.
-int kv_map_for(CUtensorMap* out, const void* pool, long long rows) {
-    static std::unordered_map<const void*, std::pair<long long, CUtensorMap>> cache;
+// One layer's pages seen as [rows][row_elems] bfloat16, boxes of 16 rows x 64 values.
+int kv_map_for(CUtensorMap* out, const void* pool, long long rows, int row_elems = HD) {
+    static std::unordered_map<const void*, std::pair<std::pair<long long, int>, CUtensorMap>> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(pool);
-    if (it != cache.end() && it->second.first == rows) { *out = it->second.second; return AIRUN_OK; }
+    const std::pair<long long, int> shape(rows, row_elems);
+    if (it != cache.end() && it->second.first == shape) { *out = it->second.second; return AIRUN_OK; }
     EncodeTiledFn fn = encode_fn();
     if (!fn) return AIRUN_ERR_UNSUPPORTED;
-    cuuint64_t dims[2] = {(cuuint64_t)HD, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)HD * 2};
+    cuuint64_t dims[2] = {(cuuint64_t)row_elems, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)row_elems * 2};
     cuuint32_t box[2] = {64, 16};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pool), dims, strides, box, estr,
@@ -968,7 +1181,7 @@ int kv_map_for(CUtensorMap* out, const void* pool, long long rows) {
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return AIRUN_ERR_ARG;
     if (cache.size() > 4096) cache.clear();
-    cache[pool] = std::make_pair(rows, *out);
+    cache[pool] = std::make_pair(shape, *out);
     return AIRUN_OK;
 }
 
@@ -1025,12 +1238,101 @@ AIRUN_EXPORT int airun_attn_prefill_wide(const void* q, void* out, const void* p
     if (r != AIRUN_OK) return r;
     static unsigned long long configured = 0;            // one bit per device
     if (first_on_device(configured)) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_wide_kernel<W_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_TOTAL);
         if (e != cudaSuccess) return (int)e;
     }
-    airun_launch(attn_prefill_wide_kernel, dim3(n_tiles, nkv), dim3(TC_THREADS), W_SMEM_TOTAL, stream, p, (const int4*)tiles, map, n_tiles_dev);
+    airun_launch(attn_prefill_wide_kernel<W_PLAIN>, dim3(n_tiles, nkv), dim3(TC_THREADS), W_SMEM_TOTAL, stream, p, (const int4*)tiles, map, n_tiles_dev, WideExtra{});
     return airun_launch_status();
 }
+
+#if HD == 128
+// The wide kernel for the softmax attention with its options and for the attention without softmax (head and value size
+// 128); tiles of up to tile_rows / G tokens, tile_rows 128 or 256.  kind: W_OPTIONS, W_TABLE or W_SIGMOID.  tail >= 0: the
+// pages hold one row of 128 + tail elements for key and value.  out, gate: rows of out_stride and gate_stride elements,
+// 16-byte aligned.
+AIRUN_EXPORT int airun_attn_prefill_kinds(int kind, const void* q, void* out, long long out_stride, const void* pool,
+                                          const int32_t* block_table, int max_blocks, const int32_t* positions, int num_pages,
+                                          int page_size, int nh, int nkv, float scale, int window, const float* table, int table_len,
+                                          const float* sink, const float* gate, long long gate_stride, float out_scale,
+                                          const float* dist_a, const float* dist_b, const float* head_c, int tail, const void* tiles,
+                                          int n_tiles, const int32_t* n_tiles_dev, int tile_rows, int* err, cudaStream_t stream) {
+    if (n_tiles < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || nh / nkv > QM || !err || (tile_rows != QM && tile_rows != 2 * QM) ||
+        out_stride < (long long)nh * HD || (dist_a && !dist_b))
+        return AIRUN_ERR_ARG;
+    if ((kind != W_OPTIONS && kind != W_TABLE && kind != W_SIGMOID) || (kind == W_TABLE && (!table || table_len <= 0))) return AIRUN_ERR_ARG;
+    if (out_stride % 8 || ((uintptr_t)out & 15) || ((uintptr_t)q & 15) || (tail >= 0 && tail % 8)) return AIRUN_ERR_ARG;
+    if (gate && (gate_stride % 4 || ((uintptr_t)gate & 15))) return AIRUN_ERR_ARG;
+    int shift = -1;
+    for (int s = 4; s < 20; ++s) if ((1 << s) == page_size) shift = s;
+    if (shift < 0) return AIRUN_ERR_UNSUPPORTED;
+    if (n_tiles == 0) return AIRUN_OK;
+    if (nkv > 65535) return AIRUN_ERR_ARG;
+    TcParams p;
+    p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out; p.block_table = block_table; p.positions = positions;
+    p.max_blocks = max_blocks; p.num_pages = num_pages; p.page_size = page_size; p.page_shift = shift;
+    p.nh = nh; p.nkv = nkv; p.G = nh / nkv; p.scale_log2 = scale * LOG2E; p.window = window; p.err = err;
+    WideExtra ex = {};
+    ex.out_stride = out_stride; ex.table = table; ex.table_len = table_len; ex.sink = sink; ex.gate = gate; ex.gate_stride = gate_stride;
+    ex.out_scale = out_scale; ex.dist_a = dist_a; ex.dist_b = dist_b; ex.head_c = head_c; ex.tail = tail;
+    int smem = W_SMEM_TOTAL;
+    if (kind != W_OPTIONS) {
+        // the lanes of a warp are 32 / G tokens of G heads: with this stride they read 32 different banks
+        ex.tab_toks = QM / p.G + 2;
+        ex.tab_stride = (ex.tab_toks + 127 + 31) / 32 * 32 + (p.G < 32 ? 32 / p.G : 1);
+        smem += 4 * p.G * ex.tab_stride * (int)sizeof(float);
+        if (smem > 227 * 1024) return AIRUN_ERR_UNSUPPORTED;         // G up to 12
+    }
+    CUtensorMap map;
+    const int width = tail >= 0 ? HD + tail : HD;
+    const int r = kv_map_for(&map, pool, (long long)num_pages * (tail >= 0 ? 1 : 2) * nkv * page_size, width);
+    if (r != AIRUN_OK) return r;
+    static unsigned long long configured[3];             // one bit per device
+    auto go = [&](auto kern, int i) -> int {
+        if (first_on_device(configured[i])) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (e != cudaSuccess) return (int)e;
+        }
+        airun_launch(kern, dim3(n_tiles, nkv), dim3(TC_THREADS), smem, stream, p, (const int4*)tiles, map, n_tiles_dev, ex);
+        return airun_launch_status();
+    };
+    if (kind == W_OPTIONS) return go(attn_prefill_wide_kernel<W_OPTIONS>, 0);
+    if (kind == W_TABLE) return go(attn_prefill_wide_kernel<W_TABLE>, 1);
+    return go(attn_prefill_wide_kernel<W_SIGMOID>, 2);
+}
+
+// Differential attention: q [T][nh][2 * 64], pages of keys [nkv][page][2 * 64] then values [nkv][page][128]; cap > 0; tiles of
+// up to 128 / G tokens.
+AIRUN_EXPORT int airun_attn_prefill_diff(const void* q, void* out, long long out_stride, const void* pool, const int32_t* block_table,
+                                         int max_blocks, const int32_t* positions, int num_pages, int page_size, int nh, int nkv,
+                                         float scale, float cap, float lambda, float eps, float out_scale, int chunk, int window,
+                                         const void* tiles, int n_tiles, const int32_t* n_tiles_dev, int* err, cudaStream_t stream) {
+    if (n_tiles < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || nh / nkv > QM || !err || out_stride < (long long)nh * HD || !(cap > 0.0f) ||
+        chunk < 0 || window < 0 || out_stride % 8 || (((uintptr_t)out | (uintptr_t)q) & 15))
+        return AIRUN_ERR_ARG;
+    int shift = -1;
+    for (int s = 4; s < 20; ++s) if ((1 << s) == page_size) shift = s;
+    if (shift < 0) return AIRUN_ERR_UNSUPPORTED;
+    if (n_tiles == 0) return AIRUN_OK;
+    if (nkv > 65535) return AIRUN_ERR_ARG;
+    TcParams p;
+    p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out; p.block_table = block_table; p.positions = positions;
+    p.max_blocks = max_blocks; p.num_pages = num_pages; p.page_size = page_size; p.page_shift = shift;
+    p.nh = nh; p.nkv = nkv; p.G = nh / nkv; p.scale_log2 = scale * LOG2E; p.window = window; p.err = err;
+    WideExtra ex = {};
+    ex.out_stride = out_stride; ex.out_scale = out_scale; ex.tail = -1; ex.cap_c = cap * LOG2E; ex.cap_k = 2.0f * scale * LOG2E / cap;
+    ex.lambda = lambda; ex.eps = eps; ex.chunk = chunk;
+    CUtensorMap map;
+    const int r = kv_map_for(&map, pool, (long long)num_pages * 2 * nkv * page_size);
+    if (r != AIRUN_OK) return r;
+    static unsigned long long configured = 0;
+    if (first_on_device(configured)) {
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_wide_kernel<W_DIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_TOTAL);
+        if (e != cudaSuccess) return (int)e;
+    }
+    airun_launch(attn_prefill_wide_kernel<W_DIFF>, dim3(n_tiles, nkv), dim3(TC_THREADS), W_SMEM_TOTAL, stream, p, (const int4*)tiles, map, n_tiles_dev, ex);
+    return airun_launch_status();
+}
+#endif
 
 // The shared prefix of a batch of decoded tokens on tcgen05: see TcShared.  Same contract as
 // airun_attn_shared_prefix of attention_mma.cu (slots n_splits .. n_splits+slices-1 of every unit of the

@@ -695,6 +695,27 @@ def diff_attention_supported(D: int, Dv: int) -> bool:
     return "diff_attention" not in DISABLED and D <= 128 and Dv <= 128
 
 
+def diff_prefill_tc(ctx, q, out, cache, part) -> bool:
+    """The prompt portions of a differential attention with maps of 64 and values of 128 on tcgen05 (``W_DIFF`` of
+    csrc/attention_tcgen05.cu); single tokens are left alone.  False: the sizes, the pages or the alignment are not this
+    kernel's, or the batch is too small for it."""
+    T, nh, nkv = q.shape[0], part.nh, part.nkv
+    if (part.D != 64 or part.Dv != 128 or T < PROMPT_TC_MIN_TOKENS or not hasattr(ctx, "extras") or not part.cap > 0 or not part.scale > 0
+            or not prefill_tc_supported(128, int(cache.page_size)) or out.stride(0) % 8 or out.data_ptr() % 16 or q.data_ptr() % 16
+            or cache.pool.data_ptr() % 16):
+        return False
+    tiles, n, n_dev = _prompt_tiles(ctx, nh // nkv, PREFILL_ROWS, T)
+    pool, bt = cache.pool, cache.block_table
+    f = _fn("attention_tcgen05", "airun_attn_prefill_diff",
+            [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float,
+             c_float, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p], {"HD": 128})
+    _check(f(_p(q), _p(out), out.stride(0) if T > 1 else max(out.shape[1], out.stride(0)), _p(pool), _p(bt), bt.stride(0), _p(ctx.positions),
+             pool.shape[0], int(cache.page_size), nh, nkv, float(part.scale), float(part.cap), float(part.lam), float(part.eps),
+             1.0 - float(part.lambda_init), int(part.chunk), int(part.window), _p(tiles), n, _p(n_dev), _p(ctx.err), _stream()),
+           "attn_prefill_diff")
+    return True
+
+
 def diff_attention_bf16(ctx, q, out, cache, part) -> bool:
     """Differential attention on the tensor cores (csrc/diff_attention_mma.cu) for every row of the batch, prompt
     portions and single tokens alike; False: the caller runs the plain kernel (head sizes above 128)."""
@@ -724,6 +745,8 @@ def diff_attention_bf16(ctx, q, out, cache, part) -> bool:
         f = _fn("diff_attention_mma", "airun_diff_attention_group", sig + csig + [c_void_p, c_void_p])
         _check(f(*common, *consts, _p(ctx.err), _stream()), "diff_attention_group")
     if single and getattr(ctx, "decode_only", False):
+        return True
+    if single and diff_prefill_tc(ctx, q, out, cache, part):
         return True
     # every other request's tokens are cut into tiles of 64; the kernel walks cu_tokens to find its tile, so the
     # launch only needs an upper bound of their number
@@ -801,6 +824,55 @@ def linear_act_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mo
     return True
 
 
+PROMPT_KINDS = dict(options=1, table=2, sigmoid=3)     # of csrc/attention_tcgen05.cu: airun_attn_prefill_kinds
+PROMPT_TC_MIN_TOKENS = 192
+
+
+def _prompt_tiles(ctx, G: int, tile_rows: int, T: int):
+    """(tiles, their largest number, their number on the device): the portions of the batch cut into tiles of tile_rows // G
+    tokens by csrc/attention_plan.cu, the tiles with the most keys first; made once per step, group size and tile size."""
+    key = ("prompt_tiles", G, tile_rows)
+    got = ctx.extras.get(key)
+    if got is None:
+        per, shape = max(1, tile_rows // G), ctx.extras.get("device_plan") or {}
+        portions = min(int(shape.get("max_portions", ctx.num_reqs)), int(ctx.num_reqs), T // 2)
+        n = T // per + portions + 1
+        ws = getattr(ctx, "ws_main", None)
+        buf = ws.alloc((4 + 4 * n + T,), torch.int32) if ws is not None else torch.empty(4 + 4 * n + T, dtype=torch.int32, device=ctx.err.device)
+        tiles = buf[4:4 + 4 * n].view(n, 4)
+        attn_plan(ctx, per, tiles, buf[4 + 4 * n:], buf[:4])
+        got = ctx.extras[key] = (tiles, n, buf[0:1])
+    return got
+
+
+def attn_prompt_kind(ctx, kind: str, q, out, cache, part, tail: int = -1, gate: Optional[torch.Tensor] = None, gate_stride: int = 0) -> bool:
+    """The prompt portions of the attentions with heads of 128 on tcgen05 (``attn_prefill_wide_kernel`` and its kinds); single
+    tokens are left alone.  False: the sizes, the pages or the alignment are not this kernel's, or the batch is too small
+    for it."""
+    T, D, Dv, nh, nkv = q.shape[0], part.D, part.Dv, part.nh, part.nkv
+    G = nh // nkv
+    if (D != 128 or Dv != 128 or T < PROMPT_TC_MIN_TOKENS or not hasattr(ctx, "extras") or (kind == "options" and not part.scale > 0) or not prefill_tc_supported(D, int(cache.page_size)) or G > (16 if kind == "options" else 12)
+            or out.stride(0) % 8 or out.data_ptr() % 16 or q.data_ptr() % 16 or cache.pool.data_ptr() % 16 or (tail >= 0 and tail % 8)
+            or (gate is not None and (gate_stride % 4 or gate.data_ptr() % 16))):
+        return False
+    # two Q tiles a CTA share every key tile; with fewer than a CTA for nearly every SM one Q tile each gives twice as many
+    rows = PREFILL_ROWS_WIDE if T // (PREFILL_ROWS_WIDE // G) * nkv >= machine(q.device).wide_min_ctas else PREFILL_ROWS
+    tiles, n, n_dev = _prompt_tiles(ctx, G, rows, T)
+    pool, bt = cache.pool, cache.block_table
+    table, sink = getattr(part, "table", None), getattr(part, "sink", None)
+    f = _fn("attention_tcgen05", "airun_attn_prefill_kinds",
+            [c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p,
+             c_int, c_void_p, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
+             c_void_p], {"HD": 128})
+    sig = kind == "sigmoid"
+    _check(f(PROMPT_KINDS[kind], _p(q), _p(out), out.stride(0) if T > 1 else max(out.shape[1], out.stride(0)), _p(pool), _p(bt), bt.stride(0),
+             _p(ctx.positions), pool.shape[0], int(cache.page_size), nh, nkv, float(part.scale), int(part.window),
+             None if sig else _p(table), 0 if sig or table is None else table.shape[1], None if sig else _p(sink), _p(gate), int(gate_stride),
+             1.0 if sig else float(part.out_scale), _p(part.dist_a) if sig else None, _p(part.dist_b) if sig else None,
+             _p(part.head_c) if sig else None, tail, _p(tiles), n, _p(n_dev), rows, _p(ctx.err), _stream()), "attn_prefill_kinds")
+    return True
+
+
 SIGMOID_TILE_ROWS = 64
 SIGMOID_MIN_KEYS_PER_SLICE = 256       # a slice of a single token's keys is at least this long
 
@@ -872,6 +944,8 @@ def sigmoid_attention_bf16(ctx, q, out, cache, part) -> bool:
         _check(f(*common, *consts, splits, _p(partial), T, _p(ctx.err), _stream()), "sigmoid_attention_group")
     if single and decode_only:
         return True
+    if single and attn_prompt_kind(ctx, "sigmoid", q, out, cache, part):
+        return True
     # every other request's tokens are cut into tiles of 64; the kernel walks cu_tokens to find its tile, so the
     # launch only needs an upper bound of their number
     max_tiles = (T + SIGMOID_TILE_ROWS - 1) // SIGMOID_TILE_ROWS + int(ctx.num_reqs)
@@ -927,6 +1001,9 @@ def softmax_attention_bf16(ctx, q, out, cache, part, gate: Optional[torch.Tensor
         f = _fn("softmax_attention_mma", "airun_softmax_attention_group", sig + csig + [c_int, c_void_p, c_int, c_void_p, c_void_p])
         _check(f(*common, *consts, splits, _p(partial), T, _p(ctx.err), _stream()), "softmax_attention_group")
     if single and decode_only:
+        return True
+    if single and attn_prompt_kind(ctx, "options" if part.table is None else "table", q, out, cache, part, tail=tail, gate=gate,
+                                   gate_stride=ops.attention_gate(gate, T, nh * Dv)):
         return True
     # every other request's tokens are cut into tiles of 64; the kernel walks cu_tokens to find its tile, so the
     # launch only needs an upper bound of their number

@@ -1,0 +1,128 @@
+"""The prompt attention on tcgen05 for heads of 128 (csrc/attention_tcgen05.cu: attn_prefill_wide_kernel and its kinds)
+against the plain kernels, which work in float32 from the same bfloat16 q and pages: softmax with a window, a distance
+table, a sink, a factor, a gate and rows that are key and value; attention without softmax.
+
+Tolerance: both sides round the result to bfloat16 (half a unit, 2^-8 of it at most, each) and the tensor cores take the weights
+as bfloat16 (2^-8 of each at most; a row's weighted mean of values moves by at most that times the largest value): 3 * 2^-8
+of the largest value.  Without softmax a row's weights do not sum to one: n weights rounded one by one move the sum of n
+values by about sqrt(n) 2^-9 of the largest weight and value, few of up to 2,048 keys weigh much; 3 * 2^-8 of the larger of the
+largest result and the largest value."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_pirerax import batch_ctx, scrambled_table
+
+gpu = pytest.mark.gpu
+
+# heads, kv heads, page, window, tail, table rows, sink, gate, out_scale, spans (first position, end) of the requests
+CASES = [
+    (1, 1, 16, 0, -1, 0, False, False, 1.0, [(0, 193)]),
+    (2, 1, 16, 0, -1, 0, True, False, 0.7, [(0, 128), (3, 67)]),
+    (4, 2, 32, 0, -1, 0, True, True, 1.0, [(0, 129), (500, 501), (77, 205)]),
+    (3, 1, 16, 100, -1, 0, False, True, 1.0, [(130, 500)]),
+    (6, 1, 64, 1, -1, 0, False, False, 1.0, [(0, 200)]),
+    (16, 1, 16, 0, -1, 0, True, False, 1.0, [(1000, 1255)]),
+    (16, 8, 16, 1024, -1, 0, False, False, 1.0, [(0, 2048)]),
+    (2, 2, 16, 0, -1, 40, True, False, 1.3, [(0, 300), (5, 6)]),
+    (16, 8, 16, 0, -1, 700, True, False, 1.0, [(0, 1027), (0, 2), (900, 1300)]),
+    (12, 1, 32, 0, -1, 5, False, False, 1.0, [(250, 449)]),
+    (5, 1, 16, 333, -1, 1, True, True, 1.0, [(0, 700)]),
+    (4, 2, 16, 90, 64, 0, True, False, 1.0, [(0, 257), (40, 140)]),
+    (3, 3, 16, 0, 8, 0, False, False, 1.0, [(10, 211)]),
+]
+SIGMOID_CASES = [(1, 1, 16, 0, True, True, [(0, 193)]), (2, 1, 32, 0, True, False, [(0, 128), (3, 67), (9, 10)]), (16, 8, 16, 0, True, True, [(0, 2048)]),
+                 (12, 1, 16, 200, False, True, [(250, 449)]), (3, 1, 64, 1, True, True, [(5, 300)]), (4, 2, 16, 0, False, False, [(0, 255), (1, 300)])]
+
+
+def made(nh, nkv, page, tail, spans, seed):
+    g = torch.Generator().manual_seed(seed)
+    bt, num_pages = scrambled_table([e for _, e in spans], page, g)
+    width = 128 + tail if tail >= 0 else 256
+    pool = (0.8 * torch.randn(num_pages, nkv * page * width, generator=g)).to("cuda", torch.bfloat16)
+    ctx = batch_ctx(spans)
+    T = ctx.num_tokens
+    q = torch.randn(T, nh * 128, generator=g).to("cuda", torch.bfloat16)
+    return g, SimpleNamespace(pool=pool, block_table=bt, page_size=page, shared=False), ctx, q
+
+
+def run_both(ctx, q, nh, tc, plain):
+    got = torch.full((q.shape[0], nh * 128 + 16), 7.0, device="cuda", dtype=torch.bfloat16)
+    want = torch.zeros(q.shape[0], nh * 128, device="cuda", dtype=torch.bfloat16)
+    assert tc(got[:, 8:8 + nh * 128])
+    plain(want)
+    assert int(ctx.err.item()) == 0
+    assert bool((got[:, :8] == 7.0).all()) and bool((got[:, 8 + nh * 128:] == 7.0).all())
+    lens = [n for n in ctx.query_lens for _ in range(n)]
+    rows = torch.tensor([n > 1 for n in lens], device="cuda")
+    assert bool((got[~rows][:, 8:8 + nh * 128] == 7.0).all())          # single tokens are another kernel's
+    return got[rows][:, 8:8 + nh * 128].float(), want[rows].float()
+
+
+@gpu
+@pytest.mark.parametrize("nh,nkv,page,window,tail,rows,sink,gated,scale,spans", CASES)
+def test_softmax_kinds(nh, nkv, page, window, tail, rows, sink, gated, scale, spans):
+    from airun_b200.kernels import fast, ops
+    g, cache, ctx, q = made(nh, nkv, page, tail, spans, nh * 100 + len(spans) + window)
+    T = q.shape[0]
+    part = SimpleNamespace(D=128, Dv=128, nh=nh, nkv=nkv, scale=0.13, window=window, out_scale=scale, tail=tail,
+                           table=(2.0 * torch.randn(nh, rows, generator=g)).cuda() if rows else None,
+                           sink=(2.0 * torch.randn(nh, generator=g)).cuda() if sink else None)
+    gate = torch.randn(T, nh * 128 + 4, generator=g).cuda()[:, 4:] if gated else None
+    got, want = run_both(
+        ctx, q, nh,
+        lambda o: fast.attn_prompt_kind(ctx, "table" if rows else "options", q, o, cache, part, tail=tail, gate=gate,
+                                        gate_stride=ops.attention_gate(gate, T, nh * 128)),
+        lambda o: ops.softmax_attention(q, o, cache, ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, scale, tail=tail, gate=gate))
+    assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * scale * float(cache.pool.abs().max())
+
+
+@gpu
+@pytest.mark.parametrize("nh,nkv,page,window,dist,offset,spans", SIGMOID_CASES)
+def test_attention_without_softmax(nh, nkv, page, window, dist, offset, spans):
+    from airun_b200.kernels import fast, ops
+    g, cache, ctx, q = made(nh, nkv, page, -1, spans, nh * 7 + len(spans))
+    a, b, c = ((0.2 + torch.rand(nh, generator=g)).cuda(), (0.1 + torch.rand(nh, generator=g)).cuda(), (-2.0 + torch.randn(nh, generator=g)).cuda())
+    part = SimpleNamespace(D=128, Dv=128, nh=nh, nkv=nkv, scale=0.13, window=window, dist_a=a if dist else None, dist_b=b if dist else None,
+                           head_c=c if offset else None)
+    got, want = run_both(
+        ctx, q, nh, lambda o: fast.attn_prompt_kind(ctx, "sigmoid", q, o, cache, part),
+        lambda o: ops.sigmoid_attention(q, o, cache, ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, part.head_c, window))
+    assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * max(float(want.abs().max()), float(cache.pool.abs().max()))
+
+
+DIFF_CASES = [(1, 1, 16, 0, 0, [(0, 193)]), (4, 2, 32, 64, 0, [(0, 129), (500, 501), (77, 205)]), (3, 1, 16, 37, 0, [(130, 500)]),
+              (16, 8, 16, 2048, 0, [(0, 2100)]), (16, 1, 16, 0, 50, [(1000, 1255)]), (6, 3, 64, 300, 90, [(250, 700), (0, 2)])]
+
+
+@gpu
+@pytest.mark.parametrize("nh,nkv,page,chunk,window,spans", DIFF_CASES)
+def test_differential(nh, nkv, page, chunk, window, spans):
+    """Two maps, a soft cap and the difference's norm, against the plain kernel.  A result is a difference over its root mean
+    square, so what bounds it is the rounding of the two means (2^-9 of the largest value each, with the weights') over the
+    smallest root mean square among the rows, times the factor, and the result's own 2^-9."""
+    from airun_b200.kernels import fast, ops
+    g, cache, ctx, q = made(nh, nkv, page, -1, spans, nh * 31 + chunk)
+    part = SimpleNamespace(D=64, Dv=128, nh=nh, nkv=nkv, scale=0.3, cap=20.0, chunk=chunk, window=window, lam=0.45, eps=1e-5, lambda_init=0.2)
+
+    def plain(o):
+        ops.diff_attention(q, o, cache.pool, cache.block_table, ctx.positions, ctx.req_of_token, ctx.num_reqs, page, nh, nkv, 64, 128, 0.3, 20.0,
+                           chunk, window, 0.45, 1e-5, 0.8, ctx.err)
+
+    got, want = run_both(ctx, q, nh, lambda o: fast.diff_prefill_tc(ctx, q, o, cache, part), plain)
+    err = (got - want).view(-1, nh, 128).square().mean(-1).sqrt()
+    assert float(err.max()) < 0.03 and float(err.mean()) < 0.004
+
+
+@gpu
+def test_what_the_kernel_does_not_take_stays_with_the_other():
+    """Small batches, other head sizes, pages of 24, wide groups and unaligned rows are refused, not run."""
+    from airun_b200.kernels import fast
+    for nh, nkv, page, D, T, off in ((2, 1, 16, 128, 100, 8), (2, 1, 24, 128, 300, 8), (2, 1, 16, 64, 300, 8), (17, 1, 16, 128, 300, 8), (2, 1, 16, 128, 300, 4)):
+        bt, pages = scrambled_table([T], page, torch.Generator().manual_seed(1))
+        cache = SimpleNamespace(pool=torch.zeros(pages, nkv * page * 2 * D, device="cuda", dtype=torch.bfloat16), block_table=bt, page_size=page)
+        part = SimpleNamespace(D=D, Dv=D, nh=nh, nkv=nkv, scale=1.0, window=0, out_scale=1.0, tail=-1, table=None, sink=None)
+        q = torch.zeros(T, nh * D, device="cuda", dtype=torch.bfloat16)
+        out = torch.zeros(T, nh * D + 8, device="cuda", dtype=torch.bfloat16)[:, off:off + nh * D]
+        assert not fast.attn_prompt_kind(batch_ctx([(0, T)]), "options", q, out, cache, part)

@@ -68,7 +68,7 @@ DISABLED = set(filter(None, os.environ.get("AIRUN_DISABLE_FAST", "").split(","))
 def all_libraries():
     return [("gemm_tcgen05", None), ("gemm_tcgen05", {"AIRUN_FOLD_NORM": 1}), ("gemm_rows", None), ("attention_plan", None), ("attention_mma", {"HD": 128}), ("attention_mma", {"HD": 64}),
             ("attention_tcgen05", {"HD": 128}), ("attention_tcgen05", {"HD": 64}), ("diff_attention_mma", None),
-            ("latent_attention_mma", None), ("sigmoid_attention_mma", None), ("softmax_attention_mma", None)]
+            ("latent_attention_mma", None), ("latent_attention_tcgen05", None), ("sigmoid_attention_mma", None), ("softmax_attention_mma", None)]
 
 
 def scratch_for(device: torch.device) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -796,8 +796,31 @@ def latent_attention_bf16(ctx, qlat, out, cache, part, gate: Optional[torch.Tens
         _check(f(*common, *consts, splits, _p(partial), _p(ctx.err), _stream()), "latent_attention_group")
     if single and decode_only:
         return True
+    if single and latent_prefill_tc(ctx, qlat, out, cache, part, gate):
+        return True
     f = _fn("latent_attention_mma", "airun_latent_attention_mma", sig + [c_void_p] + csig + [c_int, c_void_p, c_void_p])
     _check(f(*common, _p(ctx.req_of_token), *consts, 1 if single else 0, _p(ctx.err), _stream()), "latent_attention_mma")
+    return True
+
+
+LATENT_TC_MIN_TOKENS = 64
+
+
+def latent_prefill_tc(ctx, qlat, out, cache, part, gate: Optional[torch.Tensor] = None) -> bool:
+    """The prompt portions of an attention over a cached latent on tcgen05 (csrc/latent_attention_tcgen05.cu); single tokens
+    are left alone.  False: the sizes, the pages or the alignment are not this kernel's, or the batch is too small for it."""
+    H, R, KD, page, T = part.nh, part.R, part.R + part.rd, int(cache.page_size), qlat.shape[0]
+    if ("latent_tc" in DISABLED or T < LATENT_TC_MIN_TOKENS or R % 64 or KD % 64 or R > 512 or KD > 576 or H > PREFILL_ROWS or page < 16
+            or page & (page - 1) or not hasattr(ctx, "context_lens") or not hasattr(ctx, "extras") or out.data_ptr() % 16 or qlat.data_ptr() % 16 or cache.pool.data_ptr() % 16):
+        return False
+    tiles, n, n_dev = _prompt_tiles(ctx, H, PREFILL_ROWS, T)
+    pool, bt = cache.pool, cache.block_table
+    f = _fn("latent_attention_tcgen05", "airun_latent_prefill",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p,
+             c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p])
+    _check(f(_p(qlat), _p(out), _p(pool), _p(bt), bt.stride(0), _p(ctx.positions), T, pool.shape[0], page, H, R, part.rd, float(part.scale),
+             int(part.window), _p(part.sink), _p(gate), ops.attention_gate(gate, T, H), _p(tiles), n, _p(n_dev), _p(ctx.err), _stream()),
+           "latent_prefill")
     return True
 
 

@@ -115,6 +115,38 @@ def test_differential(nh, nkv, page, chunk, window, spans):
     assert float(err.max()) < 0.03 and float(err.mean()) < 0.004
 
 
+LATENT_CASES = [  # heads, R, rd, page, window, sink, gate, spans
+    (16, 512, 64, 16, 0, True, True, [(0, 300)]), (16, 512, 64, 32, 0, True, False, [(0, 129), (400, 401), (63, 193)]),
+    (1, 64, 0, 16, 0, False, False, [(0, 257)]), (33, 320, 64, 16, 100, True, True, [(70, 171)]), (128, 512, 64, 16, 0, False, False, [(190, 260)]),
+    (2, 256, 64, 64, 1, False, True, [(0, 65), (3, 5)]), (20, 448, 128, 16, 0, True, True, [(1000, 1064)]), (3, 128, 0, 16, 0, True, False, [(0, 64)]),
+    (16, 512, 64, 16, 2048, True, False, [(0, 1100)])]
+
+
+@gpu
+@pytest.mark.parametrize("H,R,rd,page,window,sink,gated,spans", LATENT_CASES)
+def test_latent(H, R, rd, page, window, sink, gated, spans):
+    """The attention over a cached latent (csrc/latent_attention_tcgen05.cu) against its plain twin."""
+    from airun_b200.kernels import fast, ops
+    g = torch.Generator().manual_seed(H + R)
+    bt, num_pages = scrambled_table([e for _, e in spans], page, g)
+    pool = (0.8 * torch.randn(num_pages, page * (R + rd), generator=g)).to("cuda", torch.bfloat16)
+    cache = SimpleNamespace(pool=pool, block_table=bt, page_size=page, shared=False)
+    ctx = batch_ctx(spans)
+    T = ctx.num_tokens
+    q = torch.randn(T, H * (R + rd), generator=g).to("cuda", torch.bfloat16)
+    sd = (2.0 * torch.randn(H, generator=g)).cuda() if sink else None
+    gate = torch.randn(T, H + 3, generator=g).cuda()[:, 3:] if gated else None
+    part = SimpleNamespace(nh=H, R=R, rd=rd, scale=1.2 * (R + rd) ** -0.5, window=window, sink=sd)
+    got = torch.full((T, H * R), 7.0, device="cuda", dtype=torch.bfloat16)
+    want = torch.zeros_like(got)
+    assert fast.latent_prefill_tc(ctx, q, got, cache, part, gate)
+    ops.latent_attention(q, want, cache, ctx, H, R, rd, part.scale, window, sd, gate)
+    assert int(ctx.err.item()) == 0
+    rows = torch.tensor([n > 1 for n in ctx.query_lens for _ in range(n)], device="cuda")
+    assert bool((got[~rows] == 7.0).all())
+    assert float((got[rows].float() - want[rows].float()).abs().max()) < 3 * 2.0 ** -8 * float(pool.abs().max())
+
+
 @gpu
 def test_what_the_kernel_does_not_take_stays_with_the_other():
     """Small batches, other head sizes, pages of 24, wide groups and unaligned rows are refused, not run."""

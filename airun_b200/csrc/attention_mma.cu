@@ -371,13 +371,46 @@ struct DecodeExtra {
                                 //   chain of launches this one belongs to began (a step replayed as one graph)
 };
 
+// What a key weighs and what becomes of a row, for the attentions whose single tokens share this kernel (head size 128, TMA):
+//   D_PLAIN    the softmax of the reference's models
+//   D_OPTIONS  softmax with a distance table, a sink, a factor and a gate on the result, rows of a wider output, keys that
+//              are values as well (one cached row: the value begins `tail` elements into the key's row)
+//   D_SIGMOID  no softmax: a key weighs sigmoid(scale * qk - a_h ln(1 + b_h * distance) + c_h)
+// The formulas are those of softmax_attention.cu and sigmoid_attention.cu.  The kernels these took before ask for every key and
+// value row with a copy of its own, 64 keys at a time for the whole CTA, and bring the slices together in a launch of their own:
+// 64 tokens over 500 to 1,000 rows of 192 elements (8 KV heads) 53 + 4 us, 38 us here.
+enum { D_PLAIN = 0, D_OPTIONS = 1, D_SIGMOID = 2 };
+struct DecodeKind {
+    long long out_stride;
+    const float* table;           // [nh][table_len] or null
+    int table_len;
+    const float* sink;            // [nh] or null
+    const float* gate;            // [T][gate_stride] or null, columns head * HD + d
+    long long gate_stride;
+    float out_scale;
+    const float *dist_a, *dist_b, *head_c;      // D_SIGMOID: [nh] each, or null
+    int tail;                     // >= 0: one cached row for key and value
+};
+__device__ __forceinline__ float lg2_approx(float v) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+// 1 / (1 + 2^v): 2^v = inf gives 0, 2^v = 0 gives 1
+__device__ __forceinline__ float sigmoid_weight(float v) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return r;
+}
+
 // TMA = true: K/V tiles arrive by cp.async.bulk.tensor (one lane of each warp issues HD/64 boxes per
 // tile, three stages per warp, an mbarrier per stage); TMA = false: cp.async, two stages, any page size.
 // WITH_PREFIX: the build that leaves a shared prefix to another kernel and merges its results
 // (k_begin_dev, extra_slices); a build of its own so that the plain one carries none of that code.
-template <bool TMA, bool WITH_PREFIX>
+template <bool TMA, bool WITH_PREFIX, int KIND = D_PLAIN>
 __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p, const DecodeExtra x,
-                                                              const __grid_constant__ CUtensorMap kv_map) {
+                                                              const __grid_constant__ CUtensorMap kv_map, const DecodeKind kd) {
     pdl_trigger();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -425,9 +458,11 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     if (x.n_rows_dev) {
         const int fit = max(1, x.dyn_slots / max(1, n_rows_used * (int)gridDim.y));
         ns_stride = min(x.n_splits, fit);
-        ns = max(1, min(ns_stride, (n_tiles_all + 7) / 8));
-        if (split >= ns) return;
     }
+    // a slice has eight tiles or more: a context far below the one the launch was planned for takes fewer slices, a short one
+    // a single slice and no merge (one token over 100 keys planned for 2,048: 10.2 us, 5.5 with one slice)
+    ns = max(1, min(ns_stride, (n_tiles_all + 7) / 8));
+    if (split >= ns) return;
 
     // key tiles of this token, this slice, this warp
     const int per_split = (n_tiles_all + ns - 1) / ns;
@@ -475,15 +510,16 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
         const int blk = j0 >> p.page_shift;
         int page = blk < p.max_blocks ? __ldg(bt + blk) : -1;
         if (page < 0 || page >= p.num_pages) { atomicOr(p.err, AIRUN_DEV_BAD_PAGE); page = 0; }
-        const int krow = (((page * 2) * p.nkv + kvh) << p.page_shift) + (j0 & (p.page_size - 1));
-        const int vrow = krow + (p.nkv << p.page_shift);
+        const bool one_row = KIND != D_PLAIN && kd.tail >= 0;
+        const int krow = (((page * (one_row ? 1 : 2)) * p.nkv + kvh) << p.page_shift) + (j0 & (p.page_size - 1));
+        const int vrow = one_row ? krow : krow + (p.nkv << p.page_shift), v_x = one_row ? kd.tail : 0;
         const uint32_t bar = smem_u32(bars + stage);
         const uint32_t kb = smem_u32(wbase + stage * 2 * TILE_BYTES), vb = kb + TILE_BYTES;
         mbar_expect_tx(bar, 2 * TILE_BYTES);
 #pragma unroll
         for (int h = 0; h < HD / 64; ++h) {
             tma_load_2d(kb + h * 2048, &kv_map, bar, h * 64, krow);
-            tma_load_2d(vb + h * 2048, &kv_map, bar, h * 64, vrow);
+            tma_load_2d(vb + h * 2048, &kv_map, bar, v_x + h * 64, vrow);
         }
     };
     if (TMA) {
@@ -521,6 +557,20 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     for (int k = 0; k < HD / 16; ++k)
         ldsm4(qf[k], smem_u32(sQ) + tile_off((lane & 7) + ((lane >> 3) & 1) * 8, 2 * k + (lane >> 4)));
 
+    // this thread's rows g and g + 8: their heads' numbers
+    const float* table[2] = {nullptr, nullptr};
+    float dist_a[2] = {0.0f, 0.0f}, dist_b[2] = {0.0f, 0.0f}, offset[2] = {0.0f, 0.0f};
+    if constexpr (KIND != D_PLAIN) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int hd = head0 + min(g + 8 * h, heads - 1);
+            if (KIND == D_OPTIONS && kd.table) table[h] = kd.table + (size_t)hd * kd.table_len;
+            if (KIND == D_SIGMOID) {
+                if (kd.dist_a) { dist_a[h] = __ldg(kd.dist_a + hd); dist_b[h] = __ldg(kd.dist_b + hd); }
+                if (kd.head_c) offset[h] = -LOG2E * __ldg(kd.head_c + hd);
+            }
+        }
+    }
     bool timed_out = false;
     for (int it = 0; it < my_n; ++it) {
         const int stage = TMA ? it % DSTAGES : (it & 1);
@@ -546,42 +596,60 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             mma16816(s[0], qf[k], b[0], b[1]);
             mma16816(s[1], qf[k], b[2], b[3]);
         }
-        float mx0 = m0, mx1 = m1;
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = j0 + n * 8 + 2 * t + (e & 1);
-                const bool vis = j <= pos && j >= k_first;
-                const float v = vis ? s[n][e] * p.scale_log2 : NEG_BIG;
-                s[n][e] = v;
-                if (e < 2) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
-            }
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float c0 = exp2f(m0 - mx0), c1 = exp2f(m1 - mx1);
-        m0 = mx0; m1 = mx1;
         uint32_t pf[4];
-        float rs0 = 0.0f, rs1 = 0.0f;
+        if constexpr (KIND == D_SIGMOID) {
+            // nothing is normalised over the keys: no maximum, no sum, no rescaling
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const float p00 = s[n][0] > 0.5f * NEG_BIG ? exp2f(s[n][0] - mx0) : 0.0f;
-            const float p01 = s[n][1] > 0.5f * NEG_BIG ? exp2f(s[n][1] - mx0) : 0.0f;
-            const float p10 = s[n][2] > 0.5f * NEG_BIG ? exp2f(s[n][2] - mx1) : 0.0f;
-            const float p11 = s[n][3] > 0.5f * NEG_BIG ? exp2f(s[n][3] - mx1) : 0.0f;
-            rs0 += p00 + p01;
-            rs1 += p10 + p11;
-            pf[n * 2 + 0] = pack_bf16(p00, p01);
-            pf[n * 2 + 1] = pack_bf16(p10, p11);
-        }
-        l0 = l0 * c0 + rs0;
-        l1 = l1 * c1 + rs1;
-        if (__any_sync(0xffffffffu, c0 != 1.0f || c1 != 1.0f)) {      // the maximum moved somewhere in the warp
+            for (int n = 0; n < 2; ++n) {
+                float w[4];
 #pragma unroll
-            for (int n = 0; n < HD / 8; ++n) { o[n][0] *= c0; o[n][1] *= c0; o[n][2] *= c1; o[n][3] *= c1; }
+                for (int e = 0; e < 4; ++e) {
+                    const int j = j0 + n * 8 + 2 * t + (e & 1), h = e >> 1;
+                    const float d = (float)max(pos - j, 0);
+                    const float v = fmaf(-s[n][e], p.scale_log2, fmaf(dist_a[h], lg2_approx(fmaf(dist_b[h], d, 1.0f)), offset[h]));
+                    w[e] = j <= pos && j >= k_first ? sigmoid_weight(v) : 0.0f;
+                }
+                pf[n * 2 + 0] = pack_bf16(w[0], w[1]);
+                pf[n * 2 + 1] = pack_bf16(w[2], w[3]);
+            }
+        } else {
+            float mx0 = m0, mx1 = m1;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = j0 + n * 8 + 2 * t + (e & 1);
+                    const bool vis = j <= pos && j >= k_first;
+                    float v = vis ? s[n][e] * p.scale_log2 : NEG_BIG;
+                    if (KIND == D_OPTIONS && kd.table && vis) v = fmaf(LOG2E, __ldg(table[e >> 1] + min(pos - j, kd.table_len - 1)), v);
+                    s[n][e] = v;
+                    if (e < 2) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
+                }
+            }
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+            const float c0 = exp2f(m0 - mx0), c1 = exp2f(m1 - mx1);
+            m0 = mx0; m1 = mx1;
+            float rs0 = 0.0f, rs1 = 0.0f;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const float p00 = s[n][0] > 0.5f * NEG_BIG ? exp2f(s[n][0] - mx0) : 0.0f;
+                const float p01 = s[n][1] > 0.5f * NEG_BIG ? exp2f(s[n][1] - mx0) : 0.0f;
+                const float p10 = s[n][2] > 0.5f * NEG_BIG ? exp2f(s[n][2] - mx1) : 0.0f;
+                const float p11 = s[n][3] > 0.5f * NEG_BIG ? exp2f(s[n][3] - mx1) : 0.0f;
+                rs0 += p00 + p01;
+                rs1 += p10 + p11;
+                pf[n * 2 + 0] = pack_bf16(p00, p01);
+                pf[n * 2 + 1] = pack_bf16(p10, p11);
+            }
+            l0 = l0 * c0 + rs0;
+            l1 = l1 * c1 + rs1;
+            if (__any_sync(0xffffffffu, c0 != 1.0f || c1 != 1.0f)) {      // the maximum moved somewhere in the warp
+#pragma unroll
+                for (int n = 0; n < HD / 8; ++n) { o[n][0] *= c0; o[n][1] *= c0; o[n][2] *= c1; o[n][3] *= c1; }
+            }
         }
 #pragma unroll
         for (int n2 = 0; n2 < HD / 16; ++n2) {
@@ -594,6 +662,8 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
         __syncwarp();
     }
     if (timed_out && lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+    // without softmax the merges below add sums up as they are: every warp and slice at one maximum, its weights' sum positive
+    if constexpr (KIND == D_SIGMOID) { m0 = m1 = 0.0f; l0 = l1 = 0.25f; }
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
@@ -611,6 +681,19 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
         wo[(g + 8) * HD + n * 8 + 2 * t + 1] = o[n][3];
     }
     __syncthreads();
+    // what a row's sums are multiplied by: 1 / (their weights' sum and the sink's), with the factor; the result with its gate
+    auto row_factor = [&](int r, float gm, float sum) -> float {
+        if (KIND == D_SIGMOID) return 1.0f;
+        const float sink2 = kd.sink ? __ldg(kd.sink + head0 + r) * LOG2E : NEG_BIG;
+        const float top = fmaxf(gm, sink2), f = gm > 0.5f * NEG_BIG ? exp2f(gm - top) : 0.0f;
+        const float den = sum * f + (kd.sink ? exp2f(sink2 - top) : 0.0f);
+        return den > 0.0f ? kd.out_scale * f / den : 0.0f;
+    };
+    auto put = [&](int r, int d, float v) {
+        const int c = (head0 + r) * HD + d;
+        if (kd.gate) v /= 1.0f + __expf(-kd.gate[(size_t)tok * kd.gate_stride + c]);
+        p.out[(size_t)tok * kd.out_stride + c] = __float2bfloat16_rn(v);
+    };
     // thread i handles element(s) (row, d): row = e / HD
     const int unit = blockIdx.z * gridDim.y + blockIdx.y;
     const int extra = WITH_PREFIX ? x.extra_slices : 0;
@@ -632,7 +715,8 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             part[r * (HD + 2) + 2 + d] = acc;
             if (d == 0) { part[r * (HD + 2)] = gm; part[r * (HD + 2) + 1] = sum; }
         } else {
-            p.out[((size_t)tok * p.nh + head0 + r) * HD + d] = __float2bfloat16_rn(sum > 0.0f ? acc / sum : 0.0f);
+            if constexpr (KIND == D_PLAIN) p.out[((size_t)tok * p.nh + head0 + r) * HD + d] = __float2bfloat16_rn(sum > 0.0f ? acc / sum : 0.0f);
+            else put(r, d, acc * row_factor(r, gm, sum));
         }
     }
     if (!part) return;
@@ -670,7 +754,7 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             s_f[sp][r] = f;
             sum = fmaf(l, f, sum);
         }
-        s_inv[r] = sum > 0.0f ? 1.0f / sum : 0.0f;
+        s_inv[r] = KIND != D_PLAIN ? row_factor(r, gm, sum) : sum > 0.0f ? 1.0f / sum : 0.0f;
     }
     __syncthreads();
     constexpr int EG = 4, SG = 8;                                // elements and slices per round of loads
@@ -704,7 +788,8 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             const int e = e0 + k * 32 * DW;
             if (e < total) {
                 const int r = e / HD, d = e - r * HD;
-                p.out[((size_t)tok * p.nh + head0 + r) * HD + d] = __float2bfloat16_rn(acc[k] * s_inv[r]);
+                if constexpr (KIND == D_PLAIN) p.out[((size_t)tok * p.nh + head0 + r) * HD + d] = __float2bfloat16_rn(acc[k] * s_inv[r]);
+                else put(r, d, acc[k] * s_inv[r]);
             }
         }
     }
@@ -728,14 +813,15 @@ EncodeTiledFn encode_fn() {
 }
 
 // Tensor map of one layer's pages seen as [rows][HD] bfloat16, boxes of 16 rows x 64 values.
-int kv_map_for(CUtensorMap* out, const void* pool, long long rows) {
-    static std::unordered_map<const void*, std::pair<long long, CUtensorMap>> cache;
+int kv_map_for(CUtensorMap* out, const void* pool, long long rows, int width = HD) {
+    static std::unordered_map<const void*, std::pair<std::pair<long long, int>, CUtensorMap>> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(pool);
-    if (it != cache.end() && it->second.first == rows) { *out = it->second.second; return AIRUN_OK; }
-    cuuint64_t dims[2] = {(cuuint64_t)HD, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)HD * 2};
+    const std::pair<long long, int> shape(rows, width);
+    if (it != cache.end() && it->second.first == shape) { *out = it->second.second; return AIRUN_OK; }
+    cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)width * 2};
     cuuint32_t box[2] = {64, DN};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode_fn()(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pool), dims, strides, box, estr,
@@ -743,7 +829,7 @@ int kv_map_for(CUtensorMap* out, const void* pool, long long rows) {
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return AIRUN_ERR_ARG;
     if (cache.size() > 4096) cache.clear();
-    cache[pool] = std::make_pair(rows, *out);
+    cache[pool] = std::make_pair(shape, *out);
     return AIRUN_OK;
 }
 
@@ -865,6 +951,45 @@ AIRUN_EXPORT int airun_attn_decode(const void* q, void* out, const void* pool, c
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
     }
-    airun_launch(kern, dim3(n_splits, nkv * hgroups, n_rows), dim3(32 * DW), smem, stream, p, x, map);
+    airun_launch(kern, dim3(n_splits, nkv * hgroups, n_rows), dim3(32 * DW), smem, stream, p, x, map, DecodeKind{});
     return airun_launch_status();
 }
+
+#if HD == 128
+// Single tokens of the softmax attention with its options (kind 1) and of the attention without softmax (kind 2): see
+// DecodeKind; pages of a power of two >= 16 tokens; the other arguments as above (a q row is [nh][HD], an output row has
+// out_stride elements).
+AIRUN_EXPORT int airun_attn_decode_kind(int kind, const void* q, void* out, long long out_stride, const void* pool, const int32_t* block_table,
+                                        int max_blocks, const int32_t* positions, const int32_t* req_of_token, int num_reqs, int num_pages,
+                                        int page_size, int nh, int nkv, float scale, int window, const float* table, int table_len,
+                                        const float* sink, const float* gate, long long gate_stride, float out_scale, const float* dist_a,
+                                        const float* dist_b, const float* head_c, int tail, const int32_t* rows, int n_rows, int n_splits,
+                                        float* scratch, int* counters, const int32_t* n_rows_dev, int dyn_slots, int early_ok, int* err,
+                                        cudaStream_t stream) {
+    if ((kind != D_OPTIONS && kind != D_SIGMOID) || (n_rows_dev && (dyn_slots <= 0 || !rows))) return AIRUN_ERR_ARG;
+    if (n_rows < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || n_splits < 1 || n_splits > MAX_SPLITS || !err ||
+        out_stride < (long long)nh * HD || (table && table_len <= 0) || (dist_a && !dist_b) || (tail >= 0 && tail % 8) || window < 0)
+        return AIRUN_ERR_ARG;
+    if (n_splits > 1 && (!scratch || !counters)) return AIRUN_ERR_ARG;
+    if (n_rows == 0) return AIRUN_OK;
+    const int hgroups = (nh / nkv + 15) / 16;
+    if (nkv * hgroups > 65535 || n_rows > 65535) return AIRUN_ERR_ARG;
+    const AttnParams p = make_params(q, out, pool, block_table, max_blocks, positions, req_of_token, num_reqs,
+                                     num_pages, page_size, nh, nkv, scale, window, err);
+    if (p.page_shift < 4 || encode_fn() == nullptr) return AIRUN_ERR_UNSUPPORTED;
+    DecodeExtra x{rows, n_splits, scratch, counters, n_rows_dev, dyn_slots, nullptr, 0, early_ok};
+    DecodeKind kd{out_stride, table, table_len, sink, gate, gate_stride, out_scale, dist_a, dist_b, head_c, tail};
+    CUtensorMap map;
+    const int r = kv_map_for(&map, pool, (long long)num_pages * (tail >= 0 ? 1 : 2) * nkv * page_size, tail >= 0 ? HD + tail : HD);
+    if (r != AIRUN_OK) return r;
+    const int smem = DW * 3 * 2 * DN * HD * 2 + 16 * HD * 2 + DW * 3 * 8 + 1024;
+    static unsigned long long configured[2] = {0, 0};
+    auto kern = kind == D_OPTIONS ? attn_decode_kernel<true, false, D_OPTIONS> : attn_decode_kernel<true, false, D_SIGMOID>;
+    if (first_on_device(configured[kind - 1])) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    airun_launch(kern, dim3(n_splits, nkv * hgroups, n_rows), dim3(32 * DW), smem, stream, p, x, map, kd);
+    return airun_launch_status();
+}
+#endif

@@ -704,7 +704,7 @@ def diff_prefill_tc(ctx, q, out, cache, part) -> bool:
             or not prefill_tc_supported(128, int(cache.page_size)) or out.stride(0) % 8 or out.data_ptr() % 16 or q.data_ptr() % 16
             or cache.pool.data_ptr() % 16):
         return False
-    tiles, n, n_dev = _prompt_tiles(ctx, nh // nkv, PREFILL_ROWS, T)
+    tiles, n, n_dev = _prompt_tiles(ctx, nh // nkv, PREFILL_ROWS, T)[:3]
     pool, bt = cache.pool, cache.block_table
     f = _fn("attention_tcgen05", "airun_attn_prefill_diff",
             [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float,
@@ -813,7 +813,7 @@ def latent_prefill_tc(ctx, qlat, out, cache, part, gate: Optional[torch.Tensor] 
     if ("latent_tc" in DISABLED or T < LATENT_TC_MIN_TOKENS or R % 64 or KD % 64 or R > 512 or KD > 576 or H > PREFILL_ROWS or page < 16
             or page & (page - 1) or not hasattr(ctx, "context_lens") or not hasattr(ctx, "extras") or out.data_ptr() % 16 or qlat.data_ptr() % 16 or cache.pool.data_ptr() % 16):
         return False
-    tiles, n, n_dev = _prompt_tiles(ctx, H, PREFILL_ROWS, T)
+    tiles, n, n_dev = _prompt_tiles(ctx, H, PREFILL_ROWS, T)[:3]
     pool, bt = cache.pool, cache.block_table
     f = _fn("latent_attention_tcgen05", "airun_latent_prefill",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p,
@@ -851,9 +851,15 @@ PROMPT_KINDS = dict(options=1, table=2, sigmoid=3)     # of csrc/attention_tcgen
 PROMPT_TC_MIN_TOKENS = 192
 
 
+def _prompt_tile_rows(T: int, G: int, nkv: int, device) -> int:
+    """Two Q tiles a CTA share every key tile; with fewer than a CTA for nearly every SM one Q tile each gives twice as many."""
+    return PREFILL_ROWS_WIDE if T // max(1, PREFILL_ROWS_WIDE // G) * nkv >= machine(device).wide_min_ctas else PREFILL_ROWS
+
+
 def _prompt_tiles(ctx, G: int, tile_rows: int, T: int):
-    """(tiles, their largest number, their number on the device): the portions of the batch cut into tiles of tile_rows // G
-    tokens by csrc/attention_plan.cu, the tiles with the most keys first; made once per step, group size and tile size."""
+    """(tiles, their largest number, their number on the device, rows of single tokens, their number on the device): the
+    portions of the batch cut into tiles of tile_rows // G tokens by csrc/attention_plan.cu, the tiles with the most keys
+    first; made once per step, group size and tile size."""
     key = ("prompt_tiles", G, tile_rows)
     got = ctx.extras.get(key)
     if got is None:
@@ -864,8 +870,54 @@ def _prompt_tiles(ctx, G: int, tile_rows: int, T: int):
         buf = ws.alloc((4 + 4 * n + T,), torch.int32) if ws is not None else torch.empty(4 + 4 * n + T, dtype=torch.int32, device=ctx.err.device)
         tiles = buf[4:4 + 4 * n].view(n, 4)
         attn_plan(ctx, per, tiles, buf[4 + 4 * n:], buf[:4])
-        got = ctx.extras[key] = (tiles, n, buf[0:1])
+        got = ctx.extras[key] = (tiles, n, buf[0:1], buf[4 + 4 * n:], buf[1:2])
     return got
+
+
+def attn_single_kind(ctx, kind: str, q, out, cache, part, decode_only: bool, tail: int = -1, gate: Optional[torch.Tensor] = None,
+                     gate_stride: int = 0) -> bool:
+    """The single tokens of the attentions with heads of 128 through the kernel of the Qwen3 part (csrc/attention_mma.cu:
+    ``attn_decode_kernel`` and its kinds); portions are left alone.  False: the sizes, the pages or the alignment are not
+    this kernel's."""
+    T, nh, nkv, page = q.shape[0], part.nh, part.nkv, int(cache.page_size)
+    G = nh // nkv
+    if ("single_kind" in DISABLED or part.D != 128 or part.Dv != 128 or page < 16 or page & (page - 1) or not hasattr(ctx, "extras") or G > 16
+            or not hasattr(ctx, "context_lens") or q.data_ptr() % 16 or cache.pool.data_ptr() % 16 or (tail >= 0 and tail % 8)):
+        return False
+    context = int(ctx.extras.get("planning_context_len", ctx.max_context_len))
+    if part.window > 0:
+        context = min(context, int(part.window))
+    slots = machine(q.device).decode_slots_tma
+    rows = rows_dev = None
+    n_rows, dyn = T, 0
+    if decode_only:
+        splits = plan_decode_splits(T, nkv, 1, context, 128, slots)
+    else:
+        shape = ctx.extras.get("device_plan") or {}
+        _, _, _, rows, rows_dev = _prompt_tiles(ctx, G, _prompt_tile_rows(T, G, nkv, q.device), T)
+        n_rows, dyn = min(int(shape.get("max_rows", ctx.num_reqs)), int(ctx.num_reqs), T), slots
+        if n_rows == 0:
+            return True
+        # no row takes more slices than fit when the fewest rows of this shape are there
+        fit = max(1, slots // (max(1, int(shape.get("min_rows", 1))) * nkv))
+        splits = max(1, min(64, (context + DECODE_MIN_KEYS_PER_SPLIT - 1) // DECODE_MIN_KEYS_PER_SPLIT, fit))
+    scratch, counters = scratch_for(q.device)
+    if n_rows * nkv > counters.numel() or (n_rows * nkv * splits if decode_only else max(dyn, n_rows * nkv)) * 16 * 130 > scratch.numel():
+        return False
+    pool, bt = cache.pool, cache.block_table
+    sig = kind == "sigmoid"
+    table, sink = (None, None) if sig else (part.table, part.sink)
+    f = _fn("attention_mma", "airun_attn_decode_kind",
+            [c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
+             c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
+             c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p], {"HD": 128})
+    _check(f(2 if sig else 1, _p(q), _p(out), out.stride(0) if T > 1 else max(out.shape[1], out.stride(0)), _p(pool), _p(bt), bt.stride(0),
+             _p(ctx.positions), _p(ctx.req_of_token), int(ctx.num_reqs), pool.shape[0], page, nh, nkv, float(part.scale), int(part.window),
+             _p(table), 0 if table is None else table.shape[1], _p(sink), _p(gate), int(gate_stride), 1.0 if sig else float(part.out_scale),
+             _p(part.dist_a) if sig else None, _p(part.dist_b) if sig else None, _p(part.head_c) if sig else None, tail, _p(rows), n_rows, splits,
+             _p(scratch), _p(counters), _p(rows_dev), dyn, 1 if torch.cuda.is_current_stream_capturing() else 0, _p(ctx.err), _stream()),
+           "attn_decode_kind")
+    return True
 
 
 def attn_prompt_kind(ctx, kind: str, q, out, cache, part, tail: int = -1, gate: Optional[torch.Tensor] = None, gate_stride: int = 0) -> bool:
@@ -878,9 +930,8 @@ def attn_prompt_kind(ctx, kind: str, q, out, cache, part, tail: int = -1, gate: 
             or out.stride(0) % 8 or out.data_ptr() % 16 or q.data_ptr() % 16 or cache.pool.data_ptr() % 16 or (tail >= 0 and tail % 8)
             or (gate is not None and (gate_stride % 4 or gate.data_ptr() % 16))):
         return False
-    # two Q tiles a CTA share every key tile; with fewer than a CTA for nearly every SM one Q tile each gives twice as many
-    rows = PREFILL_ROWS_WIDE if T // (PREFILL_ROWS_WIDE // G) * nkv >= machine(q.device).wide_min_ctas else PREFILL_ROWS
-    tiles, n, n_dev = _prompt_tiles(ctx, G, rows, T)
+    rows = _prompt_tile_rows(T, G, nkv, q.device)
+    tiles, n, n_dev = _prompt_tiles(ctx, G, rows, T)[:3]
     pool, bt = cache.pool, cache.block_table
     table, sink = getattr(part, "table", None), getattr(part, "sink", None)
     f = _fn("attention_tcgen05", "airun_attn_prefill_kinds",
@@ -957,7 +1008,7 @@ def sigmoid_attention_bf16(ctx, q, out, cache, part) -> bool:
     single = "sigmoid_group" not in DISABLED and nh // nkv <= 16
     decode_only = bool(getattr(ctx, "decode_only", False))
     lens = None if ctx.extras.get("device_plan") else getattr(ctx, "query_lens", None)
-    if single and (decode_only or lens is None or 1 in list(lens)):
+    if single and (decode_only or lens is None or 1 in list(lens)) and not attn_single_kind(ctx, "sigmoid", q, out, cache, part, decode_only):
         context = ctx.extras.get("planning_context_len", ctx.max_context_len)
         if part.window > 0:
             context = min(context, part.window)
@@ -1015,7 +1066,8 @@ def softmax_attention_bf16(ctx, q, out, cache, part, gate: Optional[torch.Tensor
     single = "softmax_group" not in DISABLED and nh // nkv <= 16
     decode_only = bool(getattr(ctx, "decode_only", False))
     lens = None if ctx.extras.get("device_plan") else getattr(ctx, "query_lens", None)
-    if single and (decode_only or lens is None or 1 in list(lens)):
+    if single and (decode_only or lens is None or 1 in list(lens)) and not attn_single_kind(
+            ctx, "options", q, out, cache, part, decode_only, tail=tail, gate=gate, gate_stride=ops.attention_gate(gate, T, nh * Dv)):
         context = ctx.extras.get("planning_context_len", ctx.max_context_len)
         if part.window > 0:
             context = min(context, part.window)

@@ -147,6 +147,46 @@ def test_latent(H, R, rd, page, window, sink, gated, spans):
     assert float((got[rows].float() - want[rows].float()).abs().max()) < 3 * 2.0 ** -8 * float(pool.abs().max())
 
 
+# heads, kv heads, page, window, tail, table rows, sink, gate, spans
+SINGLE_CASES = [(1, 1, 16, 0, -1, 0, False, False, [(0, 1)]), (2, 1, 16, 0, -1, 0, True, True, [(1499, 1500), (14, 15), (15, 16), (699, 700)]),
+                (16, 8, 32, 100, -1, 0, True, False, [(99, 100), (100, 101), (2000, 2001)]), (3, 1, 16, 0, -1, 90, True, True, [(128, 129), (899, 900)]),
+                (16, 1, 64, 1, -1, 5, False, False, [(300, 301), (0, 1)]), (4, 2, 16, 0, 64, 0, True, False, [(1023, 1024), (31, 32)]),
+                (6, 2, 16, 333, 8, 0, False, True, [(1200, 1201), (17, 18), (0, 1)])]
+
+
+@gpu
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("nh,nkv,page,window,tail,rows,sink,gated,spans", SINGLE_CASES)
+def test_single_tokens(nh, nkv, page, window, tail, rows, sink, gated, spans, mixed):
+    """Single tokens alone and beside a portion (csrc/attention_mma.cu: attn_decode_kernel and its kinds), softmax with its options
+    and without softmax, against the plain kernels."""
+    from airun_b200.kernels import fast, ops
+    if mixed:
+        spans = spans[:1] + [(3, 30)] + spans[1:]
+    g, cache, ctx, q = made(nh, nkv, page, tail, spans, nh + window)
+    T = q.shape[0]
+    one = torch.tensor([n == 1 for n in ctx.query_lens for _ in range(n)], device="cuda")
+    part = SimpleNamespace(D=128, Dv=128, nh=nh, nkv=nkv, scale=0.13, window=window, out_scale=1.3, tail=tail,
+                           table=(2.0 * torch.randn(nh, rows, generator=g)).cuda() if rows else None,
+                           sink=(2.0 * torch.randn(nh, generator=g)).cuda() if sink else None)
+    gate = torch.randn(T, nh * 128 + 4, generator=g).cuda()[:, 4:] if gated else None
+    stride = ops.attention_gate(gate, T, nh * 128)
+    got = torch.full((T, nh * 128 + 16), 7.0, device="cuda", dtype=torch.bfloat16)
+    want = torch.zeros(T, nh * 128, device="cuda", dtype=torch.bfloat16)
+    assert fast.attn_single_kind(ctx, "options", q, got[:, 8:8 + nh * 128], cache, part, not mixed, tail=tail, gate=gate, gate_stride=stride)
+    ops.softmax_attention(q, want, cache, ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, 1.3, tail=tail, gate=gate)
+    assert int(ctx.err.item()) == 0 and bool((got[~one][:, 8:8 + nh * 128] == 7.0).all()) and bool((got[:, :8] == 7.0).all())
+    assert float((got[one][:, 8:8 + nh * 128].float() - want[one].float()).abs().max()) < 3 * 2.0 ** -8 * 1.3 * float(cache.pool.abs().max())
+    if tail >= 0:
+        return
+    part.dist_a, part.dist_b, part.head_c = (0.2 + torch.rand(nh, generator=g)).cuda(), (0.1 + torch.rand(nh, generator=g)).cuda(), None
+    assert fast.attn_single_kind(ctx, "sigmoid", q, got[:, 8:8 + nh * 128], cache, part, not mixed)
+    ops.sigmoid_attention(q, want, cache, ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, None, window)
+    assert int(ctx.err.item()) == 0
+    most = max(float(want[one].abs().max()), float(cache.pool.abs().max()))
+    assert float((got[one][:, 8:8 + nh * 128].float() - want[one].float()).abs().max()) < 3 * 2.0 ** -8 * most
+
+
 @gpu
 def test_what_the_kernel_does_not_take_stays_with_the_other():
     """Small batches, other head sizes, pages of 24, wide groups and unaligned rows are refused, not run."""

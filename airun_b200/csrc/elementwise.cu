@@ -56,22 +56,58 @@ AIRUN_EXPORT int airun_embed(const void* table, int table_dtype, const int32_t* 
 // sum x + delta is normed; it is written back to x only when write_back is set
 // (a gathered final norm leaves x alone).  VEC = 4 reads float4 (n % 4 == 0) and keeps up to
 // KEEP vectors per thread in registers between the two passes; longer rows are read again.
+// What bounds a few rows is the chain of loads, not bytes.  The weights, which no kernel writes, are cold in a decode
+// step (the products have streamed through the cache since), so they are asked for ahead of the wait for the kernel in
+// front: 8 rows of 2048 take 2.6 us with nothing in front to overlap with; with the weights read after the sums, as single
+// numbers, they took 3.5.
 #define KEEP 4
+template <int VEC>
+__device__ __forceinline__ void load_vec(const float* __restrict__ p, int i, float (&v)[VEC]) {
+    if (VEC == 4) {
+        const float4 f = reinterpret_cast<const float4*>(p)[i];
+        v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
+    } else {
+        v[0] = p[i];
+    }
+}
 template <typename TOut, int VEC>
-__global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta,
+__device__ __forceinline__ void store_vec(TOut* __restrict__ p, int i, const float (&v)[VEC]) {
+    if (VEC == 4 && sizeof(TOut) == 4) {
+        reinterpret_cast<float4*>(p)[i] = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
+    } else if (VEC == 4) {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1 % VEC]), hi = __floats2bfloat162_rn(v[2 % VEC], v[3 % VEC]);
+        reinterpret_cast<uint2*>(p)[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    } else {
+        p[i] = from_f32<TOut>(v[0]);
+    }
+}
+
+template <typename TOut, int VEC>
+__global__ __launch_bounds__(VEC == 4 ? 512 : 1024) void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta,
                                const float* __restrict__ w, TOut* __restrict__ out,
                                const int32_t* __restrict__ rows, int n, float eps, int write_back,
                                const float* __restrict__ w2, TOut* __restrict__ out2) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float red[33];
+    const int nv = n / VEC;                       // vectors in the row
+    float wk[KEEP][VEC], wk2[KEEP][VEC];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) { wk[k][e] = 1.0f; wk2[k][e] = 1.0f; }
+        if (i < nv) {
+            if (w) load_vec<VEC>(w, i, wk[k]);
+            if (w2) load_vec<VEC>(w2, i, wk2[k]);
+        }
+    }
+    pdl_wait();
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
     float* xr = x + (size_t)src * n;
     const float* dr = delta ? delta + (size_t)src * n : nullptr;
     TOut* outr = out + (size_t)r * n;
     TOut* outr2 = out2 ? out2 + (size_t)r * n : nullptr;      // the same row under a second weight
-    const int nv = n / VEC;                       // vectors in the row
     float keep[KEEP][VEC];
     float ss = 0.0f;
     // All loads of x and delta first, then the sums and the stores: a load issued after a store through the
@@ -84,17 +120,8 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
 #pragma unroll
         for (int e = 0; e < VEC; ++e) { keep[k][e] = 0.0f; dk[k][e] = 0.0f; }
         if (i < nv) {
-            if (VEC == 4) {
-                const float4 v = reinterpret_cast<const float4*>(xr)[i];
-                keep[k][0] = v.x; keep[k][1 % VEC] = v.y; keep[k][2 % VEC] = v.z; keep[k][3 % VEC] = v.w;
-                if (dr) {
-                    const float4 d = reinterpret_cast<const float4*>(dr)[i];
-                    dk[k][0] = d.x; dk[k][1 % VEC] = d.y; dk[k][2 % VEC] = d.z; dk[k][3 % VEC] = d.w;
-                }
-            } else {
-                keep[k][0] = xr[i];
-                if (dr) dk[k][0] = dr[i];
-            }
+            load_vec<VEC>(xr, i, keep[k]);
+            if (dr) load_vec<VEC>(dr, i, dk[k]);
         }
     }
 #pragma unroll
@@ -104,10 +131,7 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
             if (dr) {
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) keep[k][e] += dk[k][e];
-                if (write_back) {
-                    if (VEC == 4) reinterpret_cast<float4*>(xr)[i] = make_float4(keep[k][0], keep[k][1 % VEC], keep[k][2 % VEC], keep[k][3 % VEC]);
-                    else xr[i] = keep[k][0];
-                }
+                if (write_back) store_vec<float, VEC>(xr, i, keep[k]);
             }
 #pragma unroll
             for (int e = 0; e < VEC; ++e) ss = fmaf(keep[k][e], keep[k][e], ss);
@@ -127,12 +151,14 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ 
     for (int k = 0; k < KEEP; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i < nv) {
+            float o[VEC];
 #pragma unroll
-            for (int e = 0; e < VEC; ++e)
-                outr[i * VEC + e] = from_f32<TOut>(keep[k][e] * inv * (w ? w[i * VEC + e] : 1.0f));
+            for (int e = 0; e < VEC; ++e) o[e] = keep[k][e] * inv * wk[k][e];
+            store_vec<TOut, VEC>(outr, i, o);
             if (outr2) {
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) outr2[i * VEC + e] = from_f32<TOut>(keep[k][e] * inv * w2[i * VEC + e]);
+                for (int e = 0; e < VEC; ++e) o[e] = keep[k][e] * inv * wk2[k][e];
+                store_vec<TOut, VEC>(outr2, i, o);
             }
         }
     }
@@ -248,8 +274,8 @@ static int rmsnorm_launch(float* x, const float* delta, const float* w, void* ou
     if (n_rows < 0 || n <= 0 || ((w2 == nullptr) != (out2 == nullptr))) return AIRUN_ERR_ARG;
     if (rows && write_back) return AIRUN_ERR_ARG;
     if (n_rows == 0) return AIRUN_OK;
-    const bool vec = n % 4 == 0 && (((uintptr_t)x | (uintptr_t)delta) & 15) == 0;
-    if (vec && !rows && n_rows >= 256 && n >= 512 && (((uintptr_t)out | (uintptr_t)w | (uintptr_t)out2 | (uintptr_t)w2) & 15) == 0) {
+    const bool vec = n % 4 == 0 && (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)out | (uintptr_t)w | (uintptr_t)out2 | (uintptr_t)w2) & 15) == 0;
+    if (vec && !rows && n_rows >= 256 && n >= 512) {
         // enough warps per block that the blocks still cover the SMs twice
         const int wpb = n_rows >= 2368 ? 8 : n_rows >= 1184 ? 4 : 2;
         const int blocks = (n_rows + wpb - 1) / wpb;
@@ -263,7 +289,7 @@ static int rmsnorm_launch(float* x, const float* delta, const float* w, void* ou
     }
     const int nv = vec ? n / 4 : n;
     int threads = (nv + 31) / 32 * 32;
-    if (threads > 1024) threads = 1024;
+    if (threads > (vec ? 512 : 1024)) threads = vec ? 512 : 1024;
     if (threads < 32) threads = 32;
     if (n_rows <= 64 && threads > 256 && vec) threads = 256;      // few rows: more loads in flight per thread
 #define LAUNCH(TOut, VEC) \
@@ -429,17 +455,29 @@ AIRUN_EXPORT int airun_soft_cap(float* x, long long n, float cap, cudaStream_t s
 
 // Copies whole cache pages inside the pools of one cache group: for every pair (src, dst) and every
 // owner layer, page dst = page src.  pool: [owners][pages][page_words] 16-byte words.  Pairs whose
-// ids are outside the pool set the bad-page bit and are skipped.
+// ids are outside the pool set the bad-page bit and are skipped.  Four words a thread, read before the first is written: a
+// fork copies a page or two, which leaves most of the chip idle, so what counts is how often a thread waits for memory (one
+// block a page and layer, a word at a time: 7.4 us for pages of 48 KB; 2.1 us).
+#define COPY_WORDS 4
 __global__ void copy_pages_kernel(uint4* __restrict__ pool, long long owner_words, long long page_words,
                                   const int32_t* __restrict__ pairs, int num_pages, int* __restrict__ err) {
     const int src = pairs[2 * blockIdx.x], dst = pairs[2 * blockIdx.x + 1];
     if (src < 0 || src >= num_pages || dst < 0 || dst >= num_pages) {
-        if (threadIdx.x == 0 && err) atomicOr(err, AIRUN_DEV_BAD_PAGE);
+        if (threadIdx.x == 0 && blockIdx.z == 0 && err) atomicOr(err, AIRUN_DEV_BAD_PAGE);
         return;
     }
     const uint4* s = pool + (long long)blockIdx.y * owner_words + (long long)src * page_words;
     uint4* d = pool + (long long)blockIdx.y * owner_words + (long long)dst * page_words;
-    for (long long i = threadIdx.x; i < page_words; i += blockDim.x) d[i] = s[i];
+    const long long step = (long long)gridDim.z * COPY_WORDS * blockDim.x;
+    for (long long i0 = (long long)blockIdx.z * COPY_WORDS * blockDim.x + threadIdx.x; i0 < page_words; i0 += step) {
+        uint4 v[COPY_WORDS];
+#pragma unroll
+        for (int k = 0; k < COPY_WORDS; ++k)
+            if (i0 + k * blockDim.x < page_words) v[k] = s[i0 + k * blockDim.x];
+#pragma unroll
+        for (int k = 0; k < COPY_WORDS; ++k)
+            if (i0 + k * blockDim.x < page_words) d[i0 + k * blockDim.x] = v[k];
+    }
 }
 
 AIRUN_EXPORT int airun_copy_pages(void* pool, int owners, int num_pages, long long page_bytes, const int32_t* pairs,
@@ -448,8 +486,9 @@ AIRUN_EXPORT int airun_copy_pages(void* pool, int owners, int num_pages, long lo
         return AIRUN_ERR_ARG;
     if (n_pairs == 0) return AIRUN_OK;
     if (owners > 65535) return AIRUN_ERR_ARG;
-    copy_pages_kernel<<<dim3(n_pairs, owners), 256, 0, stream>>>((uint4*)pool, (long long)num_pages * (page_bytes / 16),
-                                                                 page_bytes / 16, pairs, num_pages, err);
+    const long long parts = (page_bytes / 16 + 256 * COPY_WORDS - 1) / (256 * COPY_WORDS);
+    copy_pages_kernel<<<dim3(n_pairs, owners, (unsigned)(parts < 64 ? parts : 64)), 256, 0, stream>>>(
+        (uint4*)pool, (long long)num_pages * (page_bytes / 16), page_bytes / 16, pairs, num_pages, err);
     return airun_launch_status();
 }
 
@@ -568,54 +607,78 @@ AIRUN_EXPORT int airun_glu_clamped(const void* in, int in_dtype, void* out, int 
 
 // Norm on a sub-layer's OUTPUT: x[t] += mult * y[t] / sqrt(mean(y[t]^2) + eps) * w, and, when `cast` is given,
 // cast[t] = x[t] in the compute type (the input of the sub-layer that follows, which reads x itself).  One block
-// per row; the row of y stays in registers between the two passes while it is short enough.
-template <typename TCast>
+// per row; up to KEEP vectors a thread of y, x and w, all asked for before the first is used (the weights, which no
+// kernel writes, ahead of the wait for the kernel in front), stay in registers between the two passes.  2026 rows
+// and 3 rows of 2048, 12 calls each: 122 us; one number a load, with x read and written in turn after the sum, 228 us.
+template <typename TCast, int VEC>
 __global__ __launch_bounds__(256) void postnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y,
                                                            const float* __restrict__ w, TCast* __restrict__ cast,
                                                            int n, float eps, float mult) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float red[33];
+    const int nv = n / VEC;
+    float wk[KEEP][VEC], yk[KEEP][VEC], xk[KEEP][VEC];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < nv) load_vec<VEC>(w, i, wk[k]);
+    }
+    pdl_wait();
     const int r = blockIdx.x;
     float* xr = x + (size_t)r * n;
     const float* yr = y + (size_t)r * n;
-    float keep[8];
     float ss = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int i = threadIdx.x + k * 256;
-        keep[k] = i < n ? yr[i] : 0.0f;
-        ss = fmaf(keep[k], keep[k], ss);
+    for (int k = 0; k < KEEP; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) yk[k][e] = 0.0f;
+        if (i < nv) { load_vec<VEC>(yr, i, yk[k]); load_vec<VEC>(xr, i, xk[k]); }
     }
-    for (int i = threadIdx.x + 8 * 256; i < n; i += 256) ss = fmaf(yr[i], yr[i], ss);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) ss = fmaf(yk[k][e], yk[k][e], ss);
+    const int tail0 = (threadIdx.x + KEEP * blockDim.x) * VEC, tstep = blockDim.x * VEC;       // a row longer than the registers hold
+    for (int i = tail0; i < n; i += tstep)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) ss = fmaf(yr[i + e], yr[i + e], ss);
     ss = block_sum(ss, red);
     const float inv = 1.0f / sqrtf(ss / (float)n + eps);
+    TCast* cr = cast ? cast + (size_t)r * n : nullptr;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int i = threadIdx.x + k * 256;
-        if (i < n) {
-            const float v = xr[i] + mult * (keep[k] * inv * w[i]);
-            xr[i] = v;
-            if (cast) cast[(size_t)r * n + i] = from_f32<TCast>(v);
+    for (int k = 0; k < KEEP; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < nv) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) xk[k][e] += mult * (yk[k][e] * inv * wk[k][e]);
+            store_vec<float, VEC>(xr, i, xk[k]);
+            if (cr) store_vec<TCast, VEC>(cr, i, xk[k]);
         }
     }
-    for (int i = threadIdx.x + 8 * 256; i < n; i += 256) {
-        const float v = xr[i] + mult * (yr[i] * inv * w[i]);
-        xr[i] = v;
-        if (cast) cast[(size_t)r * n + i] = from_f32<TCast>(v);
-    }
+    for (int i = tail0; i < n; i += tstep)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            const float v = xr[i + e] + mult * (yr[i + e] * inv * w[i + e]);
+            xr[i + e] = v;
+            if (cr) cr[i + e] = from_f32<TCast>(v);
+        }
 }
 
 AIRUN_EXPORT int airun_postnorm_add(float* x, const float* y, const float* w, void* cast, int cast_dtype, int T, int n,
                                     float eps, float mult, cudaStream_t stream) {
     if (T < 0 || n <= 0 || !x || !y || !w) return AIRUN_ERR_ARG;
     if (T == 0) return AIRUN_OK;
-    if (!cast || cast_dtype == AIRUN_DT_F32)
-        airun_launch(postnorm_add_kernel<float>, dim3(T), dim3(256), 0, stream, x, y, w, (float*)cast, n, eps, mult);
-    else if (cast_dtype == AIRUN_DT_BF16)
-        airun_launch(postnorm_add_kernel<__nv_bfloat16>, dim3(T), dim3(256), 0, stream, x, y, w, (__nv_bfloat16*)cast, n, eps, mult);
-    else
-        return AIRUN_ERR_UNSUPPORTED;
+    const bool vec = n % 4 == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)cast) & 15) == 0;
+    // many rows: as few threads as hold the row in registers; few rows: more of them, with fewer loads each
+    const int nv = vec ? n / 4 : n;
+    int threads = ((T > 64 ? (nv + KEEP - 1) / KEEP : nv) + 31) / 32 * 32;
+    if (threads > 256) threads = 256;
+#define PN_LAUNCH(TC, VEC) airun_launch(postnorm_add_kernel<TC, VEC>, dim3(T), dim3(threads), 0, stream, x, y, w, (TC*)cast, n, eps, mult)
+    if (!cast || cast_dtype == AIRUN_DT_F32) { if (vec) PN_LAUNCH(float, 4); else PN_LAUNCH(float, 1); }
+    else if (cast_dtype == AIRUN_DT_BF16) { if (vec) PN_LAUNCH(__nv_bfloat16, 4); else PN_LAUNCH(__nv_bfloat16, 1); }
+    else return AIRUN_ERR_UNSUPPORTED;
+#undef PN_LAUNCH
     return airun_launch_status();
 }
 

@@ -1,0 +1,53 @@
+"""The kernels between the products at the sizes where their forms change: norms whose rows, weights and results do or do not
+allow 16-byte accesses, copies of pages that one block or several take."""
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n", [(1, 4), (3, 130), (1, 4096), (64, 1024), (65, 4096), (200, 8200), (2, 9000), (300, 512), (5, 33)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_norms_on_and_off_their_alignment(rows, n, off, dtype):
+    """float32: a sum of n squares in chains of at most n / 32 and six levels of adds, halved by the root, and three
+    products: (n / 64 + 8) units of 2^-24 of the value; bfloat16 rounds once more, to half a unit: 2^-8 of the value at most."""
+    from airun_b200.kernels import ops
+    g = torch.Generator().manual_seed(rows + n)
+
+    def shifted(t):                                      # the same numbers, `off` elements into their storage
+        store = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")
+        store[off:off + t.numel()] = t.reshape(-1).cuda()
+        return store[off:off + t.numel()].view(t.shape)
+
+    x, d = torch.randn(rows, n, generator=g), torch.randn(rows, n, generator=g)
+    w, w2 = torch.randn(n, generator=g), torch.randn(n, generator=g)
+    tol = (n / 64 + 8) * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    norm = lambda v, weight: v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * weight
+    ok = lambda got, want: bool(((got.cpu().double() - want).abs() <= tol * want.abs() + 1e-30).all())
+    X, out, out2 = shifted(x), shifted(torch.zeros(rows, n, dtype=dtype)), shifted(torch.zeros(rows, n, dtype=dtype))
+    ops.rmsnorm_pair(X, shifted(w), out, shifted(w2), out2, 1e-5, delta=shifted(d))
+    s = (x + d).double()
+    assert torch.equal(X.cpu(), x + d) and ok(out, norm(s, w.double())) and ok(out2, norm(s, w2.double()))
+    pick = torch.tensor([rows - 1, 0], dtype=torch.int32, device="cuda")
+    gathered = shifted(torch.zeros(2, n, dtype=dtype))
+    ops.rmsnorm(X, shifted(w), 1e-5, gathered, rows=pick)
+    assert ok(gathered, norm(s, w.double())[[rows - 1, 0]]) and torch.equal(X.cpu(), x + d)
+    Y, cast = shifted(x), shifted(torch.zeros(rows, n, dtype=dtype))
+    ops.postnorm_add(Y, shifted(d), shifted(w), 1e-5, 0.7, cast=cast)
+    part = 0.7 * norm(d.double(), w.double())
+    want, size = x.double() + part, x.abs().double() + part.abs()
+    assert bool(((Y.cpu().double() - want).abs() <= (n / 64 + 8) * 2.0 ** -24 * size).all())
+    assert torch.equal(cast.cpu(), Y.cpu().to(dtype))
+
+
+@gpu
+@pytest.mark.parametrize("words", [1, 1023, 1024, 1025, 70000])
+def test_pages_of_one_block_and_of_several(words):
+    from airun_b200.kernels import ops
+    pool = torch.randint(-2 ** 31, 2 ** 31 - 1, (3, 6, 4 * words), dtype=torch.int32, device="cuda")
+    want = pool.clone()
+    want[:, 5], want[:, 0] = pool[:, 1], pool[:, 4]
+    ops.copy_pages(pool, torch.tensor([[1, 5], [4, 0]], dtype=torch.int32, device="cuda"))
+    assert torch.equal(pool, want)

@@ -1027,7 +1027,7 @@ def moe_route(logits: torch.Tensor, top: int, softmax_scores: bool, renorm: bool
               bias: Optional[torch.Tensor] = None) -> None:
     """ids / wts [T, top]: every token's ``top`` experts by score (sigmoid or softmax of the router's ``logits``
     [T, E], float32) and their weights; rank [T, top]: the row's place among its expert's rows; seg [E + 1]: where each
-    expert's rows begin.  ``counts`` (int32 [E]) must be zero on entry.  ``bias`` (float32 [E]) is added to the logits first."""
+    expert's rows begin.  ``counts`` (int32 [E]) receives the rows of every expert.  ``bias`` (float32 [E]) is added to the logits first."""
     _cuda(logits, req_of_token, ids, wts, rank, counts, seg, bias)
     _rows_f32(logits, "logits")
     T, E = logits.shape
@@ -1083,7 +1083,7 @@ def moe_route_grouped(logits: torch.Tensor, num_real: int, top: int, groups: int
     float32 [T, n_out]: the first ``num_real`` outputs are experts with matrices, the rest return their input.  Scores
     are the softmax over all outputs; the choice is by score + ``correction`` inside the ``keep`` best of ``groups``
     equal runs of neighbouring outputs; weights are the chosen scores over their sum (+ 1e-20) times ``weight_scale``.
-    ``counts`` (int32 [num_real]) must be zero on entry; seg [num_real + 1].  ``sigmoid_scores``: scores are sigmoids of
+    ``counts`` (int32 [num_real]) receives the rows of every expert; seg [num_real + 1].  ``sigmoid_scores``: scores are sigmoids of
     the logits; ``group_best`` 2: a group's score is the sum of its two largest; without ``renorm`` the weights are the
     chosen scores times ``weight_scale``."""
     _cuda(logits, correction, req_of_token, ids, wts, rank, counts, seg)

@@ -135,7 +135,6 @@ class RoutedExperts(FeedForward):
         ids, rank, row_of = (ws.alloc((T, top), torch.int32) for _ in range(3))
         wts = ws.alloc((T, top), torch.float32)
         seg = ws.alloc((self.E + 1,), torch.int32)
-        self.counts.zero_()
         logits = ws.alloc((T, self.n_out + self.extra_rows), torch.float32)
         linear(ctx, h, self.w_router, logits)
         if self.grouped_routing:

@@ -1,9 +1,54 @@
-"""The kernels between the products at the sizes where their forms change: norms whose rows, weights and results do or do not
-allow 16-byte accesses, copies of pages that one block or several take."""
+"""The kernels between the products at the sizes where their forms change: the router's single block and its many, norms whose
+rows, weights and results do or do not allow 16-byte accesses, copies of pages that one block or several take."""
 import pytest
 import torch
 
 gpu = pytest.mark.gpu
+
+
+@gpu
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("T,E,top", [(1, 16, 4), (31, 16, 16), (32, 40, 3), (33, 40, 3), (70, 16, 1), (7, 64, 40), (40, 64, 33), (32, 700, 8), (2, 1024, 8)])
+def test_router_of_one_block_and_of_many(T, E, top, grouped):
+    """Scores in float32 differ from float64 by a few units of their last place (expf: 2) and by the sum over E of them;
+    8 + E / 16 units of 2^-24 of the score hold."""
+    from airun_b200.kernels import ops
+    g = torch.Generator().manual_seed(T + E)
+    z = torch.randn(T, E, generator=g)
+    off = torch.randn(E, generator=g) * 0.1
+    req = torch.zeros(T, dtype=torch.int32)
+    if T > 2:
+        req[[1, T - 1]] = -1
+    live = req >= 0
+    ids, rank = (torch.full((T, top), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    wts = torch.zeros(T, top, device="cuda")
+    real = E - 3 if grouped else E
+    counts, seg = torch.zeros(real, dtype=torch.int32, device="cuda"), torch.full((real + 1,), -1, dtype=torch.int32, device="cuda")
+    if grouped:
+        s = torch.softmax(z.double(), -1)
+        choice = s + off.double()
+        ops.moe_route_grouped(z.cuda(), real, top, 1, 1, 1.5, off.cuda(), req.cuda(), ids, wts, rank, counts, seg)
+    else:
+        s = torch.sigmoid(z.double() + off.double())
+        choice = z.double() + off.double()
+        ops.moe_route(z.cuda(), top, False, True, req.cuda(), ids, wts, rank, counts, seg, bias=off.cuda())
+    got, r, c, sg = ids.cpu().long(), rank.cpu().long(), counts.cpu().long(), seg.cpu().long()
+    assert (got[~live] == -1).all()
+    # the order of the choice, up to float32's doubt about two scores
+    order = choice.gather(1, got.clamp(min=0))[live]
+    doubt = 1e-6
+    assert bool((order[:, 1:] <= order[:, :-1] + doubt).all())
+    assert bool((order[:, -1] >= torch.topk(choice[live], top, -1).values[:, -1] - doubt).all())
+    assert all(len(set(row.tolist())) == top for row in got[live])
+    chosen = s.gather(1, got.clamp(min=0))[live]
+    want = chosen / chosen.sum(-1, keepdim=True) * (1.5 if grouped else 1.0)
+    assert bool(((wts.cpu().double()[live] - want).abs() <= (8 + E / 16 + top) * 2.0 ** -24 * want).all())
+    flat, fr = got[live].reshape(-1), r[live].reshape(-1)
+    here = flat < real
+    assert torch.equal(c, torch.bincount(flat[here], minlength=real))
+    assert torch.equal(sg, torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(c, 0)]))
+    rows = sg[flat[here]] + fr[here]
+    assert sorted(rows.tolist()) == list(range(int(here.sum())))                    # every row of the segments is used once
 
 
 @gpu

@@ -33,6 +33,7 @@
 #include <unordered_map>
 #include <string>
 #include <cstring>
+#include <type_traits>
 
 #define BM 128
 #define BK 64
@@ -304,14 +305,17 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float* v,
                 for (int i = 0; i < 16; ++i) if (n0 + i < p.b_rows) o[i] = __float2bfloat16_rn(v[i]);
             }
         }
-    } else {
+    } else if (a_row < p.a_rows) {
+        // one warp a scheduler: what counts is the instructions between two stores
+        const int n = p.b_rows - (b0 + c0);                  // tokens from here on
+        typedef typename std::conditional<EPI == EPI_F32, float, __nv_bfloat16>::type TOut;
+        TOut* o = (TOut*)p.out + (size_t)(b0 + c0) * p.ldc + a_row;
+        if (n >= 16) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int tok = b0 + c0 + i;
-            if (tok < p.b_rows && a_row < p.a_rows) {
-                if (EPI == EPI_F32) ((float*)p.out)[(size_t)tok * p.ldc + a_row] = v[i];
-                else ((__nv_bfloat16*)p.out)[(size_t)tok * p.ldc + a_row] = __float2bfloat16_rn(v[i]);
-            }
+            for (int i = 0; i < 16; ++i, o += p.ldc) *o = from_f32<TOut>(v[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i, o += p.ldc) if (i < n) *o = from_f32<TOut>(v[i]);
         }
     }
 }
@@ -344,17 +348,18 @@ __device__ __forceinline__ void store_swiglu_normal(const GemmParams& p, const f
 }
 
 // SwiGLU, swapped mode: this lane's row is a gate row when (a_row / 16) is even, and lane + 16
-// holds the matching up row.  v: 16 columns (tokens).
+// holds the matching up row.  v: 16 columns (tokens).  The gate lanes take the first eight tokens, the up lanes the others:
+// one exchange brings each the other half of its pairs.
 __device__ __forceinline__ void store_swiglu_swapped(const GemmParams& p, const float* v, int a_row, int b0, int c0) {
     const int lane = threadIdx.x & 31;
+    const bool low = lane < 16;
+    const int first = b0 + c0 + (low ? 0 : 8), n = a_row < p.a_rows ? p.b_rows - first : 0;
+    __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)first * p.ldc + (a_row >> 5) * 16 + (lane & 15);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float up = __shfl_down_sync(0xffffffffu, v[i], 16);
-        const int tok = b0 + c0 + i;
-        if (lane < 16 && tok < p.b_rows && a_row < p.a_rows) {
-            const int n_out = (a_row / 32) * 16 + (a_row % 32);
-            ((__nv_bfloat16*)p.out)[(size_t)tok * p.ldc + n_out] = __float2bfloat16_rn(gated_unit(p.glu_limit, p.glu_slope, v[i], up));
-        }
+    for (int i = 0; i < 8; ++i, o += p.ldc) {
+        const float other = __shfl_xor_sync(0xffffffffu, low ? v[i + 8] : v[i], 16);
+        const float g = low ? v[i] : other, u = low ? other : v[i + 8];
+        if (i < n) *o = __float2bfloat16_rn(gated_unit(p.glu_limit, p.glu_slope, g, u));
     }
 }
 
@@ -497,6 +502,53 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     const bool direct = p.ksplit == 1;
     const bool clustered = CLUSTER && !direct;
     const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    const int cols = SWAP ? min(BN, p.b_rows - b0) : BN;      // columns of the tile that stand for tokens (swapped)
+    // One slice: the next 32 columns are on their way from tensor memory while these are stored.  (Sixteen at a time, each
+    // waited for, and a bounds check a store: [2048, 512] with 24, 64 and 128 tokens took 4.9, 6.5 and 9.3 us; 3.9, 4.3 and
+    // 5.1 now.  [12288, 2048] gated, 64 tokens: 22.5 -> 18.3 us.)
+    auto finish_direct = [&]() {
+        auto put = [&](const uint32_t (&r)[32], int c) {
+            float v[16], u[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                v[i] = __uint_as_float(r[i]);
+                u[i] = __uint_as_float(r[16 + i]);
+            }
+            if (AIRUN_FOLD_NORM && p.ssq_in) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    v[i] *= SWAP ? s_scale[c + i] : row_scale;
+                    u[i] *= SWAP ? s_scale[c + 16 + i] : row_scale;
+                }
+            }
+            if constexpr (EPI == EPI_SWIGLU) {
+                if (SWAP) {
+                    store_swiglu_swapped(p, v, a_row, b0, c);
+                    if (c + 16 < cols) store_swiglu_swapped(p, u, a_row, b0, c + 16);
+                } else {
+                    store_swiglu_normal(p, v, u, a_row, b0, c);
+                }
+            } else {
+                if (p.act) { epilogue_act(v, p.act - 1); epilogue_act(u, p.act - 1); }
+                store_chunk<EPI, SWAP>(p, v, a_row, b0, c);
+                if (c + 16 < cols) store_chunk<EPI, SWAP>(p, u, a_row, b0, c + 16);
+            }
+        };
+        uint32_t r0[32], r1[32];
+        tmem_ld32_async(lane_addr, r0);
+#pragma unroll 1
+        for (int c = 0; c < cols; c += 64) {
+            __syncwarp();
+            tmem_wait32(r0);
+            if (c + 32 < cols) tmem_ld32_async(lane_addr + c + 32, r1);
+            put(r0, c);
+            if (c + 32 >= cols) break;
+            __syncwarp();
+            tmem_wait32(r1);
+            if (c + 64 < cols) tmem_ld32_async(lane_addr + c + 64, r0);
+            put(r1, c + 32);
+        }
+    };
     // Sums the slices of the tile (or takes the accumulator as it is), applies the epilogue and stores.
     // rank < 0: all columns, slices from tensor memory (one slice) or from the scratch; rank >= 0: the
     // chunks of columns that fall to this CTA of the cluster, slices from the peers' shared memory.
@@ -505,7 +557,11 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
         const float* all = (direct || rank >= 0) ? nullptr : p.scratch + (size_t)tile * p.ksplit * (BN * BM);
         const uint32_t mine = smem_u32(smem);
         constexpr int STEP = (EPI == EPI_SWIGLU && !SWAP) ? 32 : 16;
-        for (int c = 0; c < BN; c += STEP) {
+        if (EPI != EPI_RESID && BN >= 32 && direct && n_kb > 0) {
+            finish_direct();
+            return;
+        }
+        for (int c = 0; c < cols; c += STEP) {
             if (rank >= 0 && (c / STEP) % p.ksplit != rank) continue;
             float v[16], u[16];
             if (direct) {
@@ -658,15 +714,35 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
             float* part = clustered ? reinterpret_cast<float*>(smem)
                                     : p.scratch + ((size_t)tile * p.ksplit + split) * (BN * BM);
             if (ok) {
-                for (int c = 0; c < BN; c += 16) {
-                    float v[16];
-                    if (n_kb > 0) tmem_ld16(lane_addr + c, v);
-                    else {
+                if (BN >= 32 && n_kb > 0) {
+                    uint32_t r0[32], r1[32];
+                    float* to = part + quad * 32 + lane;
+                    auto put = [&](const uint32_t (&r)[32], int c) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+                        for (int i = 0; i < 32; ++i) to[(c + i) * BM] = __uint_as_float(r[i]);
+                    };
+                    tmem_ld32_async(lane_addr, r0);
+#pragma unroll 1
+                    for (int c = 0; c < cols; c += 64) {
+                        tmem_wait32(r0);
+                        if (c + 32 < cols) tmem_ld32_async(lane_addr + c + 32, r1);
+                        put(r0, c);
+                        if (c + 32 >= cols) break;
+                        tmem_wait32(r1);
+                        if (c + 64 < cols) tmem_ld32_async(lane_addr + c + 64, r0);
+                        put(r1, c + 32);
                     }
+                } else {
+                    for (int c = 0; c < cols; c += 16) {
+                        float v[16];
+                        if (n_kb > 0) tmem_ld16(lane_addr + c, v);
+                        else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) part[(size_t)(c + i) * BM + quad * 32 + lane] = v[i];
+                            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) part[(size_t)(c + i) * BM + quad * 32 + lane] = v[i];
+                    }
                 }
             }
             if (clustered) {

@@ -1,5 +1,6 @@
 """The kernels between the products at the sizes where their forms change: the router's single block and its many, norms whose
-rows, weights and results do or do not allow 16-byte accesses, copies of pages that one block or several take."""
+rows, weights and results do or do not allow 16-byte accesses, copies of pages that one block or several take, and the
+epilogue of the products for up to 128 tokens."""
 import pytest
 import torch
 
@@ -96,3 +97,33 @@ def test_pages_of_one_block_and_of_several(words):
     want[:, 5], want[:, 0] = pool[:, 1], pool[:, 4]
     ops.copy_pages(pool, torch.tensor([[1, 5], [4, 0]], dtype=torch.int32, device="cuda"))
     assert torch.equal(pool, want)
+
+
+@gpu
+@pytest.mark.parametrize("ksplit", [1, 3, 10])           # one slice, a cluster, slices through the scratch
+@pytest.mark.parametrize("epi", [0, 1, 2])
+@pytest.mark.parametrize("M,bn", [(1, 32), (8, 32), (9, 32), (16, 32), (17, 32), (31, 32), (33, 64), (40, 64), (48, 64), (49, 64), (64, 64),
+                                  (65, 128), (80, 128), (97, 128), (127, 128), (128, 128), (70, 64), (200, 128)])
+def test_products_with_the_tokens_as_columns(M, bn, epi, ksplit):
+    """The epilogue of the swapped product takes the tile's tokens 32, 16 and 8 at a time.  Rows behind the last token stay as
+    they are.  float32: sums of K products in the tensor core, 2^-14 of the largest possible sum; bfloat16 results round
+    to half a unit more; the gated unit g sigmoid(g) u has slopes of at most 1.1 |u| and |g|."""
+    from airun_b200.kernels import fast
+    N, K = 288, 712
+    g = torch.Generator().manual_seed(M + epi)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((M + 3, N // 2 if epi == 2 else N), 7.0, dtype=torch.float32 if epi == 0 else torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        fast.gemm_tcgen05(x.cuda(), w.cuda(), out[:M], epi, True, bn, ksplit, err)
+    want = x.double() @ w.double().T
+    e = 2.0 ** -14 * (x.double().abs() @ w.double().abs().T)
+    if epi == 2:
+        a, b = (t.view(M, N // 32, 2, 16) for t in (want, e))
+        (gate, up), (eg, eu) = ((t[:, :, 0].reshape(M, -1), t[:, :, 1].reshape(M, -1)) for t in (a, b))
+        want = gate * torch.sigmoid(gate) * up
+        e = 1.1 * up.abs() * eg + gate.abs() * eu
+    if epi:
+        e = e + 2.0 ** -8 * want.abs()
+    assert int(err.item()) == 0 and bool(((out[:M].cpu().double() - want).abs() <= e + 1e-30).all())
+    assert bool((out[M:] == 7.0).all())

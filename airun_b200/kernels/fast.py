@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from functools import lru_cache
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -168,8 +169,8 @@ def plan_gemm(M: int, N: int, K: int, mach: Optional[Machine] = None) -> Tuple[b
     memory: as many as keep the CTAs within SPLIT_CTAS (all clusters must be resident at once; 288
     CTAs in clusters of 6 were not and took half as long again) and a slice at 8 K-steps or more.  Above
     128 tokens, tiles of 128 x 256 on the persistent kernel once there are 96 of them; fewer tiles
-    leave SMs idle, so the tile narrows to 128 x 128, and only if that still fills less than one
-    wave and a slice keeps 32 K-steps is K cut as well.  Both rules come from sweeps over the
+    leave SMs idle, so the tile narrows to 128 x 128 or K is cut, whichever takes less time (_plan_few_tiles).
+    All rules come from sweeps over the
     Qwen3-1.7B and -8B shapes, 1 to 2048 tokens, timed inside CUDA graphs."""
     mach = mach or machine()
     kb = (K + 63) // 64
@@ -188,8 +189,27 @@ def plan_gemm(M: int, N: int, K: int, mach: Optional[Machine] = None) -> Tuple[b
     mt = (M + 127) // 128
     if N >= 256 and mt * ((N + 255) // 256) >= mach.sms * 96 // B200_SMS:
         return False, 256, 1
-    tiles = mt * ((N + 127) // 128)
-    return False, 128, max(1, min(mach.sms // tiles, kb // 32))
+    return _plan_few_tiles(mt, N, kb, mach.sms)
+
+
+@lru_cache(maxsize=4096)
+def _plan_few_tiles(mt: int, N: int, kb: int, sms: int) -> Tuple[bool, int, int]:
+    """Tile width and K slices of ``mt`` rows of tiles over N weight rows that do not fill the chip as they are.  The time is
+    that of a CTA's K-steps, bound by what an SM takes in (0.28 us a step of 128 x 128, 0.36 us of 128 x 256, which is fewer
+    bytes per result), and of bringing the slices together (5 and 8 us); slices run as clusters, which must all be
+    resident: 128 CTAs on 148 SMs.  B200, us, slices as K alone would have them (one from 32 K-steps each) and by this rule:
+    512 tokens x [2048, 6144] 22.6, 19.6; 256 x [2048, 2048] 12.5, 10.2; 384 x [4096, 12288] 59.8, 48.3; 1024 x [2048, 6144]
+    30.6, 27.7."""
+    best = None
+    for bn, step, merge in ((128, 0.28, 5.0), (256, 0.36, 8.0)):
+        if N < bn and bn > 128:
+            continue
+        tiles = mt * ((N + bn - 1) // bn)
+        for ks in range(1, max(1, min(sms * 128 // B200_SMS // tiles, kb // 8, 8)) + 1):
+            us = ((tiles + sms - 1) // sms if ks == 1 else 1) * ((kb + ks - 1) // ks) * step + (merge if ks > 1 else 0.0)
+            if best is None or us < best[0]:
+                best = us, bn, ks
+    return False, best[1], best[2]
 
 
 def _usable(x: torch.Tensor, w: torch.Tensor) -> bool:

@@ -64,6 +64,21 @@ static inline void airun_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block,
     if (e != cudaSuccess && airun_launch_rc == 0) airun_launch_rc = (int)e;
 }
 
+// The same once everything before it in the stream is done.  For kernels of fewer blocks than the chip holds at once whose
+// blocks run long: blocks that become resident while the kernel in front still runs go where it leaves room, several to an
+// SM while others stay empty, and stay there.
+template <typename... KArgs, typename... Args>
+static inline void airun_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                      Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    if (e != cudaSuccess && airun_launch_rc == 0) airun_launch_rc = (int)e;
+}
+
 // The same with thread-block clusters of (1, 1, cluster_z) CTAs (grid.z must be a multiple of it).
 template <typename... KArgs, typename... Args>
 static inline void airun_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -380,8 +380,11 @@ static int gla_recurrent_launch(const float* q, const float* k, const float* v, 
     const int tiles = ceil_div_i(Dv, GLA_COLS);
     if (tiles > 65535) return AIRUN_ERR_ARG;
     GlaSegments segs = {};
-#define GLA_LAUNCH(NS, C, SEG) airun_launch(gla_recurrent_kernel<NS, C, SEG>, grid, dim3(256), 0, stream, q, k, v, row_stride, decay, state, \
+#define GLA_LAUNCH_BY(BY, NS, C, SEG) BY(gla_recurrent_kernel<NS, C, SEG>, grid, dim3(256), 0, stream, q, k, v, row_stride, decay, state, \
         slot_stride, cu_tokens, state_slots, max_slots, out, heads, D, Dv, q_scale, err, head_decay, in_silu, num_reqs, segs)
+    // segments run long, with fewer blocks than the chip holds: they wait for the kernel in front (airun_launch_after).  A step
+    // of 2048 tokens with three layers of one decay per head took 3.38 ms instead of 3.24 with them packed where it leaves room.
+#define GLA_LAUNCH(NS, C, SEG) do { if (SEG) GLA_LAUNCH_BY(airun_launch_after, NS, C, SEG); else GLA_LAUNCH_BY(airun_launch, NS, C, SEG); } while (0)
     if (work) {
         if (max_segments <= 0 || D > 128 || D % 4 || Dv % 4 || slot_stride % 4 || (((uintptr_t)state | (uintptr_t)out | (uintptr_t)work) & 15))
             return AIRUN_ERR_ARG;
@@ -399,7 +402,7 @@ static int gla_recurrent_launch(const float* q, const float* k, const float* v, 
                 const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (GLA_SEG * 132 + 128 * 64) * (int)sizeof(float));
                 if (e != cudaSuccess) return (int)e;
             }
-            airun_launch(kern, dim3(max_segments, heads, ceil_div_i(Dv, 64)), dim3(256), smem, stream, q, row_stride, decay, state, slot_stride,
+            airun_launch_after(kern, dim3(max_segments, heads, ceil_div_i(Dv, 64)), dim3(256), smem, stream, q, row_stride, decay, state, slot_stride,
                          cu_tokens, state_slots, max_slots, out, heads, D, Dv, q_scale, head_decay, in_silu, num_reqs, segs);
             return airun_launch_status();
         };
@@ -412,6 +415,7 @@ static int gla_recurrent_launch(const float* q, const float* k, const float* v, 
     else GLA_PICK(false);
 #undef GLA_PICK
 #undef GLA_LAUNCH
+#undef GLA_LAUNCH_BY
     return airun_launch_status();
 }
 

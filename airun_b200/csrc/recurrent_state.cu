@@ -708,6 +708,114 @@ __global__ __launch_bounds__(128) void delta_chunk_coef_kernel(RecurrentArgs a, 
     }
 }
 
+// The same for a decay per key channel (delta rule) and for the time mix.  The decays no longer leave the sums over key
+// channels, so they go into the vectors: with G_i[d] = g_0 .. g_i and L_ij[d] = g_(j+1) .. g_i of a channel,
+//     pred_i = S0^T (G_i k_i),   o_i = S0^T (G_i q_i) + sum_{j<=i} (sum_d q_i L_ij k_j) u_j,   S = G_7 S0 + sum_j (L_7j k_j) u_j
+// (time mix: u_j = v_j, the query meets the decays up to the token before it, and the token itself counts with its bonus).
+// This kernel writes G_i k_i, G_i q_i, L_7j k_j and G_7, and the rows of the inverse and of the products, for all chunks
+// of all requests at once.  Every decay product is formed as a product, so a decay near zero only wipes.
+struct ChunkVectors { float *q, *k, *k_end, *whole; };         // [T][heads * D] each; whole: at a chunk's first token; k: delta rule only
+enum { CHUNK_HEAD = 0, CHUNK_CHANNEL = 1, CHUNK_MIX = 2 };
+template <int SL, bool MIX>      // D <= 32 * SL
+__global__ __launch_bounds__(128) void chunk_vectors_kernel(RecurrentArgs a, int num_reqs, float* __restrict__ coef, ChunkVectors vec) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float s_dot[4][64], s_m[4][RS_CHUNK][RS_CHUNK];
+    int b = blockIdx.x, row0 = -1, nt = 0;
+    for (int r = 0; r < num_reqs; ++r) {
+        const int t0 = a.cu_tokens[r], n = a.cu_tokens[r + 1] - t0;
+        if (n <= 0) continue;
+        const int chunks = (n + RS_CHUNK - 1) / RS_CHUNK;
+        if (b < chunks) { row0 = t0 + b * RS_CHUNK; nt = min(RS_CHUNK, n - b * RS_CHUNK); break; }
+        b -= chunks;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.y * 4 + warp;
+    if (row0 < 0 || head >= a.heads) return;
+    const float* qh = a.q + (size_t)(head / a.kv_rep) * a.D;
+    const float* kh = a.k + (size_t)(head / a.kv_rep) * a.D;
+    const float* gh = a.g + (size_t)head * a.D;
+    float acc[64];                                       // 28 products of keys (j < i), then 36 of a query and a key (j <= i)
+#pragma unroll
+    for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+#pragma unroll
+    for (int sl = 0; sl < SL; ++sl) {
+        const int d = lane + 32 * sl;
+        const bool d_on = d < a.D;
+        float kk[RS_CHUNK], qq[RS_CHUNK], gg[RS_CHUNK];
+#pragma unroll
+        for (int i = 0; i < RS_CHUNK; ++i) {
+            const bool on = i < nt && d_on;
+            kk[i] = on ? kh[(size_t)(row0 + i) * a.k_stride + d] : 0.0f;
+            qq[i] = on ? qh[(size_t)(row0 + i) * a.q_stride + d] : 0.0f;
+            gg[i] = on ? gh[(size_t)(row0 + i) * a.g_stride + d] : 1.0f;
+        }
+        const size_t at = ((size_t)row0 * a.heads + head) * a.D + d, step = (size_t)a.heads * a.D;
+        const float bonus = MIX && d_on ? a.bonus[(size_t)head * a.D + d] : 0.0f;
+        float G = 1.0f;
+#pragma unroll
+        for (int i = 0; i < RS_CHUNK; ++i) {
+            if (!MIX) G *= gg[i];
+            if (i < nt && d_on) {
+                vec.q[at + i * step] = qq[i] * G;
+                if (!MIX) vec.k[at + i * step] = kk[i] * G;
+            }
+            if (MIX) G *= gg[i];
+        }
+        if (d_on) vec.whole[at] = G;
+#pragma unroll
+        for (int j = 0; j < RS_CHUNK; ++j) {
+            float x = kk[j];
+            acc[28 + j * (j + 1) / 2 + j] = fmaf(MIX ? qq[j] * bonus : qq[j], x, acc[28 + j * (j + 1) / 2 + j]);
+#pragma unroll
+            for (int i = j + 1; i < RS_CHUNK; ++i) {
+                if (!MIX) {
+                    x *= gg[i];
+                    acc[i * (i - 1) / 2 + j] = fmaf(kk[i], x, acc[i * (i - 1) / 2 + j]);
+                }
+                acc[28 + i * (i + 1) / 2 + j] = fmaf(qq[i], x, acc[28 + i * (i + 1) / 2 + j]);
+                if (MIX) x *= gg[i];
+            }
+            if (j < nt && d_on) vec.k_end[at + j * step] = x;
+        }
+    }
+    float half[2][32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) { half[0][e] = acc[2 * e]; half[1][e] = acc[2 * e + 1]; }
+    rs_scatter_sum<32>(half[0], lane);
+    rs_scatter_sum<32>(half[1], lane);
+    s_dot[warp][2 * lane] = half[0][0];
+    s_dot[warp][2 * lane + 1] = half[1][0];
+    __syncwarp();
+    const int c = lane & (RS_CHUNK - 1);                 // lanes 8.. repeat what lanes 0..7 do and store nothing
+    const float beta = MIX ? 1.0f : c < nt ? 1.0f / (1.0f + expf(-a.beta[(size_t)(row0 + c) * a.beta_stride + head])) : 0.0f;
+    float qk[RS_CHUNK];
+#pragma unroll
+    for (int i = 0; i < RS_CHUNK; ++i) {
+        qk[i] = i >= c ? s_dot[warp][28 + i * (i + 1) / 2 + c] : 0.0f;
+        if (!MIX && lane < RS_CHUNK) s_m[warp][i][c] = i > c ? s_dot[warp][i * (i - 1) / 2 + c] : 0.0f;
+    }
+    __syncwarp();
+    float x[RS_CHUNK];
+#pragma unroll
+    for (int i = 0; i < RS_CHUNK; ++i) {
+        const float bi = __shfl_sync(0xffffffffu, beta, i);
+        float sum = 0.0f;
+        if (!MIX) {
+#pragma unroll
+            for (int j = 0; j < i; ++j) sum = fmaf(s_m[warp][i][j], x[j], sum);
+        }
+        x[i] = i < c ? 0.0f : i == c ? bi : -bi * sum;
+    }
+    if (lane < RS_CHUNK) {
+        float* dst = coef + ((size_t)row0 * a.heads + head) * RS_COEF;
+        const size_t step = (size_t)a.heads * RS_COEF;
+#pragma unroll
+        for (int i = 0; i < RS_CHUNK; ++i)
+            if (i < nt) { dst[i * step + c] = x[i]; dst[i * step + RS_CHUNK + c] = qk[i]; }
+        if (c < nt) { dst[c * step + 2 * RS_CHUNK] = 1.0f; dst[c * step + 2 * RS_CHUNK + 1] = 1.0f; }
+    }
+}
+
 // two float32 numbers in a register pair: d = a * b + c and a * b, both halves at once
 typedef unsigned long long rs_pair;
 __device__ __forceinline__ rs_pair rs_fma2(rs_pair a, rs_pair b, rs_pair c) {
@@ -731,17 +839,28 @@ __device__ __forceinline__ float2 rs_unpack(rs_pair v) {
     return d;
 }
 
-// One block per (request, head, 16 value columns), 256 threads: a column is shared by sixteen neighbouring lanes with NS key
-// channels each.  After the sums over key channels lane l < 8 of a column holds token l's prediction and stands for its
-// write, lane l >= 8 holds token l - 8's read-out of the old state and stands for its output.  (What bounds a prompt is how
-// long one chunk takes, with few warps an SM: sixteen lanes a column instead of eight are twice the warps for the same work.)
-template <int NS>
-__global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(RecurrentArgs a, const float* __restrict__ coef) {
+// One block per (request, head, 16 value columns): a column is shared by DG neighbouring lanes with NS key channels each.
+// After the sums over key channels lane l of a column holds token l's prediction and its read-out of the old state and stands
+// for its write and its output; where DG is sixteen, one half of the lanes does the one and one the other.  What bounds a
+// prompt is how long one chunk takes, and with more blocks than SMs how often it reads shared memory.  With eight lanes a
+// column a read of keys or queries serves four columns of a warp; sixteen lanes and twice the warps read twice as often for
+// it.  Three requests of 811, 675 and 540 tokens, 16 heads of 64 x 128: sixteen lanes 247 us, eight 188; one of 2048: 232
+// and 213; heads of 256 channels, 500 tokens: 149 and 221 (a lane's chain of 32 channels is the longer one there).
+// MINB blocks an SM: named, the compiler gives a thread up to 200 registers and reads ahead (unnamed it took 71).  One decay a
+// head: two where the blocks fit (1536 tokens, 16 heads: 129 us, four 155), else four (4 x 300 tokens 84, four 77).
+// The launch waits for the kernel in front (airun_launch_after): packed on the SMs that it leaves first, the 128 blocks of
+// one request of 2048 tokens took 374 us instead of 232.
+// CHUNK_CHANNEL, CHUNK_MIX: over the vectors of chunk_vectors_kernel, whose decays are theirs already.
+template <int NS, int KIND, int DG, int MINB>
+__global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArgs a, const float* __restrict__ coef, ChunkVectors vec) {
     pdl_trigger();
     pdl_wait();
-    constexpr int DG = 16, DP = NS * DG, COLS = 16, TT = NS >= 16 ? 8 : 16, NT = 256;
-    constexpr bool KEEP_K = NS <= 8;              // the keys of a chunk stay in registers from the dot products to the update
+    constexpr bool VECS = KIND != CHUNK_HEAD, MIX = KIND == CHUNK_MIX;
+    constexpr int DP = NS * DG, NT = 16 * DG, COLS = 16, TT = DP >= 256 || (VECS && DP >= 128) ? 8 : 16;
+    constexpr bool KEEP_K = NS <= 8 && !VECS;     // the keys of a chunk stay in registers from the dot products to the update
     __shared__ __align__(16) float s_q[2][TT][DP], s_k[2][TT][DP], s_v[2][TT][COLS], s_c[2][TT][RS_COEF];
+    __shared__ __align__(16) float s_e[VECS && !MIX ? 2 : 1][VECS && !MIX ? TT : 1][VECS && !MIX ? DP : 4];     // keys decayed to their chunk's end
+    __shared__ __align__(16) float s_w[VECS ? 2 : 1][VECS ? TT / RS_CHUNK : 1][VECS ? DP : 4];                  // a chunk's whole decay
     __shared__ __align__(16) float s_x[NT / 32][32 / DG][3][RS_CHUNK];        // per warp and column: what its lanes tell one another
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS;
     const int t0 = a.cu_tokens[r], n = a.cu_tokens[r + 1] - t0;
@@ -757,17 +876,26 @@ __global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(Recur
     const bool col_ok = col < Dv;
     const int ncol = min(COLS, Dv - col0);
     // both stages start as zeros: padding and rows beyond the last token hold numbers whose weight is zero
-    for (int e = threadIdx.x; e < 2 * TT * DP; e += NT) { (&s_q[0][0][0])[e] = 0.0f; (&s_k[0][0][0])[e] = 0.0f; }
+    for (int e = threadIdx.x; e < 2 * TT * DP; e += NT) {
+        (&s_q[0][0][0])[e] = 0.0f; (&s_k[0][0][0])[e] = 0.0f;
+        if (VECS && !MIX) (&s_e[0][0][0])[e] = 0.0f;
+    }
+    if (VECS)
+        for (int e = threadIdx.x; e < 2 * (TT / RS_CHUNK) * DP; e += NT) (&s_w[0][0][0])[e] = 0.0f;
     for (int e = threadIdx.x; e < 2 * TT * COLS; e += NT) (&s_v[0][0][0])[e] = 0.0f;
     __syncthreads();
-    const float* qh = a.q + (size_t)(head / a.kv_rep) * D + (size_t)t0 * a.q_stride;
-    const float* kh = a.k + (size_t)(head / a.kv_rep) * D + (size_t)t0 * a.k_stride;
+    // (time mix: the keys that are staged are the decayed ones of the update, there is nothing to predict)
+    const long long q_stride = VECS ? (long long)a.heads * D : a.q_stride, k_stride = VECS ? (long long)a.heads * D : a.k_stride;
+    const float* qh = (VECS ? vec.q + (size_t)head * D : a.q + (size_t)(head / a.kv_rep) * D) + (size_t)t0 * q_stride;
+    const float* kh = (VECS ? (MIX ? vec.k_end : vec.k) + (size_t)head * D : a.k + (size_t)(head / a.kv_rep) * D) + (size_t)t0 * k_stride;
+    const float* eh = VECS ? vec.k_end + (size_t)head * D + (size_t)t0 * k_stride : nullptr;
+    const float* wh = VECS ? vec.whole + (size_t)head * D + (size_t)t0 * k_stride : nullptr;
     const float* vh = a.v + (size_t)head * Dv + col0 + (size_t)t0 * a.v_stride;
     const float* ch = coef + ((size_t)t0 * a.heads + head) * RS_COEF;
     // A thread copies the same piece of a row, of every step-th row: 16 bytes, or one number where the rows allow no more.
-    const bool vec = (D % 4 == 0) && ((a.q_stride | a.k_stride) % 4 == 0) && ((((uintptr_t)qh | (uintptr_t)kh) & 15) == 0);
+    const bool vec16 = (D % 4 == 0) && ((q_stride | k_stride) % 4 == 0) && ((((uintptr_t)qh | (uintptr_t)kh) & 15) == 0);
     const bool vvec = (ncol % 4 == 0) && (a.v_stride % 4 == 0) && (((uintptr_t)vh & 15) == 0);
-    const int dper = vec ? D / 4 : min(D, NT), drows = NT / dper, drow = threadIdx.x / dper, dcol = (threadIdx.x - drow * dper) * (vec ? 4 : 1);
+    const int dper = vec16 ? D / 4 : min(D, NT), drows = NT / dper, drow = threadIdx.x / dper, dcol = (threadIdx.x - drow * dper) * (vec16 ? 4 : 1);
     const int vper = vvec ? ncol / 4 : ncol, vrows = NT / vper, vrow = threadIdx.x / vper, vcol = (threadIdx.x - vrow * vper) * (vvec ? 4 : 1);
     constexpr int CPER = RS_COEF / 4, CROWS = NT / CPER;
     const int crow = threadIdx.x / CPER, ccol = (threadIdx.x - crow * CPER) * 4;
@@ -775,13 +903,21 @@ __global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(Recur
         const int nt = min(TT, n - base);
         if (drow < drows)
             for (int tt = drow; tt < nt; tt += drows) {
-                const float* qr = qh + (size_t)(base + tt) * a.q_stride;
-                const float* kr = kh + (size_t)(base + tt) * a.k_stride;
-                if (vec) {
+                const float* qr = qh + (size_t)(base + tt) * q_stride;
+                const float* kr = kh + (size_t)(base + tt) * k_stride;
+                const float* er = VECS ? eh + (size_t)(base + tt) * k_stride : nullptr;
+                const float* wr = VECS && tt % RS_CHUNK == 0 ? wh + (size_t)(base + tt) * k_stride : nullptr;
+                if (vec16) {
                     rs_cp16(&s_q[buf][tt][dcol], qr + dcol);
                     rs_cp16(&s_k[buf][tt][dcol], kr + dcol);
+                    if (VECS && !MIX) rs_cp16(&s_e[buf][tt][dcol], er + dcol);
+                    if (VECS && wr) rs_cp16(&s_w[buf][tt / RS_CHUNK][dcol], wr + dcol);
                 } else {
-                    for (int d = dcol; d < D; d += dper) { rs_cp4(&s_q[buf][tt][d], qr + d); rs_cp4(&s_k[buf][tt][d], kr + d); }
+                    for (int d = dcol; d < D; d += dper) {
+                        rs_cp4(&s_q[buf][tt][d], qr + d); rs_cp4(&s_k[buf][tt][d], kr + d);
+                        if (VECS && !MIX) rs_cp4(&s_e[buf][tt][d], er + d);
+                        if (VECS && wr) rs_cp4(&s_w[buf][tt / RS_CHUNK][d], wr + d);
+                    }
                 }
             }
         if (vrow < vrows)
@@ -831,8 +967,9 @@ __global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(Recur
                     const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(&s_k[buf][c0 + i][(i4 * DG + dg) * 4]);
                     const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(&s_q[buf][c0 + i][(i4 * DG + dg) * 4]);
                     if (KEEP_K) kr[KEEP_K ? i : 0][KEEP_K ? i4 : 0] = k4;
-                    p2[i] = rs_fma2(S[2 * i4], k4.x, p2[i]); o2[i] = rs_fma2(S[2 * i4], q4.x, o2[i]);
-                    p2[i] = rs_fma2(S[2 * i4 + 1], k4.y, p2[i]); o2[i] = rs_fma2(S[2 * i4 + 1], q4.y, o2[i]);
+                    if (!MIX) { p2[i] = rs_fma2(S[2 * i4], k4.x, p2[i]); p2[i] = rs_fma2(S[2 * i4 + 1], k4.y, p2[i]); }
+                    o2[i] = rs_fma2(S[2 * i4], q4.x, o2[i]);
+                    o2[i] = rs_fma2(S[2 * i4 + 1], q4.y, o2[i]);
                 }
             }
             float sum[2 * RS_CHUNK];
@@ -841,40 +978,76 @@ __global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(Recur
                 const float2 pv = rs_unpack(p2[i]), ov = rs_unpack(o2[i]);
                 sum[i] = pv.x + pv.y; sum[RS_CHUNK + i] = ov.x + ov.y;
             }
-            rs_scatter_sum<2 * RS_CHUNK>(sum, lane);
-            // this lane's token from here on: c0 + tok; its row of the inverse (its write) or of the products (its output)
+            float pred, read;                                 // of this lane's token
+            if (DG == 2 * RS_CHUNK) {
+                rs_scatter_sum<2 * RS_CHUNK>(sum, lane);
+                pred = read = sum[0];
+            } else {
+                float (&ps)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum), (&os)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum + RS_CHUNK);
+                if (!MIX) rs_scatter_sum<RS_CHUNK>(ps, lane);
+                rs_scatter_sum<RS_CHUNK>(os, lane);
+                pred = ps[0]; read = os[0];
+            }
+            const bool writes = dg < RS_CHUNK, reads = DG == RS_CHUNK || dg >= RS_CHUNK;
+            // this lane's token from here on: c0 + tok; its rows of the inverse (its write) and of the products (its output)
             const float* cf = &s_c[buf][c0 + tok][0];
-            const float2 dec = *reinterpret_cast<const float2*>(cf + 16);         // decay up to the token; from after it to the chunk's end
-            const ulonglong2 ra = *reinterpret_cast<const ulonglong2*>(cf + (dg & RS_CHUNK)), rb = *reinterpret_cast<const ulonglong2*>(cf + (dg & RS_CHUNK) + 4);
-            if (dg < RS_CHUNK) sx[0][tok] = fmaf(-dec.x, sum[0], s_v[buf][c0 + tok][cl]);
-            __syncwarp();
-            auto row_times = [&](const float* v) {
-                const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(v), vb = *reinterpret_cast<const ulonglong2*>(v + 4);
+            const float2 dec = VECS ? make_float2(1.0f, 1.0f) : *reinterpret_cast<const float2*>(cf + 16);   // decay up to the token; from after it to the chunk's end
+            auto row_times = [&](const float* row, const ulonglong2& va, const ulonglong2& vb) {
+                const ulonglong2 ra = *reinterpret_cast<const ulonglong2*>(row), rb = *reinterpret_cast<const ulonglong2*>(row + 4);
                 const float2 t = rs_unpack(rs_fma2(rb.y, vb.y, rs_fma2(rb.x, vb.x, rs_fma2(ra.y, va.y, rs_mul2(ra.x, va.x)))));
                 return t.x + t.y;
             };
-            const float u = row_times(sx[0]);
-            if (dg < RS_CHUNK) { sx[1][tok] = u; sx[2][tok] = u * dec.y; }
-            const float whole = s_c[buf][c0 + nt - 1][16];
-            const rs_pair w2 = rs_pack(whole, whole);
+            auto eight = [&](const float* v, ulonglong2& va, ulonglong2& vb) {
+                va = *reinterpret_cast<const ulonglong2*>(v);
+                vb = *reinterpret_cast<const ulonglong2*>(v + 4);
+            };
+            ulonglong2 va, vb;
+            float u = s_v[buf][c0 + tok][cl];
+            if (MIX) {
+                u = tok < nt ? u : 0.0f;
+            } else {
+                if (writes) sx[0][tok] = fmaf(-dec.x, pred, u);
+                __syncwarp();
+                eight(sx[0], va, vb);
+                u = row_times(cf, va, vb);
+            }
+            if (writes) {
+                sx[1][tok] = u;
+                if (!VECS) sx[2][tok] = u * dec.y;
+            }
+            if constexpr (VECS) {
 #pragma unroll
-            for (int i = 0; i < NS / 2; ++i) S[i] = rs_mul2(S[i], w2);
+                for (int i4 = 0; i4 < NS / 4; ++i4) {
+                    const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(&s_w[buf][c0 / RS_CHUNK][(i4 * DG + dg) * 4]);
+                    S[2 * i4] = rs_mul2(S[2 * i4], w4.x);
+                    S[2 * i4 + 1] = rs_mul2(S[2 * i4 + 1], w4.y);
+                }
+            } else {
+                const float whole = s_c[buf][c0 + nt - 1][16];
+                const rs_pair w2 = rs_pack(whole, whole);
+#pragma unroll
+                for (int i = 0; i < NS / 2; ++i) S[i] = rs_mul2(S[i], w2);
+            }
             __syncwarp();
-            const float4 wa = *reinterpret_cast<const float4*>(&sx[2][0]), wb = *reinterpret_cast<const float4*>(&sx[2][4]);
-            const float w[RS_CHUNK] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+            eight(sx[1], va, vb);
+            ulonglong2 wa = va, wb = vb;
+            if (!VECS) eight(sx[2], wa, wb);
+            const float2 w01 = rs_unpack(wa.x), w23 = rs_unpack(wa.y), w45 = rs_unpack(wb.x), w67 = rs_unpack(wb.y);
+            const float w[RS_CHUNK] = {w01.x, w01.y, w23.x, w23.y, w45.x, w45.y, w67.x, w67.y};
 #pragma unroll
             for (int j = 0; j < RS_CHUNK; ++j) {
                 const rs_pair wj = rs_pack(w[j], w[j]);
 #pragma unroll
                 for (int i4 = 0; i4 < NS / 4; ++i4) {
                     const ulonglong2 k4 = KEEP_K ? kr[KEEP_K ? j : 0][KEEP_K ? i4 : 0]
-                                                 : *reinterpret_cast<const ulonglong2*>(&s_k[buf][c0 + j][(i4 * DG + dg) * 4]);
+                                                 : *reinterpret_cast<const ulonglong2*>(VECS && !MIX ? &s_e[buf][c0 + j][(i4 * DG + dg) * 4]
+                                                                                                     : &s_k[buf][c0 + j][(i4 * DG + dg) * 4]);
                     S[2 * i4] = rs_fma2(k4.x, wj, S[2 * i4]);
                     S[2 * i4 + 1] = rs_fma2(k4.y, wj, S[2 * i4 + 1]);
                 }
             }
-            const float o = fmaf(dec.x, sum[0], row_times(sx[1]));
-            if (col_ok && dg >= RS_CHUNK && tok < nt) orow[(size_t)(base + c0 + tok) * ((size_t)a.heads * Dv)] = o;
+            const float o = fmaf(dec.x, read, row_times(cf + RS_CHUNK, va, vb));
+            if (col_ok && reads && tok < nt) orow[(size_t)(base + c0 + tok) * ((size_t)a.heads * Dv)] = o;
             __syncwarp();                                     // the lanes' numbers are read before the next chunk's are written
         }
     }
@@ -892,7 +1065,8 @@ __global__ __launch_bounds__(256, NS <= 8 ? 2 : 1) void delta_chunk_kernel(Recur
     rs_move_tail(a, slot, t0, n);
 }
 
-// `coef` (delta with one decay per head; [T][heads][RS_COEF] floats, 16-byte aligned, may be null): chunks of eight tokens.
+// `coef` ([T][heads][RS_COEF] floats, 16-byte aligned, may be null): chunks of eight tokens.  The modes with a decay per
+// channel also need `vectors`, 4 * T * heads * D floats, 16-byte aligned, and D up to 128.
 AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k, const float* v, const float* g,
                                        long long q_stride, long long k_stride, long long v_stride, long long g_stride,
                                        const float* beta, long long beta_stride, const float* a_log, const float* dt_bias,
@@ -900,7 +1074,7 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
                                        long long slot_stride, int max_slots, const int32_t* cu_tokens, const int32_t* state_slots,
                                        int num_reqs, float* out, int heads, int kv_rep, int D, int Dv, const float* tail_src,
                                        long long tail_src_stride, long long tail_off, int tail_rows, int tail_width,
-                                       int long_chains, float* coef, int T, int* err, cudaStream_t stream) {
+                                       int long_chains, float* coef, float* vectors, int T, int* err, cudaStream_t stream) {
     if (num_reqs < 0 || heads <= 0 || heads > 65535 || kv_rep <= 0 || heads % kv_rep || D <= 0 || D > 256 || Dv <= 0 || !state ||
         !cu_tokens || !state_slots || !err || !q || !k || !v || !g || !out || slot_stride < (long long)heads * D * Dv)
         return AIRUN_ERR_ARG;
@@ -919,32 +1093,67 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
                        tail_width, err, 0};
     a.vec_cols = Dv % 4 == 0 && slot_stride % 4 == 0 && v_stride % 4 == 0 && (((uintptr_t)state | (uintptr_t)v | (uintptr_t)out) & 15) == 0;
     if (coef) {
-        if (mode != RS_DELTA_HEAD || T <= 0 || ((uintptr_t)coef & 15)) return AIRUN_ERR_ARG;
+        if (T <= 0 || ((uintptr_t)coef & 15)) return AIRUN_ERR_ARG;
+        if (mode != RS_DELTA_HEAD && (!vectors || D > 128 || ((uintptr_t)vectors & 15))) return AIRUN_ERR_ARG;
         const dim3 cgrid(T / RS_CHUNK + num_reqs, ceil_div_i(heads, 4)), mgrid(num_reqs, heads, ceil_div_i(Dv, 16));
         if (mgrid.z > 65535) return AIRUN_ERR_ARG;
 #define RS_COEFS(SL) airun_launch(delta_chunk_coef_kernel<SL>, cgrid, dim3(128), 0, stream, a, num_reqs, coef)
-#define RS_CHUNKS(NS) airun_launch(delta_chunk_kernel<NS>, mgrid, dim3(256), 0, stream, a, (const float*)coef)
+#define RS_CHUNKS(NS, KIND, DG, MINB) airun_launch_after(delta_chunk_kernel<NS, KIND, DG, MINB>, mgrid, dim3(16 * DG), 0, stream, a, (const float*)coef, vec)
+        ChunkVectors vec = {};
+        if (mode != RS_DELTA_HEAD) {
+            const size_t n = (size_t)T * heads * D;
+            vec = {vectors, vectors + n, vectors + 2 * n, vectors + 3 * n};
+#define RS_VECTORS(SL, MIX) airun_launch(chunk_vectors_kernel<SL, MIX>, cgrid, dim3(128), 0, stream, a, num_reqs, coef, vec)
+            if (mode == RS_WKV) {
+                if (D <= 32) RS_VECTORS(1, true);
+                else if (D <= 64) RS_VECTORS(2, true);
+                else RS_VECTORS(4, true);
+                if (D <= 32) RS_CHUNKS(4, CHUNK_MIX, 8, 4);
+                else if (D <= 64) RS_CHUNKS(8, CHUNK_MIX, 8, 4);
+                else RS_CHUNKS(16, CHUNK_MIX, 8, 4);
+            } else {
+                if (D <= 32) RS_VECTORS(1, false);
+                else if (D <= 64) RS_VECTORS(2, false);
+                else RS_VECTORS(4, false);
+                if (D <= 32) RS_CHUNKS(4, CHUNK_CHANNEL, 8, 4);
+                else if (D <= 64) RS_CHUNKS(8, CHUNK_CHANNEL, 8, 4);
+                else RS_CHUNKS(16, CHUNK_CHANNEL, 8, 4);
+            }
+#undef RS_VECTORS
+            return airun_launch_status();
+        }
         if (D <= 32) RS_COEFS(1);
         else if (D <= 64) RS_COEFS(2);
         else if (D <= 128) RS_COEFS(4);
         else RS_COEFS(8);
-        if (D <= 64) RS_CHUNKS(4);
-        else if (D <= 128) RS_CHUNKS(8);
-        else RS_CHUNKS(16);
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const bool few = (long long)mgrid.x * mgrid.y * mgrid.z <= 2LL * sms;
+#define RS_HEAD_CHUNKS(NS) do { if (few) RS_CHUNKS(NS, CHUNK_HEAD, 8, 2); else RS_CHUNKS(NS, CHUNK_HEAD, 8, 4); } while (0)
+        if (D <= 32) RS_HEAD_CHUNKS(4);
+        else if (D <= 64) RS_HEAD_CHUNKS(8);
+        else if (D <= 128) RS_HEAD_CHUNKS(16);
+        else RS_CHUNKS(16, CHUNK_HEAD, 16, 1);
+#undef RS_HEAD_CHUNKS
 #undef RS_COEFS
 #undef RS_CHUNKS
         return airun_launch_status();
     }
     dim3 grid(num_reqs, heads, tiles);
+    // long chains: see airun_launch_after
+#define RS_PICK(KERNEL) \
+    do { if (long_chains) airun_launch_after(KERNEL, grid, dim3(128), 0, stream, a); else airun_launch(KERNEL, grid, dim3(128), 0, stream, a); } while (0)
 #define RS_LAUNCH(NS, DG) \
-    do { if (mode == RS_DELTA) airun_launch(recurrent_state_kernel<RS_DELTA, NS, DG>, grid, dim3(128), 0, stream, a); \
-         else if (mode == RS_DELTA_HEAD) airun_launch(recurrent_state_kernel<RS_DELTA_HEAD, NS, DG>, grid, dim3(128), 0, stream, a); \
-         else airun_launch(recurrent_state_kernel<RS_WKV, NS, DG>, grid, dim3(128), 0, stream, a); } while (0)
+    do { if (mode == RS_DELTA) RS_PICK((recurrent_state_kernel<RS_DELTA, NS, DG>)); \
+         else if (mode == RS_DELTA_HEAD) RS_PICK((recurrent_state_kernel<RS_DELTA_HEAD, NS, DG>)); \
+         else RS_PICK((recurrent_state_kernel<RS_WKV, NS, DG>)); } while (0)
     if (D <= 16) RS_LAUNCH(4, 4);
     else if (D <= 32) RS_LAUNCH(8, 4);
     else if (D <= 64) { if (dg == 8) RS_LAUNCH(8, 8); else RS_LAUNCH(16, 4); }
     else if (D <= 128) { if (dg == 8) RS_LAUNCH(16, 8); else RS_LAUNCH(32, 4); }
     else { if (dg == 8) RS_LAUNCH(32, 8); else RS_LAUNCH(64, 4); }
 #undef RS_LAUNCH
+#undef RS_PICK
     return airun_launch_status();
 }

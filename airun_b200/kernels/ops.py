@@ -931,13 +931,17 @@ def recurrent_state(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     f = _fn("recurrent_state", "airun_recurrent_state",
             [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p, c_longlong,
              c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-             c_longlong, c_longlong, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p])
+             c_longlong, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p])
     long_chains = 1 if T > 2 * int(ctx.num_reqs) else 0          # requests bring many tokens each, not one
-    # one decay per head: such chains run in chunks of eight tokens over coefficients worked out ahead of the recurrence
-    coef = ctx.ws.alloc((T, heads, RS_COEF), torch.float32) if head_decay and long_chains else None
+    # such chains run in chunks of eight tokens over coefficients (and, with a decay per channel, vectors) worked out ahead
+    # of the recurrence; with the vectors from 64 tokens a request on, below which they cost about what the chunks save
+    ws = getattr(ctx, "ws", None)
+    chunks = long_chains and (head_decay or (D <= 128 and T >= 64 * int(ctx.num_reqs) and ws is not None))
+    coef = ws.alloc((T, heads, RS_COEF), torch.float32) if chunks else None
+    vectors = ws.alloc((4, T, heads * D), torch.float32) if chunks and not head_decay else None
     _check(f(int(mode), _p(q), _p(k), _p(v), _p(g), _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(g), _p(beta), bs,
              _p(a_log), _p(dt_bias), _p(bonus), _p(state), state.stride(0), state.shape[0], _p(ctx.cu_tokens), _p(ctx.state_slots), int(ctx.num_reqs),
-             _p(out), heads, kv_rep, D, Dv, _p(tail_src), ts, int(tail_off), int(tail_rows), tw, long_chains, _p(coef), T,
+             _p(out), heads, kv_rep, D, Dv, _p(tail_src), ts, int(tail_off), int(tail_rows), tw, long_chains, _p(coef), _p(vectors), T,
              _p(ctx.err), _stream()), "recurrent_state")
 
 

@@ -69,3 +69,61 @@ def test_segments_against_token_by_token(heads, D, Dv, per_head, first, second):
             assert bool(((state[slots[r]].cpu().double() - want_state[r]).abs() <= 2e-5 * bound_state[r] + 1e-30).all())
             at += n
     assert float(state[[s for s in range(len(first) + 1) if s not in slots]].abs().max()) == 0
+
+
+# ----------------------------------------------------------------------------- chunks of eight tokens, a decay per channel
+CHUNK_CASES = [  # heads, q/k heads, D, Dv, tokens of the requests in the first and in the second step
+    (2, 1, 64, 128, (140, 7), (1, 190)), (3, 3, 32, 20, (200, 9, 16), (15, 0, 223)), (1, 1, 128, 33, (77,), (64,)),
+    (4, 2, 12, 8, (150, 3), (5, 130)), (2, 2, 100, 64, (1, 150), (133, 2)), (1, 1, 7, 5, (90,), (71,)), (2, 1, 128, 128, (257,), (130,)),
+    (1, 1, 33, 16, (65, 64), (8, 121))]
+
+
+@gpu
+@pytest.mark.parametrize("mix", [False, True])
+@pytest.mark.parametrize("heads,kv,D,Dv,first,second", CHUNK_CASES)
+def test_chunks_with_a_decay_per_channel(heads, kv, D, Dv, first, second, mix):
+    """The delta rule and the time mix in chunks (csrc/recurrent_state.cu) over two steps and then one token each, against token by token in float64;
+    decays from 1e-20 to a hair below one.  Tolerance: unit keys and beta in (0, 1) let no error grow in the delta rule,
+    each token adds a few roundings of the state's size, 2e-5 of the largest entry so far; the time mix as above."""
+    import plain_pogarax as P
+    from test_pirerax import batch_ctx
+    from airun_b200.kernels import ops
+    if mix:
+        kv, Dv = heads, D
+    g = torch.Generator().manual_seed(heads + 10 * D)
+    slots = list(range(len(first) + 1))[::-1][:len(first)]
+    n_state = heads * D * Dv
+    state = torch.zeros(len(first) + 1, n_state + 4, device="cuda")
+    want_state = [torch.zeros(heads, D, Dv, dtype=torch.float64) for _ in first]
+    bonus = torch.randn(heads, D, generator=g)
+    ends = [0] * len(first)
+    for lens in (first, second, [1] * len(first)):
+        live = [r for r, n in enumerate(lens) if n]
+        ctx = batch_ctx([(ends[r], ends[r] + lens[r]) for r in live], [slots[r] for r in live])
+        T = ctx.num_tokens
+        q, k = (torch.nn.functional.normalize(torch.randn(T, kv, D, generator=g), dim=-1) for _ in range(2))
+        v, beta = torch.randn(T, heads, Dv, generator=g), torch.randn(T, heads, generator=g)
+        decay = torch.rand(T, heads, D, generator=g) ** (0.02 + torch.rand(heads, D, generator=g) ** 4 * 3)
+        decay[:, :, ::5] = 1e-20 ** torch.rand(T, heads, (D + 4) // 5, generator=g)
+        out = torch.empty(T, heads * Dv, device="cuda")
+        args = [t.reshape(T, -1).cuda() for t in (q, k, v, decay)]
+        if mix:
+            ops.recurrent_state(ops.RECURRENCE_WKV, *args, state, ctx, out, heads, 1, D, Dv, bonus=bonus.cuda())
+        else:
+            ops.recurrent_state(ops.RECURRENCE_DELTA, *args, state, ctx, out, heads, heads // kv, D, Dv, beta=beta.cuda())
+        assert int(ctx.err.item()) == 0
+        at = 0
+        for r in live:
+            rows = slice(at, at + lens[r])
+            qq, kk = (t[rows].double().repeat_interleave(heads // kv, dim=1) for t in (q, k))
+            if mix:
+                o, S = P.plain_wkv_recurrence(qq, kk, v[rows].double(), decay[rows].double(), bonus.double(), state=want_state[r])
+            else:
+                o, S = P.plain_delta_recurrence(qq, kk, v[rows].double(), decay[rows].double(), torch.sigmoid(beta[rows].double()), state=want_state[r])
+            want_state[r] = S
+            size = max(1.0, float(S.abs().max()), float(o.abs().max()))
+            assert float((out[rows].cpu().double().view(-1, heads, Dv) - o).abs().max()) < 2e-5 * size
+            assert float((state[slots[r], :n_state].cpu().double().view(heads, D, Dv) - S).abs().max()) < 2e-5 * size
+            ends[r] += lens[r]
+            at += lens[r]
+    assert float(state[:, n_state:].abs().max()) == 0

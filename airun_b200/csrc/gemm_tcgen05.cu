@@ -93,25 +93,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 }
 // ---- thread-block clusters: the rank of this CTA, a barrier over all threads of all CTAs, and loads
 // from a peer's shared memory
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -131,16 +112,20 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
+// 16 columns of this thread's row, asked for and not waited for, and the wait (see tmem_wait32).
+__device__ __forceinline__ void tmem_ld_async(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.wait::ld.sync.aligned;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+        :: "memory");
 }
 
 // 32 columns of this thread's row, asked for and not waited for; tmem_wait32 waits for every load asked for so far and
@@ -164,6 +149,9 @@ __device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
           "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
         :: "memory");
 }
+
+__device__ __forceinline__ void tmem_ld_async(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32_async(taddr, r); }
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[32]) { tmem_wait32(r); }
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 bf16) with the
 // 128-byte swizzle: 8-row groups 1024 bytes apart, version 1, layout type SWIZZLE_128B.
@@ -306,17 +294,11 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float* v,
             }
         }
     } else if (a_row < p.a_rows) {
-        // one warp a scheduler: what counts is the instructions between two stores
         const int n = p.b_rows - (b0 + c0);                  // tokens from here on
         typedef typename std::conditional<EPI == EPI_F32, float, __nv_bfloat16>::type TOut;
         TOut* o = (TOut*)p.out + (size_t)(b0 + c0) * p.ldc + a_row;
-        if (n >= 16) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i, o += p.ldc) *o = from_f32<TOut>(v[i]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i, o += p.ldc) if (i < n) *o = from_f32<TOut>(v[i]);
-        }
+        for (int i = 0; i < 16; ++i, o += p.ldc) if (i < n) *o = from_f32<TOut>(v[i]);
     }
 }
 
@@ -499,88 +481,48 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     __shared__ float s_ssq[4][(SWAP && AIRUN_FOLD_NORM) ? BN : 1];       // per epilogue warp: sums of squares per token
     float row_scale = 1.0f;
     bool ok = true;
-    const bool direct = p.ksplit == 1;
-    const bool clustered = CLUSTER && !direct;
+    const bool direct = !CLUSTER && p.ksplit == 1;           // (a clustered launch has two slices or more)
+    constexpr bool clustered = CLUSTER;
     const int tile = blockIdx.y * gridDim.x + blockIdx.x;
     const int cols = SWAP ? min(BN, p.b_rows - b0) : BN;      // columns of the tile that stand for tokens (swapped)
-    // One slice: the next 32 columns are on their way from tensor memory while these are stored.  (Sixteen at a time, each
-    // waited for, and a bounds check a store: [2048, 512] with 24, 64 and 128 tokens took 4.9, 6.5 and 9.3 us; 3.9, 4.3 and
-    // 5.1 now.  [12288, 2048] gated, 64 tokens: 22.5 -> 18.3 us.)
-    auto finish_direct = [&]() {
-        auto put = [&](const uint32_t (&r)[32], int c) {
-            float v[16], u[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                v[i] = __uint_as_float(r[i]);
-                u[i] = __uint_as_float(r[16 + i]);
-            }
-            if (AIRUN_FOLD_NORM && p.ssq_in) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    v[i] *= SWAP ? s_scale[c + i] : row_scale;
-                    u[i] *= SWAP ? s_scale[c + 16 + i] : row_scale;
-                }
-            }
-            if constexpr (EPI == EPI_SWIGLU) {
-                if (SWAP) {
-                    store_swiglu_swapped(p, v, a_row, b0, c);
-                    if (c + 16 < cols) store_swiglu_swapped(p, u, a_row, b0, c + 16);
-                } else {
-                    store_swiglu_normal(p, v, u, a_row, b0, c);
-                }
-            } else {
-                if (p.act) { epilogue_act(v, p.act - 1); epilogue_act(u, p.act - 1); }
-                store_chunk<EPI, SWAP>(p, v, a_row, b0, c);
-                if (c + 16 < cols) store_chunk<EPI, SWAP>(p, u, a_row, b0, c + 16);
-            }
-        };
-        uint32_t r0[32], r1[32];
-        tmem_ld32_async(lane_addr, r0);
-#pragma unroll 1
-        for (int c = 0; c < cols; c += 64) {
-            __syncwarp();
-            tmem_wait32(r0);
-            if (c + 32 < cols) tmem_ld32_async(lane_addr + c + 32, r1);
-            put(r0, c);
-            if (c + 32 >= cols) break;
-            __syncwarp();
-            tmem_wait32(r1);
-            if (c + 64 < cols) tmem_ld32_async(lane_addr + c + 64, r0);
-            put(r1, c + 32);
-        }
-    };
+    // The loops over columns are kept rolled, one body for all of them, with the next columns on their way from tensor memory
+    // while these are stored.  Between other kernels the code comes cold: unrolled to 64 columns, which was as fast when the
+    // same product ran again and again, the epilogue cost 1.5 to 3.5 us more inside a model's step.
     // Sums the slices of the tile (or takes the accumulator as it is), applies the epilogue and stores.
     // rank < 0: all columns, slices from tensor memory (one slice) or from the scratch; rank >= 0: the
     // chunks of columns that fall to this CTA of the cluster, slices from the peers' shared memory.
     auto finish_tile = [&](int rank) {
         float ssq_acc = 0.0f;
-        const float* all = (direct || rank >= 0) ? nullptr : p.scratch + (size_t)tile * p.ksplit * (BN * BM);
+        const float* all = (direct || CLUSTER) ? nullptr : p.scratch + (size_t)tile * p.ksplit * (BN * BM);
         const uint32_t mine = smem_u32(smem);
         constexpr int STEP = (EPI == EPI_SWIGLU && !SWAP) ? 32 : 16;
-        if (EPI != EPI_RESID && BN >= 32 && direct && n_kb > 0) {
-            finish_direct();
-            return;
-        }
+        uint32_t next[STEP];
+#pragma unroll
+        for (int i = 0; i < STEP; ++i) next[i] = 0;
+        if (direct && n_kb > 0) tmem_ld_async(lane_addr, next);
+#pragma unroll 1
         for (int c = 0; c < cols; c += STEP) {
-            if (rank >= 0 && (c / STEP) % p.ksplit != rank) continue;
+            if (CLUSTER && (c / STEP) % p.ksplit != rank) continue;
             float v[16], u[16];
             if (direct) {
-                if (n_kb > 0) {
-                    tmem_ld16(lane_addr + c, v);
-                    if (STEP == 32) tmem_ld16(lane_addr + c + 16, u);
-                } else {
+                __syncwarp();
+                if (n_kb > 0) tmem_wait(next);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) { v[i] = 0.0f; u[i] = 0.0f; }
+                for (int i = 0; i < 16; ++i) {
+                    v[i] = __uint_as_float(next[i]);
+                    if (STEP == 32) u[i] = __uint_as_float(next[(STEP == 32 ? 16 : 0) + i]);
                 }
+                if (n_kb > 0 && c + STEP < cols) tmem_ld_async(lane_addr + c + STEP, next);
             } else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) { v[i] = 0.0f; u[i] = 0.0f; }
                 // slices are added in order; loads of four slices are in flight at a time
+#pragma unroll 1
                 for (int s0 = 0; s0 < p.ksplit; s0 += 4) {
                     float t[4][STEP];
 #pragma unroll
                     for (int d = 0; d < 4; ++d) {
-                        if (CLUSTER && rank >= 0) {
+                        if (CLUSTER) {
                             const uint32_t peer = s0 + d < p.ksplit ? map_to_cta(mine, (uint32_t)(s0 + d)) : 0u;
 #pragma unroll
                             for (int i = 0; i < STEP; ++i)
@@ -714,35 +656,20 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
             float* part = clustered ? reinterpret_cast<float*>(smem)
                                     : p.scratch + ((size_t)tile * p.ksplit + split) * (BN * BM);
             if (ok) {
-                if (BN >= 32 && n_kb > 0) {
-                    uint32_t r0[32], r1[32];
-                    float* to = part + quad * 32 + lane;
-                    auto put = [&](const uint32_t (&r)[32], int c) {
+                uint32_t next[16];
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) to[(c + i) * BM] = __uint_as_float(r[i]);
-                    };
-                    tmem_ld32_async(lane_addr, r0);
+                for (int i = 0; i < 16; ++i) next[i] = 0;
+                float* to = part + quad * 32 + lane;
+                if (n_kb > 0) tmem_ld_async(lane_addr, next);
 #pragma unroll 1
-                    for (int c = 0; c < cols; c += 64) {
-                        tmem_wait32(r0);
-                        if (c + 32 < cols) tmem_ld32_async(lane_addr + c + 32, r1);
-                        put(r0, c);
-                        if (c + 32 >= cols) break;
-                        tmem_wait32(r1);
-                        if (c + 64 < cols) tmem_ld32_async(lane_addr + c + 64, r0);
-                        put(r1, c + 32);
-                    }
-                } else {
-                    for (int c = 0; c < cols; c += 16) {
-                        float v[16];
-                        if (n_kb > 0) tmem_ld16(lane_addr + c, v);
-                        else {
+                for (int c = 0; c < cols; c += 16, to += 16 * BM) {
+                    if (n_kb > 0) tmem_wait(next);
+                    float v[16];
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-                        }
+                    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(next[i]);
+                    if (n_kb > 0 && c + 16 < cols) tmem_ld_async(lane_addr + c + 16, next);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) part[(size_t)(c + i) * BM + quad * 32 + lane] = v[i];
-                    }
+                    for (int i = 0; i < 16; ++i) to[i * BM] = v[i];
                 }
             }
             if (clustered) {

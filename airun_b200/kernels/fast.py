@@ -185,6 +185,11 @@ def plan_gemm(M: int, N: int, K: int, mach: Optional[Machine] = None) -> Tuple[b
         tiles = (N + 127) // 128
         if M <= 16:
             return True, bn, max(1, min(mach.stream_ctas // tiles, kb // 10))
+        if 2 * tiles > mach.sms:
+            # not even clusters of two would all be resident (one CTA an SM), and slices through the scratch cost more than
+            # they save: 96 tiles of [12288, 2048], 24, 64 and 128 tokens 14.6, 18.1 and 26.5 us in two slices, 13.3, 15.7
+            # and 19.9 in one
+            return True, bn, 1
         return True, bn, max(1, min(mach.split_ctas // tiles, kb // 8, 8))
     mt = (M + 127) // 128
     if N >= 256 and mt * ((N + 255) // 256) >= mach.sms * 96 // B200_SMS:

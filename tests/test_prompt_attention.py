@@ -92,6 +92,34 @@ def test_attention_without_softmax(nh, nkv, page, window, dist, offset, spans):
     assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * max(float(want.abs().max()), float(cache.pool.abs().max()))
 
 
+SPLIT_CASES = [  # head size, heads, kv heads, page, window, spans: key tiles a query tile has, 1 to 17
+    (128, 16, 8, 16, 0, [(900, 1143), (872, 1107)]), (128, 2, 1, 16, 0, [(0, 193)]), (128, 4, 1, 16, 0, [(300, 364)]), (64, 1, 1, 16, 0, [(0, 128)]),
+    (128, 2, 2, 32, 0, [(500, 600), (3, 4), (380, 390)]), (64, 8, 2, 32, 0, [(1000, 1100)]), (128, 3, 1, 16, 200, [(700, 900)]),
+    (128, 2, 2, 64, 0, [(2000, 2070), (5, 300)]), (64, 20, 4, 16, 0, [(1024, 1100)]), (128, 8, 8, 16, 129, [(0, 700)])]
+
+
+@gpu
+@pytest.mark.parametrize("hd,nh,nkv,page,window,spans", SPLIT_CASES)
+def test_few_tiles_whose_keys_are_cut(hd, nh, nkv, page, window, spans):
+    """attn_prefill_tc_kernel with the keys of a tile in slices that meet in a cluster: slices of two key tiles and of more, last
+    slices that are shorter or empty, tiles too short to be cut beside others that are not."""
+    from airun_b200.kernels import fast, ops
+    g = torch.Generator().manual_seed(hd + nh + window)
+    bt, num_pages = scrambled_table([e for _, e in spans], page, g)
+    pool = (0.8 * torch.randn(num_pages, 2, nkv, page, hd, generator=g)).to("cuda", torch.bfloat16)
+    ctx = batch_ctx(spans)
+    ctx.token_ids = ctx.positions
+    q = (2.0 * torch.randn(ctx.num_tokens, nh * hd, generator=g)).to("cuda", torch.bfloat16)
+    got, want = torch.full_like(q, 7.0), torch.zeros_like(q)
+    plan = fast._attention_plan(ctx, nh // nkv, fast.PREFILL_ROWS)
+    fast.attn_prefill_tc(ctx, q, got, SimpleNamespace(pool=pool, block_table=bt, page_size=page), nh, nkv, hd, 0.13, window, plan["tiles"], plan["n_tiles"])
+    ops.softmax_attention(q, want, SimpleNamespace(pool=pool.view(num_pages, -1), block_table=bt, page_size=page, shared=False), ctx, nh, nkv, hd, hd,
+                          0.13, None, None, window, 1.0)
+    rows = torch.tensor([n > 1 for n in ctx.query_lens for _ in range(n)], device="cuda")
+    assert int(ctx.err.item()) == 0 and bool((got[~rows] == 7.0).all())
+    assert float((got[rows].float() - want[rows].float()).abs().max()) < 3 * 2.0 ** -8 * float(pool.abs().max())
+
+
 DIFF_CASES = [(1, 1, 16, 0, 0, [(0, 193)]), (4, 2, 32, 64, 0, [(0, 129), (500, 501), (77, 205)]), (3, 1, 16, 37, 0, [(130, 500)]),
               (16, 8, 16, 2048, 0, [(0, 2100)]), (16, 1, 16, 0, 50, [(1000, 1255)]), (6, 3, 64, 300, 90, [(250, 700), (0, 2)])]
 

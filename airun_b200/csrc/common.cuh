@@ -34,6 +34,11 @@
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A weight that no kernel writes: on its way to the L2 cache while the kernel in front still runs.
+__device__ __forceinline__ void prefetch_l2(const float* p, int n) {
+    for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+}
+
 static thread_local int airun_launch_rc = 0;
 
 static inline bool airun_pdl_enabled() {

@@ -49,9 +49,21 @@ __device__ __forceinline__ void lat_put_piece(const LatAngles& a, const float* _
 template <typename TC>
 __device__ __forceinline__ void lat_put_query(const LatAngles& a, const float* __restrict__ q, TC* __restrict__ qn, TC* __restrict__ qlat,
                                               int H, int D, int R, int rd, int rot_dims, int rope_kind) {
-    for (int e = threadIdx.x; e < H * D; e += blockDim.x) {
-        const int h = e / D, d = e - h * D;
-        qn[e] = from_f32<TC>(q[(size_t)h * (D + rd) + d]);
+    if (((D | rd) & 3) == 0 && (((uintptr_t)q | (uintptr_t)qn) & 15) == 0) {
+        const int per = D >> 2;
+#pragma unroll 2
+        for (int e = threadIdx.x; e < H * per; e += blockDim.x) {
+            const int h = e / per, d = (e - h * per) * 4;
+            const float4 v = *reinterpret_cast<const float4*>(q + (size_t)h * (D + rd) + d);
+            __align__(16) TC o[4] = {from_f32<TC>(v.x), from_f32<TC>(v.y), from_f32<TC>(v.z), from_f32<TC>(v.w)};
+            if (sizeof(TC) == 2) *reinterpret_cast<uint2*>(qn + 4 * e) = *reinterpret_cast<uint2*>(o);
+            else *reinterpret_cast<uint4*>(qn + 4 * e) = *reinterpret_cast<uint4*>(o);
+        }
+    } else {
+        for (int e = threadIdx.x; e < H * D; e += blockDim.x) {
+            const int h = e / D, d = e - h * D;
+            qn[e] = from_f32<TC>(q[(size_t)h * (D + rd) + d]);
+        }
     }
     const int half = (rd + 1) / 2;
     for (int e = threadIdx.x; e < H * half; e += blockDim.x) {
@@ -94,15 +106,17 @@ __global__ __launch_bounds__(256) void latent_prepare_kernel(
     TC* __restrict__ pool, const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int store, int* __restrict__ err) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float red[33];
     __shared__ LatAngles angles;
     const int t = blockIdx.x;
+    // what no kernel in front writes, ahead of the wait: the angles, and the norms' weights on their way
     const int req = req_of_token[t], pos = positions[t];
+    if (store) lat_angles(angles, rot_dims, inv_freq, rot_mult, pos);
+    if (t == 0) { prefetch_l2(wq, q_rank); if (store) prefetch_l2(wkv, R); }
+    pdl_wait();
     if (req < 0 || pos < 0) return;
     if (req >= num_reqs) { if (threadIdx.x == 0) atomicOr(err, AIRUN_DEV_BAD_REQ); return; }
     const float* row = proj + (size_t)t * stride;
-    if (store) lat_angles(angles, rot_dims, inv_freq, rot_mult, pos);
     float ss = 0.0f;
     for (int i = threadIdx.x; i < q_rank; i += blockDim.x) ss = fmaf(row[i], row[i], ss);
     ss = block_sum(ss, red);                 // (its barriers also publish the angles)
@@ -142,14 +156,16 @@ __global__ __launch_bounds__(256) void latent_query_kernel(
     const int32_t* __restrict__ req_of_token, const float* __restrict__ wkv, float eps, TC* __restrict__ pool,
     const int32_t* __restrict__ block_table, int max_blocks, int num_reqs, int num_pages, int page_size, int* __restrict__ err) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float red[33];
     __shared__ LatAngles angles;
     const int t = blockIdx.x;
+    // what no kernel in front writes, ahead of the wait: the angles, and the norm's weights on their way
     const int pos = positions[t], req = req_of_token[t];
+    lat_angles(angles, rot_dims, inv_freq, rot_mult, pos);
+    if (t == 0 && pool) prefetch_l2(wkv, R);
+    pdl_wait();
     if (req < 0 || pos < 0) return;
     if (pool && req >= num_reqs) { if (threadIdx.x == 0) atomicOr(err, AIRUN_DEV_BAD_REQ); return; }
-    lat_angles(angles, rot_dims, inv_freq, rot_mult, pos);
     __syncthreads();
     const float* row = q + (size_t)t * q_stride;
     lat_put_query<TC>(angles, row, qn + (size_t)t * H * D, qlat + (size_t)t * H * (R + rd), H, D, R, rd, rot_dims, rope_kind);

@@ -40,11 +40,6 @@ struct MoeChoices {
     }
 };
 
-// A weight that no kernel writes: on its way to the L2 cache while the kernel in front still runs.
-__device__ __forceinline__ void moe_prefetch(const float* p, int n) {
-    for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
-}
-
 // A block that holds all tokens of the step counts in shared memory and writes the segments itself: 32 threads scan.
 __device__ __forceinline__ void moe_segments(const int32_t* s_counts, int32_t* __restrict__ counts, int32_t* __restrict__ seg, int E) {
     const int lane = threadIdx.x & 31;
@@ -114,7 +109,7 @@ __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_kernel(
     const int32_t* __restrict__ req_of_token, int32_t* __restrict__ ids, float* __restrict__ wts, int32_t* __restrict__ rank,
     int32_t* __restrict__ counts, int32_t* __restrict__ seg) {
     pdl_trigger();
-    if (bias) moe_prefetch(bias, E);
+    if (bias) prefetch_l2(bias, E);
     pdl_wait();
     extern __shared__ float s_all[];                     // [warps][E], ONE: and the counts
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,7 +232,7 @@ __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_grouped_kernel(
     int groups, int keep, int sigmoid_scores, int group_best, int renorm, float weight_scale, const int32_t* __restrict__ req_of_token,
     int32_t* __restrict__ ids, float* __restrict__ wts, int32_t* __restrict__ rank, int32_t* __restrict__ counts, int32_t* __restrict__ seg) {
     pdl_trigger();
-    if (correction) moe_prefetch(correction, n_out);
+    if (correction) prefetch_l2(correction, n_out);
     pdl_wait();
     extern __shared__ float s_all[];                     // [warps][2 * n_out + groups], ONE: and the counts
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 2 * n_out + groups;

@@ -49,10 +49,21 @@ __global__ __launch_bounds__(32 * XA_PREP_WARPS) void qkv_prepare_kernel(
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv, int D, int Dv,
     int store, int one_row, int* __restrict__ err) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float s_x[XA_PREP_WARPS][32 * XA_MAX_PER_LANE];
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // what no kernel in front writes, ahead of the wait: the angles, which are the same for every head of the token (one sine
+    // and cosine per rotated pair), and the norms' weights on their way
     const int req = req_of_token[t], pos = positions[t];
+    __shared__ float s_cos[16 * XA_MAX_PER_LANE], s_sin[16 * XA_MAX_PER_LANE];
+    auto turn = [&](float at) {
+        if (rope_kind != XA_ROPE_NONE)
+            for (int i = threadIdx.x; i < (rdim >> 1); i += blockDim.x) sincosf(at * inv_freq[i], &s_sin[i], &s_cos[i]);
+    };
+    if (!rope_positions) turn((float)pos);
+    if (t == 0 && q_w) prefetch_l2(q_w, whole_norm ? nh * D : D);
+    if (t == 0 && k_w && store) prefetch_l2(k_w, whole_norm ? nkv * D : D);
+    pdl_wait();
+    if (rope_positions) turn((float)rope_positions[t]);
     if (req < 0 || pos < 0) return;
     if (req >= num_reqs) {
         if (threadIdx.x == 0) atomicOr(err, AIRUN_DEV_BAD_REQ);
@@ -75,11 +86,6 @@ __global__ __launch_bounds__(32 * XA_PREP_WARPS) void qkv_prepare_kernel(
     }
     const float* row = proj + (size_t)t * proj_stride;
     const int krow = one_row ? D + rdim : D;              // elements from one token's key to the next
-    const float rpos = (float)(rope_positions ? rope_positions[t] : pos);
-    // the angles are the same for every head of the token: one sine and cosine per rotated pair, worked out once
-    __shared__ float s_cos[16 * XA_MAX_PER_LANE], s_sin[16 * XA_MAX_PER_LANE];
-    if (rope_kind != XA_ROPE_NONE)
-        for (int i = threadIdx.x; i < (rdim >> 1); i += blockDim.x) sincosf(rpos * inv_freq[i], &s_sin[i], &s_cos[i]);
     // one root mean square over all rows of q and one over all rows of k, worked out ahead of the heads
     float whole_q = 1.0f, whole_k = 1.0f;
     if (whole_norm) {

@@ -276,8 +276,8 @@ struct TcShared {
 // 900, 16 heads on 8 KV heads: 25.6 us on 64 CTAs, 21.9 on 128.
 template <bool SHARED, bool SPLIT>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
-    const TcParams p, const int4* __restrict__ tiles, const __grid_constant__ CUtensorMap kv_map,
-    const int* __restrict__ n_tiles_dev, const TcShared sh) {
+    const TcParams p, const int4* tiles, const __grid_constant__ CUtensorMap kv_map,
+    const int* n_tiles_dev, const TcShared sh) {
     pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -318,7 +318,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
     // heads started last, on top of a machine already half done).
     const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int tile_idx = SHARED ? (int)blockIdx.x : lin / (int)gridDim.y;
-    if (!SHARED && n_tiles_dev && tile_idx >= *n_tiles_dev) {       // a CTA beyond the tiles in use: nothing to do
+    if (!SHARED && n_tiles_dev && tile_idx >= load_fresh(n_tiles_dev)) {       // a CTA beyond the tiles in use: nothing to do
         leave();
         return;
     }
@@ -331,7 +331,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
         n_tok = min(per, sh.n_tok - tok0);
         req = sh.req_of_token[tok0];
     } else {
-        const int4 t4 = tiles[tile_idx];
+        const int4 t4 = load_fresh(tiles + tile_idx);
         req = t4.x; tok0 = t4.y; n_tok = t4.z;
     }
     const int kvh = SHARED ? (int)blockIdx.y : lin % (int)gridDim.y;
@@ -747,8 +747,8 @@ enum { W_KFULL = 0, W_KEMPTY = 2, W_VFULL = 4, W_VEMPTY = 6, W_SFULL = 8, W_PFUL
 
 template <int KIND>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
-    const TcParams p, const int4* __restrict__ tiles, const __grid_constant__ CUtensorMap kv_map,
-    const int* __restrict__ n_tiles_dev, const WideExtra ex) {
+    const TcParams p, const int4* tiles, const __grid_constant__ CUtensorMap kv_map,
+    const int* n_tiles_dev, const WideExtra ex) {
     constexpr bool TABLE = KIND == W_TABLE || KIND == W_SIGMOID, DIFF = KIND == W_DIFF;
     pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -777,7 +777,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     // the KV heads of a tile before the next tile: the tiles with the most keys, of all heads, start first
     const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int tile_idx = lin / (int)gridDim.y;
-    if (n_tiles_dev && tile_idx >= *n_tiles_dev) {       // a CTA beyond the tiles in use: nothing to do
+    if (n_tiles_dev && tile_idx >= load_fresh(n_tiles_dev)) {       // a CTA beyond the tiles in use: nothing to do
         tc_fence_before();
         __syncthreads();
         if (warp == 1) {
@@ -788,7 +788,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     }
 
     const int G = p.G;
-    const int4 t4 = tiles[tile_idx];
+    const int4 t4 = load_fresh(tiles + tile_idx);
     const int req = t4.x, tok0 = t4.y, n_tok = t4.z;
     const int kvh = lin % (int)gridDim.y;
     const int n_rows = n_tok * G;

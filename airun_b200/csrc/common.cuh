@@ -34,6 +34,15 @@
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// What the kernel in front has written is read through volatile after pdl_wait(): a load through a const __restrict__ pointer
+// counts as the same for the whole kernel, from before the wait on, and may be moved ahead of it or answered from an L1
+// line that another kernel left.
+__device__ __forceinline__ int load_fresh(const int* p) { return *(const volatile int*)p; }
+__device__ __forceinline__ int4 load_fresh(const int4* p) {
+    const volatile int* v = (const volatile int*)p;
+    return make_int4(v[0], v[1], v[2], v[3]);
+}
+
 // A weight that no kernel writes: on its way to the L2 cache while the kernel in front still runs.
 __device__ __forceinline__ void prefetch_l2(const float* p, int n) {
     for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));

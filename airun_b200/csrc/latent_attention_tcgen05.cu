@@ -163,8 +163,8 @@ struct LatParams {
 enum { L_QFULL = 0, L_NFULL = 1, L_NEMPTY = 3, L_VFULL = 5, L_VEMPTY = 7, L_SFULL = 9, L_PFULL = 11, L_FINAL = 12, L_BARS = 13 };
 
 __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
-    const LatParams p, const int4* __restrict__ tiles, const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-    const int* __restrict__ n_tiles_dev) {
+    const LatParams p, const int4* tiles, const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
+    const int* n_tiles_dev) {
     pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -189,8 +189,8 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
     // the halves of a tile before the next tile: the tiles with the most keys start first
     const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int tile_idx = lin / (int)gridDim.y, half = lin % (int)gridDim.y;
-    if (tile_idx < *n_tiles_dev) {
-        const int4 t4 = tiles[tile_idx];
+    if (tile_idx < load_fresh(n_tiles_dev)) {
+        const int4 t4 = load_fresh(tiles + tile_idx);
         const int req = t4.x, tok0 = t4.y, n_rows = t4.z * p.H;
         const int pos_lo = p.positions[tok0], pos_hi = p.positions[tok0 + t4.z - 1];
         const int k_first = p.window > 0 ? max(0, pos_lo - p.window + 1) : 0;

@@ -1350,6 +1350,7 @@ AIRUN_EXPORT int airun_attn_prefill_kinds(int kind, const void* q, void* out, lo
         out_stride < (long long)nh * HD || (dist_a && !dist_b))
         return AIRUN_ERR_ARG;
     if ((kind != W_OPTIONS && kind != W_TABLE && kind != W_SIGMOID) || (kind == W_TABLE && (!table || table_len <= 0))) return AIRUN_ERR_ARG;
+    if (kind == W_OPTIONS && !(scale > 0.0f)) return AIRUN_ERR_ARG;          // the largest score is taken ahead of the scaling
     if (out_stride % 8 || ((uintptr_t)out & 15) || ((uintptr_t)q & 15) || (tail >= 0 && tail % 8)) return AIRUN_ERR_ARG;
     if (gate && (gate_stride % 4 || ((uintptr_t)gate & 15))) return AIRUN_ERR_ARG;
     int shift = -1;
@@ -1396,7 +1397,7 @@ AIRUN_EXPORT int airun_attn_prefill_diff(const void* q, void* out, long long out
                                          int max_blocks, const int32_t* positions, int num_pages, int page_size, int nh, int nkv,
                                          float scale, float cap, float lambda, float eps, float out_scale, int chunk, int window,
                                          const void* tiles, int n_tiles, const int32_t* n_tiles_dev, int* err, cudaStream_t stream) {
-    if (n_tiles < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || nh / nkv > QM || !err || out_stride < (long long)nh * HD || !(cap > 0.0f) ||
+    if (n_tiles < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || nh / nkv > QM || !err || out_stride < (long long)nh * HD || !(cap > 0.0f) || !(scale > 0.0f) ||
         chunk < 0 || window < 0 || out_stride % 8 || (((uintptr_t)out | (uintptr_t)q) & 15))
         return AIRUN_ERR_ARG;
     int shift = -1;

@@ -426,14 +426,15 @@ int row_map(CUtensorMap* out, const void* ptr, long long rows, int width, int bo
 
 // qlat [T][H][R + rd] and out [T][H][R] bfloat16, contiguous, 16-byte aligned; pool [pages][page_size][R + rd]; R and R + rd in
 // multiples of 64, R up to 512, R + rd up to 576; H up to 128; pages of a power of two >= 16 tokens.  tiles: {request, first
-// token, tokens (up to 128 / H), -}, of which *n_tiles_dev are in use.
+// token, tokens (up to 128 / H), -}, of which *n_tiles_dev are in use.  scale > 0: the largest score of a row is taken ahead of
+// the scaling.
 AIRUN_EXPORT int airun_latent_prefill(const void* qlat, void* out, const void* pool, const int32_t* block_table, int max_blocks,
                                       const int32_t* positions, int T, int num_pages, int page_size, int H, int R, int rd, float scale,
                                       int window, const float* sink, const float* gate, long long gate_stride, const void* tiles,
                                       int n_tiles, const int32_t* n_tiles_dev, int* err, cudaStream_t stream) {
     const int KD = R + rd;
     if (T < 0 || n_tiles < 0 || H <= 0 || H > LT_ROWS || R <= 0 || rd < 0 || R % 64 || KD % 64 || R > 512 || KD > 64 * LT_MAX_BLOCKS || !err ||
-        !n_tiles_dev || (gate && gate_stride < H) || (((uintptr_t)qlat | (uintptr_t)out | (uintptr_t)pool) & 15))
+        !n_tiles_dev || !(scale > 0.0f) || (gate && gate_stride < H) || (((uintptr_t)qlat | (uintptr_t)out | (uintptr_t)pool) & 15))
         return AIRUN_ERR_ARG;
     int shift = -1;
     for (int s = 4; s < 20; ++s) if ((1 << s) == page_size) shift = s;

@@ -833,10 +833,11 @@ LATENT_TC_MIN_TOKENS = 64
 
 def latent_prefill_tc(ctx, qlat, out, cache, part, gate: Optional[torch.Tensor] = None) -> bool:
     """The prompt portions of an attention over a cached latent on tcgen05 (csrc/latent_attention_tcgen05.cu); single tokens
-    are left alone.  False: the sizes, the pages or the alignment are not this kernel's, or the batch is too small for it."""
+    are left alone.  False: the sizes, the pages or the alignment are not this kernel's, the batch is too small for it, or the
+    scale is not positive (a row's largest score is taken, and hidden keys are marked, ahead of the scaling)."""
     H, R, KD, page, T = part.nh, part.R, part.R + part.rd, int(cache.page_size), qlat.shape[0]
     if ("latent_tc" in DISABLED or T < LATENT_TC_MIN_TOKENS or R % 64 or KD % 64 or R > 512 or KD > 576 or H > PREFILL_ROWS or page < 16
-            or page & (page - 1) or not hasattr(ctx, "context_lens") or not hasattr(ctx, "extras") or out.data_ptr() % 16 or qlat.data_ptr() % 16 or cache.pool.data_ptr() % 16):
+            or page & (page - 1) or not part.scale > 0 or not hasattr(ctx, "context_lens") or not hasattr(ctx, "extras") or out.data_ptr() % 16 or qlat.data_ptr() % 16 or cache.pool.data_ptr() % 16):
         return False
     tiles, n, n_dev = _prompt_tiles(ctx, H, PREFILL_ROWS, T)[:3]
     pool, bt = cache.pool, cache.block_table

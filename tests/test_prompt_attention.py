@@ -226,3 +226,24 @@ def test_what_the_kernel_does_not_take_stays_with_the_other():
         q = torch.zeros(T, nh * D, device="cuda", dtype=torch.bfloat16)
         out = torch.zeros(T, nh * D + 8, device="cuda", dtype=torch.bfloat16)[:, off:off + nh * D]
         assert not fast.attn_prompt_kind(batch_ctx([(0, T)]), "options", q, out, cache, part)
+
+
+@gpu
+@pytest.mark.parametrize("scale", [-0.11, 0.0])
+def test_latent_with_a_scale_that_is_not_positive(scale):
+    """The kernel takes a row's largest score before it scales: such a scale goes to the other kernel, and the result is the plain
+    kernel's (tolerance as above)."""
+    from airun_b200.kernels import fast, ops
+    H, R, rd, spans = 4, 128, 64, [(0, 200), (70, 130)]
+    g = torch.Generator().manual_seed(5)
+    bt, num_pages = scrambled_table([e for _, e in spans], 16, g)
+    cache = SimpleNamespace(pool=(0.8 * torch.randn(num_pages, 16 * (R + rd), generator=g)).to("cuda", torch.bfloat16), block_table=bt, page_size=16,
+                            shared=False)
+    ctx = batch_ctx(spans)
+    q = torch.randn(ctx.num_tokens, H * (R + rd), generator=g).to("cuda", torch.bfloat16)
+    part = SimpleNamespace(nh=H, R=R, rd=rd, scale=scale, window=0, sink=None)
+    got, want = (torch.zeros(ctx.num_tokens, H * R, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    assert fast.latent_attention_bf16(ctx, q, got, cache, part)
+    ops.latent_attention(q, want, cache, ctx, H, R, rd, scale, 0, None)
+    assert int(ctx.err.item()) == 0 and bool(torch.isfinite(got).all())
+    assert float((got.float() - want.float()).abs().max()) < 3 * 2.0 ** -8 * float(cache.pool.abs().max())

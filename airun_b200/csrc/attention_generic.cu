@@ -170,9 +170,14 @@ __global__ __launch_bounds__(32 * ROWS_WARPS) void attention_rows_f32_kernel(
             const bool ok = page >= 0 && page < num_pages;
             if (j <= pos && !ok) bad = true;
             on |= ok ? 1u << u : 0u;
-            const float* kj = pool + (((size_t)(ok ? page : 0) * 2 * nkv + kvh) * page_size + j % page_size) * HD + lane * PL;
-            kv[u] = lane_load<PL>(kj);
-            vv[u] = lane_load<PL>(kj + (size_t)nkv * page_size * HD);
+            // (a key that is not there is not read: its weight of zero would not make a NaN of another request harmless)
+#pragma unroll
+            for (int i = 0; i < PL; ++i) kv[u].v[i] = vv[u].v[i] = 0.0f;
+            if (ok) {
+                const float* kj = pool + (((size_t)page * 2 * nkv + kvh) * page_size + j % page_size) * HD + lane * PL;
+                kv[u] = lane_load<PL>(kj);
+                vv[u] = lane_load<PL>(kj + (size_t)nkv * page_size * HD);
+            }
         }
         float s[NV];
 #pragma unroll
@@ -248,7 +253,7 @@ __global__ __launch_bounds__(32 * ROWS_WARPS) void attention_rows_f32_kernel(
             gsum += s_sum[w][h] * weight;
             v = fmaf(s_acc[w][h][d], weight, v);
         }
-        dst[e] = gsum > 0.0f ? v * (1.0f / gsum) : 0.0f;
+        dst[e] = v * (gsum > 0.0f ? 1.0f / gsum : 0.0f);           // (a NaN in the sums stays one)
     }
 }
 

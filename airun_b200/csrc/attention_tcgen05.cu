@@ -733,15 +733,12 @@ __device__ __forceinline__ float w_log2(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// 1 / (1 + 2^x) of two scores with one reciprocal: 1/a = b / (ab).  x is kept at most 60 (a NaN stays one), so that the
-// product stays finite; such a weight is below 1e-18 either way.
-__device__ __forceinline__ float2 w_sigmoid2(float x, float y) {
-    asm("min.NaN.f32 %0, %0, 0f42700000;" : "+f"(x));
-    asm("min.NaN.f32 %0, %0, 0f42700000;" : "+f"(y));
-    const float a = 1.0f + ex2(x), b = 1.0f + ex2(y);
+// 1 / (1 + 2^x): 2^x = inf gives 0, 2^x = 0 gives 1.  (One reciprocal of a product for two scores would be a quarter fewer special
+// operations, but rounds four times more, cannot tell weights below 2^-60 apart and lets a NaN score spoil its neighbour.)
+__device__ __forceinline__ float w_sigmoid(float x) {
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
-    return make_float2(b * r, a * r);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + ex2(x)));
+    return r;
 }
 enum { W_KFULL = 0, W_KEMPTY = 2, W_VFULL = 4, W_VEMPTY = 6, W_SFULL = 8, W_PFULL = 10, W_FINAL = 12, W_PHALF = 13 };
 
@@ -986,7 +983,8 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     uint32_t pw[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        float2 w = w_sigmoid2(fmaf(v[2 * i], -sc, tb[-(c * 64 + 2 * i)]), fmaf(v[2 * i + 1], -sc, tb[-(c * 64 + 2 * i + 1)]));
+                        float2 w = make_float2(w_sigmoid(fmaf(v[2 * i], -sc, tb[-(c * 64 + 2 * i)])),
+                                               w_sigmoid(fmaf(v[2 * i + 1], -sc, tb[-(c * 64 + 2 * i + 1)])));
                         if (!full) {
                             const int j = j0 + c * 64 + 2 * i;
                             if (!(j <= pos && (p.window == 0 || pos - j < p.window))) w.x = 0.0f;
@@ -1028,7 +1026,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             }
             const float raw = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
             // (with a table the scores are scaled already; a cap keeps their order, so the largest is capped alone)
-            const float capped = TABLE ? raw : DIFF ? ex.cap_c - 2.0f * ex.cap_c * w_sigmoid2(ex.cap_k * raw, 0.0f).x : raw * sc;
+            const float capped = TABLE ? raw : DIFF ? ex.cap_c - 2.0f * ex.cap_c * w_sigmoid(ex.cap_k * raw) : raw * sc;
             const float mx = raw > 0.5f * NEG_BIG ? capped : NEG_BIG;
             const bool raise = mx > m + 8.0f;
             if (it == 0) {
@@ -1076,7 +1074,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 for (int i = 0; i < 32; ++i) {
                     float2 e;
                     if constexpr (DIFF) {
-                        const float2 w = w_sigmoid2(ex.cap_k * v[2 * i], ex.cap_k * v[2 * i + 1]);
+                        const float2 w = make_float2(w_sigmoid(ex.cap_k * v[2 * i]), w_sigmoid(ex.cap_k * v[2 * i + 1]));
                         e = __ffma2_rn(w, make_float2(-2.0f * ex.cap_c, -2.0f * ex.cap_c), make_float2(ex.cap_c + nm, ex.cap_c + nm));
                     } else {
                         e = TABLE ? __fadd2_rn(make_float2(v[2 * i], v[2 * i + 1]), nm2) : __ffma2_rn(make_float2(v[2 * i], v[2 * i + 1]), sc2, nm2);

@@ -587,6 +587,18 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
         }
         const uint32_t kb = smem_u32(wbase + stage * 2 * TILE_BYTES), vb = kb + TILE_BYTES;
         const int j0 = (tb + warp + it * DW) * DN;
+        if (KIND != D_PLAIN && (j0 < k_first || j0 + DN - 1 > pos)) {
+            // Value rows that this token does not see may be another request's or left over: as zeros they add nothing, as NaN times
+            // a weight of zero they would be NaN.  Lane r + 16 h blanks the h-th half of row r.
+            const int j = j0 + (lane & 15);
+            if (j < k_first || j > pos) {
+                uint4* const vrow = reinterpret_cast<uint4*>(wbase + stage * 2 * TILE_BYTES + TILE_BYTES + (lane >> 4) * 2048 + (lane & 15) * 128);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) vrow[c] = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // ahead of the copy that fills this stage again
+            }
+            __syncwarp();
+        }
         float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {

@@ -814,7 +814,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     const int blk = j >> p.page_shift;
                     int page = (j <= pos_hi && blk < p.max_blocks) ? __ldg(bt + blk) : 0;
                     if (page < 0 || page >= p.num_pages) {
-                        if (j >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
+                        if (j + 15 >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                         page = 0;
                     }
                     const int parts = KIND != W_PLAIN && ex.tail >= 0 ? 1 : 2;       // key rows, then value rows; or rows that are both
@@ -972,6 +972,25 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             }
             tc_fence_after();
             const int j0 = (tile_first + it) * KN;
+            if (KIND != W_PLAIN && x == 0 && (j0 < k_first || j0 + KN - 1 > pos_hi)) {
+                // Value rows that no token of the tile sees may be another request's or left over: as zeros they add nothing, as
+                // NaN times a weight of zero they would be NaN.  Thread r blanks the row of key r; the products of both Q tiles
+                // begin after this warpgroup's weights.
+                if (!mbar_wait(BAR(W_VFULL + (it & 1)), (it >> 1) & 1)) {
+                    ok = false;
+                    if (TABLE) continue;
+                    break;
+                }
+                if (j0 + r < k_first || j0 + r > pos_hi) {
+                    uint8_t* const vrow = smem + W_OFF_V + (it & 1) * KV_BYTES + r * 128;
+#pragma unroll
+                    for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(vrow + h * ROWBLK + c * 16) = make_uint4(0, 0, 0, 0);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                __syncwarp();
+            }
             // every key visible to every row: no masks
             const bool full = DIFF ? j0 >= all_lo && j0 + KN - 1 <= pos_lo : p.window == 0 && j0 + KN - 1 <= pos_lo;
             float v[64];

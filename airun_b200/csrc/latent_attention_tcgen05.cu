@@ -215,7 +215,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                         const int j = (tile_first + it) * LT_KEYS + g * 16, blk = j >> p.page_shift;
                         int page = (j <= pos_hi && blk < p.max_blocks) ? __ldg(bt + blk) : 0;
                         if (page < 0 || page >= p.num_pages) {
-                            if (j >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
+                            if (j + 15 >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                             page = 0;
                         }
                         rows[g] = (page << p.page_shift) + (j & (p.page_size - 1));
@@ -302,6 +302,16 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                 tmem_wait32(raw);
                 tmem_wait32(raw + 32);
                 const int j0 = (tile_first + it) * LT_KEYS;
+                if (r < LT_KEYS && (j0 + r < k_first || j0 + r > pos_hi)) {
+                    // A cached row that no token of the tile sees may be another request's or left over: as zeros its values add
+                    // nothing, as NaN times a weight of zero they would be NaN.  S has been formed, so all blocks have landed.
+                    uint8_t* const row = smem_k + (it % p.stages) * p.blocks * LT_KBLK + r * 128;
+                    for (int b = 0; b < nv; ++b)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(row + b * LT_KBLK + c * 16) = make_uint4(0, 0, 0, 0);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                __syncwarp();
                 float v[LT_KEYS];
                 const bool full = p.window == 0 && j0 + LT_KEYS - 1 <= pos_lo;      // every key visible to every row
 #pragma unroll

@@ -93,6 +93,20 @@ def spoil(kind, pages, page, row):
 
 
 @gpu
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3.0e38])
+@pytest.mark.parametrize("spans", [PROMPTS, SINGLES], ids=["prompts", "singles"])
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_rows_that_no_token_sees(kind, spans, bad):
+    run, _, pages, seen, rows, _, _, _ = made(kind, spans, len(kind))
+    unseen = ~seen[:, None, :, None].expand_as(pages)
+    zeros = run(pages.masked_fill(unseen, 0.0))
+    if zeros is None:
+        pytest.skip("single tokens of this kind have a kernel of their own")
+    anything = run(pages.masked_fill(unseen, bad))
+    assert bool(torch.isfinite(zeros[rows]).all()) and torch.equal(zeros[rows], anything[rows])
+
+
+@gpu
 @pytest.mark.parametrize("hd", [32, 64, 128])
 @pytest.mark.parametrize("nh,nkv", [(1, 1), (4, 2), (8, 2)])
 def test_unseen_rows_and_nan_keys_in_float32(hd, nh, nkv):

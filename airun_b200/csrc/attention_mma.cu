@@ -545,7 +545,9 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
 
     if (!TMA && my_n > 0) load_tile(tb + warp, 0);
 
-    float m0 = NEG_BIG, m1 = NEG_BIG, l0 = 0.0f, l1 = 0.0f;
+    // with options a visible score may be as low as float32 goes (a distance table), and a NaN must stay one: hidden is -inf there
+    constexpr float HIDDEN = KIND == D_PLAIN ? NEG_BIG : -INFINITY;
+    float m0 = HIDDEN, m1 = HIDDEN, l0 = 0.0f, l1 = 0.0f;
     float o[HD / 8][4];
 #pragma unroll
     for (int n = 0; n < HD / 8; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.0f; }
@@ -632,7 +634,7 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
                 for (int e = 0; e < 4; ++e) {
                     const int j = j0 + n * 8 + 2 * t + (e & 1);
                     const bool vis = j <= pos && j >= k_first;
-                    float v = vis ? s[n][e] * p.scale_log2 : NEG_BIG;
+                    float v = vis ? s[n][e] * p.scale_log2 : HIDDEN;
                     if (KIND == D_OPTIONS && kd.table && vis) v = fmaf(LOG2E, __ldg(table[e >> 1] + min(pos - j, kd.table_len - 1)), v);
                     s[n][e] = v;
                     if (e < 2) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
@@ -642,15 +644,17 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-            const float c0 = exp2f(m0 - mx0), c1 = exp2f(m1 - mx1);
+            // (nothing seen yet: subtract nothing, so that hidden keys come out as 0)
+            const float b0 = KIND != D_PLAIN && mx0 == -INFINITY ? 0.0f : mx0, b1 = KIND != D_PLAIN && mx1 == -INFINITY ? 0.0f : mx1;
+            const float c0 = exp2f(m0 - b0), c1 = exp2f(m1 - b1);
             m0 = mx0; m1 = mx1;
             float rs0 = 0.0f, rs1 = 0.0f;
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-                const float p00 = s[n][0] > 0.5f * NEG_BIG ? exp2f(s[n][0] - mx0) : 0.0f;
-                const float p01 = s[n][1] > 0.5f * NEG_BIG ? exp2f(s[n][1] - mx0) : 0.0f;
-                const float p10 = s[n][2] > 0.5f * NEG_BIG ? exp2f(s[n][2] - mx1) : 0.0f;
-                const float p11 = s[n][3] > 0.5f * NEG_BIG ? exp2f(s[n][3] - mx1) : 0.0f;
+                const float p00 = KIND != D_PLAIN || s[n][0] > 0.5f * NEG_BIG ? exp2f(s[n][0] - b0) : 0.0f;
+                const float p01 = KIND != D_PLAIN || s[n][1] > 0.5f * NEG_BIG ? exp2f(s[n][1] - b0) : 0.0f;
+                const float p10 = KIND != D_PLAIN || s[n][2] > 0.5f * NEG_BIG ? exp2f(s[n][2] - b1) : 0.0f;
+                const float p11 = KIND != D_PLAIN || s[n][3] > 0.5f * NEG_BIG ? exp2f(s[n][3] - b1) : 0.0f;
                 rs0 += p00 + p01;
                 rs1 += p10 + p11;
                 pf[n * 2 + 0] = pack_bf16(p00, p01);
@@ -696,9 +700,9 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     // what a row's sums are multiplied by: 1 / (their weights' sum and the sink's), with the factor; the result with its gate
     auto row_factor = [&](int r, float gm, float sum) -> float {
         if (KIND == D_SIGMOID) return 1.0f;
-        const float sink2 = kd.sink ? __ldg(kd.sink + head0 + r) * LOG2E : NEG_BIG;
-        const float top = fmaxf(gm, sink2), f = gm > 0.5f * NEG_BIG ? exp2f(gm - top) : 0.0f;
-        const float den = sum * f + (kd.sink ? exp2f(sink2 - top) : 0.0f);
+        const float sink2 = kd.sink ? __ldg(kd.sink + head0 + r) * LOG2E : HIDDEN;
+        const float top = fmaxf(gm, sink2), f = gm > HIDDEN ? exp2f(gm - top) : 0.0f;
+        const float den = sum * f + (sink2 > HIDDEN ? exp2f(sink2 - top) : 0.0f);
         return den > 0.0f ? kd.out_scale * f / den : 0.0f;
     };
     auto put = [&](int r, int d, float v) {
@@ -713,7 +717,7 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     float* part = ns + extra > 1 ? x.scratch + ((size_t)unit * unit_stride + split) * (16 * (HD + 2)) : nullptr;
     for (int e = threadIdx.x; e < heads * HD; e += 32 * DW) {
         const int r = e / HD, d = e - r * HD;
-        float gm = NEG_BIG;
+        float gm = HIDDEN;
 #pragma unroll
         for (int w = 0; w < DW; ++w) gm = fmaxf(gm, s_m[w][r]);
         float acc = 0.0f, sum = 0.0f;
@@ -751,13 +755,13 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     for (int i = threadIdx.x; i < nt * 16; i += 32 * DW) {
         const int sp = i >> 4, r = i & 15;
         const float* ps = all + (size_t)slot(sp) * 16 * (HD + 2) + r * (HD + 2);
-        s_f[sp][r] = r < heads ? __ldcg(ps) : NEG_BIG;          // the slice's maximum
+        s_f[sp][r] = r < heads ? __ldcg(ps) : HIDDEN;          // the slice's maximum
         s_l2[sp][r] = r < heads ? __ldcg(ps + 1) : 0.0f;        // and its sum
     }
     __syncthreads();
     if (threadIdx.x < heads) {
         const int r = threadIdx.x;
-        float gm = NEG_BIG;
+        float gm = HIDDEN;
         for (int sp = 0; sp < nt; ++sp) gm = fmaxf(gm, s_f[sp][r]);
         float sum = 0.0f;
         for (int sp = 0; sp < nt; ++sp) {

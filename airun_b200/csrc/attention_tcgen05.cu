@@ -747,6 +747,9 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     const TcParams p, const int4* tiles, const __grid_constant__ CUtensorMap kv_map,
     const int* n_tiles_dev, const WideExtra ex) {
     constexpr bool TABLE = KIND == W_TABLE || KIND == W_SIGMOID, DIFF = KIND == W_DIFF;
+    // what a hidden key's score is and the lowest a row's maximum counts from: with a distance table a visible score may be as
+    // low as float32 goes
+    constexpr float HIDDEN = KIND == W_PLAIN ? NEG_BIG : -INFINITY, LOWEST = KIND == W_PLAIN ? 0.5f * NEG_BIG : -INFINITY;
     pdl_trigger();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -925,7 +928,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             if (lane == 0) mbar_arrive(BAR(W_PFULL + x));          // phase 0: Q is ready
         }
 
-        float m = NEG_BIG, l = 0.0f;
+        float m = HIDDEN, l = 0.0f;
         bool ok = true;
         const float sc = p.scale_log2;
         // W_DIFF: the first key this row sees, and the first that all rows see
@@ -1022,7 +1025,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             }
             // the row's maximum, as four chains that the scheduler can interleave: keys 64-127, then keys 0-63,
             // which stay in registers
-            float r0 = NEG_BIG, r1 = NEG_BIG, r2 = NEG_BIG, r3 = NEG_BIG;
+            float r0 = HIDDEN, r1 = HIDDEN, r2 = HIDDEN, r3 = HIDDEN;
 #pragma unroll
             for (int c = 1; c >= 0; --c) {
                 tmem_ld64(s_addr + c * 64, v);
@@ -1035,7 +1038,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     for (int i = 0; i < 64; ++i) {
                         const int j = j0 + c * 64 + i;
                         const bool vis = DIFF ? j <= pos && j >= vis_lo : j <= pos && (p.window == 0 || pos - j < p.window);
-                        v[i] = vis ? v[i] : NEG_BIG;
+                        v[i] = vis ? v[i] : HIDDEN;
                     }
                 }
 #pragma unroll
@@ -1046,7 +1049,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             const float raw = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
             // (with a table the scores are scaled already; a cap keeps their order, so the largest is capped alone)
             const float capped = TABLE ? raw : DIFF ? ex.cap_c - 2.0f * ex.cap_c * w_sigmoid(ex.cap_k * raw) : raw * sc;
-            const float mx = raw > 0.5f * NEG_BIG ? capped : NEG_BIG;
+            const float mx = raw > LOWEST ? capped : HIDDEN;
             const bool raise = mx > m + 8.0f;
             if (it == 0) {
                 m = mx;                                              // nothing accumulated yet
@@ -1065,10 +1068,10 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 if (raise) m = mx;
             }
             // probabilities as pairs of bfloat16 over the S tile (keys 2c, 2c+1 in column c), row sum.
-            // A hidden key holds -1e30, which the product sends to exp2(-inf) = 0 without a test; only a
-            // row that has seen no key at all (m = -1e30) must not add its -m.
+            // A hidden key holds HIDDEN, which the product sends to exp2(-inf) = 0 without a test; only a
+            // row that has seen no key at all (m = HIDDEN) must not add its -m.
             const float2 sc2 = make_float2(sc, sc);
-            const float nm = m > 0.5f * NEG_BIG ? -m : 0.0f;
+            const float nm = m > LOWEST ? -m : 0.0f;
             const float2 nm2 = make_float2(nm, nm);
             float2 rs2 = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -1084,7 +1087,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                         for (int i = 0; i < 64; ++i) {
                             const int j = j0 + 64 + i;
                             const bool vis = DIFF ? j <= pos && j >= vis_lo : j <= pos && (p.window == 0 || pos - j < p.window);
-                            v[i] = vis ? v[i] : NEG_BIG;
+                            v[i] = vis ? v[i] : HIDDEN;
                         }
                     }
                 }
@@ -1100,8 +1103,8 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     }
                     float2 pp = make_float2(ex2(e.x), ex2(e.y));
                     if (DIFF && !full) {                             // a hidden key's score is capped as well: it weighs nothing
-                        if (v[2 * i] <= 0.5f * NEG_BIG) pp.x = 0.0f;
-                        if (v[2 * i + 1] <= 0.5f * NEG_BIG) pp.y = 0.0f;
+                        if (v[2 * i] == -INFINITY) pp.x = 0.0f;
+                        if (v[2 * i + 1] == -INFINITY) pp.y = 0.0f;
                     }
                     rs2 = __fadd2_rn(rs2, pp);
                     __nv_bfloat162 h2 = __floats2bfloat162_rn(pp.x, pp.y);
@@ -1186,9 +1189,9 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 inv = 1.0f;
             } else {
                 // the sink joins the denominator; if it is above every score the sums are scaled down to it
-                const float sink2 = ex.sink ? __ldg(ex.sink + head) * LOG2E : NEG_BIG;
-                const float top = fmaxf(m, sink2), f = m > 0.5f * NEG_BIG ? ex2(m - top) : 0.0f;
-                const float den = l * f + (ex.sink ? ex2(sink2 - top) : 0.0f);
+                const float sink2 = ex.sink ? __ldg(ex.sink + head) * LOG2E : HIDDEN;
+                const float top = fmaxf(m, sink2), f = m > LOWEST ? ex2(m - top) : 0.0f;
+                const float den = l * f + (sink2 > LOWEST ? ex2(sink2 - top) : 0.0f);
                 inv = den > 0.0f ? ex.out_scale * f / den : 0.0f;
                 if (ex.gate) gate = ex.gate + (size_t)tok * ex.gate_stride + (size_t)head * HD;
             }

@@ -160,6 +160,33 @@ def test_a_nan_key_of_a_prompt_reaches_the_rows_that_see_it(kind, key):
 
 
 @gpu
+@pytest.mark.parametrize("key", [0, 13, 14, 290, 299])
+@pytest.mark.parametrize("kind", [k for k in KINDS if not k.startswith(("diff", "latent"))])
+def test_a_nan_key_of_a_single_token(kind, key):
+    run, plain, pages, seen, rows, ctx, part, bt = made(kind, SINGLES, len(kind) + key)
+    clean = run(pages)
+    sick = pages.clone()
+    spoil(kind, sick, int(bt[2, key // 16]), key % 16)
+    got, want = run(sick), torch.isnan(plain(sick))
+    assert torch.equal(torch.isnan(got), want) and torch.equal(got[~want], clean[~want])
+    if not part.window or 299 - key < part.window:
+        assert bool(want[2].any())
+
+
+@gpu
+@pytest.mark.parametrize("spans", [PROMPTS, SINGLES], ids=["prompts", "singles"])
+def test_distance_terms_near_the_lowest_number(spans):
+    """Every distance of the second head costs 1e32: a row's weights go by the differences, and no row may come out empty."""
+    run, plain, pages, seen, rows, ctx, part, bt = made("table", spans, 3)
+    part.table[1] = -1.0e32
+    part.sink = None
+    got, want = run(pages)[rows].float(), plain(pages)[rows].float()
+    assert bool(torch.isfinite(want).all()) and bool((want.view(-1, 4, 128)[:, 1].abs().amax(-1) > 0).all())
+    # both work in float32 at 1e32, where the scores vanish: the mean of the visible values, rounded (see test_prompt_attention)
+    assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * float(pages.abs().max())
+
+
+@gpu
 @pytest.mark.parametrize("spans", [PROMPTS, SINGLES], ids=["prompts", "singles"])
 def test_sigmoid_weights_far_below_one(spans):
     """A score offset of -60: weights of e^-60 times values of up to 1e25.  bfloat16 weights and results: 3 * 2^-8 of the

@@ -40,7 +40,7 @@ struct RowsParams {
 
 __device__ __forceinline__ float activation(float z, int m) {
     if (m == 0) { const float r = fmaxf(z, 0.0f); return r * r; }
-    if (m == 1) return __fdividef(z, 1.0f + __expf(-z));
+    if (m == 1) return z / (1.0f + __expf(-z));
     if (m == 2) return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
     if (m == 4) return 0.5f * z * (1.0f + erff(z * 0.7071067811865476f));
     return fmaxf(z, 0.0f);
@@ -49,9 +49,9 @@ __device__ __forceinline__ float gated_unit(float limit, float slope, float g, f
     if (limit > 0.0f) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
-        return __fdividef(g, 1.0f + __expf(-slope * g)) * (u + 1.0f);
+        return g / (1.0f + __expf(-slope * g)) * (u + 1.0f);
     }
-    return __fdividef(g, 1.0f + __expf(-g)) * u;
+    return g / (1.0f + __expf(-g)) * u;
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"

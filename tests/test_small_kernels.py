@@ -127,3 +127,73 @@ def test_products_with_the_tokens_as_columns(M, bn, epi, ksplit):
         e = e + 2.0 ** -8 * want.abs()
     assert int(err.item()) == 0 and bool(((out[:M].cpu().double() - want).abs() <= e + 1e-30).all())
     assert bool((out[M:] == 7.0).all())
+
+
+@gpu
+@pytest.mark.parametrize("how", ["rows", "rows grouped", "columns", "columns cluster", "persistent", "persistent grouped"])
+@pytest.mark.parametrize("limit", [0.0, 7.0])
+def test_gated_units_of_gates_far_below_zero(how, limit):
+    """silu(-88) is -5e-37 and is multiplied by up to 1e30: the quotient's divisor, e^88, lies beyond 2^126, where the fast
+    division gives zero.  e^x is right to 2 + 1.2 |x| units of 2^-24; bfloat16 results round to 2^-8."""
+    from types import SimpleNamespace
+
+    from airun_b200.kernels import fast
+    M, N, K = (5 if how.startswith("rows") else 40 if how.startswith("columns") else 300), 512, 64
+    g = torch.Generator().manual_seed(M)
+    gate, up = -80.0 - 8.4 * torch.rand(N // 2, generator=g), 1.0e30 * torch.randn(N // 2, generator=g)
+    w = torch.zeros(N // 32, 2, 16, K)
+    w[:, 0, :, 0], w[:, 1, :, 1] = gate.view(-1, 16), up.view(-1, 16)
+    w = w.view(N, K).bfloat16()
+    x = torch.zeros(M, K).bfloat16()
+    x[:, 0] = 1.0
+    x[:, 1] = torch.randn(M, generator=g).bfloat16()
+    z = (x.double() @ w.double().T).view(M, N // 32, 2, 16)
+    a, b = z[:, :, 0].reshape(M, -1), z[:, :, 1].reshape(M, -1)
+    if limit:
+        want = a * torch.sigmoid(a) * (b.clamp(-limit, limit) + 1)
+    else:
+        want = a * torch.sigmoid(a) * b
+    out = torch.full((M, N // 2), 7.0, dtype=torch.bfloat16, device="cuda")
+    ctx = SimpleNamespace(err=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    xd, wd, glu = x.cuda(), w.cuda(), (limit, 1.0 if limit else 0.0)
+    if "grouped" in how:
+        seg = torch.tensor([0, M], dtype=torch.int32, device="cuda")
+        old, fast.GROUPED_ROWS_MAX = fast.GROUPED_ROWS_MAX, 64 if how.startswith("rows") else 0
+        try:
+            assert fast.grouped_linear_bf16(ctx, xd, wd[None].contiguous(), out, seg, swiglu_group=16, **(dict(glu=glu) if limit else {}))
+        finally:
+            fast.GROUPED_ROWS_MAX = old
+    elif limit:
+        assert fast.linear_glu_clamped_bf16(ctx, xd, wd, out, 16, limit, 1.0)
+    elif how == "rows":
+        fast.gemm_rows(xd, wd, out, fast.EPI_SWIGLU, glu=glu)
+    else:
+        swap = how.startswith("columns")
+        fast.gemm_tcgen05(xd, wd, out, fast.EPI_SWIGLU, swap, 64 if swap else 256, 1, ctx.err)
+    assert int(ctx.err.item()) == 0 and float(want.abs().min()) > 0
+    assert bool(((out.cpu().double() - want).abs() <= (2.0 ** -8 + 2e-5) * want.abs() + 1.2e-38).all())
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M", [5, 40, 300])
+def test_silu_far_below_zero(M, dtype):
+    """z sigmoid(z) as an epilogue where e^-z lies beyond 2^126 (see above)."""
+    from types import SimpleNamespace
+
+    from airun_b200.kernels import fast, ops
+    N, K = 512, 64
+    w = torch.zeros(N, K)
+    w[:, 0] = -80.0 - 8.4 * torch.rand(N, generator=torch.Generator().manual_seed(M))
+    w, x = w.bfloat16(), torch.zeros(M, K).bfloat16()
+    x[:, 0] = 1.0
+    z = x.double() @ w.double().T
+    want = z * torch.sigmoid(z)
+    out, err = torch.full((M, N), 7.0, dtype=dtype, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    epi, silu = (fast.EPI_F32 if dtype == torch.float32 else fast.EPI_BF16), ops.ACTIVATIONS["silu"]
+    if M == 5:
+        fast.gemm_rows(x.cuda(), w.cuda(), out, epi, act=silu)
+    else:
+        fast.gemm_tcgen05(x.cuda(), w.cuda(), out, epi, M == 40, 64 if M == 40 else 256, 1, err, act=silu)
+    assert int(err.item()) == 0
+    assert bool(((out.cpu().double() - want).abs() <= ((2.0 ** -8 if dtype == torch.bfloat16 else 0) + 2e-5) * want.abs() + 1.2e-38).all())

@@ -1055,7 +1055,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 m = mx;                                              // nothing accumulated yet
             } else if (__any_sync(0xffffffffu, raise)) {
                 // rescale this warp's rows of O
-                const float f = raise ? ex2(m - mx) : 1.0f;
+                const float f = raise ? (DIFF ? exp2f(m - mx) : ex2(m - mx)) : 1.0f;
 #pragma unroll
                 for (int c = 0; c < HD; c += 32) {
                     float t[32];
@@ -1101,7 +1101,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     } else {
                         e = TABLE ? __fadd2_rn(make_float2(v[2 * i], v[2 * i + 1]), nm2) : __ffma2_rn(make_float2(v[2 * i], v[2 * i + 1]), sc2, nm2);
                     }
-                    float2 pp = make_float2(ex2(e.x), ex2(e.y));
+                    float2 pp = DIFF ? make_float2(exp2f(e.x), exp2f(e.y)) : make_float2(ex2(e.x), ex2(e.y));
                     if (DIFF && !full) {                             // a hidden key's score is capped as well: it weighs nothing
                         if (v[2 * i] == -INFINITY) pp.x = 0.0f;
                         if (v[2 * i + 1] == -INFINITY) pp.y = 0.0f;
@@ -1190,8 +1190,8 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             } else {
                 // the sink joins the denominator; if it is above every score the sums are scaled down to it
                 const float sink2 = ex.sink ? __ldg(ex.sink + head) * LOG2E : HIDDEN;
-                const float top = fmaxf(m, sink2), f = m > LOWEST ? ex2(m - top) : 0.0f;
-                const float den = l * f + (sink2 > LOWEST ? ex2(sink2 - top) : 0.0f);
+                const float top = fmaxf(m, sink2), f = m > LOWEST ? exp2f(m - top) : 0.0f;
+                const float den = l * f + (sink2 > LOWEST ? exp2f(sink2 - top) : 0.0f);
                 inv = den > 0.0f ? ex.out_scale * f / den : 0.0f;
                 if (ex.gate) gate = ex.gate + (size_t)tok * ex.gate_stride + (size_t)head * HD;
             }
@@ -1214,10 +1214,10 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 #pragma unroll
                         for (int i = 0; i < 8; i += 4) {
                             const float4 g4 = *reinterpret_cast<const float4*>(gate + c + q8 * 8 + i);
-                            o[q8 * 8 + i] = __fdividef(o[q8 * 8 + i], 1.0f + __expf(-g4.x));
-                            o[q8 * 8 + i + 1] = __fdividef(o[q8 * 8 + i + 1], 1.0f + __expf(-g4.y));
-                            o[q8 * 8 + i + 2] = __fdividef(o[q8 * 8 + i + 2], 1.0f + __expf(-g4.z));
-                            o[q8 * 8 + i + 3] = __fdividef(o[q8 * 8 + i + 3], 1.0f + __expf(-g4.w));
+                            o[q8 * 8 + i] /= 1.0f + __expf(-g4.x);
+                            o[q8 * 8 + i + 1] /= 1.0f + __expf(-g4.y);
+                            o[q8 * 8 + i + 2] /= 1.0f + __expf(-g4.z);
+                            o[q8 * 8 + i + 3] /= 1.0f + __expf(-g4.w);
                         }
                     }
 #pragma unroll

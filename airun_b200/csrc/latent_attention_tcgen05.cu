@@ -133,11 +133,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 // K-major operand, rows of 128 bytes with the 128-byte swizzle: 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
@@ -333,7 +328,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                 if (it == 0) {
                     m = mx;                                              // nothing accumulated yet
                 } else if (__any_sync(0xffffffffu, raise)) {
-                    const float f = raise ? ex2(m - mx) : 1.0f;          // rescale this warp's rows of O
+                    const float f = raise ? exp2f(m - mx) : 1.0f;          // rescale this warp's rows of O
                     for (int c = 0; c < nv * 64; c += 32) {
                         uint32_t t[32];
                         tmem_ld32_async(o_addr + c, t);
@@ -353,7 +348,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
 #pragma unroll
                 for (int i = 0; i < LT_KEYS / 2; ++i) {
                     const float2 e = __ffma2_rn(make_float2(v[2 * i], v[2 * i + 1]), sc2, nm2);
-                    const float2 pp = make_float2(ex2(e.x), ex2(e.y));
+                    const float2 pp = make_float2(exp2f(e.x), exp2f(e.y));
                     rs2 = __fadd2_rn(rs2, pp);
                     __nv_bfloat162 h2 = __floats2bfloat162_rn(pp.x, pp.y);
                     pw[i] = *reinterpret_cast<uint32_t*>(&h2);
@@ -370,10 +365,10 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
             tc_fence_after();
             // the sink joins the denominator; if it is above every score the sums are scaled down to it
             const float sink2 = p.sink ? __ldg(p.sink + head) * LOG2E : NEG_BIG;
-            const float top = fmaxf(m, sink2), f = m > 0.5f * NEG_BIG ? ex2(m - top) : 0.0f;
-            const float den = l * f + (p.sink ? ex2(sink2 - top) : 0.0f);
+            const float top = fmaxf(m, sink2), f = m > 0.5f * NEG_BIG ? exp2f(m - top) : 0.0f;
+            const float den = l * f + (p.sink ? exp2f(sink2 - top) : 0.0f);
             float inv = den > 0.0f ? f / den : 0.0f;
-            if (p.gate && row_ok) inv = __fdividef(inv, 1.0f + __expf(-p.gate[(size_t)tok * p.gate_stride + head]));
+            if (p.gate && row_ok) inv /= 1.0f + __expf(-p.gate[(size_t)tok * p.gate_stride + head]);
             uint4* dst = reinterpret_cast<uint4*>(p.out + ((size_t)tok * p.H + head) * p.R + v0 * 64);
             for (int c = 0; c < nv * 64; c += 32) {
                 uint32_t o[32];

@@ -45,7 +45,7 @@ def made(kind, spans, seed, page=16):
     part = SimpleNamespace(D=128, Dv=128, nh=nh, nkv=nkv, scale=0.13, window=window, out_scale=1.0, tail=64 if kind == "one" else -1,
                            table=torch.randn(nh, 400, generator=g).cuda() if kind == "table" else None, sink=torch.zeros(nh, device="cuda"),
                            dist_a=torch.full((nh,), 0.4, device="cuda"), dist_b=torch.full((nh,), 0.2, device="cuda"), head_c=None, R=R, rd=rd,
-                           chunk=chunk, cap=20.0, lam=0.45, eps=1e-5, lambda_init=0.2, gate=None)
+                           chunk=chunk, cap=20.0, lam=0.45, eps=1e-5, lambda_init=0.2, gate=None, q=q)
     if kind == "differential":
         part.D = 64
 
@@ -55,30 +55,30 @@ def made(kind, spans, seed, page=16):
     def run(p):
         out = torch.full((T, ow), 7.0, device="cuda", dtype=torch.bfloat16)
         if kind == "latent":
-            took = not single and fast.latent_prefill_tc(ctx, q, out, cache(p), part, part.gate)
+            took = not single and fast.latent_prefill_tc(ctx, part.q, out, cache(p), part, part.gate)
         elif kind == "differential":
-            took = not single and fast.diff_prefill_tc(ctx, q, out, cache(p), part)
+            took = not single and fast.diff_prefill_tc(ctx, part.q, out, cache(p), part)
         else:
             name = "options" if kind in ("one", "window") else kind
             more = {} if kind == "sigmoid" else dict(gate=part.gate, gate_stride=ops.attention_gate(part.gate, T, ow))
             if single:
-                took = fast.attn_single_kind(ctx, name if name == "sigmoid" else "options", q, out, cache(p), part, True, tail=part.tail, **more)
+                took = fast.attn_single_kind(ctx, name if name == "sigmoid" else "options", part.q, out, cache(p), part, True, tail=part.tail, **more)
             else:
-                took = fast.attn_prompt_kind(ctx, name, q, out, cache(p), part, tail=part.tail, **more)
+                took = fast.attn_prompt_kind(ctx, name, part.q, out, cache(p), part, tail=part.tail, **more)
         assert int(ctx.err.item()) == 0
         return out if took else None
 
     def plain(p):
         out = torch.zeros(T, ow, device="cuda", dtype=torch.bfloat16)
         if kind == "latent":
-            ops.latent_attention(q, out, cache(p), ctx, nh, R, rd, 0.13, window, part.sink, part.gate)
+            ops.latent_attention(part.q, out, cache(p), ctx, nh, R, rd, 0.13, window, part.sink, part.gate)
         elif kind == "differential":
-            ops.diff_attention(q, out, cache(p).pool, bt, ctx.positions, ctx.req_of_token, ctx.num_reqs, page, nh, nkv, 64, 128, 0.13, 20.0, chunk,
+            ops.diff_attention(part.q, out, cache(p).pool, bt, ctx.positions, ctx.req_of_token, ctx.num_reqs, page, nh, nkv, 64, 128, 0.13, 20.0, chunk,
                                window, 0.45, 1e-5, 0.8, ctx.err)
         elif kind == "sigmoid":
-            ops.sigmoid_attention(q, out, cache(p), ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, part.head_c, window)
+            ops.sigmoid_attention(part.q, out, cache(p), ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, part.head_c, window)
         else:
-            ops.softmax_attention(q, out, cache(p), ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, 1.0, tail=part.tail, gate=part.gate)
+            ops.softmax_attention(part.q, out, cache(p), ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, 1.0, tail=part.tail, gate=part.gate)
         return out
 
     rows = torch.tensor([single or n > 1 for n in ctx.query_lens for _ in range(n)], device="cuda")
@@ -196,3 +196,22 @@ def test_sigmoid_weights_far_below_one(spans):
     pages[:, 2:] *= 1.0e25
     got, want = run(pages)[rows].float(), plain(pages)[rows].float()
     assert bool(torch.isfinite(got).all()) and float((got - want).abs().max()) < 3 * 2.0 ** -8 * float(want.abs().max())
+
+
+@gpu
+@pytest.mark.parametrize("spans", [PROMPTS, SINGLES], ids=["prompts", "singles"])
+@pytest.mark.parametrize("kind", ["options", "table", "one row", "latent"])
+def test_gates_far_below_zero(kind, spans):
+    """sigmoid(-88) is 6e-39 times values of 1e30: a quotient whose divisor is beyond 2^126 must not become zero."""
+    run, plain, pages, seen, rows, ctx, part, bt = made(kind, spans, 6)
+    if kind in ("options", "table"):
+        pages[:, 2:] *= 1.0e30
+    else:
+        pages *= 1.0e30                                      # key and value at once: the queries make up for it
+        part.q = (part.q * 1.0e-30).contiguous()
+    part.gate = torch.full((ctx.num_tokens, 4 if kind == "latent" else 512), -88.0, device="cuda")
+    got = run(pages)
+    if got is None:
+        pytest.skip("single tokens of this kind have a kernel of their own")
+    got, want = got[rows].float(), plain(pages)[rows].float()
+    assert float(want.abs().max()) > 1e-10 and float((got - want).abs().max()) < 3 * 2.0 ** -8 * float(want.abs().max())

@@ -154,15 +154,15 @@ struct SharedArgs {
 
 // n_tiles_dev: null, or the number of tiles another kernel has written (the grid may be larger)
 template <bool SHARED>
-__global__ __launch_bounds__(PTHREADS, 2) void attn_prefill_kernel(const AttnParams p, const int4* __restrict__ tiles,
-                                                                   const int* __restrict__ n_tiles_dev, const SharedArgs sh) {
+__global__ __launch_bounds__(PTHREADS, 2) void attn_prefill_kernel(const AttnParams p, const int4* tiles,
+                                                                   const int* n_tiles_dev, const SharedArgs sh) {
     pdl_trigger();
     pdl_wait();
     // the KV heads of a tile before the next tile (blocks start in the order of their linear index): the
     // tiles with the most keys, of all heads, start first
     const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int tile_idx = SHARED ? (int)blockIdx.x : lin / (int)gridDim.y;
-    if (!SHARED && n_tiles_dev && tile_idx >= *n_tiles_dev) return;
+    if (!SHARED && n_tiles_dev && tile_idx >= load_fresh(n_tiles_dev)) return;
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* sQ = smem;                               // [PM][HD]
     uint8_t* sK = sQ + PM * HD * 2;                   // [2][PN][HD]
@@ -175,7 +175,7 @@ __global__ __launch_bounds__(PTHREADS, 2) void attn_prefill_kernel(const AttnPar
         n_tok = min(per, sh.n_tok - tok0);
         req = p.req_of_token[tok0];
     } else {
-        const int4 t4 = tiles[tile_idx];
+        const int4 t4 = load_fresh(tiles + tile_idx);
         req = t4.x; tok0 = t4.y; n_tok = t4.z;
     }
     const int kvh = SHARED ? (int)blockIdx.y : lin % (int)gridDim.y;
@@ -440,9 +440,9 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
     const int split = blockIdx.x;
     const int hgroups = (p.G + 15) / 16;
     const int kvh = blockIdx.y / hgroups, hg = blockIdx.y - kvh * hgroups;
-    const int n_rows_used = x.n_rows_dev ? *x.n_rows_dev : (int)gridDim.z;
+    const int n_rows_used = x.n_rows_dev ? load_fresh(x.n_rows_dev) : (int)gridDim.z;
     if ((int)blockIdx.z >= n_rows_used) return;
-    const int tok = x.rows ? x.rows[blockIdx.z] : (int)blockIdx.z;     // no list: row i is token i
+    const int tok = x.rows ? load_fresh(x.rows + blockIdx.z) : (int)blockIdx.z;     // no list: row i is token i
     const int pos = p.positions[tok];
     const int req = p.req_of_token[tok];
     const int heads = min(16, p.G - hg * 16);          // valid rows

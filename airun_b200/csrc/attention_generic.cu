@@ -20,8 +20,8 @@
 
 template <typename TQ, typename TKV>
 __global__ __launch_bounds__(32 * ATTN_WARPS) void attention_generic_kernel(
-    const TQ* __restrict__ q, TQ* __restrict__ out,
-    const TKV* __restrict__ pool, const int32_t* __restrict__ block_table, int max_blocks,
+    const TQ* q, TQ* __restrict__ out,
+    const TKV* pool, const int32_t* __restrict__ block_table, int max_blocks,
     const int32_t* __restrict__ positions, const int32_t* __restrict__ req_of_token,
     int num_reqs, int num_pages, int page_size, int nh, int nkv, int hd,
     float scale, int window, int* __restrict__ err) {
@@ -127,7 +127,7 @@ template <int PL> __device__ __forceinline__ LaneVec<PL> lane_load(const float* 
 
 template <int PL, int GH>
 __global__ __launch_bounds__(32 * ROWS_WARPS) void attention_rows_f32_kernel(
-    const float* __restrict__ q, float* __restrict__ out, const float* __restrict__ pool,
+    const float* q, float* __restrict__ out, const float* pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv,
     float scale, int window, int* __restrict__ err) {

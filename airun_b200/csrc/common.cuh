@@ -29,14 +29,18 @@
 // global memory that an earlier kernel writes or reads (the wait returns when the earlier kernels
 // have finished and their writes are visible).  Every kernel calls pdl_trigger() first, which lets
 // the kernel after it become resident as soon as room is free.  What a kernel does before
-// pdl_wait() (shared-memory barriers, tensor-memory allocation, loads of WEIGHTS, which no kernel
-// writes) overlaps the tail of the kernel before it.  AIRUN_PDL=0 in the environment turns it off.
+// pdl_wait() (shared-memory barriers, tensor-memory allocation, loads of WEIGHTS and of the batch's
+// layout, which no kernel of a step writes) overlaps the tail of the kernel before it.  AIRUN_PDL=0 in
+// the environment turns it off.
+//
+// const __restrict__ is for weights and the batch's layout only: it says that nothing writes there while the kernel
+// lives, and a kernel lives from ahead of its wait on, so such loads may be moved ahead of the wait or answered from a
+// line that the L1 cache has kept.  What the kernels of a step write (activations, cache pages, states, lists, counters)
+// is read through plain pointers; results that a kernel does not read may be __restrict__.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// What the kernel in front has written is read through volatile after pdl_wait(): a load through a const __restrict__ pointer
-// counts as the same for the whole kernel, from before the wait on, and may be moved ahead of it or answered from an L1
-// line that another kernel left.
+// Lists and counters of the kernel in front, which say where a kernel reads and writes, are read through volatile as well.
 __device__ __forceinline__ int load_fresh(const int* p) { return *(const volatile int*)p; }
 __device__ __forceinline__ int4 load_fresh(const int4* p) {
     const volatile int* v = (const volatile int*)p;

@@ -22,7 +22,7 @@
 // q_out = proj[:, :q_width] + q_bias in the storage type; keys and values (with their biases) into the
 // token's page.  One block per token.
 template <typename T>
-__global__ void qkv_bias_store_kernel(const float* __restrict__ proj, long long proj_stride,
+__global__ void qkv_bias_store_kernel(const float* proj, long long proj_stride,
                                       const float* __restrict__ q_bias, const float* __restrict__ k_bias,
                                       const float* __restrict__ v_bias, T* __restrict__ q_out, T* __restrict__ pool,
                                       const int32_t* __restrict__ block_table, int max_blocks,
@@ -86,7 +86,7 @@ AIRUN_EXPORT int airun_qkv_bias_store(const float* proj, long long proj_stride, 
 // position and the keys it sees.
 template <typename T>
 __global__ __launch_bounds__(32 * DA_WARPS) void diff_attention_kernel(
-    const T* __restrict__ q, T* __restrict__ out, long long out_stride, const T* __restrict__ pool,
+    const T* q, T* __restrict__ out, long long out_stride, const T* pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv, int D, int Dv,
     float scale, float cap, int chunk, int window, float lambda, float eps, float out_scale, int* __restrict__ err) {

@@ -11,7 +11,7 @@
 #include <type_traits>
 
 template <typename TTab>
-__global__ void embed_kernel(const TTab* __restrict__ table, const int32_t* __restrict__ ids,
+__global__ void embed_kernel(const TTab* __restrict__ table, const int32_t* ids,
                              float* __restrict__ out, int H, int V, float scale, int* __restrict__ err) {
     pdl_trigger();
     pdl_wait();
@@ -62,7 +62,7 @@ AIRUN_EXPORT int airun_embed(const void* table, int table_dtype, const int32_t* 
 // numbers, they took 3.5.
 #define KEEP 4
 template <int VEC>
-__device__ __forceinline__ void load_vec(const float* __restrict__ p, int i, float (&v)[VEC]) {
+__device__ __forceinline__ void load_vec(const float* p, int i, float (&v)[VEC]) {
     if (VEC == 4) {
         const float4 f = reinterpret_cast<const float4*>(p)[i];
         v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
@@ -71,7 +71,7 @@ __device__ __forceinline__ void load_vec(const float* __restrict__ p, int i, flo
     }
 }
 template <typename TOut, int VEC>
-__device__ __forceinline__ void store_vec(TOut* __restrict__ p, int i, const float (&v)[VEC]) {
+__device__ __forceinline__ void store_vec(TOut* p, int i, const float (&v)[VEC]) {
     if (VEC == 4 && sizeof(TOut) == 4) {
         reinterpret_cast<float4*>(p)[i] = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
     } else if (VEC == 4) {
@@ -83,7 +83,7 @@ __device__ __forceinline__ void store_vec(TOut* __restrict__ p, int i, const flo
 }
 
 template <typename TOut, int VEC>
-__global__ __launch_bounds__(VEC == 4 ? 512 : 1024) void rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta,
+__global__ __launch_bounds__(VEC == 4 ? 512 : 1024) void rmsnorm_kernel(float* x, const float* delta,
                                const float* __restrict__ w, TOut* __restrict__ out,
                                const int32_t* __restrict__ rows, int n, float eps, int write_back,
                                const float* __restrict__ w2, TOut* __restrict__ out2) {
@@ -179,7 +179,7 @@ __global__ __launch_bounds__(VEC == 4 ? 512 : 1024) void rmsnorm_kernel(float* _
 // written back and read again (from cache) for the second pass.
 #define RB 8
 template <typename TOut>
-__global__ __launch_bounds__(256) void rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ delta,
+__global__ __launch_bounds__(256) void rmsnorm_rows_kernel(float* x, const float* delta,
                                                            const float* __restrict__ w, TOut* __restrict__ out,
                                                            int n_rows, int n, float eps, int write_back,
                                                            const float* __restrict__ w2, TOut* __restrict__ out2) {
@@ -319,7 +319,7 @@ AIRUN_EXPORT int airun_rmsnorm_pair(float* x, const float* delta, const float* w
 // in: [T][2*I] where blocks of `group` gate columns alternate with blocks of
 // `group` up columns (group == I means plain [gate | up] halves).  out: [T][I].
 template <typename TIn, typename TOut>
-__global__ void swiglu_kernel(const TIn* __restrict__ in, TOut* __restrict__ out,
+__global__ void swiglu_kernel(const TIn* in, TOut* __restrict__ out,
                               long long total, int I, int group) {
     pdl_trigger();
     pdl_wait();
@@ -353,7 +353,7 @@ AIRUN_EXPORT int airun_swiglu(const void* in, int in_dtype, void* out, int out_d
 }
 
 // out[r] = in[rows[r]] for rows of n elements of `elt` bytes (n*elt a multiple of 4).
-__global__ void gather_rows_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+__global__ void gather_rows_kernel(const uint32_t* in, uint32_t* __restrict__ out,
                                    const int32_t* __restrict__ rows, int words) {
     pdl_trigger();
     pdl_wait();
@@ -431,7 +431,7 @@ AIRUN_EXPORT int airun_fill_random(void* out, int out_dtype, long long n, unsign
 
 // x = cap * tanh(x / cap), in place: a soft limit on logits.  The dense Qwen3 head has none (the
 // reference applies no cap, crates/airun-core/src/runtime.rs:2632-2651); a head part may ask for one.
-__global__ void soft_cap_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void soft_cap_kernel(float* x, long long n, float cap) {
     pdl_trigger();
     pdl_wait();
     const long long i = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
@@ -497,7 +497,7 @@ AIRUN_EXPORT int airun_copy_pages(void* pool, int owners, int num_pages, long lo
 // vectors.  `vec` is one row added to every token (a per-pass offset of the residual stream).  With
 // write_back the sum v becomes the new x.  Source row = rows ? rows[r] : r.  The accurate tanhf is used.
 template <typename TOut>
-__global__ void dyt_norm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ vec,
+__global__ void dyt_norm_kernel(float* x, const float* delta, const float* __restrict__ vec,
                                 const float* __restrict__ alpha, const float* __restrict__ w, const float* __restrict__ b,
                                 TOut* __restrict__ out, const int32_t* __restrict__ rows, int n, int write_back) {
     pdl_trigger();
@@ -550,7 +550,7 @@ AIRUN_EXPORT int airun_dyt_norm(float* x, const float* delta, const float* vec, 
 
 // x[t] += delta[t] + vec for every row t (delta and vec may each be absent), and a += b elementwise
 // (vec == nullptr, delta = b): the plain forms of adds that norms otherwise carry out on the way.
-__global__ void add_rows_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ vec,
+__global__ void add_rows_kernel(float* x, const float* delta, const float* __restrict__ vec,
                                 long long total, int n) {
     pdl_trigger();
     pdl_wait();
@@ -574,7 +574,7 @@ AIRUN_EXPORT int airun_add_rows(float* x, const float* delta, const float* vec, 
 // out = g * sigmoid(slope * g) * (u + 1).  Gate and up columns alternate in blocks of `group` (as for
 // SwiGLU above); the output rows may be strided (a slice of a wider activation buffer).
 template <typename TIn, typename TOut>
-__global__ void glu_clamped_kernel(const TIn* __restrict__ in, TOut* __restrict__ out, long long total, int I, int group,
+__global__ void glu_clamped_kernel(const TIn* in, TOut* __restrict__ out, long long total, int I, int group,
                                    long long out_stride, float limit, float slope) {
     pdl_trigger();
     pdl_wait();
@@ -611,7 +611,7 @@ AIRUN_EXPORT int airun_glu_clamped(const void* in, int in_dtype, void* out, int 
 // kernel writes, ahead of the wait for the kernel in front), stay in registers between the two passes.  2026 rows
 // and 3 rows of 2048, 12 calls each: 122 us; one number a load, with x read and written in turn after the sum, 228 us.
 template <typename TCast, int VEC>
-__global__ __launch_bounds__(256) void postnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y,
+__global__ __launch_bounds__(256) void postnorm_add_kernel(float* x, const float* y,
                                                            const float* __restrict__ w, TCast* __restrict__ cast,
                                                            int n, float eps, float mult) {
     pdl_trigger();
@@ -709,15 +709,15 @@ __device__ __forceinline__ void sandwich_put(TOut* __restrict__ out, int i, int 
 
 // PAIR: two results join at once, x + mult * (y / rms(y) * w_post + y2 / rms(y2) * w_post2); without it mult is not read.
 template <typename TOut, int VEC, bool PAIR>
-__global__ __launch_bounds__(512) void sandwich_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w_post,
-                                     const float* __restrict__ y2, const float* __restrict__ w_post2, float mult,
+__global__ __launch_bounds__(512) void sandwich_norm_kernel(float* x, const float* y, const float* __restrict__ w_post,
+                                     const float* y2, const float* __restrict__ w_post2, float mult,
                                      const float* __restrict__ w_pre, TOut* __restrict__ out, const int32_t* __restrict__ rows,
                                      int n, float eps_post, float eps_pre, int write_back, int mode) {
     pdl_trigger();
     __shared__ float red[33];
     const int nv = n / VEC;
     float v[KEEP][VEC], yk[KEEP][VEC], wa[KEEP][VEC], wb[KEEP][VEC];
-    auto load = [&](const float* __restrict__ p, float (&d)[VEC], int i, float none) {
+    auto load = [&](const float* p, float (&d)[VEC], int i, float none) {
         if (!p || i >= nv) {
 #pragma unroll
             for (int e = 0; e < VEC; ++e) d[e] = none;
@@ -852,7 +852,7 @@ AIRUN_EXPORT int airun_sandwich_norm(float* x, const float* y, const float* w_po
 
 // out = in in another type (float32 -> bfloat16 or a plain copy), n elements.
 template <typename TOut>
-__global__ void cast_kernel(const float* __restrict__ in, TOut* __restrict__ out, long long n) {
+__global__ void cast_kernel(const float* in, TOut* __restrict__ out, long long n) {
     pdl_trigger();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -881,7 +881,7 @@ __device__ __forceinline__ float unit_act(float z, int mode) {
 }
 
 template <typename TOut>
-__global__ void act_kernel(const float* __restrict__ in, TOut* __restrict__ out, long long total, int n, long long out_stride,
+__global__ void act_kernel(const float* in, TOut* __restrict__ out, long long total, int n, long long out_stride,
                            int mode) {
     pdl_trigger();
     pdl_wait();
@@ -908,9 +908,9 @@ AIRUN_EXPORT int airun_act(const float* in, void* out, int out_dtype, int T, int
 //   out = s1 * sigmoid(g1 + c1) * y1 [+ s2 * sigmoid(g2 + c2) * y2]
 // y: a sub-layer's result [T][n], g: its gate's product [T][gate stride] (a column slice of a wider buffer is fine), c:
 // the gate's bias [n], s: the sub-layer's scale per channel [n]; gates and scales may each be absent (null).  All float32.
-__global__ void gated_sum_kernel(const float* __restrict__ y1, const float* __restrict__ g1, long long g1_stride,
-                                 const float* __restrict__ c1, const float* __restrict__ s1, const float* __restrict__ y2,
-                                 const float* __restrict__ g2, long long g2_stride, const float* __restrict__ c2,
+__global__ void gated_sum_kernel(const float* y1, const float* g1, long long g1_stride,
+                                 const float* __restrict__ c1, const float* __restrict__ s1, const float* y2,
+                                 const float* g2, long long g2_stride, const float* __restrict__ c2,
                                  const float* __restrict__ s2, float* __restrict__ out, long long total, int n) {
     pdl_trigger();
     pdl_wait();
@@ -944,7 +944,7 @@ AIRUN_EXPORT int airun_gated_sum(const float* y1, const float* g1, long long g1_
 }
 
 // x *= factor, in place (a head whose logits carry a fixed factor).
-__global__ void scale_kernel(float* __restrict__ x, long long n, float factor) {
+__global__ void scale_kernel(float* x, long long n, float factor) {
     pdl_trigger();
     pdl_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -28,7 +28,7 @@ struct GemmExtra {
 
 template <typename TA, typename TW, typename TC, int FORM>      // FORM 0 plain, 1 batched, 2 grouped
 __global__ __launch_bounds__(256) void gemm_simt_kernel(
-    const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C,
+    const TA* A, const TW* __restrict__ W, TC* __restrict__ C,
     int M, int N, int K, long long lda, long long ldw, long long ldc, GemmExtra ex) {
     pdl_trigger();
     pdl_wait();
@@ -138,7 +138,7 @@ template <int NV> __device__ __forceinline__ int halving_sum(float (&v)[NV], int
 // are formed in a fixed order (lanes by halving, then warps in turn).
 template <int MR, int NC, int FORM>
 __global__ __launch_bounds__(32 * GV_WARPS) void gemv_f32_kernel(
-    const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+    const float* A, const float* __restrict__ W, float* __restrict__ C,
     int M, int N, int K, long long lda, long long ldw, long long ldc, GemmExtra ex) {
     pdl_trigger();
     __shared__ float red[GV_WARPS][MR * NC];
@@ -218,7 +218,7 @@ __device__ __forceinline__ void f32_cp16(float* smem, const float* gmem, bool on
 }
 template <int FORM>
 __global__ __launch_bounds__(256, 2) void gemm_f32_kernel(
-    const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+    const float* A, const float* __restrict__ W, float* __restrict__ C,
     int M, int N, int K, long long lda, long long ldw, long long ldc, GemmExtra ex) {
     pdl_trigger();
     pdl_wait();

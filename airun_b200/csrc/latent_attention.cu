@@ -31,7 +31,7 @@ __device__ __forceinline__ void lat_angles(LatAngles& a, int rot_dims, const flo
 
 // Piece i (two elements) of a rotated part: i < rot_dims / 2 is a rotated pair, the pieces behind them pass unchanged.
 template <typename TC>
-__device__ __forceinline__ void lat_put_piece(const LatAngles& a, const float* __restrict__ src, TC* __restrict__ dst, int i, int rd,
+__device__ __forceinline__ void lat_put_piece(const LatAngles& a, const float* src, TC* __restrict__ dst, int i, int rd,
                                               int rot_dims, int rope_kind) {
     if (i < rot_dims / 2) {
         const int e0 = rope_kind == LAT_ROPE_NEOX ? i : 2 * i, e1 = rope_kind == LAT_ROPE_NEOX ? i + rot_dims / 2 : 2 * i + 1;
@@ -47,7 +47,7 @@ __device__ __forceinline__ void lat_put_piece(const LatAngles& a, const float* _
 // One token's queries, q [H][D + rd] float32: the unrotated parts into qn [H][D], the rotated parts, turned, behind the
 // first R elements of qlat's rows [H][R + rd] (which the product with Wuk^T fills).
 template <typename TC>
-__device__ __forceinline__ void lat_put_query(const LatAngles& a, const float* __restrict__ q, TC* __restrict__ qn, TC* __restrict__ qlat,
+__device__ __forceinline__ void lat_put_query(const LatAngles& a, const float* q, TC* __restrict__ qn, TC* qlat,
                                               int H, int D, int R, int rd, int rot_dims, int rope_kind) {
     if (((D | rd) & 3) == 0 && (((uintptr_t)q | (uintptr_t)qn) & 15) == 0) {
         const int per = D >> 2;
@@ -74,7 +74,7 @@ __device__ __forceinline__ void lat_put_query(const LatAngles& a, const float* _
 
 // One token's cached row: c / rms(c) * wkv, then the rotated key part (kr lies behind c).
 template <typename TC>
-__device__ __forceinline__ void lat_put_row(const LatAngles& a, const float* __restrict__ c, const float* __restrict__ wkv, float eps,
+__device__ __forceinline__ void lat_put_row(const LatAngles& a, const float* c, const float* __restrict__ wkv, float eps,
                                             TC* __restrict__ dst, int R, int rd, int rot_dims, int rope_kind, float* red) {
     float ss = 0.0f;
     for (int i = threadIdx.x; i < R; i += blockDim.x) ss = fmaf(c[i], c[i], ss);
@@ -101,7 +101,7 @@ __device__ __forceinline__ TC* lat_slot(TC* pool, const int32_t* __restrict__ bl
 // `store`.  cq = dq / rms(dq) * wq in the compute type; the cache row = [dkv / rms(dkv) * wkv | rotate(kr)].
 template <typename TC>
 __global__ __launch_bounds__(256) void latent_prepare_kernel(
-    const float* __restrict__ proj, long long stride, const float* __restrict__ wq, const float* __restrict__ wkv, float eps,
+    const float* proj, long long stride, const float* __restrict__ wq, const float* __restrict__ wkv, float eps,
     TC* __restrict__ cq, int q_rank, int R, int rd, int rot_dims, int rope_kind, const float* __restrict__ inv_freq, float rot_mult,
     TC* __restrict__ pool, const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int store, int* __restrict__ err) {
@@ -151,7 +151,7 @@ AIRUN_EXPORT int airun_latent_prepare(const float* proj, long long stride, const
 // heads' queries, and the token's cache row is written in the same pass (a query without a low-rank product of its own).
 template <typename TC>
 __global__ __launch_bounds__(256) void latent_query_kernel(
-    const float* __restrict__ q, long long q_stride, TC* __restrict__ qn, TC* __restrict__ qlat, int H, int D, int R, int rd, int rot_dims,
+    const float* q, long long q_stride, TC* __restrict__ qn, TC* qlat, int H, int D, int R, int rd, int rot_dims,
     int rope_kind, const float* __restrict__ inv_freq, float rot_mult, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, const float* __restrict__ wkv, float eps, TC* __restrict__ pool,
     const int32_t* __restrict__ block_table, int max_blocks, int num_reqs, int num_pages, int page_size, int* __restrict__ err) {
@@ -199,9 +199,9 @@ AIRUN_EXPORT int airun_latent_query(const float* q, long long q_stride, void* qn
 #define LAT_PER_LANE 20      // R + rd <= 640
 template <typename TC>
 __global__ __launch_bounds__(32 * LAT_WARPS) void latent_attention_kernel(
-    const TC* __restrict__ qlat, TC* __restrict__ out, const TC* __restrict__ pool, const int32_t* __restrict__ block_table,
+    const TC* qlat, TC* __restrict__ out, const TC* pool, const int32_t* __restrict__ block_table,
     int max_blocks, const int32_t* __restrict__ positions, const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages,
-    int page_size, int H, int R, int rd, float scale, int window, const float* __restrict__ sink, const float* __restrict__ gate,
+    int page_size, int H, int R, int rd, float scale, int window, const float* __restrict__ sink, const float* gate,
     long long gate_stride, int* __restrict__ err) {
     pdl_trigger();
     pdl_wait();

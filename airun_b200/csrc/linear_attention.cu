@@ -28,7 +28,7 @@
 #define LOWRANK_EXP_NEG_EXP 3
 #define DECAY_TOKENS 8        // tokens of one block: a row of w2 is read once for all of them
 template <typename TW>
-__global__ __launch_bounds__(128) void decay_kernel(const float* __restrict__ low, long long low_stride, const TW* __restrict__ w2,
+__global__ __launch_bounds__(128) void decay_kernel(const float* low, long long low_stride, const TW* __restrict__ w2,
                                                     const float* __restrict__ bias, float* __restrict__ out, int T, int n, int rank,
                                                     float inv_tau, const int32_t* __restrict__ req_of_token,
                                                     int mode, int in_tanh, const float* __restrict__ group_param, int group) {
@@ -136,8 +136,8 @@ __device__ __forceinline__ bool gla_find_segment(const int32_t* cu_tokens, int n
 }
 template <int NS, bool CONST, bool SEG>
 __global__ __launch_bounds__(256) void gla_recurrent_kernel(
-    const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, long long row_stride,
-    const float* __restrict__ decay, float* __restrict__ state, long long slot_stride,
+    const float* q, const float* k, const float* v, long long row_stride,
+    const float* decay, float* state, long long slot_stride,
     const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int max_slots,
     float* __restrict__ out, int heads, int D, int Dv, float q_scale, int* __restrict__ err,
     const float* __restrict__ head_decay, int in_silu, int num_reqs, GlaSegments segs) {
@@ -276,8 +276,8 @@ __global__ __launch_bounds__(256) void gla_recurrent_kernel(
 // output, 8 tokens x 4 columns a thread.  Only products of decays occur, never quotients, so a decay near zero only wipes.
 template <bool CONST>
 __global__ __launch_bounds__(256) void gla_segment_kernel(
-    const float* __restrict__ q, long long row_stride, const float* __restrict__ decay, float* __restrict__ state, long long slot_stride,
-    const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int max_slots, float* __restrict__ out, int heads,
+    const float* q, long long row_stride, const float* decay, float* state, long long slot_stride,
+    const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int max_slots, float* out, int heads,
     int D, int Dv, float q_scale, const float* __restrict__ head_decay, int in_silu, int num_reqs, GlaSegments segs) {
     pdl_trigger();
     pdl_wait();
@@ -448,7 +448,7 @@ AIRUN_EXPORT int airun_decay_recurrent(const float* q, const float* k, const flo
 // out[t][c] = scale * o[t][c] / sqrt(mean_c o[t]^2 + eps) * w[c] * sigmoid(gate[t][c]) over a token's whole row of n
 // numbers (all heads at once); one block per token.  o is float32 [T][n], gate float32 rows of `gate_stride`.
 template <typename TOut>
-__global__ __launch_bounds__(256) void rownorm_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate,
+__global__ __launch_bounds__(256) void rownorm_gate_kernel(const float* o, const float* gate,
                                                            long long gate_stride, const float* __restrict__ w,
                                                            TOut* __restrict__ out, long long out_stride, int n, float eps,
                                                            float scale, const int32_t* __restrict__ req_of_token) {
@@ -484,7 +484,7 @@ AIRUN_EXPORT int airun_rownorm_gate(const float* o, const float* gate, long long
 
 // out[t][h][j] = o[t][h][j] / sqrt(mean_j o^2 + eps) * w[j] * silu(gate[t][h][j]); one warp per (token, head).
 template <typename TOut>
-__global__ __launch_bounds__(128) void out_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate,
+__global__ __launch_bounds__(128) void out_gate_kernel(const float* o, const float* gate,
                                                        long long gate_stride, const float* __restrict__ w,
                                                        TOut* __restrict__ out, long long out_stride, int T, int heads,
                                                        int Dv, float eps, const int32_t* __restrict__ req_of_token,

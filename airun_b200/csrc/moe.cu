@@ -41,7 +41,7 @@ struct MoeChoices {
 };
 
 // A block that holds all tokens of the step counts in shared memory and writes the segments itself: 32 threads scan.
-__device__ __forceinline__ void moe_segments(const int32_t* s_counts, int32_t* __restrict__ counts, int32_t* __restrict__ seg, int E) {
+__device__ __forceinline__ void moe_segments(const int32_t* s_counts, int32_t* counts, int32_t* __restrict__ seg, int E) {
     const int lane = threadIdx.x & 31;
     int before = 0;
     if (lane == 0) seg[0] = 0;
@@ -58,7 +58,7 @@ __device__ __forceinline__ void moe_segments(const int32_t* s_counts, int32_t* _
     }
 }
 
-__device__ __forceinline__ void moe_route_token(const float* __restrict__ z, const float* __restrict__ bias, int E, int top,
+__device__ __forceinline__ void moe_route_token(const float* z, const float* __restrict__ bias, int E, int top,
                                                 int softmax_scores, int renorm, bool padding, float* s_score, MoeChoices chosen) {
     const int lane = chosen.lane;
     if (padding) {
@@ -105,9 +105,9 @@ __device__ __forceinline__ void moe_route_token(const float* __restrict__ z, con
 // ONE: a single block, which counts in shared memory and writes `counts` and `seg` when it is done.
 template <bool ONE>
 __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_kernel(
-    const float* __restrict__ z, long long z_stride, const float* __restrict__ bias, int T, int E, int top, int softmax_scores, int renorm,
-    const int32_t* __restrict__ req_of_token, int32_t* __restrict__ ids, float* __restrict__ wts, int32_t* __restrict__ rank,
-    int32_t* __restrict__ counts, int32_t* __restrict__ seg) {
+    const float* z, long long z_stride, const float* __restrict__ bias, int T, int E, int top, int softmax_scores, int renorm,
+    const int32_t* __restrict__ req_of_token, int32_t* ids, float* wts, int32_t* rank,
+    int32_t* counts, int32_t* __restrict__ seg) {
     pdl_trigger();
     if (bias) prefetch_l2(bias, E);
     pdl_wait();
@@ -141,7 +141,7 @@ __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_kernel(
 // Sigmoid scores without a correction are ranked by their logits: the order is the same, and scores that round to 1 are
 // still told apart.
 // Only experts with matrices are counted into segments.
-__device__ __forceinline__ void moe_route_grouped_token(const float* __restrict__ z, const float* __restrict__ correction, int n_out, int top,
+__device__ __forceinline__ void moe_route_grouped_token(const float* z, const float* __restrict__ correction, int n_out, int top,
                                                         int groups, int keep, int sigmoid_scores, int group_best, int renorm,
                                                         float weight_scale, bool padding, float* s_score, MoeChoices chosen) {
     const int lane = chosen.lane;
@@ -228,9 +228,9 @@ __device__ __forceinline__ void moe_route_grouped_token(const float* __restrict_
 // One warp per token, `ONE` as above.
 template <bool ONE>
 __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_grouped_kernel(
-    const float* __restrict__ z, long long z_stride, const float* __restrict__ correction, int T, int n_out, int num_real, int top,
+    const float* z, long long z_stride, const float* __restrict__ correction, int T, int n_out, int num_real, int top,
     int groups, int keep, int sigmoid_scores, int group_best, int renorm, float weight_scale, const int32_t* __restrict__ req_of_token,
-    int32_t* __restrict__ ids, float* __restrict__ wts, int32_t* __restrict__ rank, int32_t* __restrict__ counts, int32_t* __restrict__ seg) {
+    int32_t* ids, float* wts, int32_t* rank, int32_t* counts, int32_t* __restrict__ seg) {
     pdl_trigger();
     if (correction) prefetch_l2(correction, n_out);
     pdl_wait();
@@ -252,13 +252,13 @@ __global__ __launch_bounds__(ONE ? 1024 : 128) void moe_route_grouped_kernel(
     }
 }
 
-__global__ void moe_zero_kernel(int32_t* __restrict__ counts, int E) {
+__global__ void moe_zero_kernel(int32_t* counts, int E) {
     pdl_trigger();
     pdl_wait();
     for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
 }
 
-__global__ void moe_offsets_kernel(const int32_t* __restrict__ counts, int32_t* __restrict__ seg, int E) {
+__global__ void moe_offsets_kernel(const int32_t* counts, int32_t* __restrict__ seg, int E) {
     pdl_trigger();
     pdl_wait();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -271,8 +271,8 @@ __global__ void moe_offsets_kernel(const int32_t* __restrict__ counts, int32_t* 
 // One block per (token, choice); rows without a weight on them are copied sixteen bytes at a time (`vec`).
 template <typename TH>
 __global__ __launch_bounds__(256) void moe_scatter_kernel(
-    const TH* __restrict__ h, int W, int top, const int32_t* __restrict__ ids, const float* __restrict__ wts,
-    const int32_t* __restrict__ rank, const int32_t* __restrict__ seg, int scale_input, TH* __restrict__ xs,
+    const TH* h, int W, int top, const int32_t* ids, const float* wts,
+    const int32_t* rank, const int32_t* seg, int scale_input, TH* __restrict__ xs,
     int32_t* __restrict__ row_of, int num_real, int vec) {
     pdl_trigger();
     pdl_wait();
@@ -300,8 +300,8 @@ __global__ __launch_bounds__(256) void moe_scatter_kernel(
 // VEC columns a thread (four on 16-byte boundaries), blockIdx.y picks a token's run of columns.
 template <typename TH, int VEC>
 __global__ __launch_bounds__(256) void moe_combine_kernel(
-    const float* __restrict__ ys, int W, int top, const int32_t* __restrict__ ids, const float* __restrict__ wts,
-    const int32_t* __restrict__ row_of, int scale_output, float* __restrict__ out, const TH* __restrict__ h) {
+    const float* ys, int W, int top, const int32_t* ids, const float* wts,
+    const int32_t* row_of, int scale_output, float* __restrict__ out, const TH* h) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;

@@ -31,11 +31,11 @@
 // DPL: values of a head per lane, ceil(head_dim / 32) rounded up to 1, 2, 4 or 8.
 template <typename TQ, typename TKV, int DPL>
 __global__ __launch_bounds__(256) void qkv_post_kernel(
-    const float* __restrict__ qkv, long long ld_qkv,
+    const float* qkv, long long ld_qkv,
     TQ* __restrict__ q_out,
     const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps,
     const int32_t* __restrict__ positions, const int32_t* __restrict__ req_of_token,
-    int rope_kind, int rotary_dim, const float* __restrict__ inv_freq, const int32_t* __restrict__ rope_positions,
+    int rope_kind, int rotary_dim, const float* __restrict__ inv_freq, const int32_t* rope_positions,
     TKV* __restrict__ pool, const int32_t* __restrict__ block_table, int max_blocks,
     int num_reqs, int num_pages, int page_size, int do_store, int kv_from_qkv,
     int nh, int nkv, int hd, int* __restrict__ err) {
@@ -143,7 +143,7 @@ __global__ __launch_bounds__(256) void qkv_post_kernel(
 // shared memory.  Same arithmetic, in the same order, as the kernel above.
 template <typename TQ, typename TKV>
 __global__ __launch_bounds__(256) void qkv_post_hd128_kernel(
-    const float* __restrict__ qkv, long long ld_qkv,
+    const float* qkv, long long ld_qkv,
     TQ* __restrict__ q_out,
     const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps,
     const int32_t* __restrict__ positions, const int32_t* __restrict__ req_of_token,

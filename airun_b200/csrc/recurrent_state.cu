@@ -25,8 +25,8 @@
 // rows before the request's first row of this step come from tail[slot][taps-1][C] (the inputs that ended the
 // step before; zero at the start of a request).  One block per token.
 __global__ __launch_bounds__(256) void short_conv_kernel(
-    const float* __restrict__ in, long long in_stride, const float* __restrict__ w, int taps,
-    const float* __restrict__ state, long long slot_stride, long long tail_off, int max_slots,
+    const float* in, long long in_stride, const float* __restrict__ w, int taps,
+    const float* state, long long slot_stride, long long tail_off, int max_slots,
     const int32_t* __restrict__ req_of_token, const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots,
     int num_reqs, float* __restrict__ out, int C, int n_unit_heads, int q_heads, int unit_dim, float unit_eps,
     float q_scale, int* __restrict__ err) {
@@ -68,7 +68,7 @@ __global__ __launch_bounds__(256) void short_conv_kernel(
 // weights, which no kernel writes, before the kernel in front has finished.
 template <int TAPS, int NV, int TOK>
 __global__ __launch_bounds__(128) void short_conv_rows_kernel(
-    const float* __restrict__ in, long long in_stride, const float* __restrict__ w, const float* __restrict__ state,
+    const float* in, long long in_stride, const float* __restrict__ w, const float* state,
     long long slot_stride, long long tail_off, int max_slots, const int32_t* __restrict__ req_of_token,
     const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int num_reqs, float* __restrict__ out, int T,
     int C, int n_unit_heads, int q_heads, int unit_dim, float unit_eps, float q_scale, int* __restrict__ err) {
@@ -176,7 +176,7 @@ AIRUN_EXPORT int airun_short_conv(const float* in, long long in_stride, const fl
 // for the first row a request brings in this step, the row its state keeps (zero at the start of a request).
 template <typename TOut>
 __global__ __launch_bounds__(256) void token_shift_kernel(
-    const float* __restrict__ x, const float* __restrict__ mu, int n_mix, const float* __restrict__ state,
+    const float* x, const float* __restrict__ mu, int n_mix, const float* state,
     long long slot_stride, long long prev_off, int max_slots, const int32_t* __restrict__ req_of_token,
     const int32_t* __restrict__ cu_tokens, const int32_t* __restrict__ state_slots, int num_reqs, TOut* __restrict__ out,
     int T, int W, int* __restrict__ err) {
@@ -852,7 +852,7 @@ __device__ __forceinline__ float2 rs_unpack(rs_pair v) {
 // one request of 2048 tokens took 374 us instead of 232.
 // CHUNK_CHANNEL, CHUNK_MIX: over the vectors of chunk_vectors_kernel, whose decays are theirs already.
 template <int NS, int KIND, int DG, int MINB>
-__global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArgs a, const float* __restrict__ coef, ChunkVectors vec) {
+__global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArgs a, const float* coef, ChunkVectors vec) {
     pdl_trigger();
     pdl_wait();
     constexpr bool VECS = KIND != CHUNK_HEAD, MIX = KIND == CHUNK_MIX;

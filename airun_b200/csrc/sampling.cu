@@ -56,7 +56,7 @@ __device__ BestPair block_best(BestPair p, BestPair* sh) {
 // (crates/airun-cuda/kernels/ops.cu:118-149: 128 partial blocks, then one final block).
 #define ARGMAX_CHUNKS 64
 __global__ __launch_bounds__(256) void argmax_partial_kernel(
-    const float* __restrict__ logits, long long ld, int V, BestPair* __restrict__ partial) {
+    const float* logits, long long ld, int V, BestPair* __restrict__ partial) {
     pdl_trigger();
     pdl_wait();
     __shared__ BestPair sh_best[33];
@@ -74,9 +74,9 @@ __global__ __launch_bounds__(256) void argmax_partial_kernel(
 }
 
 __global__ __launch_bounds__(SAMPLE_THREADS) void sample_kernel(
-    const float* __restrict__ logits, long long ld, int V,
+    const float* logits, long long ld, int V,
     const float* __restrict__ temperature, const float* __restrict__ uniform,
-    int32_t* __restrict__ out, const BestPair* __restrict__ partial) {
+    int32_t* __restrict__ out, const BestPair* partial) {
     pdl_trigger();
     pdl_wait();
     __shared__ BestPair sh_best[33];
@@ -178,7 +178,7 @@ __device__ __forceinline__ unsigned long long cand_key(float v, int id) {
 }
 
 __global__ __launch_bounds__(CAND_THREADS) void largest_logits_kernel(
-    const float* __restrict__ logits, long long ld, int V, const int32_t* __restrict__ rows, int n_cand,
+    const float* logits, long long ld, int V, const int32_t* __restrict__ rows, int n_cand,
     int32_t* __restrict__ out_ids, float* __restrict__ out_vals, int32_t* __restrict__ out_flags) {
     pdl_trigger();
     extern __shared__ unsigned long long s_keys[];               // CAND_THREADS * CAND_PER_THREAD

@@ -32,7 +32,7 @@ __device__ __forceinline__ void sa_store4(__nv_bfloat16* dst, float4 v) {
 // registers across the two sums and writes four results at a time; otherwise it goes number by number.
 template <typename T>
 __global__ __launch_bounds__(256) void qk_rownorm_store_kernel(
-    const float* __restrict__ proj, long long proj_stride, const float* __restrict__ q_w, const float* __restrict__ k_w,
+    const float* proj, long long proj_stride, const float* __restrict__ q_w, const float* __restrict__ k_w,
     float eps, float temp_coef, int temp_every, T* __restrict__ q_out, T* __restrict__ pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int q_width, int nkv, int kd, int vd,
@@ -165,7 +165,7 @@ AIRUN_EXPORT int airun_qk_rownorm_store(const float* proj, long long proj_stride
 // its position and the keys it sees.
 template <typename T>
 __global__ __launch_bounds__(32 * SA_WARPS) void sigmoid_attention_kernel(
-    const T* __restrict__ q, T* __restrict__ out, long long out_stride, const T* __restrict__ pool,
+    const T* q, T* __restrict__ out, long long out_stride, const T* pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv, int D, int Dv,
     float scale, const float* __restrict__ dist_a, const float* __restrict__ dist_b, const float* __restrict__ head_c,

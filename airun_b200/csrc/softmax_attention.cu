@@ -42,9 +42,9 @@ __device__ __forceinline__ void xa_store4(__nv_bfloat16* dst, float4 v) {
 // the values.  proj is float32 [T][nh*D (+ nkv*D + nkv*Dv when store)], bias the same columns (or null).
 template <typename T>
 __global__ __launch_bounds__(32 * XA_PREP_WARPS) void qkv_prepare_kernel(
-    const float* __restrict__ proj, long long proj_stride, const float* __restrict__ bias, const float* __restrict__ q_w,
+    const float* proj, long long proj_stride, const float* __restrict__ bias, const float* __restrict__ q_w,
     const float* __restrict__ k_w, int whole_norm, int unit_norm, float eps, int rope_kind, int rdim, const float* __restrict__ inv_freq,
-    const int32_t* __restrict__ rope_positions, float temp_coef, int temp_every, T* __restrict__ q_out, T* __restrict__ pool,
+    const int32_t* rope_positions, float temp_coef, int temp_every, T* __restrict__ q_out, T* __restrict__ pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv, int D, int Dv,
     int store, int one_row, int* __restrict__ err) {
@@ -335,11 +335,11 @@ AIRUN_EXPORT int airun_qkv_prepare(const float* proj, long long proj_stride, con
 // the denominator there.  A token's result depends only on its own q, its position and the keys it sees.
 template <typename T>
 __global__ __launch_bounds__(32 * XA_WARPS) void softmax_attention_kernel(
-    const T* __restrict__ q, T* __restrict__ out, long long out_stride, const T* __restrict__ pool,
+    const T* q, T* __restrict__ out, long long out_stride, const T* pool,
     const int32_t* __restrict__ block_table, int max_blocks, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ req_of_token, int num_reqs, int num_pages, int page_size, int nh, int nkv, int D, int Dv,
     float scale, const float* __restrict__ table, int table_len, const float* __restrict__ sink, int window, float out_scale,
-    int tail, const float* __restrict__ gate, long long gate_stride, int* __restrict__ err) {
+    int tail, const float* gate, long long gate_stride, int* __restrict__ err) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ float s_acc[];           // [XA_WARPS][Dv], then [XA_WARPS] maxima and [XA_WARPS] sums

@@ -18,8 +18,8 @@
 // SMAX: the most streams this instance takes (4 or SMAX); the loops over streams are unrolled to it.
 template <typename TOut, int SMAX>
 __global__ __launch_bounds__(256) void stream_step_kernel(
-    float* __restrict__ xs, int S, int H, const float* __restrict__ y, long long y_stride, const float* __restrict__ y_bias,
-    const float* __restrict__ carry, const float* __restrict__ write, float mult, const float* __restrict__ read,
+    float* xs, int S, int H, const float* y, long long y_stride, const float* __restrict__ y_bias,
+    const float* carry, const float* write, float mult, const float* read,
     const float* __restrict__ norm_w, float eps, TOut* __restrict__ out, long long out_stride,
     const int32_t* __restrict__ req_of_token) {
     pdl_trigger();
@@ -127,7 +127,7 @@ __global__ __launch_bounds__(256) void stream_step_kernel(
 }
 
 // xs[t][s] = x[t] for every stream s.
-__global__ void stream_fill_kernel(const float* __restrict__ x, float* __restrict__ xs, long long total, int S, int H) {
+__global__ void stream_fill_kernel(const float* x, float* xs, long long total, int S, int H) {
     pdl_trigger();
     pdl_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

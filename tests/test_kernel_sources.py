@@ -21,3 +21,40 @@ def test_work_lists_are_read_fresh():
             assert re.search(r"(const )?(int|int32_t|int4|void)\s*$", before), (name, text[use.start() - 60:use.end() + 20])
         readers += len(re.findall(r"load_fresh\(", text))
     assert readers >= 8
+
+
+# what no kernel of a step writes: weights and constants of the model, the batch's layout and lists that are copied to the device
+# ahead of the step, sampling parameters
+UNWRITTEN = set("""W alpha b bias c1 c2 s1 s2 correction dist_a dist_b group_param head_c head_decay inv_freq k_bias q_bias v_bias k_norm_w
+q_norm_w k_w q_w mu norm_w sink table vec w w2 w_post w_post2 w_pre wkv wq y_bias
+block_table context_lens cu_tokens positions req_of_token rows state_slots pairs temperature uniform""".split())
+# results that their kernel does not read, or reads only what it has written itself
+WRITTEN_ONLY = set("""C cast coef counts cq dst err out out2 out_flags out_ids out_vals partial pool q_out qlat qn row_of rows seg tiles xs""".split())
+
+
+def test_what_a_step_writes_is_not_read_as_unchanging():
+    """Every __restrict__ parameter in front of a wait is one that nothing writes, or one that is not read."""
+    seen = 0
+    for name, text in SOURCES.items():
+        for m in re.finditer(r"(const\s+)?\w+\s*\*\s*__restrict__\s+(\w+)", text):
+            seen += 1
+            assert m.group(2) in (UNWRITTEN if m.group(1) else WRITTEN_ONLY), (name, m.group(0))
+        # a cached load by name counts as unchanging too
+        for m in re.finditer(r"__ldg\((?:reinterpret_cast<const \w+\*>\()?([\w.]+)", text):
+            assert m.group(1).split(".")[-1] in UNWRITTEN | {"bt", "wr", "src"}, (name, m.group(0))
+    assert seen > 100
+    head = SOURCES["linear_attention.cu"].split("gla_segment_kernel(")[1].split("{")[0]
+    assert re.search(r"float\*\s+out\b", head)                       # this one adds to what is there
+
+
+def test_kernels_wait_before_they_end_and_trigger_first():
+    """A kernel that is launched early and never waits would let the kernel behind it start over unfinished work."""
+    for name, text in SOURCES.items():
+        launched = set(re.findall(r"airun_launch(?:_cluster)?\(\(*(\w+?)(?:<|,)", text))
+        for k in launched - {"kern", "KERNEL"}:
+            at = re.search(r"__global__[^;{]*?\b%s\s*\(" % k, text)
+            if at is None:
+                continue
+            end = text.find("__global__", at.end())
+            body = text[at.end():end if end > 0 else len(text)]
+            assert "pdl_wait()" in body and "pdl_trigger()" in body and body.index("pdl_trigger()") < body.index("pdl_wait()"), (name, k)

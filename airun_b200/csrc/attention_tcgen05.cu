@@ -1214,10 +1214,10 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 #pragma unroll
                         for (int i = 0; i < 8; i += 4) {
                             const float4 g4 = *reinterpret_cast<const float4*>(gate + c + q8 * 8 + i);
-                            o[q8 * 8 + i] /= 1.0f + __expf(-g4.x);
-                            o[q8 * 8 + i + 1] /= 1.0f + __expf(-g4.y);
-                            o[q8 * 8 + i + 2] /= 1.0f + __expf(-g4.z);
-                            o[q8 * 8 + i + 3] /= 1.0f + __expf(-g4.w);
+                            o[q8 * 8 + i] = quotient(o[q8 * 8 + i], 1.0f + __expf(-g4.x));
+                            o[q8 * 8 + i + 1] = quotient(o[q8 * 8 + i + 1], 1.0f + __expf(-g4.y));
+                            o[q8 * 8 + i + 2] = quotient(o[q8 * 8 + i + 2], 1.0f + __expf(-g4.z));
+                            o[q8 * 8 + i + 3] = quotient(o[q8 * 8 + i + 3], 1.0f + __expf(-g4.w));
                         }
                     }
 #pragma unroll

@@ -165,15 +165,15 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return d;
 }
 
-// (the true division: the fast one gives 0 for divisors beyond 2^126, and two units of the last place elsewhere)
-__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + __expf(-g)) * u; }
+// (not the fast division: that gives 0 for divisors beyond 2^126, and two units of the last place elsewhere)
+__device__ __forceinline__ float silu_mul(float g, float u) { return quotient(g, 1.0f + __expf(-g)) * u; }
 // The gated unit of the epilogue.  limit == 0: SwiGLU, silu(g) * u.  limit > 0: the clamped unit,
 // g' = min(g, limit), u' = clamp(u, -limit, limit), g' * sigmoid(slope * g') * (u' + 1).
 __device__ __forceinline__ float gated_unit(float limit, float slope, float g, float u) {
     if (limit > 0.0f) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + __expf(-slope * g)) * (u + 1.0f);
+        return quotient(g, 1.0f + __expf(-slope * g)) * (u + 1.0f);
     }
     return silu_mul(g, u);
 }
@@ -229,7 +229,7 @@ __device__ __forceinline__ void epilogue_act(float* v, int m) {
         for (int i = 0; i < 16; ++i) { const float r = fmaxf(v[i], 0.0f); v[i] = r * r; }
     } else if (m == 1) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = v[i] / (1.0f + __expf(-v[i]));
+        for (int i = 0; i < 16; ++i) v[i] = quotient(v[i], 1.0f + __expf(-v[i]));
     } else if (m == 2) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));

@@ -18,6 +18,7 @@
 #define AIRUN_DEV_BAD_REQ 2       // a token naming a request outside the batch
 #define AIRUN_DEV_BAD_TOKEN 4     // a token id outside the vocabulary
 #define AIRUN_DEV_TIMEOUT 8       // a bounded wait ran out
+#define AIRUN_DEV_BAD_ROW 16      // a row of an expert, or a segment of a prompt, outside its buffer
 
 #define AIRUN_DT_F32 0
 #define AIRUN_DT_BF16 1

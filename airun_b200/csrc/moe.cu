@@ -268,12 +268,13 @@ __global__ void moe_offsets_kernel(const int32_t* counts, int32_t* __restrict__ 
     }
 }
 
-// One block per (token, choice); rows without a weight on them are copied sixteen bytes at a time (`vec`).
+// One block per (token, choice); rows without a weight on them are copied sixteen bytes at a time (`vec`).  A row that the
+// router's lists place outside xs is reported and has no place: it is neither written here nor read when the rows are summed.
 template <typename TH>
 __global__ __launch_bounds__(256) void moe_scatter_kernel(
     const TH* h, int W, int top, const int32_t* ids, const float* wts,
     const int32_t* rank, const int32_t* seg, int scale_input, TH* __restrict__ xs,
-    int32_t* __restrict__ row_of, int num_real, int vec) {
+    int32_t* __restrict__ row_of, int num_real, int vec, int* __restrict__ err) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x, k = blockIdx.y;
@@ -285,6 +286,13 @@ __global__ __launch_bounds__(256) void moe_scatter_kernel(
         return;
     }
     const int row = seg[e] + rank[at];
+    if (row < 0 || row >= (int)(gridDim.x * gridDim.y)) {
+        if (threadIdx.x == 0) {
+            row_of[at] = -1;
+            if (err) atomicOr(err, AIRUN_DEV_BAD_ROW);
+        }
+        return;
+    }
     if (threadIdx.x == 0) row_of[at] = row;
     if (vec) {
         const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)t * W);
@@ -316,7 +324,7 @@ __global__ __launch_bounds__(256) void moe_combine_kernel(
             const int r = row_of[(size_t)t * top + k];
             const float w = scale_output ? wts[(size_t)t * top + k] : 1.0f;
             float y[VEC];
-            if (r >= 0) {
+            if (r >= 0 && r < (int)gridDim.x * top) {
                 const float* src = ys + (size_t)r * W + c;
                 if (VEC == 4) {
                     const float4 v = *reinterpret_cast<const float4*>(src);
@@ -389,17 +397,17 @@ AIRUN_EXPORT int airun_moe_route_grouped(const float* z, long long z_stride, con
 
 AIRUN_EXPORT int airun_moe_scatter(const void* h, int dtype, int T, int W, int top, const int32_t* ids, const float* wts,
                                    const int32_t* rank, const int32_t* seg, int scale_input, void* xs, int32_t* row_of,
-                                   int num_real, cudaStream_t stream) {
+                                   int num_real, int* err, cudaStream_t stream) {
     if (T < 0 || W <= 0 || top <= 0 || !ids || !wts || !rank || !seg || !xs || !row_of || num_real <= 0) return AIRUN_ERR_ARG;
     if (T == 0) return AIRUN_OK;
-    if (top > 65535) return AIRUN_ERR_ARG;
+    if (top > 65535 || (long long)T * top > 0x7fffffffLL) return AIRUN_ERR_ARG;
     const int vec = !scale_input && (W * (dtype == AIRUN_DT_F32 ? 4LL : 2LL)) % 16 == 0 && (((uintptr_t)h | (uintptr_t)xs) & 15) == 0;
     if (dtype == AIRUN_DT_F32)
         airun_launch(moe_scatter_kernel<float>, dim3(T, top), dim3(256), 0, stream, (const float*)h, W, top, ids, wts, rank, seg,
-                     scale_input, (float*)xs, row_of, num_real, vec);
+                     scale_input, (float*)xs, row_of, num_real, vec, err);
     else if (dtype == AIRUN_DT_BF16)
         airun_launch(moe_scatter_kernel<__nv_bfloat16>, dim3(T, top), dim3(256), 0, stream, (const __nv_bfloat16*)h, W, top, ids, wts,
-                     rank, seg, scale_input, (__nv_bfloat16*)xs, row_of, num_real, vec);
+                     rank, seg, scale_input, (__nv_bfloat16*)xs, row_of, num_real, vec, err);
     else
         return AIRUN_ERR_UNSUPPORTED;
     return airun_launch_status();

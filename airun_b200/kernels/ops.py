@@ -24,7 +24,8 @@ ROPE_NONE, ROPE_NEOX, ROPE_INTERLEAVED = 0, 1, 2
 _DT = {torch.float32: DT_F32, torch.bfloat16: DT_BF16}
 
 DEV_ERR_BITS = {1: "a block-table entry outside the page pool", 2: "a token naming a request outside the batch",
-                4: "a token id outside the vocabulary", 8: "a bounded device-side wait ran out"}
+                4: "a token id outside the vocabulary", 8: "a bounded device-side wait ran out",
+                16: "a row of an expert or a segment of a prompt outside its buffer"}
 
 
 class KernelError(RuntimeError):
@@ -1049,18 +1050,20 @@ def moe_route(logits: torch.Tensor, top: int, softmax_scores: bool, renorm: bool
 
 
 def moe_scatter(h: torch.Tensor, top: int, ids, wts, rank, seg, scale_input: bool, xs: torch.Tensor, row_of: torch.Tensor,
-                num_real: int = 1 << 30) -> None:
+                num_real: int = 1 << 30, err: Optional[torch.Tensor] = None) -> None:
     """xs[seg[e] + rank] = h[t] (times the weight with ``scale_input``) for each of the token's experts; row_of [T, top]
-    keeps the row (-1 for an expert id of ``num_real`` or more: an expert without matrices, which gets no row)."""
-    _cuda(h, xs, row_of)
+    keeps the row (-1 for an expert id of ``num_real`` or more: an expert without matrices, which gets no row).  A row
+    outside xs is left out and sets the error word's bit for it."""
+    _cuda(h, xs, row_of, err)
     T, W = h.shape
     _need(h.is_contiguous() and xs.is_contiguous() and tuple(xs.shape) == (T * top, W) and xs.dtype == h.dtype,
           "xs must be contiguous [T*top, W] of h's type")
     _need(row_of.dtype == torch.int32 and row_of.numel() >= T * top, "row_of must be int32 [T, top]")
     f = _fn("moe", "airun_moe_scatter",
-            [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p])
+            [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
+             c_void_p])
     _check(f(_p(h), _dt(h), T, W, int(top), _p(ids), _p(wts), _p(rank), _p(seg), 1 if scale_input else 0, _p(xs), _p(row_of),
-             int(num_real), _stream()), "moe_scatter")
+             int(num_real), _p(err), _stream()), "moe_scatter")
 
 
 def moe_combine(ys: torch.Tensor, top: int, ids, wts, row_of, scale_output: bool, out: torch.Tensor,

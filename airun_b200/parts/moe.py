@@ -145,7 +145,7 @@ class RoutedExperts(FeedForward):
             ops.moe_route(logits[:, :self.E], top, self.softmax, self.renorm, ctx.req_of_token, ids, wts, rank, self.counts, seg,
                           bias=self.b_router)
         xs = ws.alloc((M, self.H), self.dtype)
-        ops.moe_scatter(h, top, ids, wts, rank, seg, self.on_input, xs, row_of, num_real=self.E)
+        ops.moe_scatter(h, top, ids, wts, rank, seg, self.on_input, xs, row_of, num_real=self.E, err=ctx.err)
         act = ws.alloc((M, self.I), self.dtype)
         fused = False
         if xs.dtype == torch.bfloat16:

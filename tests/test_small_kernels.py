@@ -197,3 +197,32 @@ def test_silu_far_below_zero(M, dtype):
         fast.gemm_tcgen05(x.cuda(), w.cuda(), out, epi, M == 40, 64 if M == 40 else 256, 1, err, act=silu)
     assert int(err.item()) == 0
     assert bool(((out.cpu().double() - want).abs() <= ((2.0 ** -8 if dtype == torch.bfloat16 else 0) + 2e-5) * want.abs() + 1.2e-38).all())
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,top,W", [(5, 2, 64), (3, 1, 10)])
+def test_rows_of_experts_that_have_no_place(T, top, W, dtype):
+    """Ranks and segments that place a row outside the buffer (an older list, say): the row is left out, the error word says so, and
+    what lies around the buffer stays."""
+    from airun_b200.kernels import ops
+    store = torch.full((T * top + 4, W), 7.0, dtype=dtype, device="cuda")
+    xs, err = store[2:-2], torch.zeros(1, dtype=torch.int32, device="cuda")
+    h = torch.randn(T, W, dtype=torch.float32).to("cuda", dtype)
+    ids, rank = torch.zeros(T, top, dtype=torch.int32), torch.arange(T * top, dtype=torch.int32).view(T, top)
+    rank[0, 0], rank[T - 1, top - 1] = -1, T * top
+    seg = torch.tensor([0, T * top], dtype=torch.int32, device="cuda")
+    row_of, wts = torch.full((T, top), -9, dtype=torch.int32, device="cuda"), torch.ones(T, top, device="cuda")
+    ids, rank = ids.cuda(), rank.cuda()
+    ops.moe_scatter(h, top, ids, wts, rank, seg, False, xs, row_of, num_real=1, err=err)
+    assert int(err.item()) == 16 and "row" in ops.describe_device_error(16)
+    assert row_of[0, 0] == -1 and row_of[T - 1, top - 1] == -1 and bool((store[:2] == 7).all()) and bool((store[-2:] == 7).all())
+    assert bool((xs[0] == 7).all()) and bool((xs[T * top - 1] == 7).all())
+    for r in range(1, T * top - 1):
+        assert torch.equal(xs[r], h[r // top]) and int(row_of.view(-1)[r]) == r
+    ys, out = torch.randn(T * top, W, device="cuda"), torch.empty(T, W, device="cuda")
+    bad = row_of.clone()
+    bad[bad < 0] = T * top + 1000                                    # and a row number from elsewhere is not read
+    ops.moe_combine(ys, top, ids, wts, bad, False, out)
+    want = torch.where((row_of >= 0)[..., None], ys.view(T, top, W), torch.zeros(1, device="cuda")).sum(1)
+    assert torch.allclose(out, want, atol=1e-6)

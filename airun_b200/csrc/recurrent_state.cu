@@ -1066,7 +1066,8 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
 }
 
 // `coef` ([T][heads][RS_COEF] floats, 16-byte aligned, may be null): chunks of eight tokens.  The modes with a decay per
-// channel also need `vectors`, 4 * T * heads * D floats, 16-byte aligned, and D up to 128.
+// channel also need `vectors`, 4 * T * heads * D floats, 16-byte aligned, and D up to 128.  `portions`: how many of the requests
+// bring several tokens, at most (0: not known).
 AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k, const float* v, const float* g,
                                        long long q_stride, long long k_stride, long long v_stride, long long g_stride,
                                        const float* beta, long long beta_stride, const float* a_log, const float* dt_bias,
@@ -1074,7 +1075,7 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
                                        long long slot_stride, int max_slots, const int32_t* cu_tokens, const int32_t* state_slots,
                                        int num_reqs, float* out, int heads, int kv_rep, int D, int Dv, const float* tail_src,
                                        long long tail_src_stride, long long tail_off, int tail_rows, int tail_width,
-                                       int long_chains, float* coef, float* vectors, int T, int* err, cudaStream_t stream) {
+                                       int long_chains, float* coef, float* vectors, int T, int portions, int* err, cudaStream_t stream) {
     if (num_reqs < 0 || heads <= 0 || heads > 65535 || kv_rep <= 0 || heads % kv_rep || D <= 0 || D > 256 || Dv <= 0 || !state ||
         !cu_tokens || !state_slots || !err || !q || !k || !v || !g || !out || slot_stride < (long long)heads * D * Dv)
         return AIRUN_ERR_ARG;
@@ -1129,7 +1130,8 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const bool few = (long long)mgrid.x * mgrid.y * mgrid.z <= 2LL * sms;
+        // the blocks that run long are the portions': of a padded step's requests most may bring one token or none
+        const bool few = (long long)(portions > 0 && portions < num_reqs ? portions : num_reqs) * mgrid.y * mgrid.z <= 2LL * sms;
 #define RS_HEAD_CHUNKS(NS) do { if (few) RS_CHUNKS(NS, CHUNK_HEAD, 8, 2); else RS_CHUNKS(NS, CHUNK_HEAD, 8, 4); } while (0)
         if (D <= 32) RS_HEAD_CHUNKS(4);
         else if (D <= 64) RS_HEAD_CHUNKS(8);

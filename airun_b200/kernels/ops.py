@@ -894,6 +894,16 @@ RECURRENCE_DELTA, RECURRENCE_WKV, RECURRENCE_DELTA_HEAD = 0, 1, 2
 RS_COEF = 20            # floats a token and head between the two kernels of the chunked recurrence
 
 
+def portions_of(ctx) -> int:
+    """Requests of the step that bring several tokens, at most: counted where the host knows them, in a padded step what its
+    graph is made for.  (``num_reqs`` of a padded step is what the runner can hold, whoever is there.)"""
+    shape = getattr(ctx, "extras", {}).get("device_plan")
+    if shape:
+        return min(int(shape["max_portions"]), int(ctx.num_reqs))
+    lens = getattr(ctx, "query_lens", None)
+    return sum(1 for n in lens if n > 1) if lens else int(ctx.num_reqs)
+
+
 def recurrent_state(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, state: torch.Tensor, ctx,
                     out: torch.Tensor, heads: int, kv_rep: int, D: int, Dv: int, beta: Optional[torch.Tensor] = None,
                     bonus: Optional[torch.Tensor] = None, tail_src: Optional[torch.Tensor] = None, tail_off: int = 0,
@@ -932,17 +942,20 @@ def recurrent_state(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     f = _fn("recurrent_state", "airun_recurrent_state",
             [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p, c_longlong,
              c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-             c_longlong, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p])
+             c_longlong, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p])
     long_chains = 1 if T > 2 * int(ctx.num_reqs) else 0          # requests bring many tokens each, not one
     # such chains run in chunks of eight tokens over coefficients (and, with a decay per channel, vectors) worked out ahead
-    # of the recurrence; with the vectors from 64 tokens a request on, below which they cost about what the chunks save
-    ws = getattr(ctx, "ws", None)
-    chunks = long_chains and (head_decay or (D <= 128 and T >= 64 * int(ctx.num_reqs) and ws is not None))
+    # of the recurrence; with the vectors above 64 tokens a portion, below which they cost about what the chunks save (16
+    # heads of 64 x 64, token by token and in chunks, us: delta rule 64 tokens 22.6, 18.5, four times 64 26.9, 22.8, 512 135,
+    # 62; time mix 17.2, 16.3, 20.8, 19.1 and 93, 50).  Steps of up to 192 tokens, where chunks save 25 us a layer at most, stay
+    # token by token: the forms round differently, and short prompts are held to the rounding of the plain order.
+    ws, portions = getattr(ctx, "ws", None), portions_of(ctx)
+    chunks = ws is not None and (bool(long_chains) if head_decay else D <= 128 and portions > 0 and T > max(192, 64 * portions))
     coef = ws.alloc((T, heads, RS_COEF), torch.float32) if chunks else None
     vectors = ws.alloc((4, T, heads * D), torch.float32) if chunks and not head_decay else None
     _check(f(int(mode), _p(q), _p(k), _p(v), _p(g), _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(g), _p(beta), bs,
              _p(a_log), _p(dt_bias), _p(bonus), _p(state), state.stride(0), state.shape[0], _p(ctx.cu_tokens), _p(ctx.state_slots), int(ctx.num_reqs),
-             _p(out), heads, kv_rep, D, Dv, _p(tail_src), ts, int(tail_off), int(tail_rows), tw, long_chains, _p(coef), _p(vectors), T,
+             _p(out), heads, kv_rep, D, Dv, _p(tail_src), ts, int(tail_off), int(tail_rows), tw, long_chains, _p(coef), _p(vectors), T, portions,
              _p(ctx.err), _stream()), "recurrent_state")
 
 

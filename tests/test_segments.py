@@ -127,3 +127,48 @@ def test_chunks_with_a_decay_per_channel(heads, kv, D, Dv, first, second, mix):
             ends[r] += lens[r]
             at += lens[r]
     assert float(state[:, n_state:].abs().max()) == 0
+
+
+def test_rules_count_the_portions_that_are_there():
+    """A padded step names the requests its runner can hold; the rules go by the portions its graph is made for."""
+    from types import SimpleNamespace
+
+    from airun_b200.kernels import ops
+    assert ops.portions_of(SimpleNamespace(num_reqs=64, extras={"device_plan": dict(max_rows=8, min_rows=1, max_portions=4)})) == 4
+    assert ops.portions_of(SimpleNamespace(num_reqs=2, extras={"device_plan": dict(max_rows=0, min_rows=0, max_portions=4)})) == 2
+    assert ops.portions_of(SimpleNamespace(num_reqs=3, extras={}, query_lens=[1, 700, 2])) == 2
+    assert ops.portions_of(SimpleNamespace(num_reqs=5)) == 5
+
+
+@gpu
+@pytest.mark.parametrize("mode", ["channel", "mix", "head"])
+def test_a_prompt_takes_the_same_form_whatever_its_runner_can_hold(mode):
+    """One prompt in a step padded to 2 requests and to 64: the same bits, so the same kernels."""
+    from types import SimpleNamespace
+
+    from airun_b200.engine.batch import Workspace
+    from airun_b200.kernels import ops
+    g = torch.Generator().manual_seed(9)
+    T, heads, D, Dv = 256, 2, 64, 64
+    q, k, v = ((torch.randn(T, heads * D, generator=g) * 0.1).cuda() for _ in range(3))
+    decay, beta = (torch.rand(T, heads * D, generator=g) ** 0.1).cuda(), torch.randn(T, heads, generator=g).cuda()
+    outs = []
+    for held in (2, 64):
+        cu = torch.full((held + 1,), 230, dtype=torch.int32)
+        cu[0] = 0
+        ctx = SimpleNamespace(num_reqs=held, cu_tokens=cu.cuda(), state_slots=torch.arange(held, dtype=torch.int32).cuda(),
+                              err=torch.zeros(1, dtype=torch.int32, device="cuda"), ws=Workspace(torch.device("cuda"), 8 << 20),
+                              extras={"device_plan": dict(max_rows=0, min_rows=0, max_portions=1)})
+        state, out = torch.zeros(held, heads * D * Dv, device="cuda"), torch.zeros(T, heads * Dv, device="cuda")
+        if mode == "channel":
+            ops.recurrent_state(ops.RECURRENCE_DELTA, q, k, v, decay, state, ctx, out, heads, 1, D, Dv, beta=beta)
+        elif mode == "mix":
+            ops.recurrent_state(ops.RECURRENCE_WKV, q, k, v, decay, state, ctx, out, heads, 1, D, Dv, bonus=beta[:heads].new_ones(heads, D))
+        else:
+            ops.recurrent_state(ops.RECURRENCE_DELTA_HEAD, q, k, v, beta, state, ctx, out, heads, 1, D, Dv, beta=beta,
+                                a_log=beta.new_zeros(heads), dt_bias=beta.new_zeros(heads))
+        used = ctx.ws.bytes() and ctx.ws.off
+        assert int(ctx.err.item()) == 0
+        outs.append((out[:230].clone(), state[0].clone(), used))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert outs[0][2] == outs[1][2] > 0                                  # coefficients were made: both ran in chunks

@@ -149,7 +149,14 @@ __global__ __launch_bounds__(256) void gla_recurrent_kernel(
     __shared__ float s_p[GLA_WARPS][GLA_TT][GLA_COLS];
     int r = blockIdx.x, part = 0, parts = 1;
     const int head = blockIdx.y, col0 = blockIdx.z * GLA_COLS;
-    if (SEG && !gla_find_segment(cu_tokens, num_reqs, blockIdx.x, r, part, parts)) return;
+    if (SEG) {
+        const bool there = gla_find_segment(cu_tokens, num_reqs, blockIdx.x, r, part, parts);
+        int r2, part2, parts2;                             // a segment that no block has: said by one of the last segment's
+        if (blockIdx.x == gridDim.x - 1 && head == 0 && col0 == 0 && threadIdx.x == 0 &&
+            gla_find_segment(cu_tokens, num_reqs, gridDim.x, r2, part2, parts2))
+            atomicOr(err, AIRUN_DEV_BAD_ROW);
+        if (!there) return;
+    }
     int t0 = cu_tokens[r], n = cu_tokens[r + 1] - t0;
     if (n <= 0) return;
     if (SEG) { t0 += part * GLA_SEG; n = min(GLA_SEG, n - part * GLA_SEG); }
@@ -420,7 +427,7 @@ static int gla_recurrent_launch(const float* q, const float* k, const float* v, 
 }
 
 // `work`: null, or max_segments * heads * (D * Dv + D) floats for the segments (D up to 128, D and Dv in multiples of 4);
-// max_segments: at least the sum over the requests of ceil(tokens / GLA_SEG).
+// max_segments: at least the sum over the requests of ceil(tokens / GLA_SEG); with fewer the error word says so.
 AIRUN_EXPORT int airun_gla_segment_tokens() { return GLA_SEG; }
 
 AIRUN_EXPORT int airun_gla_recurrent(const float* q, const float* k, const float* v, long long row_stride,

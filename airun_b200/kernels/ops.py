@@ -398,17 +398,24 @@ def gla_decay(low: torch.Tensor, w2: torch.Tensor, bias: Optional[torch.Tensor],
              _stream()), "gla_decay")
 
 
-SEGMENT_TOKENS = 128                   # csrc/linear_attention.cu: GLA_SEG
-SEGMENT_MIN_TOKENS = 256               # tokens of a step from which a request's tokens run in segments side by side
+SEGMENT_MIN_TOKENS, SEGMENT_MAX_TOKENS = 256, 32768      # tokens of a step that run in segments side by side
+
+
+def segment_tokens() -> int:
+    """Tokens of a segment of the linear attentions' recurrence, as the kernels cut them."""
+    return int(_fn("linear_attention", "airun_gla_segment_tokens", [])())
 
 
 def _gla_work(ws, T: int, num_reqs: int, heads: int, D: int, Dv: int, state: torch.Tensor):
-    """(buffer for the segments of a step of T tokens, their largest number), or (None, 0): the step is short, the sizes
-    are not the segments', or no workspace is given.  The cut costs a second kernel and 1 / SEGMENT_TOKENS of a state per
-    token, so it pays once a request brings two segments."""
-    if ws is None or T < SEGMENT_MIN_TOKENS or D > 128 or D % 4 or Dv % 4 or state.stride(0) % 4 or state.data_ptr() % 16:
+    """(buffer for the segments of a step of T tokens, their largest number), or (None, 0): the step is short or very
+    long, the sizes are not the segments', or no workspace is given.  The cut costs a second kernel and, per token, a segment's
+    share of a state, so it pays once a request brings two segments; every segment brings the ends of those before it together,
+    which grows with the square: one request, 16 heads of 64 x 128, chain and segments, us: 512 tokens 78, 57; 2,048 262, 129;
+    8,192 1028, 607; 16,384 2033, 1454; 32,768 4060, 3874."""
+    if (ws is None or not SEGMENT_MIN_TOKENS <= T <= SEGMENT_MAX_TOKENS or D > 128 or D % 4 or Dv % 4 or state.stride(0) % 4
+            or state.data_ptr() % 16):
         return None, 0
-    n = T // SEGMENT_TOKENS + int(num_reqs)
+    n = T // segment_tokens() + int(num_reqs)
     return ws.alloc((n * heads * (D * Dv + D),), torch.float32), n
 
 

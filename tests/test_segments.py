@@ -129,6 +129,29 @@ def test_chunks_with_a_decay_per_channel(heads, kv, D, Dv, first, second, mix):
     assert float(state[:, n_state:].abs().max()) == 0
 
 
+@gpu
+@pytest.mark.parametrize("per_head", [False, True])
+def test_more_segments_than_were_made_room_for(per_head, monkeypatch):
+    """A launch for fewer segments than the step has says so instead of leaving the rest out in silence."""
+    from airun_b200.engine.batch import Workspace
+    from airun_b200.kernels import ops
+    heads, D, Dv, lens = 2, 32, 32, (300, 257)
+    T, n = sum(lens), 3 + 3
+    proj = torch.randn(T, 2 * heads * D + heads * Dv).cuda()
+    q, k, v = proj[:, :heads * D], proj[:, heads * D:2 * heads * D], proj[:, 2 * heads * D:]
+    cu, sl = torch.tensor([0, 300, T], dtype=torch.int32, device="cuda"), torch.arange(2, dtype=torch.int32, device="cuda")
+    ws, true = Workspace(torch.device("cuda"), 8 << 20), ops._gla_work
+    assert ops.segment_tokens() == 128
+    for room, bits in ((n, 0), (n + 5, 0), (n - 1, 16), (1, 16)):
+        monkeypatch.setattr(ops, "_gla_work", lambda *a, room=room: (true(*a)[0], room))
+        state, out, err = torch.zeros(2, heads, D, Dv, device="cuda"), torch.empty(T, heads * Dv, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        if per_head:
+            ops.decay_recurrent(q, k, v, torch.full((heads,), 0.9, device="cuda"), False, state, cu, sl, 2, out, heads, D, Dv, 1.0, err, ws=ws)
+        else:
+            ops.gla_recurrent(q, k, v, torch.full((T, heads * D), 0.9, device="cuda"), state, cu, sl, 2, out, heads, D, Dv, 1.0, err, ws=ws)
+        assert int(err.item()) == bits
+
+
 def test_rules_count_the_portions_that_are_there():
     """A padded step names the requests its runner can hold; the rules go by the portions its graph is made for."""
     from types import SimpleNamespace

@@ -421,10 +421,11 @@ def _gla_work(ws, T: int, num_reqs: int, heads: int, D: int, Dv: int, state: tor
 
 def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                   cu_tokens: torch.Tensor, state_slots: torch.Tensor, num_reqs: int, out: torch.Tensor,
-                  heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None) -> None:
+                  heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None, present: Optional[int] = None) -> None:
     """The recurrence S <- diag(a) S + k v^T, o = S^T q * q_scale for the tokens of every request in order.
     ``q``, ``k`` [T, heads*D] and ``v`` [T, heads*Dv] are float32 column slices of ONE buffer (equal row strides);
-    ``state`` is [slots, heads, D, Dv] float32 and is updated in place; ``out`` float32 [T, heads*Dv]."""
+    ``state`` is [slots, heads, D, Dv] float32 and is updated in place; ``out`` float32 [T, heads*Dv].  ``ws``: a workspace, with which
+    long prompts run in segments; ``present``: how many of the requests bring tokens, at most (all, unless given)."""
     _cuda(q, k, v, decay, state, cu_tokens, state_slots, out, err)
     for t, w, name in ((q, heads * D, "q"), (k, heads * D, "k"), (v, heads * Dv, "v")):
         _rows_f32(t, name)
@@ -441,7 +442,7 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torc
           and state_slots.numel() >= num_reqs, "cu_tokens / state_slots must be int32 [R + 1] / [R]")
     _need(D <= 256, f"{D} key channels a head are above the kernel's limit of 256")
     stride = q.stride(0) if T > 1 else max(q.stride(0), k.stride(0), v.stride(0))
-    work, segments = _gla_work(ws, T, num_reqs, heads, D, Dv, state)
+    work, segments = _gla_work(ws, T, num_reqs if present is None else present, heads, D, Dv, state)
     f = _fn("linear_attention", "airun_gla_recurrent",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int,
              c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p])
@@ -451,7 +452,7 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torc
 
 def decay_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, head_decay: torch.Tensor, in_silu: bool,
                     state: torch.Tensor, cu_tokens: torch.Tensor, state_slots: torch.Tensor, num_reqs: int, out: torch.Tensor,
-                    heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None) -> None:
+                    heads: int, D: int, Dv: int, q_scale: float, err: torch.Tensor, ws=None, present: Optional[int] = None) -> None:
     """The recurrence with one decay per head, S <- d_h S + k v^T, o = S^T q * q_scale, for the tokens of every request in
     order.  ``q``, ``k`` [T, heads*D] and ``v`` [T, heads*Dv] are float32 column slices of ONE buffer; with ``in_silu``
     they arrive without their activation z sigmoid(z), which the kernel applies.  ``head_decay`` float32 [heads];
@@ -471,7 +472,7 @@ def decay_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, head_deca
           and state_slots.numel() >= num_reqs, "cu_tokens / state_slots must be int32 [R + 1] / [R]")
     _need(D <= 256, f"{D} key channels a head are above the kernel's limit of 256")
     stride = q.stride(0) if T > 1 else max(q.stride(0), k.stride(0), v.stride(0))
-    work, segments = _gla_work(ws, T, num_reqs, heads, D, Dv, state)
+    work, segments = _gla_work(ws, T, num_reqs if present is None else present, heads, D, Dv, state)
     f = _fn("linear_attention", "airun_decay_recurrent",
             [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int,
              c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p])
@@ -909,6 +910,12 @@ def portions_of(ctx) -> int:
         return min(int(shape["max_portions"]), int(ctx.num_reqs))
     lens = getattr(ctx, "query_lens", None)
     return sum(1 for n in lens if n > 1) if lens else int(ctx.num_reqs)
+
+
+def requests_of(ctx) -> int:
+    """Requests of the step that bring any token, at most (see ``portions_of``)."""
+    shape = getattr(ctx, "extras", {}).get("device_plan")
+    return min(int(shape["max_rows"]) + int(shape["max_portions"]), int(ctx.num_reqs)) if shape else int(ctx.num_reqs)
 
 
 def recurrent_state(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, state: torch.Tensor, ctx,

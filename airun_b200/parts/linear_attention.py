@@ -83,7 +83,8 @@ class GatedLinearAttention(Mixer):
         ops.gla_decay(low, self.w_decay, self.decay_bias, self.tau, decay, ctx.req_of_token)
         o = ws.alloc((T, vd), torch.float32)
         ops.gla_recurrent(q, k, v, decay, cache.state, ctx.cu_tokens, ctx.state_slots, ctx.num_reqs, o,
-                          self.nh, self.D, self.Dv, self.q_scale, ctx.err, ws=None if getattr(ctx, "decode_only", False) else ctx.ws)
+                          self.nh, self.D, self.Dv, self.q_scale, ctx.err, ws=None if getattr(ctx, "decode_only", False) else ctx.ws,
+                          present=ops.requests_of(ctx))
         ops.gla_out_gate(o, gate, self.norm_w, self.eps, act, self.nh, self.Dv, ctx.req_of_token)
 
     def forward(self, ctx, h, cache, sink=None):
@@ -160,7 +161,8 @@ class DecayLinearAttention(Mixer):
         q, k, v, gate = proj[:, :kd], proj[:, kd:2 * kd], proj[:, 2 * kd:2 * kd + vd], proj[:, 2 * kd + vd:2 * kd + 2 * vd]
         o = ws.alloc((T, vd), torch.float32)
         ops.decay_recurrent(q, k, v, self.decay, True, cache.state, ctx.cu_tokens, ctx.state_slots, ctx.num_reqs, o,
-                            self.nh, self.D, self.Dv, 1.0, ctx.err, ws=None if getattr(ctx, "decode_only", False) else ctx.ws)
+                            self.nh, self.D, self.Dv, 1.0, ctx.err, ws=None if getattr(ctx, "decode_only", False) else ctx.ws,
+                          present=ops.requests_of(ctx))
         ops.rownorm_gate(o, gate, self.norm_w, self.eps, act, ctx.req_of_token, scale=self.out_scale)
 
     def forward(self, ctx, h, cache, sink=None):

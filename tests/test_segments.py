@@ -161,6 +161,9 @@ def test_rules_count_the_portions_that_are_there():
     assert ops.portions_of(SimpleNamespace(num_reqs=2, extras={"device_plan": dict(max_rows=0, min_rows=0, max_portions=4)})) == 2
     assert ops.portions_of(SimpleNamespace(num_reqs=3, extras={}, query_lens=[1, 700, 2])) == 2
     assert ops.portions_of(SimpleNamespace(num_reqs=5)) == 5
+    assert ops.requests_of(SimpleNamespace(num_reqs=64, extras={"device_plan": dict(max_rows=8, min_rows=1, max_portions=4)})) == 12
+    assert ops.requests_of(SimpleNamespace(num_reqs=10, extras={"device_plan": dict(max_rows=8, min_rows=1, max_portions=4)})) == 10
+    assert ops.requests_of(SimpleNamespace(num_reqs=3, extras={}, query_lens=[1, 700, 2])) == 3
 
 
 @gpu

@@ -286,14 +286,18 @@ def linear_swiglu_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch.Tens
 
 
 GROUPED_MAX_TILES = 1024
-# rows a segment on average up to which the product goes to csrc/gemm_rows.cu: 16 matrices of 3072 x 2048, tcgen05 and rows,
-# 32 rows 43.2 and 33.8 us, 128 rows 43.4 and 42.0, 256 rows 43.2 and 51.1 (29, 31 and 31 us of weights)
-GROUPED_ROWS_MAX = 8
+# A product goes to csrc/gemm_rows.cu up to this many rows a segment on average and up to this many tokens, which is what one
+# segment can hold: a segment reads its matrix again for every 8 or 16 rows.  16 matrices of 3072 x 2048 as gated units, weights
+# not in the L2 cache, tcgen05 and rows, us: 8 tokens of 4 experts 44.1, 35.7; 16 of 8 44.5, 42.4; 32 of 4 44.4, 42.5.  All
+# tokens on the same experts: 8 of 4 22.6, 14.3; 16 of 8 27.2, 25.3; 32 of 4 22.6, 25.9; 128 rows of one of 16 (1,024 x 2,048
+# each) 17.3, 61.4.
+GROUPED_ROWS_MAX, GROUPED_ROWS_TOKENS = 8, 32
 
 
 def grouped_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor, swiglu_group: int = 0,
-                        act: Optional[int] = None, glu: Optional[Tuple[float, float]] = None) -> bool:
-    """Rows seg[e] .. seg[e+1]-1 of x [M, K] times w[e]^T (w [E, N, K]) on tcgen05, the segments read from the device.
+                        act: Optional[int] = None, glu: Optional[Tuple[float, float]] = None, tokens: Optional[int] = None) -> bool:
+    """Rows seg[e] .. seg[e+1]-1 of x [M, K] times w[e]^T (w [E, N, K]) on the tensor cores, the segments read from the device;
+    ``tokens``: no segment has more rows than that (None: not known, the kernel is chosen by the average alone).
     ``act`` (an ``ops.ACT_*``; not with ``swiglu_group``): the activation applied to the finished sums in the epilogue.
     ``swiglu_group`` 16: the rows of w[e] alternate between blocks of 16 gate and 16 up rows and out is the gated
     unit's result, bfloat16 [M, N/2] (SwiGLU, or the clamped unit with ``glu`` = (limit, slope)); 0: out [M, N] float32 or bfloat16.  False when the kernel does not take the
@@ -314,7 +318,7 @@ def grouped_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor
     _cuda(x, w, out, seg)
     _need(out.stride(1) == 1 and seg.dtype == torch.int32 and seg.numel() >= E + 1 and seg.is_contiguous(),
           "out must be row-major and seg int32 [E + 1]")
-    if M <= GROUPED_ROWS_MAX * E and "gemm_rows" not in DISABLED:
+    if M <= GROUPED_ROWS_MAX * E and (tokens is None or tokens <= GROUPED_ROWS_TOKENS) and "gemm_rows" not in DISABLED:
         f = _fn("gemm_rows", "airun_gemm_rows_grouped", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int,
                                                          c_void_p, c_int, c_float, c_float, c_int, c_void_p])
         lim, slope = glu if glu is not None else (0.0, 0.0)

@@ -151,22 +151,22 @@ class RoutedExperts(FeedForward):
         if xs.dtype == torch.bfloat16:
             from ..kernels import fast
             if self.gated:
-                fused = fast.grouped_linear_bf16(ctx, xs, self.w_gu, act, seg, swiglu_group=self.group, glu=self.glu)
+                fused = fast.grouped_linear_bf16(ctx, xs, self.w_gu, act, seg, swiglu_group=self.group, glu=self.glu, tokens=T)
             else:
-                fused = fast.grouped_linear_bf16(ctx, xs, self.w_up, act, seg, act=self.act_mode)
+                fused = fast.grouped_linear_bf16(ctx, xs, self.w_up, act, seg, act=self.act_mode, tokens=T)
         if not fused and self.gated:
             gu = ws.alloc((M, 2 * self.I), torch.float32)
-            grouped_linear(ctx, xs, self.w_gu, gu, seg)
+            grouped_linear(ctx, xs, self.w_gu, gu, seg, T)
             if self.glu:
                 ops.glu_clamped(gu, act, self.group, *self.glu)
             else:
                 ops.swiglu(gu, act, self.group)
         elif not fused:
             up = ws.alloc((M, self.I), torch.float32)
-            grouped_linear(ctx, xs, self.w_up, up, seg)
+            grouped_linear(ctx, xs, self.w_up, up, seg, T)
             ops.act(up, act, self.act_mode)
         ys = ws.alloc((M, self.H), torch.float32)
-        grouped_linear(ctx, act, self.w_down, ys, seg)
+        grouped_linear(ctx, act, self.w_down, ys, seg, T)
         delta = ws.alloc((T, self.H), torch.float32)
         ops.moe_combine(ys, top, ids, wts, row_of, not self.on_input, delta, passthrough=h if self.identity else None)
         if with_extra:
@@ -174,12 +174,12 @@ class RoutedExperts(FeedForward):
         return delta
 
 
-def grouped_linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor) -> None:
+def grouped_linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor, tokens: int) -> None:
     """Rows seg[e] .. seg[e+1]-1 of x times w[e]^T: x [M, K], w [E, N, K], out [M, N], seg int32 [E+1] on the device.
     bfloat16 operands go to the tensor-core kernel where it takes the sizes, everything else to the plain one."""
     if x.dtype == torch.bfloat16:
         from ..kernels import fast
-        if fast.grouped_linear_bf16(ctx, x, w, out, seg):
+        if fast.grouped_linear_bf16(ctx, x, w, out, seg, tokens=tokens):
             return
     ops.gemm_simt_grouped(x, w, out, seg)
 

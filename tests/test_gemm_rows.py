@@ -91,3 +91,21 @@ def test_segments_and_heads(lens, N, K):
         close(oh[:, :, :N], torch.einsum("thk,hnk->thn", xh.double(), w.double()), torch.einsum("thk,hnk->thn", xh.double().abs(), w.double().abs()),
               K, torch.bfloat16)
         assert bool((oh[:, :, N:] == 5.0).all())
+
+
+def test_which_products_of_segments_read_their_matrices_per_few_rows(monkeypatch):
+    """By the rows a segment has on average and by the rows it can have: with many tokens, all of which may choose one expert, the
+    matrices are read once (csrc/gemm_tcgen05.cu)."""
+    from airun_b200.kernels import fast
+    went = []
+    monkeypatch.setattr(fast, "_cuda", lambda *a: None)
+    monkeypatch.setattr(fast, "_check", lambda *a: None)
+    monkeypatch.setattr(fast, "_stream", lambda: None)
+    monkeypatch.setattr(fast, "_fn", lambda lib, name, args, defines=None: lambda *a: went.append(lib))
+    ctx = SimpleNamespace(err=torch.zeros(1, dtype=torch.int32))
+    for E, tokens, top, want in ((16, 8, 4, "gemm_rows"), (16, 32, 4, "gemm_rows"), (16, 33, 2, "gemm_tcgen05"), (64, 512, 1, "gemm_tcgen05"),
+                                 (16, 20, 8, "gemm_tcgen05"), (64, 32, 8, "gemm_rows")):
+        x, w = torch.zeros(tokens * top, 64, dtype=torch.bfloat16), torch.zeros(E, 32, 64, dtype=torch.bfloat16)
+        out, seg = torch.zeros(tokens * top, 32), torch.zeros(E + 1, dtype=torch.int32)
+        went.clear()
+        assert fast.grouped_linear_bf16(ctx, x, w, out, seg, tokens=tokens) and went == [want]

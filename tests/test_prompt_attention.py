@@ -60,6 +60,17 @@ def run_both(ctx, q, nh, tc, plain):
     return got[rows][:, 8:8 + nh * 128].float(), want[rows].float()
 
 
+def absolute(ctx, q, cache, nh, nkv, plain):
+    """What the weights give of the values' absolute values.  Rounding a weight and the two results to bfloat16 (2^-9 each) moves an
+    element by three of 2^-9 of that; 2^-7 leaves a quarter for the float32 sums and exponentials."""
+    pages = cache.pool.view(cache.pool.shape[0], 2, -1).clone()
+    pages[:, 1] = pages[:, 1].abs()
+    out = torch.zeros(q.shape[0], nh * 128, device="cuda", dtype=torch.bfloat16)
+    plain(out, SimpleNamespace(pool=pages.view_as(cache.pool), block_table=cache.block_table, page_size=cache.page_size, shared=False))
+    rows = torch.tensor([n > 1 for n in ctx.query_lens for _ in range(n)], device="cuda")
+    return out[rows].float()
+
+
 @gpu
 @pytest.mark.parametrize("nh,nkv,page,window,tail,rows,sink,gated,scale,spans", CASES)
 def test_softmax_kinds(nh, nkv, page, window, tail, rows, sink, gated, scale, spans):
@@ -76,6 +87,9 @@ def test_softmax_kinds(nh, nkv, page, window, tail, rows, sink, gated, scale, sp
                                         gate_stride=ops.attention_gate(gate, T, nh * 128)),
         lambda o: ops.softmax_attention(q, o, cache, ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, scale, tail=tail, gate=gate))
     assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * scale * float(cache.pool.abs().max())
+    if tail < 0:                                             # and each element by the weights' sum of its absolute values
+        most = absolute(ctx, q, cache, nh, nkv, lambda o, c: ops.softmax_attention(q, o, c, ctx, nh, nkv, 128, 128, 0.13, part.table, part.sink, window, scale, gate=gate))
+        assert bool(((got - want).abs() <= 2.0 ** -7 * most + 1e-6).all())
 
 
 @gpu
@@ -90,6 +104,8 @@ def test_attention_without_softmax(nh, nkv, page, window, dist, offset, spans):
         ctx, q, nh, lambda o: fast.attn_prompt_kind(ctx, "sigmoid", q, o, cache, part),
         lambda o: ops.sigmoid_attention(q, o, cache, ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, part.head_c, window))
     assert float((got - want).abs().max()) < 3 * 2.0 ** -8 * max(float(want.abs().max()), float(cache.pool.abs().max()))
+    most = absolute(ctx, q, cache, nh, nkv, lambda o, c: ops.sigmoid_attention(q, o, c, ctx, nh, nkv, 128, 128, 0.13, part.dist_a, part.dist_b, part.head_c, window))
+    assert bool(((got - want).abs() <= 2.0 ** -7 * most + 1e-6).all())
 
 
 SPLIT_CASES = [  # head size, heads, kv heads, page, window, spans: key tiles a query tile has, 1 to 17
@@ -128,8 +144,9 @@ DIFF_CASES = [(1, 1, 16, 0, 0, [(0, 193)]), (4, 2, 32, 64, 0, [(0, 129), (500, 5
 @pytest.mark.parametrize("nh,nkv,page,chunk,window,spans", DIFF_CASES)
 def test_differential(nh, nkv, page, chunk, window, spans):
     """Two maps, a soft cap and the difference's norm, against the plain kernel.  A result is a difference over its root mean
-    square, so what bounds it is the rounding of the two means (2^-9 of the largest value each, with the weights') over the
-    smallest root mean square among the rows, times the factor, and the result's own 2^-9."""
+    square: the two means are rounded in their weights alone here (2^-9 of a mean of absolute values, 0.64, at the most, less by
+    the root of the keys that matter), over the difference's root mean square, which falls to about 0.04 for rows of a
+    thousand keys, times the factor 0.8: 0.03; a mean over the rows of a tenth of that, and the results' own 2^-9."""
     from airun_b200.kernels import fast, ops
     g, cache, ctx, q = made(nh, nkv, page, -1, spans, nh * 31 + chunk)
     part = SimpleNamespace(D=64, Dv=128, nh=nh, nkv=nkv, scale=0.3, cap=20.0, chunk=chunk, window=window, lam=0.45, eps=1e-5, lambda_init=0.2)

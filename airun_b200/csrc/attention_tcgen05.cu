@@ -22,7 +22,8 @@
 // probabilities rounded to 16 bits for the second product).
 //
 // Every mbarrier wait is bounded (about two seconds); on a time-out the kernel sets an error
-// bit, stops working, frees its tensor memory and returns.  No cluster, no multicast.
+// bit, stops working, frees its tensor memory and returns.  A launch of few tiles runs as clusters (SPLIT below); no load is
+// multicast.
 #include "common.cuh"
 #include <cuda.h>
 #include <mutex>
@@ -272,7 +273,7 @@ struct TcShared {
 // SPLIT: a few tiles would leave most SMs idle, so the keys of a tile are cut into gridDim.z slices, the CTAs of one cluster.
 // Every CTA leaves its rows' (maximum, sum, unnormalised output) in its own shared memory, whose K and V stages are free by
 // then, and brings one part of the head dimensions of all slices together through distributed shared memory.  A slice has
-// two key tiles or more; a tile with no more than that is one CTA's, and the others leave.  Two portions of 240 tokens after
+// two key tiles or more, the last ones fewer or none; a tile with no more than two is one CTA's, and the others leave.  Two portions of 240 tokens after
 // 900, 16 heads on 8 KV heads: 25.6 us on 64 CTAs, 21.9 on 128.
 template <bool SHARED, bool SPLIT>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
@@ -1303,21 +1304,17 @@ AIRUN_EXPORT int airun_attn_prefill_tc(const void* q, void* out, const void* poo
     const int r = kv_map_for(&map, pool, (long long)num_pages * 2 * nkv * page_size);
     if (r != AIRUN_OK) return r;
     static unsigned long long configured = 0;            // one bit per device
-    static int sms_of[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return AIRUN_ERR_ARG;
     if (first_on_device(configured)) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
         if (e != cudaSuccess) return (int)e;
         e = cudaFuncSetAttribute(attn_prefill_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
         if (e != cudaSuccess) return (int)e;
-        cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev);
     }
     // Slices of a tile's keys while the CTAs stay within the SMs.  A launch sized for a padded batch (n_tiles_dev) counts a tile
-    // for every portion its bucket may have and the bucket's own padding, of which about two thirds are there; if more are, the
-    // second round's CTAs are half as long.
-    const long long ctas = (long long)n_tiles * nkv, sms = sms_of[dev], padded = n_tiles_dev ? 1 : 0;
+    // for every portion its bucket may have and the bucket's own padding, of which about half are there (counted over prompts of 16
+    // to 2,048 tokens in up to 16 portions: 0.5 to 0.6 on average, below 0.8 in nine of ten); if more are, the second round's
+    // CTAs are half as long.
+    const long long ctas = (long long)n_tiles * nkv, sms = airun_sm_count(), padded = n_tiles_dev ? 1 : 0;
     const int slices = ctas * SPLIT_MAX <= sms + padded * sms / 4 ? SPLIT_MAX : ctas * 2 <= sms + padded * sms * 3 / 4 ? 2 : 1;
     if (slices > 1)
         airun_launch_cluster(attn_prefill_tc_kernel<false, true>, dim3(n_tiles, nkv, slices), dim3(TC_THREADS), SMEM_TOTAL, stream, (unsigned)slices,

@@ -206,6 +206,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 static inline int ceil_div_i(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Multiprocessors of the current device.  (Threads that ask for the first time at once all store the same number.)
+static inline int airun_sm_count() {
+    static int known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    if (dev >= 0 && dev < 64 && (n = __atomic_load_n(&known[dev], __ATOMIC_RELAXED)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 1;
+    if (dev >= 0 && dev < 64) __atomic_store_n(&known[dev], n, __ATOMIC_RELAXED);
+    return n;
+}
+
 // True the first time it is asked on the current device (``mask``: one bit per device, of one kernel).
 // cudaFuncSetAttribute holds for one device only, so each kernel is configured once on each.
 static inline bool first_on_device(unsigned long long& mask) {

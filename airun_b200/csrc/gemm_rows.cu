@@ -6,8 +6,9 @@
 // copy engine, hands tiles from warp to warp, and adds up its K slices through a scratch in global memory with a ticket.
 // Here the weights go straight from global memory to the registers of the warps that multiply them.  A block takes 16 or 32
 // weight rows and all tokens; its eight warps share K (each takes every eighth run of 64 values, a 128-byte line of
-// each weight row) and add up through shared memory in warp order.  The weights of a warp's first two runs are asked for
-// before the kernel in front has finished.  Both operands are used with one permutation of k, chosen so that a lane's
+// each weight row) and add up through shared memory in warp order.  The weights of a warp's first two runs are on their way
+// before anything else is done.  (The kernel is launched once the one in front is done, see launch_mt: asked for while
+// that one still runs, they cost the kernels around it more than they save.)  Both operands are used with one permutation of k, chosen so that a lane's
 // operands of two m16n8k16 products are the 16 neighbouring bytes it loads: no shared memory, no shuffles.
 //
 // Three forms, as in the other product kernels: PLAIN; GROUPED, in which the rows of x lie in segments (device memory) with
@@ -186,7 +187,7 @@ __global__ __launch_bounds__(32 * ROW_WARPS, 2) void gemm_rows_kernel(const Rows
 template <int NT, int EPI, int FORM>
 void launch_mt(const RowsParams& p, int groups, int batch, cudaStream_t stream) {
     // 32 weight rows a block (every block reads all tokens: half as often as with 16) once that gives every SM a block
-    const bool two = EPI == EPI_SWIGLU || (long long)p.N * batch * (FORM == FORM_GROUPED ? groups : 1) >= 148 * 32;
+    const bool two = EPI == EPI_SWIGLU || (long long)p.N * batch * (FORM == FORM_GROUPED ? groups : 1) >= 32LL * airun_sm_count();
     const int rows = two ? 32 : 16;
     const dim3 grid(ceil_div_i(p.N, rows), groups, batch);
     // The launch waits for the kernel in front: resident early, half of an SM's registers a block, these blocks held up the

@@ -11,8 +11,9 @@
 // State, decays, the recurrence and the norm are float32 whatever the storage of the activations.  The
 // state of a request lives in its slot of the state tensor between steps, stored per head as [D][Dv]
 // (a row per key channel, the value columns side by side), and is zero when the request starts.  The result
-// at a token depends only on the request's tokens up to it, not on how they were cut into steps or on
-// what else is in the batch: the recurrence runs token by token in every case.
+// at a token depends only on the request's tokens up to it; its rounding also depends on the form that the
+// step takes: token by token, or, from 256 tokens of all its requests on, a request's tokens in segments of 128
+// that run side by side, whose sums are added in another order.
 #include "common.cuh"
 
 // a[t][c] = exp(logsigmoid(bias[c] + sum_j low[t][j] * w2[c][j]) / tau) for c < n (= heads * D).

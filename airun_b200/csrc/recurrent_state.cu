@@ -10,8 +10,9 @@
 //     o_t[j]   = sum_d r_t[d] * (S[d][j] + u[d] * k_t[d] * v_t[j])
 //     S[d][j] <- w_t[d] * S[d][j] + k_t[d] * v_t[j]
 // Both run in float32 on a state that lives in the request's slot of a state tensor between steps, [D][Dv] per
-// head, so the result at a token depends on the request's tokens up to it and on nothing else: not on how they
-// were cut into steps, not on the batch around them.
+// head, so the result at a token depends on the request's tokens up to it and on nothing else.  Its rounding
+// also depends on the form that the step takes: token by token, or in chunks of eight when the step's requests
+// bring many tokens (the caller decides by the step's tokens and portions), whose sums are added in another order.
 //
 // The delta rule's q, k and v pass a short causal convolution over time per channel and silu, and q and k are
 // made unit vectors per head (short_conv_kernel); the last taps - 1 inputs of the convolution are state too.  The
@@ -1127,11 +1128,8 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
         else if (D <= 64) RS_COEFS(2);
         else if (D <= 128) RS_COEFS(4);
         else RS_COEFS(8);
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         // the blocks that run long are the portions': of a padded step's requests most may bring one token or none
-        const bool few = (long long)(portions > 0 && portions < num_reqs ? portions : num_reqs) * mgrid.y * mgrid.z <= 2LL * sms;
+        const bool few = (long long)(portions > 0 && portions < num_reqs ? portions : num_reqs) * mgrid.y * mgrid.z <= 2LL * airun_sm_count();
 #define RS_HEAD_CHUNKS(NS) do { if (few) RS_CHUNKS(NS, CHUNK_HEAD, 8, 2); else RS_CHUNKS(NS, CHUNK_HEAD, 8, 4); } while (0)
         if (D <= 32) RS_HEAD_CHUNKS(4);
         else if (D <= 64) RS_HEAD_CHUNKS(8);

@@ -710,9 +710,11 @@ constexpr int W_SMEM_TOTAL = W_OFF_TAB + 1024;
 //              SAME 128 packed rows, map x reads the x-th half of a key's row; soft-capped scores, keys of the query's
 //              chunk only; the two results meet in shared memory, are subtracted and normed
 // The formulas are those of softmax_attention.cu, sigmoid_attention.cu and diff_attention.cu, the plain twins.  What bounds
-// each, and one 2,048-token prompt of 16 heads over 8 KV heads (tiles of mma.sync before, us):
-//   W_OPTIONS  as W_PLAIN, window 1,024: 109 -> 56;   W_TABLE  a table entry read from shared memory per score, twice: 139 -> 77
-//   W_SIGMOID  an ex2 and half a reciprocal per score in one pass: 120 -> 96;   W_DIFF  two and a half of them: 232 -> 123
+// each, and one 2,048-token prompt of 16 heads over 8 KV heads (the kernels on mma.sync first, us):
+//   W_OPTIONS  as W_PLAIN, window 1,024: 111, 58;   W_TABLE  a table entry read from shared memory per score, twice: 120, 74
+//   W_SIGMOID  an ex2 and a reciprocal per score in one pass: 119, 98;   W_DIFF  two of each and a half: 222, 128
+// (one reciprocal for two scores, the fast division for the gates and ex2 for exp2f in W_DIFF, all of them less exact, would
+// be 56, 77, 96 and 123)
 enum { W_PLAIN = 0, W_OPTIONS = 1, W_TABLE = 2, W_SIGMOID = 3, W_DIFF = 4 };
 struct WideExtra {
     long long out_stride;          // elements from one token's row of `out` to the next

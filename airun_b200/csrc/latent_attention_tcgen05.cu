@@ -12,8 +12,8 @@
 //              values are free as soon as S has read them, so the next tile's arrive, and its S is begun, while the softmax
 //              works; the value blocks are free after O;
 //   warps 2-5: a thread a row: running maximum and sum in float32 (exp2), P as bfloat16 over S, O rescaled lazily.
-// The mma.sync kernel reads the whole tile of cached rows from shared memory once per warp, for 16 rows: 515 us for one
-// 1,536-token prompt of 16 heads (R = 512, rd = 64); here 171 us.  What bounds it now is bringing 72 KB of cached rows into
+// The mma.sync kernel reads the whole tile of cached rows from shared memory once per warp, for 16 rows: 509 us for one
+// 1,536-token prompt of 16 heads (R = 512, rd = 64), 323 for three of 811 to 540; here 168 and 122 us.  What bounds it now is bringing 72 KB of cached rows into
 // an SM for 128 rows of queries.
 //
 // Every mbarrier wait is bounded (about two seconds); on a time-out the kernel sets an error bit, stops working, frees its

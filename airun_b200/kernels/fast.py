@@ -248,12 +248,12 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, glu
 
 
 def _few_rows(M: int, N: int, K: int) -> bool:
-    """Whether a product of M tokens with an [N, K] weight goes to csrc/gemm_rows.cu.  Both kernels timed in graphs, B200, us
-    (tcgen05, rows).  Up to 8 tokens, as long as its blocks of 32 weight rows run in one wave of two an SM: 8 tokens x
-    [2048, 2048] 7.2, 4.3; [4096, 12288] 21.7, 19.0; [6144, 4096] 12.2, 11.5; a second wave costs more than the ring of
-    the tcgen05 kernel: [12288, 2048] 11.5, 12.4; [151936, 4096] 186, 203.  From 9 tokens a block reads twice the
-    tokens and both kernels are equal at 16 M weights ([4096, 4096] 9.9, 10.0; [2048, 2048] 7.5, 5.1; [6144, 4096] 12.3,
-    14.6)."""
+    """Whether a product of M tokens with an [N, K] weight goes to csrc/gemm_rows.cu.  Both kernels as they are launched, one
+    product behind another in graphs, B200, us (tcgen05, rows).  Up to 8 tokens, as long as its blocks of 32 weight rows run
+    in one wave of two an SM: 8 tokens x [2048, 2048] 7.1, 4.3; [4096, 12288] 21.9, 19.7; [6144, 4096] 12.1, 12.4; a second
+    wave costs more than the ring of the tcgen05 kernel: [12288, 2048] 11.7, 12.8; [151936, 4096] 189, 207.  From 9 tokens a
+    block reads twice the tokens, and the line lies at 16 M weights: 16 tokens x [4096, 4096] 9.8, 10.4; [2048, 2048] 7.1,
+    4.9; [6144, 4096] 12.1, 15.0."""
     if M > ROWS_MAX or "gemm_rows" in DISABLED:
         return False
     one_wave = (N + 31) // 32 <= 2 * machine().sms
@@ -832,6 +832,8 @@ def latent_attention_bf16(ctx, qlat, out, cache, part, gate: Optional[torch.Tens
     return True
 
 
+# 16 heads over a latent of 512, mma.sync and tcgen05, us: a prompt of 64 tokens 33 and 13, behind 1,000 others 186 and 72; of 16
+# tokens 28 and 13, 176 and 67.  The line could lie lower; portions below it are rare and short.
 LATENT_TC_MIN_TOKENS = 64
 
 
@@ -878,6 +880,10 @@ def linear_act_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mo
 
 
 PROMPT_KINDS = dict(options=1, table=2, sigmoid=3)     # of csrc/attention_tcgen05.cu: airun_attn_prefill_kinds
+# Where the two kernels meet for prompts without a context, 16 heads over 8, mma.sync and tcgen05, us: 128 tokens with options 14.3
+# and 11.7, with a table 14.3 and 16.5, without softmax 13.0 and 13.3, differential 20.5 and 21.6; 192 tokens 17.0 and 13.3, 17.4
+# and 19.5, 15.9 and 16.8, 26.6 and 28.2; 256 tokens 20.1 and 13.3, 20.5 and 19.0, 19.1 and 16.9, 32.3 and 27.7.  Behind 1,000
+# others tcgen05 takes 0.5 to 0.7 of the time from 16 tokens on, but the step's tokens are all that is known here.
 PROMPT_TC_MIN_TOKENS = 192
 
 

@@ -174,7 +174,7 @@ class RoutedExperts(FeedForward):
         return delta
 
 
-def grouped_linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor, tokens: int) -> None:
+def grouped_linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor, tokens: Optional[int] = None) -> None:
     """Rows seg[e] .. seg[e+1]-1 of x times w[e]^T: x [M, K], w [E, N, K], out [M, N], seg int32 [E+1] on the device.
     bfloat16 operands go to the tensor-core kernel where it takes the sizes, everything else to the plain one."""
     if x.dtype == torch.bfloat16:

@@ -97,6 +97,7 @@ def test_which_products_of_segments_read_their_matrices_per_few_rows(monkeypatch
     """By the rows a segment has on average and by the rows it can have: with many tokens, all of which may choose one expert, the
     matrices are read once (csrc/gemm_tcgen05.cu)."""
     from airun_b200.kernels import fast
+    from airun_b200.parts.moe import grouped_linear
     went = []
     monkeypatch.setattr(fast, "_cuda", lambda *a: None)
     monkeypatch.setattr(fast, "_check", lambda *a: None)
@@ -109,3 +110,6 @@ def test_which_products_of_segments_read_their_matrices_per_few_rows(monkeypatch
         out, seg = torch.zeros(tokens * top, 32), torch.zeros(E + 1, dtype=torch.int32)
         went.clear()
         assert fast.grouped_linear_bf16(ctx, x, w, out, seg, tokens=tokens) and went == [want]
+        went.clear()
+        grouped_linear(ctx, x, w, out, seg)                  # without the number of tokens: by the average alone
+        assert went == ["gemm_rows" if tokens * top <= fast.GROUPED_ROWS_MAX * E else "gemm_tcgen05"]

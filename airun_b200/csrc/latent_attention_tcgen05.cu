@@ -314,7 +314,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                     v[i] = __uint_as_float(raw[i]);
                     if (!full) {
                         const int j = j0 + i;
-                        if (!(j <= pos && (p.window == 0 || pos - j < p.window))) v[i] = NEG_BIG;
+                        if (!(j <= pos && (p.window == 0 || pos - j < p.window))) v[i] = -INFINITY;      // hidden under every scale above 0
                     }
                 }
                 float r0 = NEG_BIG, r1 = NEG_BIG, r2 = NEG_BIG, r3 = NEG_BIG;
@@ -340,7 +340,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                     l *= f;
                     if (raise) m = mx;
                 }
-                // hidden keys hold -1e30 and come out as 0; only a row that has seen no key at all must not add its -m
+                // hidden keys are minus infinity and come out as 0; a row that has seen no key at all must not add its -m
                 const float nm = m > 0.5f * NEG_BIG ? -m : 0.0f;
                 const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(nm, nm);
                 float2 rs2 = make_float2(0.0f, 0.0f);

@@ -246,10 +246,10 @@ def test_what_the_kernel_does_not_take_stays_with_the_other():
 
 
 @gpu
-@pytest.mark.parametrize("scale", [-0.11, 0.0])
+@pytest.mark.parametrize("scale", [-0.11, 0.0, 1e-32])
 def test_latent_with_a_scale_that_is_not_positive(scale):
-    """The kernel takes a row's largest score before it scales: such a scale goes to the other kernel, and the result is the plain
-    kernel's (tolerance as above)."""
+    """The kernel takes a row's largest score before it scales: a scale of 0 or less goes to the other kernel, and hidden keys stay
+    hidden under the smallest ones (the result is the plain kernel's, tolerance as above)."""
     from airun_b200.kernels import fast, ops
     H, R, rd, spans = 4, 128, 64, [(0, 200), (70, 130)]
     g = torch.Generator().manual_seed(5)

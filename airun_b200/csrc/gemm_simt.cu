@@ -8,7 +8,7 @@
 // crates/airun-core/src/runtime.rs:5344-5352).  The tile kernels form every
 // output element as one sequential sum over k; the kernel for few float32 rows
 // cuts it over the block in a fixed order.
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 #define TM 64
 #define TN 64
@@ -309,6 +309,340 @@ __global__ __launch_bounds__(256, 2) void gemm_f32_kernel(
     }
 }
 
+// ------------------------------------------------------------------ float32 on the tensor cores, without rounding an operand
+// More than a few rows of float32 products are bound by the FMA pipe, so they go to the tensor cores with every operand
+// cut into three bfloat16 parts whose sum it is: the leading 8 bits of the significand (cut off, so that nothing overflows), the
+// next 8 (rounded) and the remaining 8, which is the whole significand of 24 bits down to 2^-133.  Of the nine products of parts the six
+// of 2^-17 and more are formed, x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; the three left out are below 2^-23 of x w, of either sign, half a
+// unit of the last place (the split of S. Markidis et al., IPDPS Workshops 2018, in bfloat16 and three parts: G. Henry, P. T. P. Tang and
+// A. Heinecke, ARITH 2019).  The tensor cores add up in float32 but cut off where float32 rounds, so they hold a sum over 64 k-values at most, the
+// small products first; the sums of these steps are added up in registers, rounded.
+//
+// A tile is 128 weight rows by `bn` rows of A (16 .. 128), its K range cut into `ks` slices that run as one cluster and are added up in order
+// through distributed shared memory.
+//   warps 0-7  : read the step sums from tensor memory (a quadrant of lanes each, every other 16 columns) and add them up; they store the tile;
+//   warps 8-15 : cut the 64 k-values of a step of every row of both operands.  The parts of W go to tensor memory, those of A to shared memory
+//                (128-byte swizzle): with both there, what the products, the cutting and the loads move through shared memory is the bound (390 KB a
+//                step of 128 x 112, 3,300 clocks for 1,540 of products).  They load nothing themselves: their fence would wait for loads under way;
+//   warp 16    : one thread issues the 24 tcgen05.mma of a step (in a warp that adds up, no product would run while it does);
+//   warp 17    : one thread issues the TMA loads, two steps ahead.
+// An infinite operand has no parts; its row is noted and its results are formed by a plain loop.
+#define XT 128                    // weight rows of a tile
+#define XB 128                    // most rows of A
+#define XK 64                     // k-values of a step
+#define X_STAGES 2                // steps of parts
+#define X_RING 2                  // steps of operands on their way to the threads that cut them
+#define X_SUM_WARPS 8
+#define X_CUT_WARPS 8
+#define X_THREADS (32 * (X_SUM_WARPS + X_CUT_WARPS + 2))   // 18 warps: 96 registers a thread
+#define X_PART (XB * XK * 2)      // bytes of one part of A
+#define X_WCOLS (XK / 2)          // columns of tensor memory of one part of W, after the two step sums
+#define X_STAGE (3 * X_PART)
+#define X_SUM_SPACE (XT * XB * 4) // the slices' sums take the place of the stages and of the ring
+#define X_RING_STEP ((XT + XB) * XK * 4)
+#define X_SMEM (X_STAGES * X_STAGE + X_RING * X_RING_STEP + 1024)
+static_assert(X_SUM_SPACE <= X_STAGES * X_STAGE + X_RING * X_RING_STEP && X_STAGE % 1024 == 0, "");
+
+// The product with the rows of A (here W) in tensor memory: 8 columns of 32 bits hold 16 k-values of a lane's row.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint2 (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[1].x),
+                 "r"(v[1].y), "r"(v[2].x), "r"(v[2].y), "r"(v[3].x), "r"(v[3].y) : "memory");
+}
+
+// One float4's three parts, packed to bfloat16 (8 bytes each).  False when one of the values is infinite or not a number.
+__device__ __forceinline__ bool f32_parts(const float4& v, uint2 (&part)[3]) {
+    const uint32_t x[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+    const float2 minus = make_float2(-1.0f, -1.0f);
+    float2 r[2];
+    uint32_t m[2], l[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {                              // packed: x - h is exact, as a multiply-add too
+        const float2 h = make_float2(__uint_as_float(x[2 * i] & 0xffff0000u), __uint_as_float(x[2 * i + 1] & 0xffff0000u));
+        r[i] = __ffma2_rn(h, minus, i == 0 ? make_float2(v.x, v.y) : make_float2(v.z, v.w));
+        const __nv_bfloat162 b = __floats2bfloat162_rn(r[i].x, r[i].y);
+        m[i] = *reinterpret_cast<const uint32_t*>(&b);
+        const float2 g = make_float2(__uint_as_float(m[i] << 16), __uint_as_float(m[i] & 0xffff0000u));
+        const float2 d = __ffma2_rn(g, minus, r[i]);
+        const __nv_bfloat162 c = __floats2bfloat162_rn(d.x, d.y);
+        l[i] = *reinterpret_cast<const uint32_t*>(&c);
+    }
+    part[0] = make_uint2(__byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x7632));
+    part[1] = make_uint2(m[0], m[1]);
+    part[2] = make_uint2(l[0], l[1]);
+    const float t = (r[0].x + r[0].y) + (r[1].x + r[1].y);     // infinity less itself is not a number
+    return t == t;
+}
+__device__ __forceinline__ bool any_inf(const float4& v) { return isinf(v.x) || isinf(v.y) || isinf(v.z) || isinf(v.w); }
+
+// The results of a tile that have an infinite operand, each by itself: columns first, first + step, .. of the tile.
+__device__ __noinline__ void f32_infinite_rows(const float* A, const float* W, float* C, int K, long long lda, long long ldw, long long ldc, int m0,
+                                               int cols, int n0, int rows, const uint32_t* marks, int first, int step) {
+    uint32_t any = 0;
+    for (int i = 0; i < 8; ++i) any |= marks[i];
+    if (any == 0) return;
+    for (int i = threadIdx.x; i < cols * rows; i += blockDim.x) {
+        const int col = i / rows, r = i % rows;
+        if (col % step != first || !(((marks[r >> 5] >> (r & 31)) | (marks[4 + (col >> 5)] >> (col & 31))) & 1u)) continue;
+        const float *a = A + (size_t)(m0 + col) * lda, *w = W + (size_t)(n0 + r) * ldw;
+        float v = 0.0f;
+        for (int k = 0; k < K; ++k) v = fmaf(a[k], w[k], v);
+        C[(size_t)(m0 + col) * ldc + n0 + r] = v;
+    }
+}
+
+template <int FORM>                                            // 0 plain, 2 grouped
+__global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const float* A, const float* __restrict__ W,
+    float* __restrict__ C, int M, int N, int K, long long lda, long long ldw, long long ldc, GemmExtra ex, int bn, int ks, int* err) {
+    pdl_trigger();
+    extern __shared__ uint8_t x_raw[];
+    uint8_t* tiles = (uint8_t*)(((uintptr_t)x_raw + 1023) & ~(uintptr_t)1023);
+    // full, empty of the stages of parts; full, empty of the two step sums; landed, read of the ring
+    __shared__ __align__(8) uint64_t bars[2 * X_STAGES + 4 + 2 * X_RING];
+    __shared__ uint32_t tmem_slot, inf_rows[2][4], all_rows[8];    // infinite operands: bit r of [0] weight row, of [1] row of A
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slice = blockIdx.z, n0 = blockIdx.x * XT;
+    int m0 = blockIdx.y * bn, m_end = M, set_w = 0;
+    if (FORM == 2) {
+        pdl_wait();                                            // the segments are the kernel's in front
+        int tile = blockIdx.y, e = 0, found = 0;
+        for (; e < ex.n_seg; ++e) {
+            const int lo = ex.seg[e], hi = ex.seg[e + 1];
+            const int n = (hi - lo + bn - 1) / bn;
+            if (tile < n) { m0 = lo + tile * bn; m_end = min(M, hi); found = 1; break; }
+            tile -= n;
+        }
+        if (!found) return;
+        W += (size_t)e * ex.sw;
+        set_w = e;
+    }
+    const int steps_all = (K + XK - 1) / XK, per = (steps_all + ks - 1) / ks;
+    const int step0 = min(slice * per, steps_all), steps = min(step0 + per, steps_all) - step0;
+    const uint32_t full = smem_u32(bars), empty = full + 8 * X_STAGES, sfull = empty + 8 * X_STAGES, sempty = sfull + 16, landed = sempty + 16, taken = landed + 8 * X_RING;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < X_STAGES; ++s) { mbar_init(full + 8 * s, X_CUT_WARPS); mbar_init(empty + 8 * s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(sfull + 8 * b, 1); mbar_init(sempty + 8 * b, X_SUM_WARPS); }
+        for (int r = 0; r < X_RING; ++r) { mbar_init(landed + 8 * r, 1); mbar_init(taken + 8 * r, X_CUT_WARPS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x < 8) (&inf_rows[0][0])[threadIdx.x] = 0;
+    if (warp == X_SUM_WARPS) tmem_alloc(smem_u32(&tmem_slot), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    const int cols = min(bn, m_end - m0);
+    float* sums = reinterpret_cast<float*>(tiles);             // of this slice, [column][128], once the products are done
+    if (warp < X_SUM_WARPS) {
+        const int quad = warp & 3, half = warp >> 2;
+        float2 acc[XB / 4];                                    // columns 16 (2 j + half) + 2 i and the next at [8 j + i]
+#pragma unroll
+        for (int i = 0; i < XB / 4; ++i) acc[i] = make_float2(0.0f, 0.0f);
+        const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
+        for (int it = 0; it < steps; ++it) {
+            const int buf = it & 1;
+            if (!mbar_wait(sfull + 8 * buf, (it >> 1) & 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+            tc_fence_after();
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < XB / 32; ++j) {
+                const int c = 16 * (2 * j + half);
+                if (c >= bn) break;
+                uint32_t r[16];
+                tmem_ld_async(lanes + buf * XB + c, r);
+                tmem_wait(r);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[8 * j + i] = __fadd2_rn(acc[8 * j + i], make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sempty + 8 * buf) : "memory");
+        }
+        // the last step's products are done, so the stages may be written over
+        const int r = quad * 32 + lane;
+        if (ks > 1) {
+#pragma unroll
+            for (int j = 0; j < XB / 32; ++j) {
+                const int c0 = 16 * (2 * j + half);
+                if (c0 >= bn) break;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sums[(c0 + i) * XT + r] = i & 1 ? acc[8 * j + i / 2].y : acc[8 * j + i / 2].x;
+            }
+        } else if (n0 + r < N) {
+            float* c = C + (size_t)(m0 + 16 * half) * ldc + n0 + r;
+#pragma unroll
+            for (int j = 0; j < XB / 32; ++j, c += 32 * ldc) {
+                const int n = cols - 16 * (2 * j + half);
+                float* o = c;
+#pragma unroll
+                for (int i = 0; i < 16; ++i, o += ldc)
+                    if (i < n) *o = i & 1 ? acc[8 * j + i / 2].y : acc[8 * j + i / 2].x;
+            }
+        }
+    } else if (warp < X_SUM_WARPS + X_CUT_WARPS) {
+        // W: this thread's row is lane `lane` of its quadrant, 32 of the step's k-values.  A: rows row + 32 i, k-values 4 q .. 4 q + 3 and 32 more on.
+        // The ring holds boxes of 32 k-values; 16 bytes j of a row lie at place j ^ (row % 8) (the loads' 128-byte swizzle).
+        const int t = threadIdx.x - 32 * X_SUM_WARPS, quad = warp & 3, half = t >> 7;
+        const int row = t >> 3, q = t & 7;
+        constexpr int RP = X_CUT_WARPS * 4;                    // 32: rows of a pass over A, four passes
+        static_assert(RP == 32 && XT == 128 && XB == 128 && XK == 64, "two threads a row of W, four passes over A");
+        const uint32_t w_at = half * (XT * 128) + (quad * 32 + lane) * 128, a_at = 2 * XT * 128 + row * 128 + ((q ^ (row & 7)) << 4);
+        for (int it = 0; it < steps; ++it) {
+            const int s = it % X_STAGES, g = it % X_RING;
+            if (!mbar_wait(landed + 8 * g, (it / X_RING) & 1) || !mbar_wait(empty + 8 * s, ((it / X_STAGES) & 1) ^ 1)) {
+                atomicOr(err, AIRUN_DEV_TIMEOUT);
+                break;
+            }
+            tc_fence_after();
+            __syncwarp();
+            const uint8_t* from = tiles + X_STAGES * X_STAGE + g * X_RING_STEP;
+            uint8_t* to = tiles + s * X_STAGE + row * (XK * 2) + ((q & 1) << 3);
+            // four values at a time, read, cut and stored: their chains of dependent instructions run side by side
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 v[4];
+                uint2 part[4][3];
+                bool fine[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(from + w_at + (((4 * h + i) ^ (lane & 7)) << 4));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fine[i] = f32_parts(v[i], part[i]);
+                if (!(fine[0] && fine[1] && fine[2] && fine[3]))
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (any_inf(v[i])) atomicOr(&inf_rows[0][quad], 1u << lane);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const uint2 p[4] = {part[0][j], part[1][j], part[2][j], part[3][j]};
+                    tmem_st8(tmem + ((uint32_t)(quad * 32) << 16) + 2 * XB + (3 * s + j) * X_WCOLS + 16 * half + 8 * h, p);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 v[4];
+                uint2 part[4][3];
+                bool fine[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(from + a_at + h * (XB * 128) + RP * i * 128);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fine[i] = f32_parts(v[i], part[i]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (row + RP * i >= bn) continue;
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        *reinterpret_cast<uint2*>(to + j * X_PART + RP * i * (XK * 2) + (((4 * h + (q >> 1)) ^ (row & 7)) << 4)) = part[i][j];
+                }
+                if (!(fine[0] && fine[1] && fine[2] && fine[3]))
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (row + RP * i < bn && any_inf(v[i])) atomicOr(&inf_rows[1][i], 1u << row);
+            }
+            __syncwarp();
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full + 8 * s) : "memory");
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(taken + 8 * g) : "memory");
+            }
+        }
+    } else if (warp == X_SUM_WARPS + X_CUT_WARPS && lane == 0) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(XT >> 4) << 24);
+        for (int it = 0; it < steps; ++it) {
+            const int s = it % X_STAGES, buf = it & 1;
+            if (!mbar_wait(sempty + 8 * buf, ((it >> 1) & 1) ^ 1) || !mbar_wait(full + 8 * s, (it / X_STAGES) & 1)) {
+                atomicOr(err, AIRUN_DEV_TIMEOUT);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t base = smem_u32(tiles) + s * X_STAGE;
+            constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, AP[6] = {0, 2, 1, 0, 1, 0};     // the smallest products first
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const uint32_t tw = tmem + 2 * XB + (3 * s + WP[j]) * X_WCOLS;
+                const uint64_t da = smem_desc_sw128(base + AP[j] * X_PART);
+#pragma unroll
+                for (int k = 0; k < XK / 16; ++k)
+                    umma_bf16_ts(tmem + buf * XB, tw + 8 * k, da + (uint64_t)(k * 2), idesc, (j > 0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit(empty + 8 * s);
+            umma_commit(sfull + 8 * buf);
+        }
+    } else if (lane == 0) {
+        const uint32_t ring = smem_u32(tiles) + X_STAGES * X_STAGE;
+        auto ask = [&](int it, bool w, bool a) {
+            const uint32_t to = ring + (it % X_RING) * X_RING_STEP, bar = landed + 8 * (it % X_RING);
+            const int k = (step0 + it) * XK;
+            if (w) {
+                mbar_expect_tx(bar, (XT + bn) * XK * 4);
+                tma_load_3d(to, &map_w, bar, k, n0, set_w);
+                tma_load_3d(to + XT * 128, &map_w, bar, k + 32, n0, set_w);
+            }
+            if (a) {
+                tma_load_3d(to + 2 * XT * 128, &map_a, bar, k, m0, 0);
+                tma_load_3d(to + (2 * XT + XB) * 128, &map_a, bar, k + 32, m0, 0);
+            }
+        };
+        const int first = min(steps, X_RING);
+        for (int it = 0; it < first; ++it) ask(it, true, false);
+        if (FORM != 2) pdl_wait();
+        for (int it = 0; it < first; ++it) ask(it, false, true);
+        for (int it = X_RING; it < steps; ++it) {
+            if (!mbar_wait(taken + 8 * (it % X_RING), ((it / X_RING) & 1) ^ 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+            ask(it, true, true);
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();                                           // every step has been added up: no product is under way any more
+    if (warp == X_SUM_WARPS) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+    if (ks == 1) {
+        f32_infinite_rows(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), &inf_rows[0][0], 0, 1);
+        return;
+    }
+    // the slices of the tile are added up in order, every CTA taking every ks-th column
+    cluster_sync_all();
+    {
+        const int r = threadIdx.x & (XT - 1);
+        if (n0 + r < N) {
+            for (int col = slice + ks * (threadIdx.x / XT); col < cols && threadIdx.x < 4 * XT; col += ks * 4) {
+                const uint32_t mine = smem_u32(sums + col * XT + r);
+                float v[8];                                    // all slices are asked for before one is added
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = q < ks ? ld_cluster_f32(map_to_cta(mine, q)) : 0.0f;
+                float t = v[0];
+#pragma unroll
+                for (int q = 1; q < 8; ++q) if (q < ks) t += v[q];
+                C[(size_t)(m0 + col) * ldc + n0 + r] = t;
+            }
+        }
+        if (threadIdx.x < 8) {                                 // the rows noted by all slices
+            uint32_t marks = 0;
+            for (int q = 0; q < ks; ++q) marks |= __float_as_uint(ld_cluster_f32(map_to_cta(smem_u32(&inf_rows[0][0] + threadIdx.x), q)));
+            all_rows[threadIdx.x] = marks;
+        }
+        __syncthreads();
+        f32_infinite_rows(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), all_rows, slice, ks);
+    }
+    __syncwarp();
+    cluster_sync_all();                                        // nobody leaves while a peer may still read its memory
+}
+
 template <int FORM, int MR>
 static void launch_gemv(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
                         int gy, int gz, const GemmExtra& ex, cudaStream_t stream) {
@@ -319,11 +653,76 @@ static void launch_gemv(const float* A, const float* W, float* C, int M, int N, 
         airun_launch(gemv_f32_kernel<MR, 4, FORM>, dim3(ceil_div_i(N, 4), gy, gz), dim3(32 * GV_WARPS), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, ex);
 }
 
+// How many clusters of `ks` CTAs the GPU holds at once, one CTA an SM.
+static int f32_clusters(int ks) {
+    static int known[64][9];
+    int dev = 0, n = 0;
+    if (ks < 2 || ks > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if ((n = __atomic_load_n(&known[dev][ks], __ATOMIC_RELAXED)) != 0) return n > 0 ? n : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, ks);
+    cfg.blockDim = dim3(X_THREADS);
+    cfg.dynamicSmemBytes = X_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = ks;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_f32_parts_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_f32_parts_kernel<0>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    __atomic_store_n(&known[dev][ks], n > 0 ? n : -1, __ATOMIC_RELAXED);
+    return n;
+}
+
+// Rows of A in a tile and K slices of the products on the tensor cores, by the time they take (B200, us): 1.26 a step of 64 k-values, 0.1 more at 128 rows;
+// bringing the slices together 2 to 7, the more the larger the share of the tile's columns that a CTA adds up.  24 rows x [1024, 1024] in 1, 2, 4 and 8
+// slices 22.9, 14.9, 9.9, 7.6; 642 x [1024, 2048] as 112 tiles of 48 rows 43.5, as 56 of 96 rows in two slices 30.2; 642 x [3072, 1024] in tiles of
+// 64, 96, 112 and 128 rows 48.3, 48.9, 25.5, 26.0.
+struct F32Plan { int bn, ks; };
+static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
+    const int sms = airun_sm_count(), steps = ceil_div_i(K, XK);
+    const long long nt = (N + XT - 1) / XT * sets;
+    F32Plan best = {XB, 1};
+    double best_us = 1e30;
+    for (int bn = 16; bn <= XB; bn += 16) {
+        const long long tiles = nt * ((rows + bn - 1) / bn);
+        for (int ks = 1; ks <= 8 && (ks == 1 || 2 * ks <= steps); ++ks) {
+            const int per = (steps + ks - 1) / ks;
+            if ((steps + per - 1) / per != ks || (ks > 1 && tiles > f32_clusters(ks))) continue;   // an empty slice, or not all resident
+            const double step = 1.25 + 0.0008 * bn, merge = ks > 1 ? 1.2 + bn * (0.015 + 0.06 / ks) : 0.0;
+            const double us = (double)((tiles * ks + sms - 1) / sms) * per * step + merge;
+            if (us < best_us) { best_us = us; best = {bn, ks}; }
+        }
+    }
+    return best;
+}
+
+// Fewest k-values of a product on the tensor cores.  Error against 64 bits (2-norm), FMA kernel and parts: operands of either sign, K = 128, 512, 1024,
+// 2048, 8192: 1.1e-7, 2.1e-7, 2.9e-7, 4.1e-7, 8.1e-7 and 0.9e-7, 1.0e-7, 1.1e-7, 1.3e-7, 1.3e-7; operands of one sign: 0.5e-7, 0.85e-7, 1.3e-7, 1.6e-7, 3.1e-7 and
+// 0.9e-7, 0.93e-7, 1.1e-7, 1.1e-7, 0.9e-7, so below 1,024 the tensor cores' cut-off sums would be the less exact ones there.
+#define X_MIN_K 1024
+// A tensor map of `sets` row-major float32 matrices [rows][K], rows `ld` and matrices `set` elements apart, boxes of box_rows x 32.
+static bool f32_map(CUtensorMap* out, const float* ptr, long long K, long long rows, long long sets, long long ld, long long set, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)sets};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)(sets > 1 ? set : ld) * 4};
+    cuuint32_t box[3] = {32, (cuuint32_t)box_rows, 1}, estr[3] = {1, 1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // True when the aligned float32 kernels took the product.  Up to 16 rows (an average of up to four a segment) the bytes
 // of W are the bound; from there on a row group's further reading of W from the L2 cache costs more than the tiles.
+// Long ones of those go to the tensor cores where the caller gives the error word that their bounded waits need, the others to the FMA pipe.
 template <int FORM>
 static bool f32_product(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int M, int N, int K, long long lda,
-                        long long ldw, long long ldc, int batch, const GemmExtra& ex, cudaStream_t stream) {
+                        long long ldw, long long ldc, int batch, const GemmExtra& ex, int* err, cudaStream_t stream) {
     if (a_dtype != AIRUN_DT_F32 || w_dtype != AIRUN_DT_F32 || c_dtype != AIRUN_DT_F32) return false;
     if ((K | lda | ldw | ex.sa | ex.sw) & 3 || ((uintptr_t)A | (uintptr_t)W) & 15) return false;
     const float *a = (const float*)A, *w = (const float*)W;
@@ -339,10 +738,35 @@ static bool f32_product(const void* A, int a_dtype, const void* W, int w_dtype, 
         else launch_gemv<FORM, 8>(a, w, c, M, N, K, lda, ldw, ldc, gy, gz, ex, stream);
         return true;
     }
+    static unsigned long long configured = 0;
+    [[maybe_unused]] static unsigned long long configured_x = 0;
+    if constexpr (FORM != 1) {
+        if (err && K >= X_MIN_K) {
+            const F32Plan plan = f32_plan(FORM == 2 ? ceil_div_i(M, segs) : M, segs, N, K);
+            const long long gy = (M + plan.bn - 1) / plan.bn + (FORM == 2 ? segs : 0);
+            CUtensorMap mw, ma;
+            bool ready = gy <= 65535 && f32_map(&mw, w, K, N, segs, ldw, ex.sw, XT) && f32_map(&ma, a, K, M, 1, lda, 0, plan.bn);
+            if (ready && first_on_device(configured_x) &&
+                cudaFuncSetAttribute(gemm_f32_parts_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, X_SMEM) != cudaSuccess) {
+                cudaGetLastError();
+                configured_x = 0;
+                ready = false;
+            }
+            if (ready) {
+                const dim3 grid(ceil_div_i(N, XT), (unsigned)gy, (unsigned)plan.ks);
+                if (plan.ks > 1)
+                    airun_launch_cluster(gemm_f32_parts_kernel<FORM>, grid, dim3(X_THREADS), X_SMEM, stream, (unsigned)plan.ks, mw, ma, a, w, c, M, N,
+                                         K, lda, ldw, ldc, ex, plan.bn, plan.ks, err);
+                else
+                    airun_launch(gemm_f32_parts_kernel<FORM>, grid, dim3(X_THREADS), X_SMEM, stream, mw, ma, a, w, c, M, N, K, lda, ldw, ldc, ex,
+                                 plan.bn, 1, err);
+                return true;
+            }
+        }
+    }
     const dim3 grid(ceil_div_i(N, FT), ceil_div_i(M, FT) + (FORM == 2 ? segs : 0), FORM == 1 ? batch : 1);
     if (grid.y > 65535) return false;
     constexpr int SMEM = F_STAGES * 2 * FT * FS * (int)sizeof(float);
-    static unsigned long long configured = 0;
     if (first_on_device(configured) &&
         cudaFuncSetAttribute(gemm_f32_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
         cudaGetLastError();
@@ -353,16 +777,16 @@ static bool f32_product(const void* A, int a_dtype, const void* W, int w_dtype, 
     return true;
 }
 
-// dtypes: a_dtype == w_dtype in {f32, bf16}; c_dtype in {f32, bf16}.
+// dtypes: a_dtype == w_dtype in {f32, bf16}; c_dtype in {f32, bf16}.  err: error word of the device, or null (see f32_product).
 AIRUN_EXPORT int airun_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype,
                                  void* C, int c_dtype, int M, int N, int K,
-                                 long long lda, long long ldw, long long ldc, cudaStream_t stream) {
+                                 long long lda, long long ldw, long long ldc, int* err, cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N) return AIRUN_ERR_ARG;
     if (M == 0) return AIRUN_OK;
     dim3 grid(ceil_div_i(N, TN), ceil_div_i(M, TM));
     if (grid.y > 65535) return AIRUN_ERR_ARG;
     GemmExtra ex = {};
-    if (f32_product<0>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, 1, ex, stream)) return airun_launch_status();
+    if (f32_product<0>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, 1, ex, err, stream)) return airun_launch_status();
 #define LAUNCH(TA, TW, TC) \
     airun_launch(gemm_simt_kernel<TA, TW, TC, 0>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, (TC*)C, M, N, K, lda, ldw, ldc, ex)
     if (a_dtype == AIRUN_DT_F32 && w_dtype == AIRUN_DT_F32 && c_dtype == AIRUN_DT_F32) LAUNCH(float, float, float);
@@ -383,7 +807,7 @@ AIRUN_EXPORT int airun_gemm_simt_batched(const void* A, int a_dtype, const void*
     if (grid.y > 65535) return AIRUN_ERR_ARG;
     GemmExtra ex = {};
     ex.sa = sa; ex.sw = sw; ex.sc = sc;
-    if (f32_product<1>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, batch, ex, stream)) return airun_launch_status();
+    if (f32_product<1>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, batch, ex, nullptr, stream)) return airun_launch_status();
 #define LAUNCH(TA, TW, TC) \
     airun_launch(gemm_simt_kernel<TA, TW, TC, 1>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, (TC*)C, M, N, K, lda, ldw, ldc, ex)
     if (a_dtype == AIRUN_DT_F32 && w_dtype == AIRUN_DT_F32 && c_dtype == AIRUN_DT_F32) LAUNCH(float, float, float);
@@ -398,14 +822,14 @@ AIRUN_EXPORT int airun_gemm_simt_batched(const void* A, int a_dtype, const void*
 // segment e times W + e*sw.  The launch covers ceil(M / TM) + n_seg row tiles, which is enough for every cut.
 AIRUN_EXPORT int airun_gemm_simt_grouped(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype,
                                          int M, int N, int K, long long lda, long long ldw, long long ldc,
-                                         const int32_t* seg, int n_seg, long long sw, cudaStream_t stream) {
+                                         const int32_t* seg, int n_seg, long long sw, int* err, cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N || !seg || n_seg <= 0) return AIRUN_ERR_ARG;
     if (M == 0) return AIRUN_OK;
     dim3 grid(ceil_div_i(N, TN), ceil_div_i(M, TM) + n_seg);
     if (grid.y > 65535) return AIRUN_ERR_ARG;
     GemmExtra ex = {};
     ex.sw = sw; ex.seg = seg; ex.n_seg = n_seg;
-    if (f32_product<2>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, 1, ex, stream)) return airun_launch_status();
+    if (f32_product<2>(A, a_dtype, W, w_dtype, C, c_dtype, M, N, K, lda, ldw, ldc, 1, ex, err, stream)) return airun_launch_status();
 #define LAUNCH(TA, TW, TC) \
     airun_launch(gemm_simt_kernel<TA, TW, TC, 2>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, (TC*)C, M, N, K, lda, ldw, ldc, ex)
     if (a_dtype == AIRUN_DT_F32 && w_dtype == AIRUN_DT_F32 && c_dtype == AIRUN_DT_F32) LAUNCH(float, float, float);

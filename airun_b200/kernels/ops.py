@@ -803,9 +803,10 @@ def softmax_attention(q: torch.Tensor, out: torch.Tensor, cache, ctx, nh: int, n
 
 
 # ---------------------------------------------------------------- products
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T on the CUDA cores, float32 accumulation."""
-    _cuda(a, w, out)
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, err: Optional[torch.Tensor] = None) -> None:
+    """out[M, N] = a[M, K] @ w[N, K]^T, float32 accumulation.  On the CUDA cores; with an error word, more than a few aligned
+    float32 rows of 1,024 values on go to the tensor cores in parts that keep all 24 bits of both operands (csrc/gemm_simt.cu)."""
+    _cuda(a, w, out, err)
     _need(a.dim() == 2 and w.dim() == 2 and out.dim() == 2, "gemm takes 2-d tensors")
     M, K = a.shape
     N = w.shape[0]
@@ -814,10 +815,10 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _need(a.dtype == w.dtype, "gemm operands must share a type")
     f = _fn("gemm_simt", "airun_gemm_simt",
             [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
-             c_longlong, c_longlong, c_longlong, c_void_p])
+             c_longlong, c_longlong, c_longlong, c_void_p, c_void_p])
     _check(f(_p(a), _dt(a), _p(w), _dt(w), _p(out), _dt(out), M, N, K,
              a.stride(0) if M > 1 else max(K, a.stride(0)), w.stride(0) if N > 1 else max(K, w.stride(0)),
-             out.stride(0) if M > 1 else max(N, out.stride(0)), _stream()), "gemm_simt")
+             out.stride(0) if M > 1 else max(N, out.stride(0)), _p(err), _stream()), "gemm_simt")
 
 
 def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
@@ -839,10 +840,11 @@ def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
              B, a.stride(1), w.stride(0), out.stride(1), _stream()), "gemm_simt_batched")
 
 
-def gemm_simt_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor) -> None:
+def gemm_simt_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: torch.Tensor,
+                      err: Optional[torch.Tensor] = None) -> None:
     """Rows seg[e] .. seg[e+1]-1 of a [M, K] times w[e]^T (w [E, N, K]) into the same rows of out [M, N]; ``seg`` is
-    int32 [E + 1] on the device.  Rows from seg[E] on are left as they are."""
-    _cuda(a, w, out, seg)
+    int32 [E + 1] on the device.  Rows from seg[E] on are left as they are.  ``err``: see ``gemm_simt``."""
+    _cuda(a, w, out, seg, err)
     _need(a.dim() == 2 and w.dim() == 3 and out.dim() == 2 and a.is_contiguous() and w.is_contiguous() and out.is_contiguous(),
           "the grouped product takes contiguous a [M, K], w [E, N, K], out [M, N]")
     M, K = a.shape
@@ -851,8 +853,8 @@ def gemm_simt_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg: 
     _need(seg.dtype == torch.int32 and seg.numel() >= E + 1 and seg.is_contiguous(), "seg must be int32 [E + 1]")
     f = _fn("gemm_simt", "airun_gemm_simt_grouped",
             [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-             c_void_p, c_int, c_longlong, c_void_p])
-    _check(f(_p(a), _dt(a), _p(w), _dt(w), _p(out), _dt(out), M, N, K, K, K, N, _p(seg), E, N * K, _stream()),
+             c_void_p, c_int, c_longlong, c_void_p, c_void_p])
+    _check(f(_p(a), _dt(a), _p(w), _dt(w), _p(out), _dt(out), M, N, K, K, K, N, _p(seg), E, N * K, _p(err), _stream()),
            "gemm_simt_grouped")
 
 

@@ -1,7 +1,8 @@
 """Matrix products y = x W^T of the projections.
 
-``linear`` picks the kernel by operand type and shape: float32 operands always
-run on the CUDA cores with float32 accumulation (the true 32-bit path);
+``linear`` picks the kernel by operand type and shape: float32 operands keep all
+their bits (the true 32-bit path: FMA kernels, and for many long rows the tensor
+cores with each operand in three parts whose sum it is);
 bfloat16 operands use the tensor-core kernels where one takes the sizes, and the
 plain CUDA-core kernel otherwise.  Both accumulate in float32.  Every projection is
 y = W x over row-major rows of length K, without a bias, as in the reference
@@ -26,7 +27,7 @@ def linear(ctx, x, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         from ..kernels import fast
         if fast.linear_bf16(ctx, x, w, out):
             return out
-    ops.gemm_simt(x, w, out)
+    ops.gemm_simt(x, w, out, ctx.err)
     return out
 
 

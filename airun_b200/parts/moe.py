@@ -181,7 +181,7 @@ def grouped_linear(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, seg
         from ..kernels import fast
         if fast.grouped_linear_bf16(ctx, x, w, out, seg, tokens=tokens):
             return
-    ops.gemm_simt_grouped(x, w, out, seg)
+    ops.gemm_simt_grouped(x, w, out, seg, ctx.err)
 
 
 register_part("feed_forward", "routed_experts", RoutedExperts)

@@ -78,6 +78,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (t1 - t0 > WAIT_NS) return false;
     }
 }
+// The same for a converged warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -286,7 +288,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
     uint32_t* tmem_slot = (uint32_t*)(bars + N_BARS);
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 8; ++i) mbar_init(BAR(i), 1);                 // K/V full and empty
@@ -364,14 +366,13 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it & 1;
                 const uint32_t ph = (it >> 1) & 1;
                 const int j0 = (tile_first + it) * KN;
                 // K tile
-                if (!mbar_wait(BAR(B_KEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                mbar_expect_tx(BAR(B_KFULL + s), KV_BYTES);
+                if (!mbar_wait_warp(BAR(B_KEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 const uint32_t kdst = smem_u32(smem + OFF_K + s * KV_BYTES);
                 int rows[KN / 16];
 #pragma unroll
@@ -380,48 +381,58 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
                     const int blk = j >> p.page_shift;
                     int page = (j <= pos_hi && blk < p.max_blocks) ? __ldg(bt + blk) : 0;
                     if (page < 0 || page >= p.num_pages) {
-                        if (j >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
+                        if (j >= k_first && lane == 0) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                         page = 0;
                     }
                     rows[gkey] = (((page * 2) * p.nkv + kvh) << p.page_shift) + (j & (p.page_size - 1));
                 }
+                if (elect_one()) {
+                    mbar_expect_tx(BAR(B_KFULL + s), KV_BYTES);
 #pragma unroll
-                for (int gkey = 0; gkey < KN / 16; ++gkey)
+                    for (int gkey = 0; gkey < KN / 16; ++gkey)
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(kdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(B_KFULL + s), h * 64, rows[gkey]);
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_2d(kdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(B_KFULL + s), h * 64, rows[gkey]);
+                }
+                __syncwarp();
                 // V tile
-                if (!mbar_wait(BAR(B_VEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                mbar_expect_tx(BAR(B_VFULL + s), KV_BYTES);
+                if (!mbar_wait_warp(BAR(B_VEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 const uint32_t vdst = smem_u32(smem + OFF_V + s * KV_BYTES);
                 const int vskip = p.nkv << p.page_shift;
+                if (elect_one()) {
+                    mbar_expect_tx(BAR(B_VFULL + s), KV_BYTES);
 #pragma unroll
-                for (int gkey = 0; gkey < KN / 16; ++gkey)
+                    for (int gkey = 0; gkey < KN / 16; ++gkey)
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(B_VFULL + s), h * 64, rows[gkey] + vskip);
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(B_VFULL + s), h * 64, rows[gkey] + vskip);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KN >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             const uint32_t q_addr = smem_u32(smem + OFF_Q), p_addr = smem_u32(smem + OFF_P);
-            bool ok = mbar_wait(BAR(B_PFULL), 0);          // first phase of P_full: the Q tile is in shared memory
+            bool ok = mbar_wait_warp(BAR(B_PFULL), 0);          // first phase of P_full: the Q tile is in shared memory
             auto issue_s = [&](int it) -> bool {
                 const int s = it & 1;
-                if (!mbar_wait(BAR(B_KFULL + s), (it >> 1) & 1)) return false;
-                if (!mbar_wait(BAR(B_SFREE + s), ((it >> 1) & 1) ^ 1)) return false;
+                if (!mbar_wait_warp(BAR(B_KFULL + s), (it >> 1) & 1)) return false;
+                if (!mbar_wait_warp(BAR(B_SFREE + s), ((it >> 1) & 1) ^ 1)) return false;
                 tc_fence_after();
                 const uint32_t k_addr = smem_u32(smem + OFF_K + s * KV_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t off = (k >> 2) * ROWBLK + (k & 3) * 32;
-                    umma_bf16(tmem_base + s * KN, desc_kmajor(q_addr + off), desc_kmajor(k_addr + off), idesc_s, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < HD / 16; ++k) {
+                        const uint32_t off = (k >> 2) * ROWBLK + (k & 3) * 32;
+                        umma_bf16(tmem_base + s * KN, desc_kmajor(q_addr + off), desc_kmajor(k_addr + off), idesc_s, k > 0 ? 1u : 0u);
+                    }
+                    umma_commit(BAR(B_KEMPTY + s));
+                    umma_commit(BAR(B_SFULL + s));
                 }
-                umma_commit(BAR(B_KEMPTY + s));
-                umma_commit(BAR(B_SFULL + s));
+                __syncwarp();
                 return true;
             };
             if (ok && n_tiles > 0) ok = issue_s(0);          // (a slice of a shared prefix may be empty)
@@ -429,20 +440,23 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_tc_kernel(
                 if (it + 1 < n_tiles) { ok = issue_s(it + 1); if (!ok) break; }
                 const int s = it & 1;
                 // P_it is in shared memory (phase it + 1 of P_full) and the O buffer has been read
-                if (!mbar_wait(BAR(B_PFULL), (it + 1) & 1)) { ok = false; break; }
-                if (!mbar_wait(BAR(B_VFULL + s), (it >> 1) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(BAR(B_PFULL), (it + 1) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(BAR(B_VFULL + s), (it >> 1) & 1)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t v_addr = smem_u32(smem + OFF_V + s * KV_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < KN / 16; ++k) {              // O accumulates over the tiles in tensor memory
-                    const uint32_t poff = (k >> 2) * ROWBLK + (k & 3) * 32;
-                    umma_bf16(tmem_base + 2 * KN, desc_kmajor(p_addr + poff), desc_mnmajor(v_addr + k * 2048), idesc_o,
-                              (it > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < KN / 16; ++k) {          // O accumulates over the tiles in tensor memory
+                        const uint32_t poff = (k >> 2) * ROWBLK + (k & 3) * 32;
+                        umma_bf16(tmem_base + 2 * KN, desc_kmajor(p_addr + poff), desc_mnmajor(v_addr + k * 2048), idesc_o,
+                                  (it > 0 || k > 0) ? 1u : 0u);
+                    }
+                    umma_commit(BAR(B_VEMPTY + s));
+                    umma_commit(BAR(B_OFULL));
                 }
-                umma_commit(BAR(B_VEMPTY + s));
-                umma_commit(BAR(B_OFULL));
+                __syncwarp();
             }
-            if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+            if (!ok && lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
         }
     } else {
         // ------------------------------------------------ softmax, correction, epilogue
@@ -760,7 +774,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     uint32_t* tmem_slot = (uint32_t*)(bars + W_N_BARS);
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 8; ++i) mbar_init(BAR(i), 1);                 // K/V full and empty
@@ -805,13 +819,12 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it & 1;
                 const uint32_t ph = (it >> 1) & 1;
                 const int j0 = (tile_first + it) * KN;
-                if (!mbar_wait(BAR(W_KEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                mbar_expect_tx(BAR(W_KFULL + s), KV_BYTES);
+                if (!mbar_wait_warp(BAR(W_KEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 const uint32_t kdst = smem_u32(smem + W_OFF_K + s * KV_BYTES);
                 int rows[KN / 16];
 #pragma unroll
@@ -820,32 +833,39 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     const int blk = j >> p.page_shift;
                     int page = (j <= pos_hi && blk < p.max_blocks) ? __ldg(bt + blk) : 0;
                     if (page < 0 || page >= p.num_pages) {
-                        if (j + 15 >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
+                        if (j + 15 >= k_first && lane == 0) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                         page = 0;
                     }
                     const int parts = KIND != W_PLAIN && ex.tail >= 0 ? 1 : 2;       // key rows, then value rows; or rows that are both
                     rows[gkey] = (((page * parts) * p.nkv + kvh) << p.page_shift) + (j & (p.page_size - 1));
                 }
+                if (elect_one()) {
+                    mbar_expect_tx(BAR(W_KFULL + s), KV_BYTES);
 #pragma unroll
-                for (int gkey = 0; gkey < KN / 16; ++gkey)
+                    for (int gkey = 0; gkey < KN / 16; ++gkey)
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(kdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_KFULL + s), h * 64, rows[gkey]);
-                if (!mbar_wait(BAR(W_VEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                mbar_expect_tx(BAR(W_VFULL + s), KV_BYTES);
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_2d(kdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_KFULL + s), h * 64, rows[gkey]);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(BAR(W_VEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 const uint32_t vdst = smem_u32(smem + W_OFF_V + s * KV_BYTES);
                 const bool one_row = KIND != W_PLAIN && ex.tail >= 0;
                 const int vskip = one_row ? 0 : p.nkv << p.page_shift, v_x = one_row ? ex.tail : 0;
+                if (elect_one()) {
+                    mbar_expect_tx(BAR(W_VFULL + s), KV_BYTES);
 #pragma unroll
-                for (int gkey = 0; gkey < KN / 16; ++gkey)
+                    for (int gkey = 0; gkey < KN / 16; ++gkey)
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_VFULL + s), v_x + h * 64, rows[gkey] + vskip);
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_2d(vdst + h * ROWBLK + gkey * 2048, &kv_map, BAR(W_VFULL + s), v_x + h * 64, rows[gkey] + vskip);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KN >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             const int last_x = two ? 1 : 0;
@@ -855,39 +875,48 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             const uint32_t q_lo = (uint32_t)qd, q_hi = (uint32_t)(qd >> 32), k_lo = (uint32_t)kd, k_hi = (uint32_t)(kd >> 32),
                            v_lo = (uint32_t)vd, v_hi = (uint32_t)(vd >> 32);
             // first phase of P_full: the Q tiles are in shared memory
-            bool ok = mbar_wait(BAR(W_PFULL), 0) && (!two || mbar_wait(BAR(W_PFULL + 1), 0));
+            bool ok = mbar_wait_warp(BAR(W_PFULL), 0) && (!two || mbar_wait_warp(BAR(W_PFULL + 1), 0));
             auto issue_s = [&](int it, int x) -> bool {          // S of Q tile x and key tile it
                 const int s = it & 1;
                 if (x == 0) {
-                    if (!mbar_wait(BAR(W_KFULL + s), (it >> 1) & 1)) return false;
+                    if (!mbar_wait_warp(BAR(W_KFULL + s), (it >> 1) & 1)) return false;
                     tc_fence_after();
                 }
                 const uint32_t qx = q_lo + x * (Q_BYTES >> 4), ks = k_lo + s * (KV_BYTES >> 4), d = tmem_base + x * KN;
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < (DIFF ? 4 : HD / 16); ++k) {
-                    const uint32_t off = ((k >> 2) * ROWBLK + (k & 3) * 32) >> 4;
-                    umma_bf16_lh(d, qx + off, q_hi, ks + off + (DIFF ? x * (ROWBLK >> 4) : 0), k_hi, idesc_s, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < (DIFF ? 4 : HD / 16); ++k) {
+                        const uint32_t off = ((k >> 2) * ROWBLK + (k & 3) * 32) >> 4;
+                        umma_bf16_lh(d, qx + off, q_hi, ks + off + (DIFF ? x * (ROWBLK >> 4) : 0), k_hi, idesc_s, k > 0 ? 1u : 0u);
+                    }
+                    if (x == last_x) umma_commit(BAR(W_KEMPTY + s));
+                    umma_commit(BAR(W_SFULL + x));
                 }
-                if (x == last_x) umma_commit(BAR(W_KEMPTY + s));
-                umma_commit(BAR(W_SFULL + x));
+                __syncwarp();
                 return true;
             };
             auto issue_o = [&](int it, int x) -> bool {          // O of Q tile x += P V of key tile it
                 const int s = it & 1;
-                if (!mbar_wait(BAR(W_PHALF + x), it & 1)) return false;           // P of keys 0-63 stands where S stood
-                if (x == 0 && !mbar_wait(BAR(W_VFULL + s), (it >> 1) & 1)) return false;
+                if (!mbar_wait_warp(BAR(W_PHALF + x), it & 1)) return false;      // P of keys 0-63 stands where S stood
+                if (x == 0 && !mbar_wait_warp(BAR(W_VFULL + s), (it >> 1) & 1)) return false;
                 tc_fence_after();
                 const uint32_t vs = v_lo + s * (KV_BYTES >> 4), d = tmem_base + (2 + x) * KN, pa = tmem_base + x * KN;
                 const uint32_t acc0 = it > 0 ? 1u : 0u;
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < KN / 32; ++k)                // 16 keys of P = 8 columns of packed pairs
-                    umma_bf16_ta_lh(d, pa + k * 8, vs + k * (2048 >> 4), v_hi, idesc_o, k > 0 ? 1u : acc0);
-                if (!mbar_wait(BAR(W_PFULL + x), (it + 1) & 1)) return false;     // and of keys 64-127
+                    for (int k = 0; k < KN / 32; ++k)            // 16 keys of P = 8 columns of packed pairs
+                        umma_bf16_ta_lh(d, pa + k * 8, vs + k * (2048 >> 4), v_hi, idesc_o, k > 0 ? 1u : acc0);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(BAR(W_PFULL + x), (it + 1) & 1)) return false;     // and of keys 64-127
                 tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int k = KN / 32; k < KN / 16; ++k)
-                    umma_bf16_ta_lh(d, pa + k * 8, vs + k * (2048 >> 4), v_hi, idesc_o, 1u);
-                if (x == last_x) umma_commit(BAR(W_VEMPTY + s));
+                    for (int k = KN / 32; k < KN / 16; ++k)
+                        umma_bf16_ta_lh(d, pa + k * 8, vs + k * (2048 >> 4), v_hi, idesc_o, 1u);
+                    if (x == last_x) umma_commit(BAR(W_VEMPTY + s));
+                }
+                __syncwarp();
                 return true;
             };
             if (ok && n_tiles > 0) {
@@ -902,8 +931,11 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                     if (ok && it + 1 < n_tiles) ok = issue_s(it + 1, 1);
                 }
             }
-            if (ok) umma_commit(BAR(W_FINAL));
-            else atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+            if (elect_one()) {
+                if (ok) umma_commit(BAR(W_FINAL));
+                else atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+            }
+            __syncwarp();
         }
     } else if (two || warp < 6) {
         // ------------------------------------------------ softmax, correction, epilogue

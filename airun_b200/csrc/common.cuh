@@ -53,6 +53,17 @@ __device__ __forceinline__ void prefetch_l2(const float* p, int n) {
     for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
 }
 
+// The warp's number, the same register for all lanes as the compiler sees it.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// True in one lane of a converged warp, the same one every time.  What issues tcgen05 and TMA instructions is a whole warp that loops and waits together, with
+// elect_one() around the instructions alone: their operands (addresses, descriptors) are then uniform registers.  Behind `lane == 0` they have to be
+// moved there one by one, 64 clocks a product and 250 a commit (B200: a step of four products 585 clocks, 280 with this).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 static thread_local int airun_launch_rc = 0;
 
 static inline bool airun_pdl_enabled() {
@@ -98,10 +109,10 @@ static inline void airun_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 
     if (e != cudaSuccess && airun_launch_rc == 0) airun_launch_rc = (int)e;
 }
 
-// The same with thread-block clusters of (1, 1, cluster_z) CTAs (grid.z must be a multiple of it).
+// The same with thread-block clusters (the grid must be a multiple of them).
 template <typename... KArgs, typename... Args>
-static inline void airun_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                        unsigned cluster_z, Args&&... args) {
+static inline void airun_launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                         dim3 cluster, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -110,9 +121,9 @@ static inline void airun_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim
     cudaLaunchAttribute attr[2];
     int n = 0;
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = 1;
-    attr[n].val.clusterDim.y = 1;
-    attr[n].val.clusterDim.z = cluster_z;
+    attr[n].val.clusterDim.x = cluster.x;
+    attr[n].val.clusterDim.y = cluster.y;
+    attr[n].val.clusterDim.z = cluster.z;
     ++n;
     if (airun_pdl_enabled()) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -123,6 +134,13 @@ static inline void airun_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim
     cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (e != cudaSuccess && airun_launch_rc == 0) airun_launch_rc = (int)e;
+}
+
+// Clusters of (1, 1, cluster_z) CTAs.
+template <typename... KArgs, typename... Args>
+static inline void airun_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                        unsigned cluster_z, Args&&... args) {
+    airun_launch_clusters(kernel, grid, block, smem, stream, dim3(1, 1, cluster_z), static_cast<KArgs>(args)...);
 }
 
 static inline int airun_launch_status() {

@@ -407,7 +407,7 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
     // full, empty of the stages of parts; full, empty of the two step sums; landed, read of the ring
     __shared__ __align__(8) uint64_t bars[2 * X_STAGES + 4 + 2 * X_RING];
     __shared__ uint32_t tmem_slot, inf_rows[2][4], all_rows[8];    // infinite operands: bit r of [0] weight row, of [1] row of A
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int slice = blockIdx.z, n0 = blockIdx.x * XT;
     int m0 = blockIdx.y * bn, m_end = M, set_w = 0;
     if (FORM == 2) {
@@ -558,49 +558,55 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(taken + 8 * g) : "memory");
             }
         }
-    } else if (warp == X_SUM_WARPS + X_CUT_WARPS && lane == 0) {
+    } else if (warp == X_SUM_WARPS + X_CUT_WARPS) {
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(XT >> 4) << 24);
         for (int it = 0; it < steps; ++it) {
             const int s = it % X_STAGES, buf = it & 1;
-            if (!mbar_wait(sempty + 8 * buf, ((it >> 1) & 1) ^ 1) || !mbar_wait(full + 8 * s, (it / X_STAGES) & 1)) {
+            if (!mbar_wait_warp(sempty + 8 * buf, ((it >> 1) & 1) ^ 1) || !mbar_wait_warp(full + 8 * s, (it / X_STAGES) & 1)) {
                 atomicOr(err, AIRUN_DEV_TIMEOUT);
                 break;
             }
             tc_fence_after();
             const uint32_t base = smem_u32(tiles) + s * X_STAGE;
             constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, AP[6] = {0, 2, 1, 0, 1, 0};     // the smallest products first
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                const uint32_t tw = tmem + 2 * XB + (3 * s + WP[j]) * X_WCOLS;
-                const uint64_t da = smem_desc_sw128(base + AP[j] * X_PART);
+                for (int j = 0; j < 6; ++j) {
+                    const uint32_t tw = tmem + 2 * XB + (3 * s + WP[j]) * X_WCOLS;
+                    const uint64_t da = smem_desc_sw128(base + AP[j] * X_PART);
 #pragma unroll
-                for (int k = 0; k < XK / 16; ++k)
-                    umma_bf16_ts(tmem + buf * XB, tw + 8 * k, da + (uint64_t)(k * 2), idesc, (j > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < XK / 16; ++k)
+                        umma_bf16_ts(tmem + buf * XB, tw + 8 * k, da + (uint64_t)(k * 2), idesc, (j > 0 || k > 0) ? 1u : 0u);
+                }
+                umma_commit(empty + 8 * s);
+                umma_commit(sfull + 8 * buf);
             }
-            umma_commit(empty + 8 * s);
-            umma_commit(sfull + 8 * buf);
+            __syncwarp();
         }
-    } else if (lane == 0) {
+    } else {
         const uint32_t ring = smem_u32(tiles) + X_STAGES * X_STAGE;
         auto ask = [&](int it, bool w, bool a) {
             const uint32_t to = ring + (it % X_RING) * X_RING_STEP, bar = landed + 8 * (it % X_RING);
             const int k = (step0 + it) * XK;
-            if (w) {
-                mbar_expect_tx(bar, (XT + bn) * XK * 4);
-                tma_load_3d(to, &map_w, bar, k, n0, set_w);
-                tma_load_3d(to + XT * 128, &map_w, bar, k + 32, n0, set_w);
+            if (elect_one()) {
+                if (w) {
+                    mbar_expect_tx(bar, (XT + bn) * XK * 4);
+                    tma_load_3d(to, &map_w, bar, k, n0, set_w);
+                    tma_load_3d(to + XT * 128, &map_w, bar, k + 32, n0, set_w);
+                }
+                if (a) {
+                    tma_load_3d(to + 2 * XT * 128, &map_a, bar, k, m0, 0);
+                    tma_load_3d(to + (2 * XT + XB) * 128, &map_a, bar, k + 32, m0, 0);
+                }
             }
-            if (a) {
-                tma_load_3d(to + 2 * XT * 128, &map_a, bar, k, m0, 0);
-                tma_load_3d(to + (2 * XT + XB) * 128, &map_a, bar, k + 32, m0, 0);
-            }
+            __syncwarp();
         };
         const int first = min(steps, X_RING);
         for (int it = 0; it < first; ++it) ask(it, true, false);
         if (FORM != 2) pdl_wait();
         for (int it = 0; it < first; ++it) ask(it, false, true);
         for (int it = X_RING; it < steps; ++it) {
-            if (!mbar_wait(taken + 8 * (it % X_RING), ((it / X_RING) & 1) ^ 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+            if (!mbar_wait_warp(taken + 8 * (it % X_RING), ((it / X_RING) & 1) ^ 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
             ask(it, true, true);
         }
     }

@@ -89,8 +89,8 @@ struct GemmParams {
                                   // distributed shared memory instead of the scratch
     float glu_limit, glu_slope;   // EPI_SWIGLU: 0, 0 for SwiGLU; a limit > 0 for the clamped gated unit
     int act;                      // EPI_F32 / EPI_BF16: 0 stores the product, 1 + m an activation of it (epilogue_act)
-    // grouped form of the persistent kernel: the rows of A are cut into n_seg segments (seg[e] .. seg[e + 1] - 1, device
-    // memory) and segment e is multiplied by rows e * b_rows .. of the B operand (one matrix per segment, stacked)
+    // grouped form of the pair kernel: the tokens are cut into n_seg segments (seg[e] .. seg[e + 1] - 1, device memory)
+    // and segment e is multiplied by rows e * a_rows .. of the weights (one matrix per segment, stacked)
     const int32_t* seg;
     int n_seg;
     int batch_a;                  // batched form: columns of A from one product to the next, and elements of the output
@@ -215,20 +215,35 @@ __device__ __forceinline__ void store_swiglu_normal(const GemmParams& p, const f
         if (b0 + c0 + 16 + i < p.b_rows) o[i] = __float2bfloat16_rn(gated_unit(p.glu_limit, p.glu_slope, g[i], u[i]));
 }
 
-// SwiGLU, swapped mode: this lane's row is a gate row when (a_row / 16) is even, and lane + 16
-// holds the matching up row.  v: 16 columns (tokens).  The gate lanes take the first eight tokens, the up lanes the others:
-// one exchange brings each the other half of its pairs.
+// Gated units where a lane is a weight row: lanes 0-15 hold gate rows, the lane 16 further on the matching up row.  v: 16 columns (tokens).  The gate lanes
+// take the first eight tokens, the up lanes the others: one exchange brings each the other half of its pairs.
+__device__ __forceinline__ void gated_units(float limit, float slope, const float* v, bool low, float (&y)[8]) {
+    float g[8], u[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, low ? v[i + 8] : v[i], 16);
+        g[i] = low ? v[i] : other;
+        u[i] = low ? other : v[i + 8];
+    }
+    if (limit > 0.0f) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = gated_unit(limit, slope, g[i], u[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = silu_mul(g[i], u[i]);
+    }
+}
+
+// SwiGLU, swapped mode: rows in turns of 16 gate and 16 up rows.
 __device__ __forceinline__ void store_swiglu_swapped(const GemmParams& p, const float* v, int a_row, int b0, int c0) {
     const int lane = threadIdx.x & 31;
     const bool low = lane < 16;
     const int first = b0 + c0 + (low ? 0 : 8), n = a_row < p.a_rows ? p.b_rows - first : 0;
     __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)first * p.ldc + (a_row >> 5) * 16 + (lane & 15);
+    float y[8];
+    gated_units(p.glu_limit, p.glu_slope, v, low, y);
 #pragma unroll
-    for (int i = 0; i < 8; ++i, o += p.ldc) {
-        const float other = __shfl_xor_sync(0xffffffffu, low ? v[i + 8] : v[i], 16);
-        const float g = low ? v[i] : other, u = low ? other : v[i + 8];
-        if (i < n) *o = __float2bfloat16_rn(gated_unit(p.glu_limit, p.glu_slope, g, u));
-    }
+    for (int i = 0; i < 8; ++i, o += p.ldc) if (i < n) *o = __float2bfloat16_rn(y[i]);
 }
 
 // rsqrt(sum of the parts / n + eps) of one token
@@ -319,7 +334,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     __shared__ int s_abort;
 
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int a0 = blockIdx.x * BM;            // first A row of the tile
     const int b0 = blockIdx.y * BN;            // first B row of the tile
     const int split = blockIdx.z;
@@ -347,7 +362,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     // weight blocks are requested before waiting for the kernel before this one: the weights keep
     // streaming across the boundary between two kernels.
     const int n_pre = n_kb < STAGES ? n_kb : STAGES;
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         for (int i = 0; i < n_pre; ++i) {
             mbar_expect_tx(full0 + 8 * i, L::STAGE_BYTES);
             const uint32_t sa = smem_u32(smem + i * L::STAGE_BYTES);
@@ -463,40 +478,44 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     };
 
     if (warp == 0) {
-        if (lane == 0) {
-            for (int i = 0; i < n_kb; ++i) {
-                const int s = i % STAGES;
-                const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
-                const int k = (kb_begin + i) * BK;
-                if (i < n_pre) {                 // the weight half of this stage is already on its way
-                    if (SWAP) tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, k, b0);
-                    else tma_load_2d(sa, &map_a, full0 + 8 * s, k, a0);
-                    continue;
+        int s = 0;
+        uint32_t phase = 0;
+        for (int i = 0; i < n_kb; ++i) {
+            if (i >= n_pre && !mbar_wait_warp(empty0 + 8 * s, phase ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); s_abort = 1; break; }
+            const uint32_t sa = smem_u32(smem) + s * L::STAGE_BYTES;
+            const int k = (kb_begin + i) * BK;
+            if (elect_one()) {
+                if (i >= n_pre) {                // (the weight half of the first stages is already on its way)
+                    mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
+                    if (SWAP) tma_load_2d(sa, &map_a, full0 + 8 * s, k, a0);
+                    else tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, k, b0);
                 }
-                const uint32_t phase = (i / STAGES) & 1;
-                if (!mbar_wait(empty0 + 8 * s, phase ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); s_abort = 1; break; }
-                mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
-                tma_load_2d(sa, &map_a, full0 + 8 * s, k, a0);
-                tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, k, b0);
+                if (SWAP) tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, k, b0);
+                else tma_load_2d(sa, &map_a, full0 + 8 * s, k, a0);
             }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; phase ^= 1; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            bool ok = true;
-            for (int i = 0; i < n_kb && ok; ++i) {
-                const int s = i % STAGES;
-                const uint32_t phase = (i / STAGES) & 1;
-                if (!mbar_wait(full0 + 8 * s, phase)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); s_abort = 1; ok = false; break; }
+            int s = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < n_kb; ++i) {
+                if (!mbar_wait_warp(full0 + 8 * s, phase)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); s_abort = 1; break; }
                 tc_fence_after();
-                const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
+                const uint32_t sa = smem_u32(smem) + s * L::STAGE_BYTES;
                 const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + L::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    umma_bf16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(empty0 + 8 * s);      // the stage is free once these MMAs have read it
+                    for (int k = 0; k < BK / 16; ++k)
+                        umma_bf16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(empty0 + 8 * s);  // the stage is free once these MMAs have read it
+                    if (i + 1 == n_kb) umma_commit(accum);     // arrives when every MMA issued so far is complete
+                }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
-            umma_commit(accum);                   // arrives when every MMA issued so far is complete
         }
     } else {
         // epilogue warps 2..5: warp w may touch the 32 TMEM lanes of quadrant w % 4
@@ -598,12 +617,6 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
 // tensor memory (2 x 256 columns): while the epilogue warps drain tile i, the MMA thread is already
 // filling tile i + 1.  Normal mode, BN = 256, no K slices.
 //
-// GROUPED: the rows of A are segments, each with a B matrix of its own (the experts of a routed feed-forward whose
-// rows have been sorted by expert).  Where the segments lie is only known on the device, so every CTA first lists
-// the row tiles of all segments in shared memory (first row, end of the segment, segment) and then walks
-// (row tile, column tile) pairs as above; a tile's rows beyond its segment's end are computed and not stored.  The
-// launch is sized for the most row tiles any cut can have, ceil(rows / 128) + segments.
-//
 // BATCHED: n_seg products of equal sizes in one launch: product e reads the columns e * batch_a .. + K - 1 of A (column
 // slices of one buffer: the heads of a per-head product), has the rows e * b_rows .. of B as its matrix and writes its
 // bfloat16 result batch_out elements further on than product e - 1.  A last K block that reaches into the next slice's
@@ -612,24 +625,19 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
 #define PSTAGES 4
 #define P_EPI_WARPS 8                         // two per quadrant of tensor-memory lanes, half of the columns each
 #define P_THREADS (64 + 32 * P_EPI_WARPS)
-#define GROUP_MAX_TILES 1024
-#define GROUP_MAX_SEGS 1024
-enum { FORM_PLAIN = 0, FORM_GROUPED = 1, FORM_BATCHED = 2 };
-template <int EPI, int FORM>
+template <int EPI, bool BATCHED>
 __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p,
     int m_tiles, int n_tiles) {
-    constexpr bool GROUPED = FORM == FORM_GROUPED, BATCHED = FORM == FORM_BATCHED;
     pdl_trigger();
-    __shared__ int s_tab[GROUPED ? 3 * GROUP_MAX_TILES : 1], s_first[GROUPED ? GROUP_MAX_SEGS + 1 : 1];
     using L = SmemLayout<PBN, PSTAGES>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = (uint64_t*)(smem + L::BAR_OFFSET);          // full[S], empty[S], acc_full[2], acc_empty[2]
     __shared__ uint32_t tmem_slot_p;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int kb_total = (p.K + BK - 1) / BK;
-    int total_tiles = m_tiles * n_tiles * (BATCHED ? p.n_seg : 1);
+    const int total_tiles = m_tiles * n_tiles * (BATCHED ? p.n_seg : 1);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + PSTAGES);
     const uint32_t accf0 = smem_u32(bars + 2 * PSTAGES), acce0 = smem_u32(bars + 2 * PSTAGES + 2);
     if (threadIdx.x == 0) {
@@ -645,9 +653,8 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
     const uint32_t tmem_base = tmem_slot_p;
     // The weights (the B operand) are written by no kernel: the first stages of this CTA's first tile
     // ask for their weight blocks before waiting for the kernel in front.
-    // (Not when grouped: which matrix a tile needs is not known before the segments are.)
-    const int n_pre = (!GROUPED && (int)blockIdx.x < total_tiles) ? (kb_total < PSTAGES ? kb_total : PSTAGES) : 0;
-    if (warp == 0 && lane == 0) {
+    const int n_pre = (int)blockIdx.x < total_tiles ? (kb_total < PSTAGES ? kb_total : PSTAGES) : 0;
+    if (warp == 0 && elect_one()) {
         const int col = (int)blockIdx.x / m_tiles;
         const int b0 = BATCHED ? (col % n_tiles) * PBN + (col / n_tiles) * p.b_rows : col * PBN;
         for (int i = 0; i < n_pre; ++i) {
@@ -656,71 +663,56 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
         }
     }
     pdl_wait();
-    if (GROUPED) {
-        for (int e = threadIdx.x; e < p.n_seg; e += P_THREADS) s_first[e + 1] = (p.seg[e + 1] - p.seg[e] + BM - 1) / BM;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int at = 0;
-            for (int e = 0; e < p.n_seg; ++e) { const int c = s_first[e + 1]; s_first[e] = at; at += c; }
-            s_first[p.n_seg] = at;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < p.n_seg; e += P_THREADS) {
-            const int lo = p.seg[e], hi = p.seg[e + 1];
-            int j = s_first[e];
-            for (int r = lo; r < hi && j < GROUP_MAX_TILES; r += BM, ++j) { s_tab[3 * j] = r; s_tab[3 * j + 1] = hi; s_tab[3 * j + 2] = e; }
-        }
-        __syncthreads();
-        m_tiles = min(s_first[p.n_seg], GROUP_MAX_TILES);
-        total_tiles = m_tiles * n_tiles;
-    }
-
     if (warp == 0) {
-        if (lane == 0) {
+        {
             int it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 const int mi = tile % m_tiles;
-                const int a0 = GROUPED ? s_tab[3 * mi] : mi * BM;
+                const int a0 = mi * BM;
                 const int col = tile / m_tiles, batch = BATCHED ? col / n_tiles : 0;
-                const int b0 = (BATCHED ? col % n_tiles : col) * PBN + (GROUPED ? s_tab[3 * mi + 2] : batch) * p.b_rows;
+                const int b0 = (BATCHED ? col % n_tiles : col) * PBN + batch * p.b_rows;
                 const int ka0 = BATCHED ? batch * p.batch_a : 0;        // where this product's columns of A begin
                 for (int kb = 0; kb < kb_total; ++kb, ++it) {
                     const int s = it % PSTAGES;
                     const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
-                    if (it < n_pre) {                // the weight half of this stage is already on its way
+                    if (it >= n_pre && !mbar_wait_warp(empty0 + 8 * s, ((it / PSTAGES) & 1) ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); ok = false; break; }
+                    if (elect_one()) {
+                        if (it >= n_pre) {           // (the weight half of the first stages is already on its way)
+                            mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
+                            tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, kb * BK, b0);
+                        }
                         tma_load_2d(sa, &map_a, full0 + 8 * s, ka0 + kb * BK, a0);
-                        continue;
                     }
-                    if (!mbar_wait(empty0 + 8 * s, ((it / PSTAGES) & 1) ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); ok = false; break; }
-                    mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
-                    tma_load_2d(sa, &map_a, full0 + 8 * s, ka0 + kb * BK, a0);
-                    tma_load_2d(sa + L::A_BYTES, &map_b, full0 + 8 * s, kb * BK, b0);
+                    __syncwarp();
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
             int it = 0, n = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++n) {
                 const int buf = n & 1;
-                if (!mbar_wait(acce0 + 8 * buf, ((n >> 1) & 1) ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
+                if (!mbar_wait_warp(acce0 + 8 * buf, ((n >> 1) & 1) ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * PBN;
                 for (int kb = 0; kb < kb_total; ++kb, ++it) {
                     const int s = it % PSTAGES;
-                    if (!mbar_wait(full0 + 8 * s, (it / PSTAGES) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); ok = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, (it / PSTAGES) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
                     const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + L::A_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        umma_bf16(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(empty0 + 8 * s);
+                        for (int k = 0; k < BK / 16; ++k)
+                            umma_bf16(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_commit(empty0 + 8 * s);
+                        if (kb + 1 == kb_total) umma_commit(accf0 + 8 * buf);
+                    }
+                    __syncwarp();
                 }
-                umma_commit(accf0 + 8 * buf);
             }
         }
     } else {
@@ -735,10 +727,9 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
             const int buf = n & 1;
             const int mi = tile % m_tiles;
             const int col = tile / m_tiles;
-            const int a0 = GROUPED ? s_tab[3 * mi] : mi * BM, b0 = (BATCHED ? col % n_tiles : col) * PBN;
+            const int a0 = mi * BM, b0 = (BATCHED ? col % n_tiles : col) * PBN;
             if (BATCHED) q.out = (__nv_bfloat16*)p.out + (size_t)(col / n_tiles) * p.batch_out;
             const int a_row = a0 + quad * 32 + lane;
-            const bool row_on = !GROUPED || a_row < s_tab[3 * mi + 1];       // grouped: rows of the tile's own segment only
             const float row_scale = (AIRUN_FOLD_NORM && p.ssq_in && a_row < p.a_rows) ? token_scale(p, a_row) : 1.0f;   // while the MMAs run
             float ssq_acc = 0.0f;
             if (!mbar_wait(accf0 + 8 * buf, (n >> 1) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
@@ -768,7 +759,7 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
                         v[i] = __uint_as_float(r[j & 1][i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
                         u[i] = __uint_as_float(r[j & 1][16 + i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
                     }
-                    if (row_on) store_swiglu_normal(p, v, u, a_row, b0, c);
+                    store_swiglu_normal(p, v, u, a_row, b0, c);
                 }
             } else {
                 // one body for all columns: unrolled, the activations' code would not stay in the instruction cache
@@ -785,8 +776,8 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
 #pragma unroll
                         for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h + i]) * (AIRUN_FOLD_NORM ? row_scale : 1.0f);
                         if (EPI == EPI_RESID) {
-                            if (row_on) ssq_acc += store_resid_normal(p, v, a_row, b0 + c + h);
-                        } else if (row_on) {
+                            ssq_acc += store_resid_normal(p, v, a_row, b0 + c + h);
+                        } else {
                             if (p.act) epilogue_act(v, p.act - 1);
                             store_chunk<EPI, false>(BATCHED ? q : p, v, a_row, b0, c + h);
                         }
@@ -808,6 +799,251 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
         tmem_dealloc(tmem_base, 2 * PBN);
     }
 }
+
+#if !AIRUN_FOLD_NORM
+// ------------------------------------------------------------------ two SMs to a tile (prompt portions, grouped products)
+// What an SM takes in from the L2 cache, about 64 bytes a clock, bounds a product whose CTAs work alone: a tile of 128 x 256 takes 48 KB a K-step of 64
+// for 512 clocks of products.  Here a pair of CTAs (a cluster of two) computes 256 weight rows x `bn` tokens (32 .. 256): each brings 128 of the
+// weight rows and half of the tokens, the leader's tcgen05.mma.cta_group::2 multiplies all of it, and each CTA gets its weight rows' results in its own tensor
+// memory: 32 KB an SM and step for the same products.  The weights are the 256-row operand so that the tokens, whose number is any, set the tile's other
+// side in steps of 32.  Pairs walk the tiles (tokens fastest: pairs side by side share weights); the stage ring runs on across tiles, the accumulator is
+// double-buffered.
+//   warp 0   : one thread issues this CTA's TMA loads (no multicast); they count towards the leader's barrier;
+//   warp 1   : allocates tensor memory; in the leader one thread issues the products and commits to both CTAs' barriers;
+//   warps 2-9: epilogue; a lane is a weight row, so a warp stores 32 neighbouring results of a token at once.
+// GROUPED: the tokens' rows are segments, each with a weight matrix of its own (the experts of a routed feed-forward whose rows have been sorted by
+// expert).  Where the segments lie is only known on the device, so every CTA first lists their tiles in shared memory.  A segment is cut into tiles of
+// equal width, the least multiple of 32 that holds its rows, so little is computed for rows that are not there; a tile's columns beyond its
+// segment's end are not stored.  The launch is sized for the most tiles any cut can have, ceil(rows / 256) + segments.
+#define GROUP_MAX_TILES 1024
+#define GROUP_MAX_SEGS 1024
+#define PAIR_STAGES 6
+#define PAIR_BN 256
+#define PAIR_BOX 64                           // tokens a load of a grouped product brings: half a tile is one or two of them
+#define PAIR_STAGE_BYTES (2 * 128 * BK * 2)
+#define PAIR_THREADS 320
+#define PAIR_SMEM (PAIR_STAGES * PAIR_STAGE_BYTES + 1024)
+
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrives at the barrier of this place in both CTAs once the products issued so far are done
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+// 16 tokens of this lane's weight row from `tok` on, of which the first n are there.
+template <int EPI>
+__device__ __forceinline__ void store_pair(const GemmParams& p, const float* v, int row, bool row_on, int tok, int n) {
+    if constexpr (EPI == EPI_SWIGLU) {
+        const int lane = threadIdx.x & 31;
+        const bool low = lane < 16;
+        if (!low) { tok += 8; n -= 8; }
+        // all units before the first store: each behind its own condition would be a chain of latencies by itself (a tile of 256 tokens
+        // 17,700 clocks, more than its products)
+        float y[8];
+        gated_units(p.glu_limit, p.glu_slope, v, low, y);
+        if (!row_on) return;
+        __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)tok * p.ldc + (row >> 5) * 16 + (lane & 15);
+        if (n >= 8) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i, o += p.ldc) *o = __float2bfloat16_rn(y[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i, o += p.ldc) if (i < n) *o = __float2bfloat16_rn(y[i]);
+        }
+    } else {
+        typedef typename std::conditional<EPI == EPI_F32, float, __nv_bfloat16>::type TOut;
+        if (!row_on) return;
+        TOut* o = (TOut*)p.out + (size_t)tok * p.ldc + row;
+        if (n >= 16) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i, o += p.ldc) *o = from_f32<TOut>(v[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i, o += p.ldc) if (i < n) *o = from_f32<TOut>(v[i]);
+        }
+    }
+}
+
+template <int EPI, bool GROUPED>
+__global__ __launch_bounds__(PAIR_THREADS, 1) void gemm_pair_kernel(
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p, int bn, int tok_tiles) {
+    pdl_trigger();
+    __shared__ int4 s_tab[GROUPED ? GROUP_MAX_TILES : 1];          // first row, end of the segment, segment, width
+    __shared__ int s_first[GROUPED ? GROUP_MAX_SEGS + 1 : 1];
+    __shared__ __align__(8) uint64_t bars[2 * PAIR_STAGES + 4];    // full (the leader's), empty of the stages; full, empty (the leader's) of the sums
+    __shared__ uint32_t tmem_slot;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int kb_total = (p.K + BK - 1) / BK, w_tiles = (p.a_rows + 255) / 256;
+    const uint32_t full = smem_u32(bars), empty = full + 8 * PAIR_STAGES, accf = empty + 8 * PAIR_STAGES, acce = accf + 16;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(accf + 8 * b, 1); mbar_init(acce + 8 * b, 16); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                            // the leader's barriers are there before anything arrives at them
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    const uint32_t full_lead = map_to_cta(full, 0), acce_lead = map_to_cta(acce, 0);
+
+    int n_tok_tiles = tok_tiles;
+    const int first_n = GROUPED ? 0 : (pair < w_tiles * tok_tiles ? min(kb_total, PAIR_STAGES) : 0);
+    if (warp == 0 && elect_one()) {                                // weights are written by no kernel
+        for (int i = 0; i < first_n; ++i) {
+            if (rank == 0) mbar_expect_tx(full + 8 * i, 2 * (128 * BK * 2) + bn * (BK * 2));
+            tma_load_2d_pair(smem_u32(smem + i * PAIR_STAGE_BYTES), &map_w, full_lead + 8 * i, i * BK, pair / tok_tiles * 256 + rank * 128);
+        }
+    }
+    pdl_wait();
+    if (GROUPED) {
+        for (int e = threadIdx.x; e < p.n_seg; e += PAIR_THREADS) s_first[e + 1] = (p.seg[e + 1] - p.seg[e] + PAIR_BN - 1) / PAIR_BN;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int at = 0;
+            for (int e = 0; e < p.n_seg; ++e) { const int c = s_first[e + 1]; s_first[e] = at; at += c; }
+            s_first[p.n_seg] = at;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < p.n_seg; e += PAIR_THREADS) {
+            const int lo = p.seg[e], hi = p.seg[e + 1];
+            int j = s_first[e];
+            const int n = s_first[e + 1] - j, width = n > 0 ? ((hi - lo + n - 1) / n + 31) / 32 * 32 : 32;
+            for (int r = lo; r < hi && j < GROUP_MAX_TILES; r += width, ++j) s_tab[j] = make_int4(r, hi, e, width);
+            // (equal widths can need a tile less than counted: its place holds nothing)
+            for (; j < s_first[e + 1] && j < GROUP_MAX_TILES; ++j) s_tab[j] = make_int4(hi, hi, e, 32);
+        }
+        __syncthreads();
+        n_tok_tiles = min(s_first[p.n_seg], GROUP_MAX_TILES);
+    }
+    const int total = w_tiles * n_tok_tiles;
+    struct Tile { int w0, t0, t_end, e, bn; };
+    auto tile_of = [&](int tile) {
+        const int ti = tile % n_tok_tiles;
+        Tile t = {tile / n_tok_tiles * 256, ti * bn, p.b_rows, 0, bn};
+        if (GROUPED) { const int4 g = s_tab[ti]; t.t0 = g.x; t.t_end = g.y; t.e = g.z; t.bn = g.w; }
+        return t;
+    };
+
+    int it = 0, s = 0;                                             // K-steps so far, and their place in the ring
+    uint32_t phase = 0;                                            // of the ring's barriers, one round after the other
+    bool ok = true;
+    if (warp == 0) {
+        for (int tile = pair; tile < total && ok; tile += pairs) {
+            const Tile t = tile_of(tile);
+            const int half = t.bn / 2, t0 = t.t0 + rank * half, w0 = t.w0 + rank * 128 + (GROUPED ? t.e * p.a_rows : 0);
+            const bool two = GROUPED && half > PAIR_BOX;           // plain: the box is the half
+            const uint32_t bytes = 2 * (128 * BK * 2) + (GROUPED ? (two ? 4 : 2) * PAIR_BOX : t.bn) * (BK * 2);
+            for (int kb = 0; kb < kb_total; ++kb, ++it) {
+                if (it >= first_n && !mbar_wait_warp(empty + 8 * s, phase ^ 1)) { ok = false; break; }
+                const uint32_t sa = smem_u32(smem) + s * PAIR_STAGE_BYTES, bar = full_lead + 8 * s;
+                if (elect_one()) {
+                    if (it >= first_n) {
+                        if (rank == 0) mbar_expect_tx(full + 8 * s, bytes);
+                        tma_load_2d_pair(sa, &map_w, bar, kb * BK, w0);
+                    }
+                    tma_load_2d_pair(sa + 128 * BK * 2, &map_x, bar, kb * BK, t0);
+                    if (two) tma_load_2d_pair(sa + (128 + PAIR_BOX) * BK * 2, &map_x, bar, kb * BK, t0 + PAIR_BOX);
+                }
+                __syncwarp();
+                if (++s == PAIR_STAGES) { s = 0; phase ^= 1; }
+            }
+        }
+        // the last commits arrive at this CTA's barriers before it may leave
+        for (int i = max(0, it - PAIR_STAGES); i < it && ok; ++i)
+            ok = mbar_wait_warp(empty + 8 * (i % PAIR_STAGES), (i / PAIR_STAGES) & 1);
+        if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+    } else if (warp == 1) {
+        if (rank == 0) {
+            int n = 0;
+            for (int tile = pair; tile < total && ok; tile += pairs, ++n) {
+                const int buf = n & 1, width = tile_of(tile).bn;
+                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+                if (!mbar_wait_warp(acce + 8 * buf, ((n >> 1) & 1) ^ 1)) { ok = false; break; }
+                tc_fence_after();
+                for (int kb = 0; kb < kb_total; ++kb) {
+                    if (!mbar_wait_warp(full + 8 * s, phase)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sa = smem_u32(smem) + s * PAIR_STAGE_BYTES;
+                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + 128 * BK * 2);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k)
+                            umma_bf16_pair(tmem + buf * PAIR_BN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_commit_pair(empty + 8 * s);
+                        if (kb + 1 == kb_total) umma_commit_pair(accf + 8 * buf);
+                    }
+                    __syncwarp();
+                    if (++s == PAIR_STAGES) { s = 0; phase ^= 1; }
+                }
+            }
+            if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+        }
+    } else {
+        const int quad = warp & 3, half = (warp - 2) >> 2;         // two warps a quadrant of lanes, every other 32 columns
+        int n = 0;
+        for (int tile = pair; tile < total; tile += pairs, ++n) {
+            const int buf = n & 1;
+            const Tile t = tile_of(tile);
+            const int row = t.w0 + rank * 128 + quad * 32 + lane;
+            const bool row_on = row < p.a_rows;
+            if (!mbar_wait(accf + 8 * buf, (n >> 1) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
+            tc_fence_after();
+            const uint32_t lanes = tmem + buf * PAIR_BN + ((uint32_t)(quad * 32) << 16);
+            auto hand_back = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(acce_lead + 8 * buf) : "memory");
+            };
+            const int cols = min(t.bn, t.t_end - t.t0);
+            if (32 * half >= cols) hand_back();                    // nothing of this tile is this warp's
+#pragma unroll 1
+            for (int c = 32 * half; c < cols; c += 64) {
+                uint32_t r[32];
+                __syncwarp();
+                tmem_ld32_async(lanes + c, r);
+                tmem_wait32(r);
+                if (c + 64 >= cols) hand_back();
+#pragma unroll
+                for (int h = 0; h < 32; h += 16) {
+                    float v[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h + i]);
+                    if (EPI != EPI_SWIGLU && p.act) epilogue_act(v, p.act - 1);
+                    store_pair<EPI>(p, v, row, row_on, t.t0 + c + h, cols - c - h);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                            // neither CTA leaves, or frees, while the other works on both
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+#endif  // !AIRUN_FOLD_NORM
 
 // ------------------------------------------------------------------ host side
 struct MapKey {
@@ -887,14 +1123,13 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
     return airun_launch_status();
 }
 
-template <int EPI, int FORM = FORM_PLAIN>
+template <int EPI, bool BATCHED = false>
 int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t stream) {
-    constexpr bool GROUPED = FORM == FORM_GROUPED;
     using L = SmemLayout<PBN, PSTAGES>;
     constexpr int SMEM = L::TOTAL + 64;
     static unsigned long long configured = 0;
     static int sms_of[64];
-    auto kern = gemm_tcgen05_persistent_kernel<EPI, FORM>;
+    auto kern = gemm_tcgen05_persistent_kernel<EPI, BATCHED>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return AIRUN_ERR_ARG;
@@ -904,14 +1139,51 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmPa
         cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev);
     }
     const int n_sm = sms_of[dev];
-    const int m_tiles = (p.a_rows + BM - 1) / BM + (GROUPED ? p.n_seg : 0), n_tiles = (p.b_rows + PBN - 1) / PBN;
-    if (GROUPED && (m_tiles > GROUP_MAX_TILES || p.n_seg > GROUP_MAX_SEGS)) return AIRUN_ERR_ARG;
-    const long long total = (long long)m_tiles * n_tiles * (FORM == FORM_BATCHED ? p.n_seg : 1);
+    const int m_tiles = (p.a_rows + BM - 1) / BM, n_tiles = (p.b_rows + PBN - 1) / PBN;
+    const long long total = (long long)m_tiles * n_tiles * (BATCHED ? p.n_seg : 1);
     if (total > 0x3fffffff) return AIRUN_ERR_ARG;
     const int grid = total < n_sm ? total : n_sm;
     airun_launch(kern, dim3(grid), dim3(P_THREADS), SMEM, stream, ma, mb, p, m_tiles, n_tiles);
     return airun_launch_status();
 }
+
+#if !AIRUN_FOLD_NORM
+// How many pairs the GPU holds at once (0: unknown).
+template <int EPI, bool GROUPED>
+int pair_capacity() {
+    static int known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if ((n = __atomic_load_n(&known[dev], __ATOMIC_RELAXED)) > 0) return n;
+    auto kern = gemm_pair_kernel<EPI, GROUPED>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.dynamicSmemBytes = PAIR_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;                              // (the hardware's pairs are neighbours in x)
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) return 0;
+    __atomic_store_n(&known[dev], n, __ATOMIC_RELAXED);
+    return n;
+}
+
+template <int EPI, bool GROUPED>
+int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int bn, int tok_tiles, cudaStream_t stream) {
+    const int cap = pair_capacity<EPI, GROUPED>();
+    if (cap <= 0) { cudaGetLastError(); return AIRUN_ERR_UNSUPPORTED; }
+    const long long total = (long long)((p.a_rows + 255) / 256) * tok_tiles;
+    if (total > 0x3fffffff) return AIRUN_ERR_ARG;
+    const int pairs = total < cap ? (int)total : cap;
+    airun_launch_clusters(gemm_pair_kernel<EPI, GROUPED>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, stream, dim3(2), mw, mx, p, bn, tok_tiles);
+    return airun_launch_status();
+}
+#endif
 
 // How many clusters of `ks` CTAs of this kernel the GPU holds at once (0: unknown or none).  A product
 // whose tiles outnumber them would run its last clusters alone in a second wave.
@@ -1071,6 +1343,36 @@ static int gemm_launch(const void* x, const void* W, void* out, int M, int N, in
     return AIRUN_ERR_UNSUPPORTED;
 }
 
+#if !AIRUN_FOLD_NORM
+// out[M][N] = x[M][K] * W[N][K]^T, two SMs to a tile of 256 weight rows x bn tokens (bn a multiple of 32 up to 256).  epi 0, 1, 2 as above; act: 0, or
+// 1 + the mode of an activation (epi 0 and 1); limit > 0: the clamped gated unit (epi 2).
+AIRUN_EXPORT int airun_gemm_pair(const void* x, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldc, int epi,
+                                 int act, float limit, float slope, int bn, int* err, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0 || !err) return M == 0 ? AIRUN_OK : AIRUN_ERR_ARG;
+    if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)W & 15)) return AIRUN_ERR_ARG;
+    if (bn < 32 || bn > PAIR_BN || bn % 32 || act < 0 || act > 5 || (epi == EPI_SWIGLU && (N % 32 != 0 || act))) return AIRUN_ERR_ARG;
+    GemmParams p = {};
+    p.a_rows = N;
+    p.b_rows = M;
+    p.K = K;
+    p.out = out;
+    p.ldc = ldc;
+    p.err = err;
+    p.act = act;
+    p.glu_limit = limit;
+    p.glu_slope = slope;
+    CUtensorMap mw, mx;
+    int r;
+    if ((r = make_map(&mw, W, N, K, ldw, 128)) != AIRUN_OK) return r;
+    if ((r = make_map(&mx, x, M, K, ldx, bn / 2)) != AIRUN_OK) return r;
+    const int tiles = (M + bn - 1) / bn;
+    if (epi == EPI_F32) return launch_pair<EPI_F32, false>(mw, mx, p, bn, tiles, stream);
+    if (epi == EPI_BF16) return launch_pair<EPI_BF16, false>(mw, mx, p, bn, tiles, stream);
+    if (epi == EPI_SWIGLU) return launch_pair<EPI_SWIGLU, false>(mw, mx, p, bn, tiles, stream);
+    return AIRUN_ERR_UNSUPPORTED;
+}
+#endif
+
 // The grouped product: rows seg[e] .. seg[e + 1] - 1 of x [M][K] times W[e] ([n_seg][N][K], contiguous) into the same
 // rows of out.  epi 0: float32 [M][N]; 1: bfloat16 [M][N]; 2: SwiGLU over interleaved gate/up rows, bfloat16 [M][N/2].
 // ``seg`` (int32 [n_seg + 1]) lives on the device; rows from seg[n_seg] on are left as they are.
@@ -1122,11 +1424,18 @@ static int gemm_grouped(const void* x, const void* W, void* out, int M, int N, i
     p.glu_slope = glu_slope;
     CUtensorMap ma, mb;
     int r;
-    if ((r = make_map(&ma, x, M, K, ldx, BM)) != AIRUN_OK) return r;
-    if ((r = make_map(&mb, W, (long long)n_seg * N, K, K, PBN)) != AIRUN_OK) return r;
-    if (epi == EPI_F32) return launch_persistent<EPI_F32, FORM_GROUPED>(ma, mb, p, stream);
-    if (epi == EPI_BF16) return launch_persistent<EPI_BF16, FORM_GROUPED>(ma, mb, p, stream);
-    if (epi == EPI_SWIGLU) return launch_persistent<EPI_SWIGLU, FORM_GROUPED>(ma, mb, p, stream);
+#if !AIRUN_FOLD_NORM
+    // (the FOLD_NORM build has no grouped products)
+    const int tiles = (M + PAIR_BN - 1) / PAIR_BN + n_seg;
+    if (tiles > GROUP_MAX_TILES || n_seg > GROUP_MAX_SEGS) return AIRUN_ERR_ARG;
+    p.a_rows = N;
+    p.b_rows = M;
+    if ((r = make_map(&ma, W, (long long)n_seg * N, K, K, 128)) != AIRUN_OK) return r;
+    if ((r = make_map(&mb, x, M, K, ldx, PAIR_BOX)) != AIRUN_OK) return r;
+    if (epi == EPI_F32) return launch_pair<EPI_F32, true>(ma, mb, p, PAIR_BN, tiles, stream);
+    if (epi == EPI_BF16) return launch_pair<EPI_BF16, true>(ma, mb, p, PAIR_BN, tiles, stream);
+    if (epi == EPI_SWIGLU) return launch_pair<EPI_SWIGLU, true>(ma, mb, p, PAIR_BN, tiles, stream);
+#endif
     return AIRUN_ERR_UNSUPPORTED;
 }
 
@@ -1155,7 +1464,7 @@ AIRUN_EXPORT int airun_gemm_tcgen05_batched(const void* x, const void* W, void* 
     int r;
     if ((r = make_map(&ma, x, M, (n_batch - 1) * sx + K, ldx, BM)) != AIRUN_OK) return r;
     if ((r = make_map(&mb, W, (long long)n_batch * N, K, K, PBN)) != AIRUN_OK) return r;
-    return launch_persistent<EPI_BF16, FORM_BATCHED>(ma, mb, p, stream);
+    return launch_persistent<EPI_BF16, true>(ma, mb, p, stream);
 }
 
 AIRUN_EXPORT int airun_gemm_tcgen05_ex(const void* x, const void* W, void* out, int M, int N, int K,

@@ -65,6 +65,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (t1 - t0 > 2000000000ull) return false;
     }
 }
+// The same for a converged warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -168,7 +170,7 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
     __shared__ uint32_t tmem_slot;
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < L_BARS; ++i) mbar_init(BAR(i), i == L_PFULL ? 4 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -196,9 +198,12 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
         auto other = [&](int i) { return i < v0 ? i : i + nv; };       // the i-th block that is no value here
 
         if (warp == 0) {
-            if (lane == 0) {
-                mbar_expect_tx(BAR(L_QFULL), (uint32_t)(p.blocks * LT_QBLK));
-                for (int b = 0; b < p.blocks; ++b) tma_load_2d(smem_u32(smem + b * LT_QBLK), &q_map, BAR(L_QFULL), b * 64, tok0 * p.H);
+            {
+                if (elect_one()) {
+                    mbar_expect_tx(BAR(L_QFULL), (uint32_t)(p.blocks * LT_QBLK));
+                    for (int b = 0; b < p.blocks; ++b) tma_load_2d(smem_u32(smem + b * LT_QBLK), &q_map, BAR(L_QFULL), b * 64, tok0 * p.H);
+                }
+                __syncwarp();
                 const int32_t* bt = p.block_table + (size_t)req * p.max_blocks;
                 for (int it = 0; it < n_tiles; ++it) {
                     const int s = it % p.stages;
@@ -210,29 +215,35 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                         const int j = (tile_first + it) * LT_KEYS + g * 16, blk = j >> p.page_shift;
                         int page = (j <= pos_hi && blk < p.max_blocks) ? __ldg(bt + blk) : 0;
                         if (page < 0 || page >= p.num_pages) {
-                            if (j + 15 >= k_first) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
+                            if (j + 15 >= k_first && lane == 0) atomicOr(p.err, AIRUN_DEV_BAD_PAGE);      // a page the window has passed may be gone
                             page = 0;
                         }
                         rows[g] = (page << p.page_shift) + (j & (p.page_size - 1));
                     }
                     if (nn) {
-                        if (!mbar_wait(BAR(L_NEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                        mbar_expect_tx(BAR(L_NFULL + s), (uint32_t)(nn * LT_KBLK));
-                        for (int i = 0; i < nn; ++i)
+                        if (!mbar_wait_warp(BAR(L_NEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
+                        if (elect_one()) {
+                            mbar_expect_tx(BAR(L_NFULL + s), (uint32_t)(nn * LT_KBLK));
+                            for (int i = 0; i < nn; ++i)
+#pragma unroll
+                                for (int g = 0; g < LT_KEYS / 16; ++g)
+                                    tma_load_2d(dst + (nv + i) * LT_KBLK + g * 2048, &k_map, BAR(L_NFULL + s), other(i) * 64, rows[g]);
+                        }
+                        __syncwarp();
+                    }
+                    if (!mbar_wait_warp(BAR(L_VEMPTY + s), ph ^ 1)) { if (lane == 0) atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
+                    if (elect_one()) {
+                        mbar_expect_tx(BAR(L_VFULL + s), (uint32_t)(nv * LT_KBLK));
+                        for (int i = 0; i < nv; ++i)
 #pragma unroll
                             for (int g = 0; g < LT_KEYS / 16; ++g)
-                                tma_load_2d(dst + (nv + i) * LT_KBLK + g * 2048, &k_map, BAR(L_NFULL + s), other(i) * 64, rows[g]);
+                                tma_load_2d(dst + i * LT_KBLK + g * 2048, &k_map, BAR(L_VFULL + s), (v0 + i) * 64, rows[g]);
                     }
-                    if (!mbar_wait(BAR(L_VEMPTY + s), ph ^ 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-                    mbar_expect_tx(BAR(L_VFULL + s), (uint32_t)(nv * LT_KBLK));
-                    for (int i = 0; i < nv; ++i)
-#pragma unroll
-                        for (int g = 0; g < LT_KEYS / 16; ++g)
-                            tma_load_2d(dst + i * LT_KBLK + g * 2048, &k_map, BAR(L_VFULL + s), (v0 + i) * 64, rows[g]);
+                    __syncwarp();
                 }
             }
         } else if (warp == 1) {
-            if (lane == 0) {
+            {
                 constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LT_KEYS >> 3) << 17) | ((uint32_t)(LT_ROWS >> 4) << 24);
                 const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(nv * 64 >> 3) << 17) | ((uint32_t)(LT_ROWS >> 4) << 24);
                 const uint64_t qd = desc_kmajor(smem_u32(smem)), kd = desc_kmajor(smem_u32(smem_k)), vd = desc_mnmajor(smem_u32(smem_k));
@@ -247,35 +258,47 @@ __global__ __launch_bounds__(LT_THREADS, 1) void latent_prefill_kernel(
                 auto issue_n = [&](int it) -> bool {
                     if (!nn) return true;
                     const int s = it % p.stages;
-                    if (!mbar_wait(BAR(L_NFULL + s), (uint32_t)(it / p.stages) & 1u)) return false;
+                    if (!mbar_wait_warp(BAR(L_NFULL + s), (uint32_t)(it / p.stages) & 1u)) return false;
                     tc_fence_after();
-                    for (int i = 0; i < nn; ++i) issue_block(it, other(i), nv + i, i == 0);
-                    umma_commit(BAR(L_NEMPTY + s));
+                    if (elect_one()) {
+                        for (int i = 0; i < nn; ++i) issue_block(it, other(i), nv + i, i == 0);
+                        umma_commit(BAR(L_NEMPTY + s));
+                    }
+                    __syncwarp();
                     return true;
                 };
                 auto issue_v = [&](int it) -> bool {
                     const int s = it % p.stages;
-                    if (!mbar_wait(BAR(L_VFULL + s), (uint32_t)(it / p.stages) & 1u)) return false;
+                    if (!mbar_wait_warp(BAR(L_VFULL + s), (uint32_t)(it / p.stages) & 1u)) return false;
                     tc_fence_after();
-                    for (int i = 0; i < nv; ++i) issue_block(it, v0 + i, i, nn == 0 && i == 0);
-                    umma_commit(BAR(L_SFULL + (it & 1)));
+                    if (elect_one()) {
+                        for (int i = 0; i < nv; ++i) issue_block(it, v0 + i, i, nn == 0 && i == 0);
+                        umma_commit(BAR(L_SFULL + (it & 1)));
+                    }
+                    __syncwarp();
                     return true;
                 };
-                bool ok = mbar_wait(BAR(L_QFULL), 0);
+                bool ok = mbar_wait_warp(BAR(L_QFULL), 0);
                 if (ok && n_tiles > 0) ok = issue_n(0) && issue_v(0);
                 for (int it = 0; it < n_tiles && ok; ++it) {
                     if (it + 1 < n_tiles) ok = issue_n(it + 1);
-                    if (!ok || !mbar_wait(BAR(L_PFULL), it & 1)) { ok = false; break; }
+                    if (!ok || !mbar_wait_warp(BAR(L_PFULL), it & 1)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t v = v_lo + (uint32_t)((it % p.stages) * p.blocks * (LT_KBLK >> 4));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < LT_KEYS / 16; ++k)            // 16 keys of P are 8 columns of packed pairs
-                        umma_ts(tmem_o, tmem_base + (it & 1) * LT_KEYS + 8 * k, v + k * (2048 >> 4), v_hi, idesc_o, it > 0 || k > 0 ? 1u : 0u);
-                    umma_commit(BAR(L_VEMPTY + it % p.stages));
+                        for (int k = 0; k < LT_KEYS / 16; ++k)        // 16 keys of P are 8 columns of packed pairs
+                            umma_ts(tmem_o, tmem_base + (it & 1) * LT_KEYS + 8 * k, v + k * (2048 >> 4), v_hi, idesc_o, it > 0 || k > 0 ? 1u : 0u);
+                        umma_commit(BAR(L_VEMPTY + it % p.stages));
+                    }
+                    __syncwarp();
                     if (it + 1 < n_tiles) ok = issue_v(it + 1);
                 }
-                if (ok) umma_commit(BAR(L_FINAL));
-                else atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+                if (elect_one()) {
+                    if (ok) umma_commit(BAR(L_FINAL));
+                    else atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+                }
+                __syncwarp();
             }
         } else {
             const int quad = warp & 3, r = quad * 32 + lane;

@@ -217,6 +217,48 @@ def _plan_few_tiles(mt: int, N: int, kb: int, sms: int) -> Tuple[bool, int, int]
     return False, best[1], best[2]
 
 
+PAIR_MIN_TOKENS = 129                  # tokens from which a product runs on pairs of SMs
+
+
+@lru_cache(maxsize=4096)
+def plan_pair(M: int, N: int, K: int, sms: int = B200_SMS) -> int:
+    """Tokens of a tile (256 weight rows wide) of the product on pairs of SMs, by the clocks that its rounds take: a K-step costs its
+    products (2 a token), or what an SM takes in from the L2 cache (16 KB of weights and 64 bytes a token at 64 bytes a clock); the last
+    tile's results about 25 a token.  B200, us, tiles of 64, 96, 128, 160, 192 and 256 tokens: 512 x [4096, 2048] 13.2, 13.1, 10.3, 11.5, 12.8,
+    15.0; 900 x [6144, 2048] 27.9, 23.8, 21.1, 18.9, 20.8, 25.2; 2,048 x [2048, 6144] 61.0, 49.0, 38.7, 41.7, 48.1, 35.9."""
+    rows, kb, pairs = (N + 255) // 256, (K + 63) // 64, sms // 2
+    best = None
+    for bn in range(32, 257, 32):
+        tiles = rows * ((M + bn - 1) // bn)
+        clocks = (tiles + pairs - 1) // pairs * kb * max(2 * bn, 256 + bn) + 25 * min(bn, M)
+        if best is None or clocks < best[0]:
+            best = clocks, bn
+    return best[1]
+
+
+def gemm_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, err: torch.Tensor, bn: Optional[int] = None,
+              act: Optional[int] = None, glu: Tuple[float, float] = (0.0, 0.0)) -> None:
+    """out = x @ w^T with two SMs to a tile of 256 weight rows x ``bn`` tokens (csrc/gemm_tcgen05.cu, the pair kernel): the epilogues of
+    ``gemm_tcgen05``, an activation (EPI_F32, EPI_BF16) or the clamped gated unit (EPI_SWIGLU)."""
+    _cuda(x, w, out, err)
+    M, K = x.shape
+    N = w.shape[0]
+    _need(x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
+          and out.stride(1) == 1, "operands must be row-major bfloat16")
+    _need(tuple(out.shape) == (M, N // 2 if epi == EPI_SWIGLU else N), "output must be [M, N], of a gated unit [M, N/2]")
+    _need(out.dtype == (torch.float32 if epi == EPI_F32 else torch.bfloat16), "output type does not match the epilogue")
+    f = _fn("gemm_tcgen05", "airun_gemm_pair", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
+                                                c_int, c_float, c_float, c_int, c_void_p, c_void_p])
+    _check(f(_p(x), _p(w), _p(out), M, N, K, x.stride(0) if M > 1 else max(K, x.stride(0)), w.stride(0),
+             out.stride(0) if M > 1 else max(out.shape[1], out.stride(0)), epi, 0 if act is None else 1 + int(act), float(glu[0]), float(glu[1]),
+             plan_pair(M, N, K, machine(x.device).sms) if bn is None else bn, _p(err), _stream()), "gemm_pair")
+
+
+def _pairs(M: int, N: int) -> bool:
+    """Whether a product of M tokens with N weight rows runs on pairs of SMs."""
+    return M >= PAIR_MIN_TOKENS and "gemm_pair" not in DISABLED
+
+
 def _usable(x: torch.Tensor, w: torch.Tensor) -> bool:
     K = x.shape[1]
     return ("gemm" not in DISABLED and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
@@ -268,6 +310,9 @@ def linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, normed
     if normed is None and _few_rows(x.shape[0], w.shape[0], x.shape[1]):
         gemm_rows(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16)
         return True
+    if normed is None and _pairs(x.shape[0], w.shape[0]):
+        gemm_pair(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16, ctx.err)
+        return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])
     gemm_tcgen05(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16, swap, bn, ksplit, ctx.err,
                  **_normed_args(normed))
@@ -279,6 +324,9 @@ def linear_swiglu_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch.Tens
         return False
     if normed is None and _few_rows(x.shape[0], w_gu.shape[0], x.shape[1]):
         gemm_rows(x, w_gu, out, EPI_SWIGLU)
+        return True
+    if normed is None and _pairs(x.shape[0], w_gu.shape[0]):
+        gemm_pair(x, w_gu, out, EPI_SWIGLU, ctx.err)
         return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w_gu.shape[0], x.shape[1])
     gemm_tcgen05(x, w_gu, out, EPI_SWIGLU, swap, bn, ksplit, ctx.err, **_normed_args(normed))
@@ -698,6 +746,9 @@ def linear_glu_clamped_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch
     if _few_rows(M, N, K):
         gemm_rows(x, w_gu, out, EPI_SWIGLU, glu=(limit, slope))
         return True
+    if _pairs(M, N):
+        gemm_pair(x, w_gu, out, EPI_SWIGLU, ctx.err, glu=(limit, slope))
+        return True
     swap, bn, ksplit = plan_gemm(M, N, K)
     scratch = counters = None
     if ksplit > 1:
@@ -873,6 +924,9 @@ def linear_act_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mo
         return False
     if _few_rows(x.shape[0], w.shape[0], x.shape[1]):
         gemm_rows(x, w, out, EPI_BF16, act=mode)
+        return True
+    if _pairs(x.shape[0], w.shape[0]):
+        gemm_pair(x, w, out, EPI_BF16, ctx.err, act=mode)
         return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])
     gemm_tcgen05(x, w, out, EPI_BF16, swap, bn, ksplit, ctx.err, act=mode)

@@ -217,11 +217,16 @@ def _plan_few_tiles(mt: int, N: int, kb: int, sms: int) -> Tuple[bool, int, int]
     return False, best[1], best[2]
 
 
-PAIR_MIN_TOKENS = 129                  # tokens from which a product runs on pairs of SMs
+@lru_cache(maxsize=4096)
+def _few_tiles_us(mt: int, N: int, kb: int, sms: int) -> float:
+    """The time that ``_plan_few_tiles`` expects of its choice, and what goes before and after."""
+    _, bn, ks = _plan_few_tiles(mt, N, kb, sms)
+    tiles, (step, merge) = mt * ((N + bn - 1) // bn), (0.28, 5.0) if bn == 128 else (0.36, 8.0)
+    return 2.5 + ((tiles + sms - 1) // sms if ks == 1 else 1) * ((kb + ks - 1) // ks) * step + (merge if ks > 1 else 0.0)
 
 
 @lru_cache(maxsize=4096)
-def plan_pair(M: int, N: int, K: int, sms: int = B200_SMS) -> int:
+def _plan_pair(M: int, N: int, K: int, sms: int) -> Tuple[int, float]:
     """Tokens of a tile (256 weight rows wide) of the product on pairs of SMs, by the clocks that its rounds take: a K-step costs its
     products (2 a token), or what an SM takes in from the L2 cache (16 KB of weights and 64 bytes a token at 64 bytes a clock); the last
     tile's results about 25 a token.  B200, us, tiles of 64, 96, 128, 160, 192 and 256 tokens: 512 x [4096, 2048] 13.2, 13.1, 10.3, 11.5, 12.8,
@@ -233,7 +238,12 @@ def plan_pair(M: int, N: int, K: int, sms: int = B200_SMS) -> int:
         clocks = (tiles + pairs - 1) // pairs * kb * max(2 * bn, 256 + bn) + 25 * min(bn, M)
         if best is None or clocks < best[0]:
             best = clocks, bn
-    return best[1]
+    return best[1], 2.2 + best[0] / 1900.0
+
+
+def plan_pair(M: int, N: int, K: int, sms: int = B200_SMS) -> int:
+    """Tokens of a tile (see ``_plan_pair``)."""
+    return _plan_pair(M, N, K, sms)[0]
 
 
 def gemm_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, err: torch.Tensor, bn: Optional[int] = None,
@@ -254,9 +264,21 @@ def gemm_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, err
              plan_pair(M, N, K, machine(x.device).sms) if bn is None else bn, _p(err), _stream()), "gemm_pair")
 
 
-def _pairs(M: int, N: int) -> bool:
-    """Whether a product of M tokens with N weight rows runs on pairs of SMs."""
-    return M >= PAIR_MIN_TOKENS and "gemm_pair" not in DISABLED
+def _pairs(M: int, N: int, K: int) -> bool:
+    """Whether a product of M tokens with an [N, K] weight runs on pairs of SMs.  Pairs do not cut K, so few long rows of tiles stay with the clustered
+    slices: above 128 tokens the estimates of both decide.  B200, weights not in the L2 cache, us, slices and pairs: 224 tokens x [2048, 6144] 13.2,
+    19.9; [4096, 12288] 32.7, 42.5; [2048, 2048] 9.3, 9.0; [4096, 2048] 10.9, 9.8; [12288, 2048] gated 19.3, 16.2.  Up to 128 tokens, where
+    the weights are the 128-row operand in either: 96 tokens x [1024, 1024] 7.3, 5.4; [2048, 2048] 7.7, 8.5; [5152, 2048] 9.7, 9.7; [12288, 2048] 16.4,
+    13.1; 128 tokens 8.2, 5.4; 8.3, 8.4; 10.9, 10.0; 17.2, 13.9; [6144, 4096] 16.1, 16.9.  64 tokens x [2048, 2048] 5.7, 8.5; [12288, 2048] 13.4, 12.8."""
+    if "gemm_pair" in DISABLED or M <= 64:
+        return False
+    kb = (K + 63) // 64
+    if M <= 128:
+        return kb <= 32 and (M > 96 or N >= 5120 or kb <= 16)
+    sms, mt = machine().sms, (M + 127) // 128
+    if N >= 256 and mt * ((N + 255) // 256) >= sms * 96 // B200_SMS:
+        return True
+    return _plan_pair(M, N, K, sms)[1] <= _few_tiles_us(mt, N, kb, sms)
 
 
 def _usable(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -310,7 +332,7 @@ def linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, normed
     if normed is None and _few_rows(x.shape[0], w.shape[0], x.shape[1]):
         gemm_rows(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16)
         return True
-    if normed is None and _pairs(x.shape[0], w.shape[0]):
+    if normed is None and _pairs(x.shape[0], w.shape[0], x.shape[1]):
         gemm_pair(x, w, out, EPI_F32 if out.dtype == torch.float32 else EPI_BF16, ctx.err)
         return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])
@@ -325,7 +347,7 @@ def linear_swiglu_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch.Tens
     if normed is None and _few_rows(x.shape[0], w_gu.shape[0], x.shape[1]):
         gemm_rows(x, w_gu, out, EPI_SWIGLU)
         return True
-    if normed is None and _pairs(x.shape[0], w_gu.shape[0]):
+    if normed is None and _pairs(x.shape[0], w_gu.shape[0], x.shape[1]):
         gemm_pair(x, w_gu, out, EPI_SWIGLU, ctx.err)
         return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w_gu.shape[0], x.shape[1])
@@ -746,7 +768,7 @@ def linear_glu_clamped_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch
     if _few_rows(M, N, K):
         gemm_rows(x, w_gu, out, EPI_SWIGLU, glu=(limit, slope))
         return True
-    if _pairs(M, N):
+    if _pairs(M, N, K):
         gemm_pair(x, w_gu, out, EPI_SWIGLU, ctx.err, glu=(limit, slope))
         return True
     swap, bn, ksplit = plan_gemm(M, N, K)
@@ -925,7 +947,7 @@ def linear_act_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mo
     if _few_rows(x.shape[0], w.shape[0], x.shape[1]):
         gemm_rows(x, w, out, EPI_BF16, act=mode)
         return True
-    if _pairs(x.shape[0], w.shape[0]):
+    if _pairs(x.shape[0], w.shape[0], x.shape[1]):
         gemm_pair(x, w, out, EPI_BF16, ctx.err, act=mode)
         return True
     swap, bn, ksplit = plan_gemm(x.shape[0], w.shape[0], x.shape[1])

@@ -106,25 +106,26 @@ struct SmemLayout {
     static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16 + 1024;   // + alignment slack
 };
 
-// An activation of 16 results in place, for feed-forwards without a gate (out = f(x W^T)):
+// An activation of N results in place, for feed-forwards without a gate (out = f(x W^T)):
 //   m = 0: relu(z)^2   1: z * sigmoid(z)   2: 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))   3: relu(z)
 //       4: 0.5 z (1 + erf(z / sqrt(2)))
+template <int N = 16>
 __device__ __forceinline__ void epilogue_act(float* v, int m) {
     if (m == 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { const float r = fmaxf(v[i], 0.0f); v[i] = r * r; }
+        for (int i = 0; i < N; ++i) { const float r = fmaxf(v[i], 0.0f); v[i] = r * r; }
     } else if (m == 1) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = quotient(v[i], 1.0f + __expf(-v[i]));
+        for (int i = 0; i < N; ++i) v[i] = quotient(v[i], 1.0f + __expf(-v[i]));
     } else if (m == 2) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
+        for (int i = 0; i < N; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
     } else if (m == 4) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + erff(v[i] * 0.7071067811865476f));
+        for (int i = 0; i < N; ++i) v[i] = 0.5f * v[i] * (1.0f + erff(v[i] * 0.7071067811865476f));
     } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
+        for (int i = 0; i < N; ++i) v[i] = fmaxf(v[i], 0.0f);
     }
 }
 
@@ -215,22 +216,44 @@ __device__ __forceinline__ void store_swiglu_normal(const GemmParams& p, const f
         if (b0 + c0 + 16 + i < p.b_rows) o[i] = __float2bfloat16_rn(gated_unit(p.glu_limit, p.glu_slope, g[i], u[i]));
 }
 
-// Gated units where a lane is a weight row: lanes 0-15 hold gate rows, the lane 16 further on the matching up row.  v: 16 columns (tokens).  The gate lanes
-// take the first eight tokens, the up lanes the others: one exchange brings each the other half of its pairs.
-__device__ __forceinline__ void gated_units(float limit, float slope, const float* v, bool low, float (&y)[8]) {
-    float g[8], u[8];
+// Gated units where a lane is a weight row: lanes 0-15 hold gate rows, the lane 16 further on the matching up row.  v: 2 H columns (tokens).  The gate lanes
+// take the first H tokens, the up lanes the others: one exchange brings each the other half of its pairs.
+template <int H>
+__device__ __forceinline__ void gated_units(float limit, float slope, const float* v, bool low, float (&y)[H]) {
+    float g[H], u[H];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float other = __shfl_xor_sync(0xffffffffu, low ? v[i + 8] : v[i], 16);
+    for (int i = 0; i < H; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, low ? v[i + H] : v[i], 16);
         g[i] = low ? v[i] : other;
-        u[i] = low ? other : v[i + 8];
+        u[i] = low ? other : v[i + H];
     }
     if (limit > 0.0f) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) y[i] = gated_unit(limit, slope, g[i], u[i]);
+        for (int i = 0; i < H; ++i) y[i] = gated_unit(limit, slope, g[i], u[i]);
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) y[i] = silu_mul(g[i], u[i]);
+        for (int i = 0; i < H; ++i) y[i] = silu_mul(g[i], u[i]);
+    }
+}
+
+// Eight tokens from `tok` on (the first n are there) of this lane's weight row, with the epilogue.
+template <int EPI>
+__device__ __forceinline__ void store_eight(const GemmParams& p, float* v, int row, int tok, int n) {
+    if constexpr (EPI == EPI_SWIGLU) {
+        const int lane = threadIdx.x & 31;
+        const bool low = lane < 16;
+        if (!low) { tok += 4; n -= 4; }
+        float y[4];
+        gated_units(p.glu_limit, p.glu_slope, v, low, y);
+        __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)tok * p.ldc + (row >> 5) * 16 + (lane & 15);
+#pragma unroll
+        for (int i = 0; i < 4; ++i, o += p.ldc) if (i < n && row < p.a_rows) *o = __float2bfloat16_rn(y[i]);
+    } else {
+        typedef typename std::conditional<EPI == EPI_F32, float, __nv_bfloat16>::type TOut;
+        if (p.act) epilogue_act<8>(v, p.act - 1);
+        TOut* o = (TOut*)p.out + (size_t)tok * p.ldc + row;
+#pragma unroll
+        for (int i = 0; i < 8; ++i, o += p.ldc) if (i < n && row < p.a_rows) *o = from_f32<TOut>(v[i]);
     }
 }
 
@@ -332,6 +355,8 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 1);
     __shared__ int s_ticket;
     __shared__ int s_abort;
+    // PUSH: the slices are brought together by stores (see push_slices)
+    constexpr bool PUSH = CLUSTER && SWAP && !AIRUN_FOLD_NORM;
 
     pdl_trigger();
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -357,6 +382,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (PUSH) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     // The weight operand (A when swapped, B otherwise) is written by no kernel, so the first stages'
     // weight blocks are requested before waiting for the kernel before this one: the weights keep
@@ -373,6 +399,10 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     }
     // from here on the results of earlier kernels are read and their buffers written
     pdl_wait();
+    if (PUSH) {
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // every CTA of the cluster runs: its memory may be written
+    }
 
     // what the epilogue warps (2..5) share between their two phases
     const int quad = warp & 3;
@@ -477,6 +507,52 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
         }
     };
 
+    // The columns of a tile in units of eight; unit u is added up by CTA u % ksplit of the cluster.  Every CTA stores its sums of a unit straight into that
+    // CTA's memory, where a place is kept for each slice, [slice][unit / ksplit][2][128 rows][4], so after one barrier each adds up what lies in its own,
+    // in slice order, and may leave: nothing is read from a peer.  (With the sums left in place and read by the peers, 64 tokens x [2048, 2048] in
+    // four slices spent 3.0 of its 6.2 us on two barriers and the reads.)
+    [[maybe_unused]] const int my_units = (BN / 8 + p.ksplit - 1) / p.ksplit;
+    [[maybe_unused]] float* const landing = reinterpret_cast<float*>(smem + L::BAR_OFFSET + 1024);
+    [[maybe_unused]] auto push_slices = [&] {
+        const uint32_t row_at = smem_u32(landing) + (uint32_t)(quad * 32 + lane) * 16u;
+        const uint32_t mine = cluster_rank() * (uint32_t)my_units;
+        int dest = 0, slot = 0;
+#pragma unroll 1
+        for (int c = 0; c < cols; c += 16) {
+            uint32_t r[16];
+            __syncwarp();
+            tmem_ld_async(lane_addr + c, r);
+            tmem_wait(r);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t to = map_to_cta(row_at + (mine + slot) * 4096u, (uint32_t)dest);
+                if (c + 8 * h < cols) {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(to + q * 2048u), "r"(r[8 * h + 4 * q]), "r"(r[8 * h + 4 * q + 1]),
+                                     "r"(r[8 * h + 4 * q + 2]), "r"(r[8 * h + 4 * q + 3]) : "memory");
+                }
+                if (++dest == p.ksplit) { dest = 0; ++slot; }
+            }
+        }
+    };
+    [[maybe_unused]] auto finish_units = [&] {
+        const float4* at = reinterpret_cast<const float4*>(landing) + quad * 32 + lane;
+        int c = 8 * (int)cluster_rank();
+        for (int j = 0; c < cols; ++j, c += 8 * p.ksplit) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+#pragma unroll 4
+            for (int q = 0; q < p.ksplit; ++q) {
+                const float4 x = at[(q * my_units + j) * 256], y = at[(q * my_units + j) * 256 + 128];
+                v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+                v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+            }
+            store_eight<EPI == EPI_RESID ? EPI_F32 : EPI>(p, v, a_row, b0 + c, cols - c);
+        }
+    };
+
     if (warp == 0) {
         int s = 0;
         uint32_t phase = 0;
@@ -555,7 +631,10 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
         if (!ok) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); }
         tc_fence_after();
         bool last = true;
-        if (!direct) {
+        if constexpr (PUSH) {
+            if (ok && n_kb > 0) push_slices();
+            last = false;
+        } else if (!direct) {
             // the partial tile goes to this CTA's own shared memory (the stages are free: every MMA is
             // complete) when the slices of a tile form a cluster, else to the scratch in global memory
             float* part = clustered ? reinterpret_cast<float*>(smem)
@@ -599,9 +678,13 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
         // and stores the result; nobody leaves while a peer may still read its memory.
         __syncwarp();
         cluster_sync_all();
-        if (warp >= 2) finish_tile((int)cluster_rank());
-        __syncwarp();
-        cluster_sync_all();
+        if constexpr (PUSH) {
+            if (warp >= 2) finish_units();
+        } else {
+            if (warp >= 2) finish_tile((int)cluster_rank());
+            __syncwarp();
+            cluster_sync_all();
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -1086,10 +1169,19 @@ int make_map(CUtensorMap* out, const void* ptr, long long rows, long long K, lon
     return AIRUN_OK;
 }
 
-// Stages of the clustered build: as many as fit in 200 KB, at most twice the plain build's.
-constexpr int cluster_stages(int bn, int stages) {
-    const int stage_bytes = (BM + bn) * BK * 2;
-    const int fit = (200 * 1024) / stage_bytes;
+// Bytes that a clustered CTA keeps for its peers' sums: for BN / 8 units, one more a slice where the units do not go round evenly (up to 8 slices).
+constexpr int landing_bytes(int bn, bool swap) {
+    int most = 0;
+    for (int ks = 2; ks <= 8; ++ks) {
+        const int n = ks * ((bn / 8 + ks - 1) / ks);
+        if (n > most) most = n;
+    }
+    return swap && !AIRUN_FOLD_NORM ? 1024 + most * 4096 : 0;
+}
+// Stages of the clustered build: as many as fit beside that in 224 KB, or 200 KB without, at most twice the plain build's.
+constexpr int cluster_stages(int bn, int stages, bool swap) {
+    const int stage_bytes = (BM + bn) * BK * 2, keep = landing_bytes(bn, swap);
+    const int fit = ((keep ? 222 : 200) * 1024 - keep) / stage_bytes;
     return fit < 2 * stages ? fit : 2 * stages;
 }
 
@@ -1101,15 +1193,14 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
         if (p.cluster_reduce) {
             // clustered CTAs are placed one to an SM at most (ncu: launch__cluster_max_active), so each
             // may as well use the whole shared memory: twice the stages
-            constexpr int CS = cluster_stages(BN, STAGES);
-            using LC = SmemLayout<BN, CS>;
+            constexpr int CS = cluster_stages(BN, STAGES, SWAP), SMEM = SmemLayout<BN, CS>::TOTAL + landing_bytes(BN, SWAP);
             static unsigned long long configured_c = 0;       // one bit per device: the attribute is the device's
             auto kern = gemm_tcgen05_kernel<BN, CS, EPI, SWAP, true>;
             if (first_on_device(configured_c)) {
-                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LC::TOTAL);
+                cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
                 if (e != cudaSuccess) return (int)e;
             }
-            airun_launch_cluster(kern, dim3(grid), dim3(GEMM_THREADS), LC::TOTAL, stream, (unsigned)p.ksplit, ma, mb, p);
+            airun_launch_cluster(kern, dim3(grid), dim3(GEMM_THREADS), SMEM, stream, (unsigned)p.ksplit, ma, mb, p);
             return airun_launch_status();
         }
     }
@@ -1194,13 +1285,13 @@ int cluster_capacity(int ks) {
     if (ks < 2 || ks > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     int* cache = per_device[dev];
     if (cache[ks] == 0) {
-        using L = SmemLayout<BN, cluster_stages(BN, STAGES)>;
-        auto kern = gemm_tcgen05_kernel<BN, cluster_stages(BN, STAGES), EPI, SWAP, true>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+        constexpr int CS = cluster_stages(BN, STAGES, SWAP), SMEM = SmemLayout<BN, CS>::TOTAL + landing_bytes(BN, SWAP);
+        auto kern = gemm_tcgen05_kernel<BN, CS, EPI, SWAP, true>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, 1, ks);
         cfg.blockDim = dim3(GEMM_THREADS);
-        cfg.dynamicSmemBytes = L::TOTAL;
+        cfg.dynamicSmemBytes = SMEM;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1;

@@ -268,13 +268,14 @@ def _pairs(M: int, N: int, K: int) -> bool:
     """Whether a product of M tokens with an [N, K] weight runs on pairs of SMs.  Pairs do not cut K, so few long rows of tiles stay with the clustered
     slices: above 128 tokens the estimates of both decide.  B200, weights not in the L2 cache, us, slices and pairs: 224 tokens x [2048, 6144] 13.2,
     19.9; [4096, 12288] 32.7, 42.5; [2048, 2048] 9.3, 9.0; [4096, 2048] 10.9, 9.8; [12288, 2048] gated 19.3, 16.2.  Up to 128 tokens, where
-    the weights are the 128-row operand in either: 96 tokens x [1024, 1024] 7.3, 5.4; [2048, 2048] 7.7, 8.5; [5152, 2048] 9.7, 9.7; [12288, 2048] 16.4,
-    13.1; 128 tokens 8.2, 5.4; 8.3, 8.4; 10.9, 10.0; 17.2, 13.9; [6144, 4096] 16.1, 16.9.  64 tokens x [2048, 2048] 5.7, 8.5; [12288, 2048] 13.4, 12.8."""
+    the weights are the rows of the tile in either, where even two slices would not be resident together, or K is short: 96 tokens x [1024, 1024] 6.4, 5.4; [2048,
+    2048] 6.3, 8.5; [5152, 2048] 8.4, 9.7; [12288, 2048] 16.4, 13.2; 128 tokens 7.2, 5.4; 6.9, 8.5; 9.1, 10.0; 17.1, 13.9; [24576, 4096] 43.0, 44.0;
+    [32768, 2048] 30.4, 28.6.  64 tokens x [1024, 1024] 5.1, 5.5."""
     if "gemm_pair" in DISABLED or M <= 64:
         return False
     kb = (K + 63) // 64
     if M <= 128:
-        return kb <= 32 and (M > 96 or N >= 5120 or kb <= 16)
+        return kb <= 16 or kb <= 32 and 2 * ((N + 127) // 128) > machine().sms
     sms, mt = machine().sms, (M + 127) // 128
     if N >= 256 and mt * ((N + 255) // 256) >= sms * 96 // B200_SMS:
         return True

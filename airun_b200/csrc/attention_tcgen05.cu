@@ -759,7 +759,13 @@ __device__ __forceinline__ float w_sigmoid(float x) {
 }
 enum { W_KFULL = 0, W_KEMPTY = 2, W_VFULL = 4, W_VEMPTY = 6, W_SFULL = 8, W_PFULL = 10, W_FINAL = 12, W_PHALF = 13 };
 
-template <int KIND>
+// SPLIT (W_SIGMOID): two CTAs (a cluster) to a tile, each with half of the tile's keys.  With no more tiles than SMs the time is that of the longest tile, of
+// twice the average's keys under a causal mask.  Afterwards CTA x takes Q tile x: the peer stores its part of the sums into this CTA's memory (the stages of K),
+// and they are added up.  Tiles of up to SPLIT_MIN_KEYS tiles of keys stay whole: the second CTA leaves at once.  A 2,048-token prompt of Gamanex (16 heads over 8 KV
+// heads, six layers) 2,636 -> 2,576 us (2,612 with tiles of up to 8 whole).  The softmax kinds, whose steps are shorter and whose sums need a common
+// scale, gained nothing: 3,050 -> 3,085 us for Tagulix, which has them with a table and with a window.
+constexpr int SPLIT_MIN_KEYS = 4;
+template <int KIND, bool SPLIT = false>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     const TcParams p, const int4* tiles, const __grid_constant__ CUtensorMap kv_map,
     const int* n_tiles_dev, const WideExtra ex) {
@@ -814,8 +820,33 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
     const int pos_lo = p.positions[tok0], pos_hi = p.positions[tok0 + n_tok - 1];
     int k_first = p.window > 0 ? max(0, pos_lo - p.window + 1) : 0;
     if (DIFF && ex.chunk > 0) k_first = max(k_first, pos_lo / ex.chunk * ex.chunk);
-    const int tile_first = k_first / KN;
-    const int n_tiles = pos_hi >= 0 ? pos_hi / KN - tile_first + 1 : 0;
+    int tile_first = k_first / KN;
+    int n_tiles = pos_hi >= 0 ? pos_hi / KN - tile_first + 1 : 0;
+    const bool halves = SPLIT && n_tiles > SPLIT_MIN_KEYS;
+    const int rank = SPLIT ? (int)cluster_rank() : 0;
+    if (SPLIT) {
+        if (halves) {
+            const int first = (n_tiles + 1) / 2;
+            if (rank == 0) n_tiles = first;
+            else { n_tiles -= first; tile_first += first; }
+        } else if (rank > 0) {
+            tc_fence_before();
+            __syncthreads();
+            if (warp == 1) {
+                tc_fence_after();
+                tmem_dealloc(tmem_base, 512);
+            }
+            return;
+        }
+    }
+    // both barriers of the two CTAs, for the warps that have no part in what lies between
+    auto pass_barriers = [&] {
+        if (halves) {
+            __syncwarp();
+            cluster_sync_all();
+            cluster_sync_all();
+        }
+    };
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -863,6 +894,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
                 __syncwarp();
             }
         }
+        pass_barriers();
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
         {
@@ -937,6 +969,7 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             }
             __syncwarp();
         }
+        pass_barriers();
     } else if (two || warp < 6) {
         // ------------------------------------------------ softmax, correction, epilogue
         const int x = (warp - 2) >> 2;                    // this warpgroup's Q tile
@@ -1164,6 +1197,27 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
         if (ok && n_tiles > 0 && !mbar_wait(BAR(W_FINAL), 0)) ok = false;
         if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
         tc_fence_after();
+        // SPLIT: what the peer has of this warpgroup's rows, [4 columns][row], or where it goes
+        float4* const landing = reinterpret_cast<float4*>(smem + W_OFF_K) + r;
+        if (SPLIT && halves) {
+            __syncwarp();
+            cluster_sync_all();                                  // every product of both CTAs is complete: the stages are free
+            if (rank != x) {
+                const uint32_t to = map_to_cta(smem_u32(landing), (uint32_t)x);
+#pragma unroll
+                for (int c = 0; c < HD; c += 32) {
+                    float o[32];
+                    tmem_ld32(o_addr + c, o);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(to + (uint32_t)((c + i) / 4) * 2048u), "f"(o[i]), "f"(o[i + 1]),
+                                     "f"(o[i + 2]), "f"(o[i + 3]) : "memory");
+                }
+            }
+            __syncwarp();
+            cluster_sync_all();
+        }
+        const bool mine = !(SPLIT && halves) || rank == x;        // this CTA stores the rows
         float inv = l > 0.0f ? 1.0f / l : 0.0f;
         if constexpr (DIFF) {
             // every product is complete: map 2's rows go through the stages of K and V to the threads of map 1
@@ -1241,7 +1295,14 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 #pragma unroll
                 for (int i = 0; i < 32; ++i) o[i] = 0.0f;
             }
-            if (row_ok && ok) {
+            if (SPLIT && halves && mine) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 t = landing[(c + i) / 4 * 128];
+                    o[i] += t.x; o[i + 1] += t.y; o[i + 2] += t.z; o[i + 3] += t.w;
+                }
+            }
+            if (row_ok && ok && mine) {
 #pragma unroll
                 for (int q8 = 0; q8 < 4; ++q8) {
                     uint32_t w[4];
@@ -1265,6 +1326,8 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
             }
         }
         }
+    } else {
+        pass_barriers();
     }
     tc_fence_before();
     __syncthreads();
@@ -1428,18 +1491,22 @@ AIRUN_EXPORT int airun_attn_prefill_kinds(int kind, const void* q, void* out, lo
     const int width = tail >= 0 ? HD + tail : HD;
     const int r = kv_map_for(&map, pool, (long long)num_pages * (tail >= 0 ? 1 : 2) * nkv * page_size, width);
     if (r != AIRUN_OK) return r;
-    static unsigned long long configured[3];             // one bit per device
+    static unsigned long long configured[4];             // one bit per device
+    // two CTAs share a tile's keys while all tiles would run at once, one to an SM, and a window leaves them enough keys
+    const bool split = kind == W_SIGMOID && tile_rows == 2 * QM && (long long)n_tiles * nkv <= airun_sm_count() &&
+                       (window == 0 || window > 2 * SPLIT_MIN_KEYS * KN);
     auto go = [&](auto kern, int i) -> int {
         if (first_on_device(configured[i])) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (e != cudaSuccess) return (int)e;
         }
-        airun_launch(kern, dim3(n_tiles, nkv), dim3(TC_THREADS), smem, stream, p, (const int4*)tiles, map, n_tiles_dev, ex);
+        if (split) airun_launch_cluster(kern, dim3(n_tiles, nkv, 2), dim3(TC_THREADS), smem, stream, 2u, p, (const int4*)tiles, map, n_tiles_dev, ex);
+        else airun_launch(kern, dim3(n_tiles, nkv), dim3(TC_THREADS), smem, stream, p, (const int4*)tiles, map, n_tiles_dev, ex);
         return airun_launch_status();
     };
     if (kind == W_OPTIONS) return go(attn_prefill_wide_kernel<W_OPTIONS>, 0);
     if (kind == W_TABLE) return go(attn_prefill_wide_kernel<W_TABLE>, 1);
-    return go(attn_prefill_wide_kernel<W_SIGMOID>, 2);
+    return split ? go(attn_prefill_wide_kernel<W_SIGMOID, true>, 3) : go(attn_prefill_wide_kernel<W_SIGMOID>, 2);
 }
 
 // Differential attention: q [T][nh][2 * 64], pages of keys [nkv][page][2 * 64] then values [nkv][page][128]; cap > 0; tiles of

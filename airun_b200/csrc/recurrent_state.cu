@@ -244,14 +244,14 @@ struct RecurrentArgs {
     int vec_cols;            // four neighbouring value columns can be read and written as 16 bytes
 };
 
-// The request's small state: its last `tail_rows` rows become the last rows of (what it held, then this step's rows).  A
+// The request's small state, moved on by `shares` blocks, this one the `share`-th: its last `tail_rows` rows become the last rows of (what it held, then this step's rows).  A
 // thread owns whole columns; row s comes from a later row, so a batch of rows that is read before it is written, in
 // ascending order, never reads what was written.
-__device__ __forceinline__ void rs_move_tail(const RecurrentArgs& a, int slot, int t0, int n) {
+__device__ __forceinline__ void rs_move_tail(const RecurrentArgs& a, int slot, int t0, int n, int share, int shares) {
     if (a.tail_rows <= 0) return;
     float* tail = a.state + (size_t)slot * a.slot_stride + a.tail_off;
-    const int R = a.tail_rows, Wd = a.tail_width, share = blockIdx.y * gridDim.z + blockIdx.z;
-    for (int c = share * blockDim.x + threadIdx.x; c < Wd; c += blockDim.x * gridDim.y * gridDim.z) {
+    const int R = a.tail_rows, Wd = a.tail_width;
+    for (int c = share * blockDim.x + threadIdx.x; c < Wd; c += blockDim.x * shares) {
         for (int s0 = 0; s0 < R; s0 += 4) {
             float v[4];
 #pragma unroll
@@ -389,7 +389,7 @@ __global__ __launch_bounds__(128) void recurrent_state_kernel(RecurrentArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (DG == 4 && n == 1 && a.vec_cols) {
         rs_one_token<MODE, DP>(a, t0, slot, head, col0);
-        rs_move_tail(a, slot, t0, 1);
+        rs_move_tail(a, slot, t0, 1, blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z);
         return;
     }
     const int dg = lane & (DG - 1), cl = warp * (32 / DG) + lane / DG, col = col0 + cl;
@@ -589,7 +589,7 @@ __global__ __launch_bounds__(128) void recurrent_state_kernel(RecurrentArgs a) {
             if (d < D) sbase[(size_t)d * Dv] = S[i];
         }
     }
-    rs_move_tail(a, slot, t0, n);
+    rs_move_tail(a, slot, t0, n, blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z);
 }
 
 // ------------------------------------------------------------------------------------------ chunks of eight tokens
@@ -840,7 +840,7 @@ __device__ __forceinline__ float2 rs_unpack(rs_pair v) {
     return d;
 }
 
-// One block per (request, head, 16 value columns): a column is shared by DG neighbouring lanes with NS key channels each.
+// One block per (request, head, 16 NC value columns): a column is shared by DG neighbouring lanes with NS key channels each, NC columns a lane.
 // After the sums over key channels lane l of a column holds token l's prediction and its read-out of the old state and stands
 // for its write and its output; where DG is sixteen, one half of the lanes does the one and one the other.  What bounds a
 // prompt is how long one chunk takes, and with more blocks than SMs how often it reads shared memory.  With eight lanes a
@@ -849,21 +849,27 @@ __device__ __forceinline__ float2 rs_unpack(rs_pair v) {
 // and 213; heads of 256 channels, 500 tokens: 149 and 221 (a lane's chain of 32 channels is the longer one there).
 // MINB blocks an SM: named, the compiler gives a thread up to 200 registers and reads ahead (unnamed it took 71).  One decay a
 // head: two where the blocks fit (1536 tokens, 16 heads: 129 us, four 155), else four (4 x 300 tokens 84, four 77).
+// Blocks of one request are neighbours: of the requests that a padded step counts some are not there, and with requests fastest the blocks of those that are came
+// several to an SM while other SMs stayed empty (three prompts of Pogarax: 406,000 cycles on one SM, 1,200 on another, 175,000 on average; its call took 3,400
+// us instead of 3,130).
 // The launch waits for the kernel in front (airun_launch_after): packed on the SMs that it leaves first, the 128 blocks of
 // one request of 2048 tokens took 374 us instead of 232.
+// NC = 2: what is read of the keys and queries serves two columns of a thread, for steps whose blocks would be more than two an SM: three prompts of 811, 676 and 541
+// tokens through Pogarax 3,345 -> 3,130 us; one of 1,536 tokens through Pirerax, where the blocks are few and a chunk's chain counts, 2,936 -> 3,047.
 // CHUNK_CHANNEL, CHUNK_MIX: over the vectors of chunk_vectors_kernel, whose decays are theirs already.
-template <int NS, int KIND, int DG, int MINB>
+template <int NS, int KIND, int DG, int MINB, int NC>
 __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArgs a, const float* coef, ChunkVectors vec) {
     pdl_trigger();
     pdl_wait();
     constexpr bool VECS = KIND != CHUNK_HEAD, MIX = KIND == CHUNK_MIX;
-    constexpr int DP = NS * DG, NT = 16 * DG, COLS = 16, TT = DP >= 256 || (VECS && DP >= 128) ? 8 : 16;
-    constexpr bool KEEP_K = NS <= 8 && !VECS;     // the keys of a chunk stay in registers from the dot products to the update
+    constexpr int DP = NS * DG, NT = 16 * DG, COLS = 16 * NC, TT = DP >= 256 || (VECS && DP >= 128) ? 8 : 16;
+    constexpr bool KEEP_K = NS <= 8 && !VECS && NC == 1;     // the keys of a chunk stay in registers from the dot products to the update
     __shared__ __align__(16) float s_q[2][TT][DP], s_k[2][TT][DP], s_v[2][TT][COLS], s_c[2][TT][RS_COEF];
     __shared__ __align__(16) float s_e[VECS && !MIX ? 2 : 1][VECS && !MIX ? TT : 1][VECS && !MIX ? DP : 4];     // keys decayed to their chunk's end
     __shared__ __align__(16) float s_w[VECS ? 2 : 1][VECS ? TT / RS_CHUNK : 1][VECS ? DP : 4];                  // a chunk's whole decay
-    __shared__ __align__(16) float s_x[NT / 32][32 / DG][3][RS_CHUNK];        // per warp and column: what its lanes tell one another
-    const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS;
+    __shared__ __align__(16) float s_x[NT / 32][32 / DG][NC][3][RS_CHUNK];    // per warp and column: what its lanes tell one another
+    const int tiles = (a.Dv + COLS - 1) / COLS, tile = (int)blockIdx.x % tiles, head = (int)blockIdx.x / tiles % a.heads;
+    const int r = (int)blockIdx.x / tiles / a.heads, col0 = tile * COLS;
     const int t0 = a.cu_tokens[r], n = a.cu_tokens[r + 1] - t0;
     if (n <= 0) return;
     const int slot = a.state_slots[r];
@@ -873,8 +879,10 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
     }
     const int D = a.D, Dv = a.Dv;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int dg = lane & (DG - 1), tok = dg & (RS_CHUNK - 1), cl = warp * (32 / DG) + lane / DG, col = col0 + cl;
-    const bool col_ok = col < Dv;
+    const int dg = lane & (DG - 1), tok = dg & (RS_CHUNK - 1), cl = warp * (32 / DG) + lane / DG, col = col0 + cl;      // and column col + 16
+    bool col_ok[NC];
+#pragma unroll
+    for (int h = 0; h < NC; ++h) col_ok[h] = col + 16 * h < Dv;
     const int ncol = min(COLS, Dv - col0);
     // both stages start as zeros: padding and rows beyond the last token hold numbers whose weight is zero
     for (int e = threadIdx.x; e < 2 * TT * DP; e += NT) {
@@ -934,20 +942,22 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0, 0);
-    float* sbase = a.state + (size_t)slot * a.slot_stride + (size_t)head * D * Dv + (col_ok ? col : 0);
-    rs_pair S[NS / 2];                            // channel of number i: group of four (i / 4) * DG + dg, element i % 4
+    float* sbase = a.state + (size_t)slot * a.slot_stride + (size_t)head * D * Dv + col;
+    rs_pair S[NC][NS / 2];                        // channel of number i: group of four (i / 4) * DG + dg, element i % 4
 #pragma unroll
-    for (int i = 0; i < NS / 2; ++i) {
-        float v[2];
+    for (int h = 0; h < NC; ++h)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int d = (((2 * i + h) >> 2) * DG + dg) * 4 + ((2 * i + h) & 3);
-            v[h] = (col_ok && d < D) ? sbase[(size_t)d * Dv] : 0.0f;
+        for (int i = 0; i < NS / 2; ++i) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int d = (((2 * i + e) >> 2) * DG + dg) * 4 + ((2 * i + e) & 3);
+                v[e] = (col_ok[h] && d < D) ? sbase[(size_t)d * Dv + 16 * h] : 0.0f;
+            }
+            S[h][i] = rs_pack(v[0], v[1]);
         }
-        S[i] = rs_pack(v[0], v[1]);
-    }
     float* orow = a.out + (size_t)t0 * ((size_t)a.heads * Dv) + (size_t)head * Dv + col;
-    float (*sx)[RS_CHUNK] = s_x[warp][lane / DG];
+    float (*sxs)[3][RS_CHUNK] = s_x[warp][lane / DG];
     int it = 0;
     for (int base = 0; base < n; base += TT, ++it) {
         const int buf = it & 1;
@@ -957,10 +967,12 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
 #pragma unroll 1
         for (int c0 = 0; c0 < TT && base + c0 < n; c0 += RS_CHUNK) {
             const int nt = min(RS_CHUNK, n - base - c0);
-            rs_pair p2[RS_CHUNK], o2[RS_CHUNK];
+            rs_pair p2[NC][RS_CHUNK], o2[NC][RS_CHUNK];
             ulonglong2 kr[KEEP_K ? RS_CHUNK : 1][KEEP_K ? NS / 4 : 1];
 #pragma unroll
-            for (int i = 0; i < RS_CHUNK; ++i) { p2[i] = 0ull; o2[i] = 0ull; }
+            for (int h = 0; h < NC; ++h)
+#pragma unroll
+                for (int i = 0; i < RS_CHUNK; ++i) { p2[h][i] = 0ull; o2[h][i] = 0ull; }
 #pragma unroll
             for (int i4 = 0; i4 < NS / 4; ++i4) {
 #pragma unroll
@@ -968,26 +980,32 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
                     const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(&s_k[buf][c0 + i][(i4 * DG + dg) * 4]);
                     const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(&s_q[buf][c0 + i][(i4 * DG + dg) * 4]);
                     if (KEEP_K) kr[KEEP_K ? i : 0][KEEP_K ? i4 : 0] = k4;
-                    if (!MIX) { p2[i] = rs_fma2(S[2 * i4], k4.x, p2[i]); p2[i] = rs_fma2(S[2 * i4 + 1], k4.y, p2[i]); }
-                    o2[i] = rs_fma2(S[2 * i4], q4.x, o2[i]);
-                    o2[i] = rs_fma2(S[2 * i4 + 1], q4.y, o2[i]);
+#pragma unroll
+                    for (int h = 0; h < NC; ++h) {
+                        if (!MIX) { p2[h][i] = rs_fma2(S[h][2 * i4], k4.x, p2[h][i]); p2[h][i] = rs_fma2(S[h][2 * i4 + 1], k4.y, p2[h][i]); }
+                        o2[h][i] = rs_fma2(S[h][2 * i4], q4.x, o2[h][i]);
+                        o2[h][i] = rs_fma2(S[h][2 * i4 + 1], q4.y, o2[h][i]);
+                    }
                 }
             }
-            float sum[2 * RS_CHUNK];
+            float pred[NC], read[NC];                         // of this lane's token
 #pragma unroll
-            for (int i = 0; i < RS_CHUNK; ++i) {
-                const float2 pv = rs_unpack(p2[i]), ov = rs_unpack(o2[i]);
-                sum[i] = pv.x + pv.y; sum[RS_CHUNK + i] = ov.x + ov.y;
-            }
-            float pred, read;                                 // of this lane's token
-            if (DG == 2 * RS_CHUNK) {
-                rs_scatter_sum<2 * RS_CHUNK>(sum, lane);
-                pred = read = sum[0];
-            } else {
-                float (&ps)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum), (&os)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum + RS_CHUNK);
-                if (!MIX) rs_scatter_sum<RS_CHUNK>(ps, lane);
-                rs_scatter_sum<RS_CHUNK>(os, lane);
-                pred = ps[0]; read = os[0];
+            for (int h = 0; h < NC; ++h) {
+                float sum[2 * RS_CHUNK];
+#pragma unroll
+                for (int i = 0; i < RS_CHUNK; ++i) {
+                    const float2 pv = rs_unpack(p2[h][i]), ov = rs_unpack(o2[h][i]);
+                    sum[i] = pv.x + pv.y; sum[RS_CHUNK + i] = ov.x + ov.y;
+                }
+                if (DG == 2 * RS_CHUNK) {
+                    rs_scatter_sum<2 * RS_CHUNK>(sum, lane);
+                    pred[h] = read[h] = sum[0];
+                } else {
+                    float (&ps)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum), (&os)[RS_CHUNK] = *reinterpret_cast<float (*)[RS_CHUNK]>(sum + RS_CHUNK);
+                    if (!MIX) rs_scatter_sum<RS_CHUNK>(ps, lane);
+                    rs_scatter_sum<RS_CHUNK>(os, lane);
+                    pred[h] = ps[0]; read[h] = os[0];
+                }
             }
             const bool writes = dg < RS_CHUNK, reads = DG == RS_CHUNK || dg >= RS_CHUNK;
             // this lane's token from here on: c0 + tok; its rows of the inverse (its write) and of the products (its output)
@@ -1002,68 +1020,92 @@ __global__ __launch_bounds__(16 * DG, MINB) void delta_chunk_kernel(RecurrentArg
                 va = *reinterpret_cast<const ulonglong2*>(v);
                 vb = *reinterpret_cast<const ulonglong2*>(v + 4);
             };
-            ulonglong2 va, vb;
-            float u = s_v[buf][c0 + tok][cl];
-            if (MIX) {
-                u = tok < nt ? u : 0.0f;
-            } else {
-                if (writes) sx[0][tok] = fmaf(-dec.x, pred, u);
+            float u[NC];
+#pragma unroll
+            for (int h = 0; h < NC; ++h) {
+                u[h] = s_v[buf][c0 + tok][cl + 16 * h];
+                if (MIX) u[h] = tok < nt ? u[h] : 0.0f;
+                else if (writes) sxs[h][0][tok] = fmaf(-dec.x, pred[h], u[h]);
+            }
+            if (!MIX) {
                 __syncwarp();
-                eight(sx[0], va, vb);
-                u = row_times(cf, va, vb);
+#pragma unroll
+                for (int h = 0; h < NC; ++h) {
+                    ulonglong2 va, vb;
+                    eight(sxs[h][0], va, vb);
+                    u[h] = row_times(cf, va, vb);
+                }
             }
             if (writes) {
-                sx[1][tok] = u;
-                if (!VECS) sx[2][tok] = u * dec.y;
+#pragma unroll
+                for (int h = 0; h < NC; ++h) {
+                    sxs[h][1][tok] = u[h];
+                    if (!VECS) sxs[h][2][tok] = u[h] * dec.y;
+                }
             }
             if constexpr (VECS) {
 #pragma unroll
                 for (int i4 = 0; i4 < NS / 4; ++i4) {
                     const ulonglong2 w4 = *reinterpret_cast<const ulonglong2*>(&s_w[buf][c0 / RS_CHUNK][(i4 * DG + dg) * 4]);
-                    S[2 * i4] = rs_mul2(S[2 * i4], w4.x);
-                    S[2 * i4 + 1] = rs_mul2(S[2 * i4 + 1], w4.y);
+#pragma unroll
+                    for (int h = 0; h < NC; ++h) { S[h][2 * i4] = rs_mul2(S[h][2 * i4], w4.x); S[h][2 * i4 + 1] = rs_mul2(S[h][2 * i4 + 1], w4.y); }
                 }
             } else {
                 const float whole = s_c[buf][c0 + nt - 1][16];
                 const rs_pair w2 = rs_pack(whole, whole);
 #pragma unroll
-                for (int i = 0; i < NS / 2; ++i) S[i] = rs_mul2(S[i], w2);
+                for (int h = 0; h < NC; ++h)
+#pragma unroll
+                    for (int i = 0; i < NS / 2; ++i) S[h][i] = rs_mul2(S[h][i], w2);
             }
             __syncwarp();
-            eight(sx[1], va, vb);
-            ulonglong2 wa = va, wb = vb;
-            if (!VECS) eight(sx[2], wa, wb);
-            const float2 w01 = rs_unpack(wa.x), w23 = rs_unpack(wa.y), w45 = rs_unpack(wb.x), w67 = rs_unpack(wb.y);
-            const float w[RS_CHUNK] = {w01.x, w01.y, w23.x, w23.y, w45.x, w45.y, w67.x, w67.y};
+            float w[NC][RS_CHUNK], o[NC];
+#pragma unroll
+            for (int h = 0; h < NC; ++h) {
+                ulonglong2 va, vb;
+                eight(sxs[h][1], va, vb);
+                o[h] = fmaf(dec.x, read[h], row_times(cf + RS_CHUNK, va, vb));
+                if (!VECS) eight(sxs[h][2], va, vb);
+                const float2 w01 = rs_unpack(va.x), w23 = rs_unpack(va.y), w45 = rs_unpack(vb.x), w67 = rs_unpack(vb.y);
+                w[h][0] = w01.x; w[h][1] = w01.y; w[h][2] = w23.x; w[h][3] = w23.y; w[h][4] = w45.x; w[h][5] = w45.y; w[h][6] = w67.x; w[h][7] = w67.y;
+            }
 #pragma unroll
             for (int j = 0; j < RS_CHUNK; ++j) {
-                const rs_pair wj = rs_pack(w[j], w[j]);
 #pragma unroll
                 for (int i4 = 0; i4 < NS / 4; ++i4) {
                     const ulonglong2 k4 = KEEP_K ? kr[KEEP_K ? j : 0][KEEP_K ? i4 : 0]
                                                  : *reinterpret_cast<const ulonglong2*>(VECS && !MIX ? &s_e[buf][c0 + j][(i4 * DG + dg) * 4]
                                                                                                      : &s_k[buf][c0 + j][(i4 * DG + dg) * 4]);
-                    S[2 * i4] = rs_fma2(k4.x, wj, S[2 * i4]);
-                    S[2 * i4 + 1] = rs_fma2(k4.y, wj, S[2 * i4 + 1]);
+#pragma unroll
+                    for (int h = 0; h < NC; ++h) {
+                        const rs_pair wj = rs_pack(w[h][j], w[h][j]);
+                        S[h][2 * i4] = rs_fma2(k4.x, wj, S[h][2 * i4]);
+                        S[h][2 * i4 + 1] = rs_fma2(k4.y, wj, S[h][2 * i4 + 1]);
+                    }
                 }
             }
-            const float o = fmaf(dec.x, read, row_times(cf + RS_CHUNK, va, vb));
-            if (col_ok && reads && tok < nt) orow[(size_t)(base + c0 + tok) * ((size_t)a.heads * Dv)] = o;
+            if (reads && tok < nt) {
+#pragma unroll
+                for (int h = 0; h < NC; ++h)
+                    if (col_ok[h]) orow[(size_t)(base + c0 + tok) * ((size_t)a.heads * Dv) + 16 * h] = o[h];
+            }
             __syncwarp();                                     // the lanes' numbers are read before the next chunk's are written
         }
     }
-    if (col_ok) {
+#pragma unroll
+    for (int h = 0; h < NC; ++h) {
+        if (!col_ok[h]) continue;
 #pragma unroll
         for (int i = 0; i < NS / 2; ++i) {
-            const float2 v = rs_unpack(S[i]);
+            const float2 v = rs_unpack(S[h][i]);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int d = (((2 * i + h) >> 2) * DG + dg) * 4 + ((2 * i + h) & 3);
-                if (d < D) sbase[(size_t)d * Dv] = h ? v.y : v.x;
+            for (int e = 0; e < 2; ++e) {
+                const int d = (((2 * i + e) >> 2) * DG + dg) * 4 + ((2 * i + e) & 3);
+                if (d < D) sbase[(size_t)d * Dv + 16 * h] = e ? v.y : v.x;
             }
         }
     }
-    rs_move_tail(a, slot, t0, n);
+    rs_move_tail(a, slot, t0, n, head * tiles + tile, a.heads * tiles);
 }
 
 // `coef` ([T][heads][RS_COEF] floats, 16-byte aligned, may be null): chunks of eight tokens.  The modes with a decay per
@@ -1097,10 +1139,17 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
     if (coef) {
         if (T <= 0 || ((uintptr_t)coef & 15)) return AIRUN_ERR_ARG;
         if (mode != RS_DELTA_HEAD && (!vectors || D > 128 || ((uintptr_t)vectors & 15))) return AIRUN_ERR_ARG;
-        const dim3 cgrid(T / RS_CHUNK + num_reqs, ceil_div_i(heads, 4)), mgrid(num_reqs, heads, ceil_div_i(Dv, 16));
-        if (mgrid.z > 65535) return AIRUN_ERR_ARG;
+        const dim3 cgrid(T / RS_CHUNK + num_reqs, ceil_div_i(heads, 4)), cols(ceil_div_i(Dv, 16), ceil_div_i(Dv, 32));
+        const long long rows_of_blocks = (long long)num_reqs * heads;                // (request, head): the columns' blocks fastest, the requests slowest
+        if (rows_of_blocks * cols.x > 0x7fffffffLL) return AIRUN_ERR_ARG;
+        const dim3 mgrid((unsigned)(rows_of_blocks * cols.x)), wgrid((unsigned)(rows_of_blocks * cols.y));
+        // the blocks that run long are the portions': of a padded step's requests most may bring one token or none
+        const long long long_blocks = (long long)(portions > 0 && portions < num_reqs ? portions : num_reqs) * heads * cols.x;
+        const bool few = long_blocks <= 2LL * airun_sm_count();
 #define RS_COEFS(SL) airun_launch(delta_chunk_coef_kernel<SL>, cgrid, dim3(128), 0, stream, a, num_reqs, coef)
-#define RS_CHUNKS(NS, KIND, DG, MINB) airun_launch_after(delta_chunk_kernel<NS, KIND, DG, MINB>, mgrid, dim3(16 * DG), 0, stream, a, (const float*)coef, vec)
+#define RS_CHUNKS(NS, KIND, DG, MINB) airun_launch_after(delta_chunk_kernel<NS, KIND, DG, MINB, 1>, mgrid, dim3(16 * DG), 0, stream, a, (const float*)coef, vec)
+#define RS_WIDE(NS, KIND, MINB) airun_launch_after(delta_chunk_kernel<NS, KIND, 8, MINB, 2>, wgrid, dim3(128), 0, stream, a, (const float*)coef, vec)
+#define RS_EITHER(NS, KIND) do { if (few) RS_CHUNKS(NS, KIND, 8, 4); else RS_WIDE(NS, KIND, 3); } while (0)
         ChunkVectors vec = {};
         if (mode != RS_DELTA_HEAD) {
             const size_t n = (size_t)T * heads * D;
@@ -1110,15 +1159,15 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
                 if (D <= 32) RS_VECTORS(1, true);
                 else if (D <= 64) RS_VECTORS(2, true);
                 else RS_VECTORS(4, true);
-                if (D <= 32) RS_CHUNKS(4, CHUNK_MIX, 8, 4);
-                else if (D <= 64) RS_CHUNKS(8, CHUNK_MIX, 8, 4);
+                if (D <= 32) RS_EITHER(4, CHUNK_MIX);
+                else if (D <= 64) RS_EITHER(8, CHUNK_MIX);
                 else RS_CHUNKS(16, CHUNK_MIX, 8, 4);
             } else {
                 if (D <= 32) RS_VECTORS(1, false);
                 else if (D <= 64) RS_VECTORS(2, false);
                 else RS_VECTORS(4, false);
-                if (D <= 32) RS_CHUNKS(4, CHUNK_CHANNEL, 8, 4);
-                else if (D <= 64) RS_CHUNKS(8, CHUNK_CHANNEL, 8, 4);
+                if (D <= 32) RS_EITHER(4, CHUNK_CHANNEL);
+                else if (D <= 64) RS_EITHER(8, CHUNK_CHANNEL);
                 else RS_CHUNKS(16, CHUNK_CHANNEL, 8, 4);
             }
 #undef RS_VECTORS
@@ -1128,15 +1177,16 @@ AIRUN_EXPORT int airun_recurrent_state(int mode, const float* q, const float* k,
         else if (D <= 64) RS_COEFS(2);
         else if (D <= 128) RS_COEFS(4);
         else RS_COEFS(8);
-        // the blocks that run long are the portions': of a padded step's requests most may bring one token or none
-        const bool few = (long long)(portions > 0 && portions < num_reqs ? portions : num_reqs) * mgrid.y * mgrid.z <= 2LL * airun_sm_count();
 #define RS_HEAD_CHUNKS(NS) do { if (few) RS_CHUNKS(NS, CHUNK_HEAD, 8, 2); else RS_CHUNKS(NS, CHUNK_HEAD, 8, 4); } while (0)
-        if (D <= 32) RS_HEAD_CHUNKS(4);
+        if (D <= 64 && !few) { if (D <= 32) RS_WIDE(4, CHUNK_HEAD, 3); else RS_WIDE(8, CHUNK_HEAD, 3); }
+        else if (D <= 32) RS_HEAD_CHUNKS(4);
         else if (D <= 64) RS_HEAD_CHUNKS(8);
         else if (D <= 128) RS_HEAD_CHUNKS(16);
         else RS_CHUNKS(16, CHUNK_HEAD, 16, 1);
 #undef RS_HEAD_CHUNKS
 #undef RS_COEFS
+#undef RS_EITHER
+#undef RS_WIDE
 #undef RS_CHUNKS
         return airun_launch_status();
     }

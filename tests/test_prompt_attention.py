@@ -108,6 +108,14 @@ def test_attention_without_softmax(nh, nkv, page, window, dist, offset, spans):
     assert bool(((got - want).abs() <= 2.0 ** -7 * most + 1e-6).all())
 
 
+@gpu
+@pytest.mark.parametrize("nh,nkv,page,window,spans", [(2, 1, 16, 0, [(900, 1143)]), (1, 1, 32, 0, [(1500, 1900), (3, 4)]), (4, 2, 32, 1100, [(1900, 2300)]),
+                                                      (16, 8, 16, 0, [(512, 640), (0, 640)])])
+def test_attention_without_softmax_in_halves(nh, nkv, page, window, spans):
+    """Few tiles of many keys, whose halves two CTAs take: tiles of one and of two query tiles, whole ones among them, a window."""
+    test_attention_without_softmax(nh, nkv, page, window, True, True, spans)
+
+
 SPLIT_CASES = [  # head size, heads, kv heads, page, window, spans: key tiles a query tile has, 1 to 17
     (128, 16, 8, 16, 0, [(900, 1143), (872, 1107)]), (128, 2, 1, 16, 0, [(0, 193)]), (128, 4, 1, 16, 0, [(300, 364)]), (64, 1, 1, 16, 0, [(0, 128)]),
     (128, 2, 2, 32, 0, [(500, 600), (3, 4), (380, 390)]), (64, 8, 2, 32, 0, [(1000, 1100)]), (128, 3, 1, 16, 200, [(700, 900)]),

@@ -198,3 +198,45 @@ def test_a_prompt_takes_the_same_form_whatever_its_runner_can_hold(mode):
         outs.append((out[:230].clone(), state[0].clone(), used))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     assert outs[0][2] == outs[1][2] > 0                                  # coefficients were made: both ran in chunks
+
+
+@gpu
+@pytest.mark.parametrize("mode", ["channel", "mix", "head"])
+@pytest.mark.parametrize("D,Dv,lens", [(64, 128, (203, 9)), (64, 40, (70, 131, 8)), (20, 33, (222,)), (32, 16, (65, 130))])
+def test_chunks_of_two_columns_a_thread(mode, D, Dv, lens):
+    """Enough heads that a thread takes two value columns, against the same heads in parts small enough for one: the sums are formed in the same
+    order, so results and states differ by the roundings of contracted multiply-adds at most (2e-6 of the largest entry)."""
+    from test_pirerax import batch_ctx
+    from airun_b200.kernels import fast, ops
+    Dv = D if mode == "mix" else Dv
+    sms = fast.machine().sms
+    n_part = 1 + max(1, sms // (len(lens) * -(-Dv // 16)))
+    heads = 4 * n_part
+    assert len(lens) * heads * -(-Dv // 16) > 2 * sms >= len(lens) * n_part * -(-Dv // 16)
+    g = torch.Generator().manual_seed(D + Dv)
+    T = sum(lens)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, heads, D, generator=g), dim=-1) for _ in range(2))
+    v, beta = torch.randn(T, heads, Dv, generator=g), torch.randn(T, heads, generator=g)
+    decay = torch.rand(T, heads, D, generator=g) ** 0.05
+    start = torch.randn(len(lens), heads, D, Dv, generator=g)
+
+    def run(lo, hi):
+        n = hi - lo
+        ctx = batch_ctx([(0, t) for t in lens], list(range(len(lens))))
+        state, out = start[:, lo:hi].reshape(len(lens), -1).cuda(), torch.empty(T, n * Dv, device="cuda")
+        flat = [t[:, lo:hi].reshape(T, -1).cuda() for t in (q, k, v, decay)]
+        b = beta[:, lo:hi].contiguous().cuda()
+        if mode == "channel":
+            ops.recurrent_state(ops.RECURRENCE_DELTA, *flat, state, ctx, out, n, 1, D, Dv, beta=b)
+        elif mode == "mix":
+            ops.recurrent_state(ops.RECURRENCE_WKV, *flat, state, ctx, out, n, 1, D, Dv, bonus=b.new_ones(n, D))
+        else:
+            ops.recurrent_state(ops.RECURRENCE_DELTA_HEAD, *flat[:3], b, state, ctx, out, n, 1, D, Dv, beta=b, a_log=b.new_zeros(n), dt_bias=b.new_zeros(n))
+        assert int(ctx.err.item()) == 0
+        return out.view(T, n, Dv), state.view(len(lens), n, D, Dv)
+
+    out, state = run(0, heads)
+    for lo in range(0, heads, n_part):
+        o, s = run(lo, lo + n_part)
+        size = max(1.0, float(s.abs().max()), float(o.abs().max()))
+        assert float((out[:, lo:lo + n_part] - o).abs().max()) <= 2e-6 * size and float((state[:, lo:lo + n_part] - s).abs().max()) <= 2e-6 * size

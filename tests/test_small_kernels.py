@@ -226,3 +226,30 @@ def test_rows_of_experts_that_have_no_place(T, top, W, dtype):
     ops.moe_combine(ys, top, ids, wts, bad, False, out)
     want = torch.where((row_of >= 0)[..., None], ys.view(T, top, W), torch.zeros(1, device="cuda")).sum(1)
     assert torch.allclose(out, want, atol=1e-6)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,n,rank", [(1, 5, 8), (8, 128, 16), (21, 300, 24), (9, 130, 32), (17, 64, 40), (10, 200, 12), (3, 33, 1), (16, 129, 1024)])
+def test_low_rank_pairs_that_end_in_a_function(T, n, rank, dtype):
+    """Rows of the second matrix in pieces of eight (up to 32 of them ahead, more in turn) and one number at a time, against 64 bits.  Tolerance: z is a sum
+    of rank products in float32 (2^-24 * rank of the sum of absolute values), and no function is steeper than 4 where it is not saturated."""
+    from airun_b200.kernels import ops
+    g = torch.Generator().manual_seed(rank + n)
+    low, w2, bias = torch.randn(T, rank + 4, generator=g)[:, :rank], (torch.randn(n, rank, generator=g) * rank ** -0.5).to(dtype), torch.randn(n, generator=g)
+    req = torch.zeros(T, dtype=torch.int32)
+    req[T // 2] = -1 if T > 4 else 0
+    param = torch.randn(n, generator=g) * 0.5
+    z = bias.double() + low.double() @ w2.double().T
+    zt = low.double().tanh() @ w2.double().T
+    err = 2.0 ** -24 * (rank + 8) * (bias.double().abs() + low.double().abs() @ w2.double().abs().T + 1)
+    soft = torch.nn.functional.softplus
+    out = torch.full((T, n), 7.0, device="cuda")
+    for mode, want, kw in ((ops.LOWRANK_EXP_SOFTPLUS, torch.exp(-torch.exp(param.double()) * soft(z)), dict(group_param=param.cuda(), group=1)),
+                           (ops.LOWRANK_SIGMOID, torch.sigmoid(z), {}), (ops.LOWRANK_EXP_NEG_EXP, torch.exp(-torch.exp(zt)), dict(in_tanh=True)),
+                           (ops.LOWRANK_POW_SIGMOID, torch.sigmoid(z) ** (1 / 16.0), dict(tau=16.0))):
+        out.fill_(7.0)
+        ops.lowrank_act(low.cuda(), w2.cuda(), None if "in_tanh" in kw else bias.cuda(), out, req.cuda(), mode, **kw)
+        got = out.cpu().double()
+        live = req >= 0
+        assert bool(((got - want).abs()[live] <= 4 * err[live] + 2e-6).all()) and bool((got[~live] == 7.0).all())

@@ -3,10 +3,11 @@
 //
 // One CTA computes one 128 x BN tile D = A * B^T of two K-major operands
 // ("rows of K contiguous values"), over one slice of K:
-//   warp 0   : one thread issues TMA loads (cp.async.bulk.tensor, 128-byte
-//              swizzle) of A and B blocks of 64 k-values into a ring of stages;
-//   warp 1   : allocates tensor memory; one thread issues tcgen05.mma
-//              (M=128, N=BN, K=16, four per block) and commits to mbarriers;
+//   warp 0   : TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of A and B
+//              blocks of 64 k-values into a ring of stages;
+//   warp 1   : allocates tensor memory; issues tcgen05.mma (M=128, N=BN, K=16,
+//              four per block) and commits to mbarriers;
+//              both loop as whole warps, one elected thread issuing (elect_one);
 //   warps 2-5: read the accumulator with tcgen05.ld, apply the epilogue, store.
 // Which operand is A decides the mode:
 //   normal (prompt portions): A = activations (128 tokens), B = weights (BN rows);
@@ -22,7 +23,8 @@
 // Every wait on an mbarrier is bounded: when it runs out the kernel sets an
 // error bit, skips the rest of its work, frees its tensor memory and returns.
 // From 17 tokens on the K slices of a tile run as one thread-block cluster and add up through distributed
-// shared memory (see cluster_reduce); no TMA load uses multicast.
+// shared memory (see push_slices); no TMA load uses multicast.
+// Most products of more than 128 tokens and all of experts run on pairs of SMs: gemm_pair_kernel.
 //
 // The reference's counterparts are its wmma prefill GEMM and its half-precision
 // matvec kernels (crates/airun-cuda/kernels/matmul.cu:518-636, :1498-1563); its

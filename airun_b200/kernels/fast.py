@@ -160,7 +160,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, 
 
 
 def plan_gemm(M: int, N: int, K: int, mach: Optional[Machine] = None) -> Tuple[bool, int, int]:
-    """(swap, bn, ksplit) for a product of M tokens with an [N, K] weight.
+    """(swap, bn, ksplit) for a product of M tokens with an [N, K] weight that does not run on pairs of SMs (``_pairs``).
 
     Up to 128 tokens the weights are the 128-row operand (swap), except for the widest products from 65 tokens on.  Up to 16 tokens the K range is cut
     until about STREAM_CTAS CTAs stream the weights (a slice keeping 10 K-steps) and the slices add

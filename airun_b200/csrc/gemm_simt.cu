@@ -1,13 +1,12 @@
-// Plain matrix product C[M][N] = A[M][K] * W[N][K]^T on the CUDA cores.
+// Plain matrix product C[M][N] = A[M][K] * W[N][K]^T.
 //
-// This is the true 32-bit path of every projection (float32 operands, FFMA
-// accumulation, no tensor cores, no reduced-precision mode) and, with bfloat16
-// operands, the plain twin the tensor-core kernels are tested against.  The
+// This is the true 32-bit path of every projection (float32 operands, no operand rounded, no reduced-precision mode): FFMA
+// kernels on the CUDA cores, and for many long rows the tensor cores with each operand in three parts that keep all its bits.
+// With bfloat16 operands it is the plain twin the tensor-core kernels are tested against.  The
 // reference keeps exact f32 FMA matvecs for the same purpose
 // (crates/airun-cuda/kernels/matmul.cu:59-141, switch at
-// crates/airun-core/src/runtime.rs:5344-5352).  The tile kernels form every
-// output element as one sequential sum over k; the kernel for few float32 rows
-// cuts it over the block in a fixed order.
+// crates/airun-core/src/runtime.rs:5344-5352).  The tile kernels on the CUDA cores form every
+// output element as one sequential sum over k or as a few in a fixed order; the others cut it over the block, steps and slices in a fixed order.
 #include "tcgen05.cuh"
 
 #define TM 64

@@ -310,32 +310,43 @@ __global__ __launch_bounds__(256, 2) void gemm_f32_kernel(
 
 // ------------------------------------------------------------------ float32 on the tensor cores, without rounding an operand
 // More than a few rows of float32 products are bound by the FMA pipe, so they go to the tensor cores with every operand
-// cut into three bfloat16 parts whose sum it is: the leading 8 bits of the significand (cut off, so that nothing overflows), the
-// next 8 (rounded) and the remaining 8, which is the whole significand of 24 bits down to 2^-133.  Of the nine products of parts the six
-// of 2^-17 and more are formed, x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; the three left out are below 2^-23 of x w, of either sign, half a
-// unit of the last place (the split of S. Markidis et al., IPDPS Workshops 2018, in bfloat16 and three parts: G. Henry, P. T. P. Tang and
-// A. Heinecke, ARITH 2019).  The tensor cores add up in float32 but cut off where float32 rounds, so they hold a sum over 64 k-values at most, the
-// small products first; the sums of these steps are added up in registers, rounded.
+// cut into three bfloat16 parts whose sum it is: its 8 leading bits (rounded), 8 of what is left (rounded) and the rest, which is the whole
+// significand of 24 bits down to 2^-133 (the split of S. Markidis et al., IPDPS Workshops 2018, in bfloat16 and three parts: G. Henry, P. T. P. Tang and
+// A. Heinecke, ARITH 2019).  Of the nine products of parts eight are formed; x3 w3, below 2^-35 of x w, is left out.
+// The tensor cores add up in float32 but cut off where float32 rounds.  So the leading product x1 w1, whose 16 bits leave room for a sum of many, has a sum
+// of its own, over the 64 k-values of a step, and the seven small ones, 2^-8 of it and less, have another over X_LOW_STEPS steps: its cuts, 28 a step, are 2^-8 of
+// those of one sum.  Both are added up in registers, rounded; a sum of one product is the rounded product, as an FMA has it.
+// Error against 64 bits (2-norm, in 1e-7), this and the FMA kernel, 300 rows: K = 1,024 dense 0.9, 2.9 (operands of one sign 0.9, 1.3); 10 % of x other than zero
+// 0.6, 1.0 (0.5, 0.6); 1 % 0.5, 0.5 (0.4, 0.4); one 0.25, 0.25.  K = 4,096 dense 1.8, 5.7 (1.6, 2.5); 10 % 1.4, 1.9 (1.3, 0.8); 1 % 0.9, 0.7 (0.7, 0.5): of many steps
+// with a few terms of one sign each, adding up the steps is the larger part.  Six products and one sum had 0.55 for one product.
+//
+// What the parts cannot hold is found and formed by a plain loop of multiply-adds (f32_plain_results): results that are not finite (an infinite operand
+// has no parts, and small products can overflow with the other sign), results below 2^-100, whose small products end at 2^-149, and the rows and columns
+// of an operand below 2^-110, whose last bits end at 2^-133.
 //
 // A tile is 128 weight rows by `bn` rows of A (16 .. 128), its K range cut into `ks` slices that run as one cluster and are added up in order
 // through distributed shared memory.
-//   warps 0-7  : read the step sums from tensor memory (a quadrant of lanes each, every other 16 columns) and add them up; they store the tile;
+//   warps 0-7  : read the sums from tensor memory (a quadrant of lanes each, every other 16 columns) and add them up; they store the tile;
 //   warps 8-15 : cut the 64 k-values of a step of every row of both operands.  The parts of W go to tensor memory, those of A to shared memory
 //                (128-byte swizzle): with both there, what the products, the cutting and the loads move through shared memory is the bound (390 KB a
 //                step of 128 x 112, 3,300 clocks for 1,540 of products).  They load nothing themselves: their fence would wait for loads under way;
-//   warp 16    : one thread issues the 24 tcgen05.mma of a step (in a warp that adds up, no product would run while it does);
-//   warp 17    : one thread issues the TMA loads, two steps ahead.
-// An infinite operand has no parts; its row is noted and its results are formed by a plain loop.
+//   warp 16    : issues the 32 tcgen05.mma of a step (in a warp that adds up, no product would run while it does), the small products first: meanwhile
+//                the leading sum of the step before is read;
+//   warp 17    : issues the TMA loads, two steps ahead.
 #define XT 128                    // weight rows of a tile
 #define XB 128                    // most rows of A
 #define XK 64                     // k-values of a step
 #define X_STAGES 2                // steps of parts
 #define X_RING 2                  // steps of operands on their way to the threads that cut them
+#define X_PRODUCTS 8              // of parts
 #define X_SUM_WARPS 8
 #define X_CUT_WARPS 8
 #define X_THREADS (32 * (X_SUM_WARPS + X_CUT_WARPS + 2))   // 18 warps: 96 registers a thread
 #define X_PART (XB * XK * 2)      // bytes of one part of A
-#define X_WCOLS (XK / 2)          // columns of tensor memory of one part of W, after the two step sums
+#define X_WCOLS (XK / 2)          // columns of tensor memory of one part of W
+#define X_WAT (2 * XB)            // their place, behind the sums of the leading and of the small products
+static_assert(X_WAT + 3 * X_STAGES * X_WCOLS <= 512, "");
+#define X_LOW_STEPS 4             // steps that the small products are added up over
 #define X_STAGE (3 * X_PART)
 #define X_SUM_SPACE (XT * XB * 4) // the slices' sums take the place of the stages and of the ring
 #define X_RING_STEP ((XT + XB) * XK * 4)
@@ -355,44 +366,49 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint2 (&v)[4]) {
                  "r"(v[1].y), "r"(v[2].x), "r"(v[2].y), "r"(v[3].x), "r"(v[3].y) : "memory");
 }
 
-// One float4's three parts, packed to bfloat16 (8 bytes each).  False when one of the values is infinite or not a number.
-__device__ __forceinline__ bool f32_parts(const float4& v, uint2 (&part)[3]) {
-    const uint32_t x[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+// One float4's three parts, packed to bfloat16 (8 bytes each).
+__device__ __forceinline__ void f32_parts(const float4& v, uint2 (&part)[3]) {
     const float2 minus = make_float2(-1.0f, -1.0f);
-    float2 r[2];
-    uint32_t m[2], l[2];
+    uint32_t b[3][2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {                              // packed: x - h is exact, as a multiply-add too
-        const float2 h = make_float2(__uint_as_float(x[2 * i] & 0xffff0000u), __uint_as_float(x[2 * i + 1] & 0xffff0000u));
-        r[i] = __ffma2_rn(h, minus, i == 0 ? make_float2(v.x, v.y) : make_float2(v.z, v.w));
-        const __nv_bfloat162 b = __floats2bfloat162_rn(r[i].x, r[i].y);
-        m[i] = *reinterpret_cast<const uint32_t*>(&b);
-        const float2 g = make_float2(__uint_as_float(m[i] << 16), __uint_as_float(m[i] & 0xffff0000u));
-        const float2 d = __ffma2_rn(g, minus, r[i]);
-        const __nv_bfloat162 c = __floats2bfloat162_rn(d.x, d.y);
-        l[i] = *reinterpret_cast<const uint32_t*>(&c);
+    for (int i = 0; i < 2; ++i) {                              // packed: what is left is exact, as a multiply-add too
+        float2 r = i == 0 ? make_float2(v.x, v.y) : make_float2(v.z, v.w);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(r.x, r.y);
+            b[j][i] = *reinterpret_cast<const uint32_t*>(&h);
+            if (j < 2) r = __ffma2_rn(make_float2(__uint_as_float(b[j][i] << 16), __uint_as_float(b[j][i] & 0xffff0000u)), minus, r);
+        }
     }
-    part[0] = make_uint2(__byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x7632));
-    part[1] = make_uint2(m[0], m[1]);
-    part[2] = make_uint2(l[0], l[1]);
-    const float t = (r[0].x + r[0].y) + (r[1].x + r[1].y);     // infinity less itself is not a number
-    return t == t;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) part[j] = make_uint2(b[j][0], b[j][1]);
 }
-__device__ __forceinline__ bool any_inf(const float4& v) { return isinf(v.x) || isinf(v.y) || isinf(v.z) || isinf(v.w); }
+// The smallest of 2 |x| - 1 as whole numbers, where zero is the largest: below X_SMALL for values other than zero below 2^-110.
+#define X_SMALL (2u * 0x08800000u - 1u)
+__device__ __forceinline__ uint32_t f32_least(uint32_t least, const float4& v) {
+    const uint32_t a = 2u * __float_as_uint(v.x) - 1u, b = 2u * __float_as_uint(v.y) - 1u, c = 2u * __float_as_uint(v.z) - 1u, d = 2u * __float_as_uint(v.w) - 1u;
+    return min(min(least, min(a, b)), min(c, d));
+}
+// Not a number for a result that the parts may not hold (see above), else zero (added up, one check answers for many results).
+__device__ __forceinline__ float f32_doubt(float v) { return fabsf(v) < 7.888609e-31f && v != 0.0f ? __int_as_float(0x7fffffff) : v * 0.0f; }
 
-// The results of a tile that have an infinite operand, each by itself: columns first, first + step, .. of the tile.
-__device__ __noinline__ void f32_infinite_rows(const float* A, const float* W, float* C, int K, long long lda, long long ldw, long long ldc, int m0,
+// The results of a tile in doubt, and those in marked rows and columns, each by itself: columns first, first + step, .. of the tile.
+__device__ __noinline__ void f32_plain_results(const float* A, const float* W, float* C, int K, long long lda, long long ldw, long long ldc, int m0,
                                                int cols, int n0, int rows, const uint32_t* marks, int first, int step) {
-    uint32_t any = 0;
-    for (int i = 0; i < 8; ++i) any |= marks[i];
-    if (any == 0) return;
     for (int i = threadIdx.x; i < cols * rows; i += blockDim.x) {
         const int col = i / rows, r = i % rows;
-        if (col % step != first || !(((marks[r >> 5] >> (r & 31)) | (marks[4 + (col >> 5)] >> (col & 31))) & 1u)) continue;
-        const float *a = A + (size_t)(m0 + col) * lda, *w = W + (size_t)(n0 + r) * ldw;
-        float v = 0.0f;
-        for (int k = 0; k < K; ++k) v = fmaf(a[k], w[k], v);
-        C[(size_t)(m0 + col) * ldc + n0 + r] = v;
+        if (col % step != first) continue;
+        float* c = C + (size_t)(m0 + col) * ldc + n0 + r;
+        const float doubt = f32_doubt(__ldcg(c));
+        if (doubt == doubt && !(((marks[r >> 5] >> (r & 31)) | (marks[4 + (col >> 5)] >> (col & 31))) & 1u)) continue;
+        const float4 *a = reinterpret_cast<const float4*>(A + (size_t)(m0 + col) * lda), *w = reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * ldw);
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int k = 0; 4 * k < K; ++k) {                      // (rows of a multiple of four values, aligned)
+            const float4 x = a[k], y = w[k];
+            s.x = fmaf(x.x, y.x, s.x); s.y = fmaf(x.y, y.y, s.y); s.z = fmaf(x.z, y.z, s.z); s.w = fmaf(x.w, y.w, s.w);
+        }
+        const float v = (s.x + s.y) + (s.z + s.w);
+        *c = v;
     }
 }
 
@@ -403,9 +419,9 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
     pdl_trigger();
     extern __shared__ uint8_t x_raw[];
     uint8_t* tiles = (uint8_t*)(((uintptr_t)x_raw + 1023) & ~(uintptr_t)1023);
-    // full, empty of the stages of parts; full, empty of the two step sums; landed, read of the ring
+    // full, empty of the stages of parts; full, empty of the leading sum and of the other; landed, read of the ring
     __shared__ __align__(8) uint64_t bars[2 * X_STAGES + 4 + 2 * X_RING];
-    __shared__ uint32_t tmem_slot, inf_rows[2][4], all_rows[8];    // infinite operands: bit r of [0] weight row, of [1] row of A
+    __shared__ uint32_t tmem_slot, marks[9], all_marks[9];         // bit r of 0-3: weight row r has an operand that is too small for its parts; 4-7: row of A; 8: a result is in doubt
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int slice = blockIdx.z, n0 = blockIdx.x * XT;
     int m0 = blockIdx.y * bn, m_end = M, set_w = 0;
@@ -424,15 +440,15 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
     }
     const int steps_all = (K + XK - 1) / XK, per = (steps_all + ks - 1) / ks;
     const int step0 = min(slice * per, steps_all), steps = min(step0 + per, steps_all) - step0;
-    const uint32_t full = smem_u32(bars), empty = full + 8 * X_STAGES, sfull = empty + 8 * X_STAGES, sempty = sfull + 16, landed = sempty + 16, taken = landed + 8 * X_RING;
+    const uint32_t full = smem_u32(bars), empty = full + 8 * X_STAGES, sfull = empty + 8 * X_STAGES, sempty = sfull + 8, lfull = sempty + 8, lempty = lfull + 8, landed = lempty + 8, taken = landed + 8 * X_RING;
     if (threadIdx.x == 0) {
         for (int s = 0; s < X_STAGES; ++s) { mbar_init(full + 8 * s, X_CUT_WARPS); mbar_init(empty + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(sfull + 8 * b, 1); mbar_init(sempty + 8 * b, X_SUM_WARPS); }
+        for (uint32_t b = sfull; b <= lfull; b += 16) { mbar_init(b, 1); mbar_init(b + 8, X_SUM_WARPS); }
         for (int r = 0; r < X_RING; ++r) { mbar_init(landed + 8 * r, 1); mbar_init(taken + 8 * r, X_CUT_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (threadIdx.x < 8) (&inf_rows[0][0])[threadIdx.x] = 0;
+    if (threadIdx.x < 9) marks[threadIdx.x] = all_marks[threadIdx.x] = 0;
     if (warp == X_SUM_WARPS) tmem_alloc(smem_u32(&tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
@@ -447,24 +463,33 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
 #pragma unroll
         for (int i = 0; i < XB / 4; ++i) acc[i] = make_float2(0.0f, 0.0f);
         const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
-        for (int it = 0; it < steps; ++it) {
-            const int buf = it & 1;
-            if (!mbar_wait(sfull + 8 * buf, (it >> 1) & 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
-            tc_fence_after();
-            __syncwarp();
+        auto add = [&](uint32_t from, uint32_t read) {
 #pragma unroll
             for (int j = 0; j < XB / 32; ++j) {
                 const int c = 16 * (2 * j + half);
                 if (c >= bn) break;
                 uint32_t r[16];
-                tmem_ld_async(lanes + buf * XB + c, r);
+                tmem_ld_async(from + c, r);
                 tmem_wait(r);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[8 * j + i] = __fadd2_rn(acc[8 * j + i], make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sempty + 8 * buf) : "memory");
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(read) : "memory");
+        };
+        for (int it = 0, group = 0; it < steps; ++it) {
+            if (!mbar_wait(sfull, it & 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+            if (it % X_LOW_STEPS == X_LOW_STEPS - 1 || it + 1 == steps) {      // (first, as the next step's products begin with it)
+                if (!mbar_wait(lfull, group & 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+                ++group;
+                tc_fence_after();
+                __syncwarp();
+                add(lanes + XB, lempty);
+            }
+            tc_fence_after();
+            __syncwarp();
+            add(lanes, sempty);
         }
         // the last step's products are done, so the stages may be written over
         const int r = quad * 32 + lane;
@@ -478,14 +503,18 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
             }
         } else if (n0 + r < N) {
             float* c = C + (size_t)(m0 + 16 * half) * ldc + n0 + r;
+            float doubt = 0.0f;
 #pragma unroll
             for (int j = 0; j < XB / 32; ++j, c += 32 * ldc) {
                 const int n = cols - 16 * (2 * j + half);
                 float* o = c;
 #pragma unroll
-                for (int i = 0; i < 16; ++i, o += ldc)
-                    if (i < n) *o = i & 1 ? acc[8 * j + i / 2].y : acc[8 * j + i / 2].x;
+                for (int i = 0; i < 16; ++i, o += ldc) {
+                    const float v = i & 1 ? acc[8 * j + i / 2].y : acc[8 * j + i / 2].x;
+                    if (i < n) { *o = v; doubt += f32_doubt(v); }
+                }
             }
+            if (doubt != doubt) atomicOr(&marks[8], 1u);
         }
     } else if (warp < X_SUM_WARPS + X_CUT_WARPS) {
         // W: this thread's row is lane `lane` of its quadrant, 32 of the step's k-values.  A: rows row + 32 i, k-values 4 q .. 4 q + 3 and 32 more on.
@@ -494,6 +523,7 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
         const int row = t >> 3, q = t & 7;
         constexpr int RP = X_CUT_WARPS * 4;                    // 32: rows of a pass over A, four passes
         static_assert(RP == 32 && XT == 128 && XB == 128 && XK == 64, "two threads a row of W, four passes over A");
+        uint32_t least_w = ~0u, least_a[4] = {~0u, ~0u, ~0u, ~0u};
         const uint32_t w_at = half * (XT * 128) + (quad * 32 + lane) * 128, a_at = 2 * XT * 128 + row * 128 + ((q ^ (row & 7)) << 4);
         for (int it = 0; it < steps; ++it) {
             const int s = it % X_STAGES, g = it % X_RING;
@@ -510,31 +540,24 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
             for (int h = 0; h < 2; ++h) {
                 float4 v[4];
                 uint2 part[4][3];
-                bool fine[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(from + w_at + (((4 * h + i) ^ (lane & 7)) << 4));
 #pragma unroll
-                for (int i = 0; i < 4; ++i) fine[i] = f32_parts(v[i], part[i]);
-                if (!(fine[0] && fine[1] && fine[2] && fine[3]))
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (any_inf(v[i])) atomicOr(&inf_rows[0][quad], 1u << lane);
-                __syncwarp();
+                for (int i = 0; i < 4; ++i) { f32_parts(v[i], part[i]); least_w = f32_least(least_w, v[i]); }
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     const uint2 p[4] = {part[0][j], part[1][j], part[2][j], part[3][j]};
-                    tmem_st8(tmem + ((uint32_t)(quad * 32) << 16) + 2 * XB + (3 * s + j) * X_WCOLS + 16 * half + 8 * h, p);
+                    tmem_st8(tmem + ((uint32_t)(quad * 32) << 16) + X_WAT + (3 * s + j) * X_WCOLS + 16 * half + 8 * h, p);
                 }
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float4 v[4];
                 uint2 part[4][3];
-                bool fine[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4*>(from + a_at + h * (XB * 128) + RP * i * 128);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) fine[i] = f32_parts(v[i], part[i]);
+                for (int i = 0; i < 4; ++i) { f32_parts(v[i], part[i]); least_a[i] = f32_least(least_a[i], v[i]); }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (row + RP * i >= bn) continue;
@@ -542,10 +565,6 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
                     for (int j = 0; j < 3; ++j)
                         *reinterpret_cast<uint2*>(to + j * X_PART + RP * i * (XK * 2) + (((4 * h + (q >> 1)) ^ (row & 7)) << 4)) = part[i][j];
                 }
-                if (!(fine[0] && fine[1] && fine[2] && fine[3]))
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (row + RP * i < bn && any_inf(v[i])) atomicOr(&inf_rows[1][i], 1u << row);
             }
             __syncwarp();
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -557,28 +576,40 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(taken + 8 * g) : "memory");
             }
         }
+        if (least_w < X_SMALL) atomicOr(&marks[quad], 1u << lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (row + RP * i < cols && least_a[i] < X_SMALL) atomicOr(&marks[4 + i], 1u << row);
     } else if (warp == X_SUM_WARPS + X_CUT_WARPS) {
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(XT >> 4) << 24);
         for (int it = 0; it < steps; ++it) {
-            const int s = it % X_STAGES, buf = it & 1;
-            if (!mbar_wait_warp(sempty + 8 * buf, ((it >> 1) & 1) ^ 1) || !mbar_wait_warp(full + 8 * s, (it / X_STAGES) & 1)) {
+            const int s = it % X_STAGES, group = it / X_LOW_STEPS;
+            const bool first = it % X_LOW_STEPS == 0, last = it % X_LOW_STEPS == X_LOW_STEPS - 1 || it + 1 == steps;
+            if ((first && !mbar_wait_warp(lempty, (group & 1) ^ 1)) || !mbar_wait_warp(full + 8 * s, (it / X_STAGES) & 1)) {
                 atomicOr(err, AIRUN_DEV_TIMEOUT);
                 break;
             }
             tc_fence_after();
             const uint32_t base = smem_u32(tiles) + s * X_STAGE;
-            constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, AP[6] = {0, 2, 1, 0, 1, 0};     // the smallest products first
+            constexpr int WP[X_PRODUCTS] = {2, 1, 2, 0, 1, 1, 0, 0}, AP[X_PRODUCTS] = {1, 2, 0, 2, 1, 0, 1, 0};     // the smallest products first, the leading one last
+            auto product = [&](int j, uint32_t sum, bool fresh) {
+                const uint32_t tw = tmem + X_WAT + (3 * s + WP[j]) * X_WCOLS;
+                const uint64_t da = smem_desc_sw128(base + AP[j] * X_PART);
+#pragma unroll
+                for (int k = 0; k < XK / 16; ++k) umma_bf16_ts(sum, tw + 8 * k, da + (uint64_t)(k * 2), idesc, fresh && k == 0 ? 0u : 1u);
+            };
             if (elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const uint32_t tw = tmem + 2 * XB + (3 * s + WP[j]) * X_WCOLS;
-                    const uint64_t da = smem_desc_sw128(base + AP[j] * X_PART);
-#pragma unroll
-                    for (int k = 0; k < XK / 16; ++k)
-                        umma_bf16_ts(tmem + buf * XB, tw + 8 * k, da + (uint64_t)(k * 2), idesc, (j > 0 || k > 0) ? 1u : 0u);
-                }
+                for (int j = 0; j < X_PRODUCTS - 1; ++j) product(j, tmem + XB, first && j == 0);
+            }
+            __syncwarp();
+            if (!mbar_wait_warp(sempty, (it & 1) ^ 1)) { atomicOr(err, AIRUN_DEV_TIMEOUT); break; }
+            tc_fence_after();
+            if (elect_one()) {
+                product(X_PRODUCTS - 1, tmem, true);
                 umma_commit(empty + 8 * s);
-                umma_commit(sfull + 8 * buf);
+                umma_commit(sfull);
+                if (last) umma_commit(lfull);
             }
             __syncwarp();
         }
@@ -617,7 +648,9 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
         tmem_dealloc(tmem, 512);
     }
     if (ks == 1) {
-        f32_infinite_rows(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), &inf_rows[0][0], 0, 1);
+        uint32_t any = 0;
+        for (int i = 0; i < 9; ++i) any |= marks[i];
+        if (any) f32_plain_results(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), marks, 0, 1);
         return;
     }
     // the slices of the tile are added up in order, every CTA taking every ks-th column
@@ -634,15 +667,19 @@ __global__ __launch_bounds__(X_THREADS, 1) void gemm_f32_parts_kernel(
 #pragma unroll
                 for (int q = 1; q < 8; ++q) if (q < ks) t += v[q];
                 C[(size_t)(m0 + col) * ldc + n0 + r] = t;
+                const float doubt = f32_doubt(t);
+                if (doubt != doubt) all_marks[8] = 1;
             }
         }
         if (threadIdx.x < 8) {                                 // the rows noted by all slices
-            uint32_t marks = 0;
-            for (int q = 0; q < ks; ++q) marks |= __float_as_uint(ld_cluster_f32(map_to_cta(smem_u32(&inf_rows[0][0] + threadIdx.x), q)));
-            all_rows[threadIdx.x] = marks;
+            uint32_t m = 0;
+            for (int q = 0; q < ks; ++q) m |= __float_as_uint(ld_cluster_f32(map_to_cta(smem_u32(marks + threadIdx.x), q)));
+            all_marks[threadIdx.x] = m;
         }
         __syncthreads();
-        f32_infinite_rows(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), all_rows, slice, ks);
+        uint32_t any = 0;
+        for (int i = 0; i < 9; ++i) any |= all_marks[i];
+        if (any) f32_plain_results(A, W, C, K, lda, ldw, ldc, m0, cols, n0, min(XT, N - n0), all_marks, slice, ks);
     }
     __syncwarp();
     cluster_sync_all();                                        // nobody leaves while a peer may still read its memory
@@ -684,10 +721,10 @@ static int f32_clusters(int ks) {
     return n;
 }
 
-// Rows of A in a tile and K slices of the products on the tensor cores, by the time they take (B200, us): 1.26 a step of 64 k-values, 0.1 more at 128 rows;
-// bringing the slices together 2 to 7, the more the larger the share of the tile's columns that a CTA adds up.  24 rows x [1024, 1024] in 1, 2, 4 and 8
-// slices 22.9, 14.9, 9.9, 7.6; 642 x [1024, 2048] as 112 tiles of 48 rows 43.5, as 56 of 96 rows in two slices 30.2; 642 x [3072, 1024] in tiles of
-// 64, 96, 112 and 128 rows 48.3, 48.9, 25.5, 26.0.
+// Rows of A in a tile and K slices of the products on the tensor cores, by the time they take (B200, us): a step of 64 k-values 1.13, 0.0006 a row and from 80
+// rows on, where the products are the bound, 0.0056 more; bringing the slices together 2 to 7, the more the larger the share of the tile's columns that a CTA
+// adds up.  64 rows x [1024, 1024] in 1, 2, 4 and 8 slices 21.8, 15.9, 10.6, 8.7; 642 x [1024, 2048] as 112 tiles of 48 rows 40.8, as 56 of 96 rows in two slices
+// 30.0; 642 x [3072, 1024] in tiles of 64, 96, 112 and 128 rows 46.1, 49.8, 28.6, 30.0; 257 x [4096, 4096] in tiles of 64, 80, 96 and 128 rows 153, 80, 88, 103.
 struct F32Plan { int bn, ks; };
 static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
     const int sms = airun_sm_count(), steps = ceil_div_i(K, XK);
@@ -699,7 +736,7 @@ static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
         for (int ks = 1; ks <= 8 && (ks == 1 || 2 * ks <= steps); ++ks) {
             const int per = (steps + ks - 1) / ks;
             if ((steps + per - 1) / per != ks || (ks > 1 && tiles > f32_clusters(ks))) continue;   // an empty slice, or not all resident
-            const double step = 1.25 + 0.0008 * bn, merge = ks > 1 ? 1.2 + bn * (0.015 + 0.06 / ks) : 0.0;
+            const double step = 1.13 + 0.0006 * bn + 0.0056 * (bn > 80 ? bn - 80 : 0), merge = ks > 1 ? 1.2 + bn * (0.015 + 0.06 / ks) : 0.0;
             const double us = (double)((tiles * ks + sms - 1) / sms) * per * step + merge;
             if (us < best_us) { best_us = us; best = {bn, ks}; }
         }
@@ -707,9 +744,9 @@ static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
     return best;
 }
 
-// Fewest k-values of a product on the tensor cores.  Error against 64 bits (2-norm), FMA kernel and parts: operands of either sign, K = 128, 512, 1024,
-// 2048, 8192: 1.1e-7, 2.1e-7, 2.9e-7, 4.1e-7, 8.1e-7 and 0.9e-7, 1.0e-7, 1.1e-7, 1.3e-7, 1.3e-7; operands of one sign: 0.5e-7, 0.85e-7, 1.3e-7, 1.6e-7, 3.1e-7 and
-// 0.9e-7, 0.93e-7, 1.1e-7, 1.1e-7, 0.9e-7, so below 1,024 the tensor cores' cut-off sums would be the less exact ones there.
+// Fewest k-values of a product on the tensor cores.  Error of the FMA kernel against 64 bits (2-norm), K = 128, 512, 1024, 2048, 8192: operands of either
+// sign 1.1e-7, 2.1e-7, 2.9e-7, 4.1e-7, 8.1e-7, of one sign 0.5e-7, 0.85e-7, 1.3e-7, 1.8e-7, 3.5e-7.  The parts have 0.9e-7 to 1.1e-7 at 1,024 of either, which the
+// cuts within a step make up, so that below 1,024 they would be the less exact ones for one sign.
 #define X_MIN_K 1024
 // A tensor map of `sets` row-major float32 matrices [rows][K], rows `ld` and matrices `set` elements apart, boxes of box_rows x 32.
 static bool f32_map(CUtensorMap* out, const float* ptr, long long K, long long rows, long long sets, long long ld, long long set, int box_rows) {

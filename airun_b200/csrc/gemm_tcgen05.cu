@@ -1001,7 +1001,9 @@ __global__ __launch_bounds__(PAIR_THREADS, 1) void gemm_pair_kernel(
     }
     pdl_wait();
     if (GROUPED) {
-        for (int e = threadIdx.x; e < p.n_seg; e += PAIR_THREADS) s_first[e + 1] = (p.seg[e + 1] - p.seg[e] + PAIR_BN - 1) / PAIR_BN;
+        // (whatever the list says, no row outside the buffers is asked for or stored)
+        auto border = [&](int e) { return min(max(p.seg[e], 0), p.b_rows); };
+        for (int e = threadIdx.x; e < p.n_seg; e += PAIR_THREADS) s_first[e + 1] = (max(border(e + 1) - border(e), 0) + PAIR_BN - 1) / PAIR_BN;
         __syncthreads();
         if (threadIdx.x == 0) {
             int at = 0;
@@ -1010,7 +1012,7 @@ __global__ __launch_bounds__(PAIR_THREADS, 1) void gemm_pair_kernel(
         }
         __syncthreads();
         for (int e = threadIdx.x; e < p.n_seg; e += PAIR_THREADS) {
-            const int lo = p.seg[e], hi = p.seg[e + 1];
+            const int lo = border(e), hi = border(e + 1);
             int j = s_first[e];
             const int n = s_first[e + 1] - j, width = n > 0 ? ((hi - lo + n - 1) / n + 31) / 32 * 32 : 32;
             for (int r = lo; r < hi && j < GROUP_MAX_TILES; r += width, ++j) s_tab[j] = make_int4(r, hi, e, width);

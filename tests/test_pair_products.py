@@ -72,6 +72,27 @@ def test_segments(cuts):
     assert bool((out[cuts[-1]:] == 7.0).all()) and ctx.err.item() == 0
 
 
+@gpu
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_segments_that_end_behind_the_rows(swiglu):
+    """A list that names more rows than there are: no row behind the last is stored, the others are as without it."""
+    from types import SimpleNamespace
+    from airun_b200.kernels import fast
+    E, M, N, K = 3, 300, 320, 200
+    x, _ = operands(M, 1, K, 4)
+    x = x.contiguous()
+    w = (torch.randn(E, N, K, device="cuda") * K ** -0.5).bfloat16()
+    ctx = SimpleNamespace(err=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    outs = []
+    for last in (M, M + 90):
+        out = torch.full((M + 100, N // 2 if swiglu else N), 7.0, device="cuda", dtype=torch.bfloat16 if swiglu else torch.float32)
+        cuts = torch.tensor([0, 40, 230, last], dtype=torch.int32, device="cuda")
+        assert fast.grouped_linear_bf16(ctx, x, w, out[:M], cuts, swiglu_group=16 if swiglu else 0)
+        assert bool((out[M:] == 7.0).all()) and ctx.err.item() == 0
+        outs.append(out[:M])
+    assert torch.equal(*outs)
+
+
 def test_plan():
     """Whatever the sizes, the width is one the kernel takes, and no narrower tile would need as few rounds."""
     from airun_b200.kernels.fast import plan_pair

@@ -695,11 +695,11 @@ static void launch_gemv(const float* A, const float* W, float* C, int M, int N, 
         airun_launch(gemv_f32_kernel<MR, 4, FORM>, dim3(ceil_div_i(N, 4), gy, gz), dim3(32 * GV_WARPS), 0, stream, A, W, C, M, N, K, lda, ldw, ldc, ex);
 }
 
-// How many clusters of `ks` CTAs the GPU holds at once, one CTA an SM.
-static int f32_clusters(int ks) {
+// How many clusters of `ks` CTAs the current device, `dev`, holds at once, one CTA an SM.
+static int f32_clusters(int ks, int dev) {
     static int known[64][9];
-    int dev = 0, n = 0;
-    if (ks < 2 || ks > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = 0;
+    if (ks < 2 || ks > 8 || dev < 0 || dev >= 64) return 0;
     if ((n = __atomic_load_n(&known[dev][ks], __ATOMIC_RELAXED)) != 0) return n > 0 ? n : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, ks);
@@ -725,8 +725,15 @@ static int f32_clusters(int ks) {
 // rows on, where the products are the bound, 0.0056 more; bringing the slices together 2 to 7, the more the larger the share of the tile's columns that a CTA
 // adds up.  64 rows x [1024, 1024] in 1, 2, 4 and 8 slices 21.8, 15.9, 10.6, 8.7; 642 x [1024, 2048] as 112 tiles of 48 rows 40.8, as 56 of 96 rows in two slices
 // 30.0; 642 x [3072, 1024] in tiles of 64, 96, 112 and 128 rows 46.1, 49.8, 28.6, 30.0; 257 x [4096, 4096] in tiles of 64, 80, 96 and 128 rows 153, 80, 88, 103.
+// The choice for the sizes of a model's products is kept, by thread (2 us a call otherwise, which a step that is not replayed from a graph would wait for).
 struct F32Plan { int bn, ks; };
 static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
+    struct Kept { long long rows, sets; int N, K, dev; F32Plan plan; };
+    static thread_local Kept table[64];                        // rows 0: empty
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); dev = -1; }
+    Kept& kept = table[((unsigned)rows * 31u + (unsigned)N * 7u + (unsigned)K / 4u + (unsigned)sets) % 64u];
+    if (kept.rows == rows && kept.sets == sets && kept.N == N && kept.K == K && kept.dev == dev) return kept.plan;
     const int sms = airun_sm_count(), steps = ceil_div_i(K, XK);
     const long long nt = (N + XT - 1) / XT * sets;
     F32Plan best = {XB, 1};
@@ -735,12 +742,13 @@ static F32Plan f32_plan(long long rows, long long sets, int N, int K) {
         const long long tiles = nt * ((rows + bn - 1) / bn);
         for (int ks = 1; ks <= 8 && (ks == 1 || 2 * ks <= steps); ++ks) {
             const int per = (steps + ks - 1) / ks;
-            if ((steps + per - 1) / per != ks || (ks > 1 && tiles > f32_clusters(ks))) continue;   // an empty slice, or not all resident
+            if ((steps + per - 1) / per != ks || (ks > 1 && tiles > f32_clusters(ks, dev))) continue;   // an empty slice, or not all resident
             const double step = 1.13 + 0.0006 * bn + 0.0056 * (bn > 80 ? bn - 80 : 0), merge = ks > 1 ? 1.2 + bn * (0.015 + 0.06 / ks) : 0.0;
             const double us = (double)((tiles * ks + sms - 1) / sms) * per * step + merge;
             if (us < best_us) { best_us = us; best = {bn, ks}; }
         }
     }
+    kept = {rows, sets, N, K, dev, best};
     return best;
 }
 

@@ -135,3 +135,16 @@ def test_grouped():
         lo, hi = cuts[e], cuts[e + 1]
         assert bool(((out[lo:hi].double() - x[lo:hi].double() @ w[e].double().T).abs() <= bound(x[lo:hi], w[e])).all())
     assert bool((out[390:] == 7.0).all()) and err.item() == 0
+
+
+@gpu
+def test_plans_that_share_a_place():
+    """Sizes in turn whose plans are kept in one place of the table (its number is 31 M + 7 N + K / 4 modulo 64)."""
+    from airun_b200.kernels import ops
+    sizes = [(17, 64, 1024), (81, 64, 1024), (145, 128, 1024), (17, 64, 1280)]
+    assert len({(31 * M + 7 * N + K // 4) % 64 for M, N, K in sizes}) == 1
+    for M, N, K in sizes * 2 + sizes[::-1]:
+        x, w = operands(M, N, K, 3)
+        out, err = torch.empty(M, N, device="cuda"), word()
+        ops.gemm_simt(x, w, out, err)
+        assert bool(((out.double() - x.double() @ w.double().T).abs() <= bound(x, w)).all()) and err.item() == 0

@@ -900,10 +900,16 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
 // expert).  Where the segments lie is only known on the device, so every CTA first lists their tiles in shared memory.  A segment is cut into tiles of
 // equal width, the least multiple of 32 that holds its rows, so little is computed for rows that are not there; a tile's columns beyond its
 // segment's end are not stored.  The launch is sized for the most tiles any cut can have, ceil(rows / 256) + segments.
+// IN_PARTS: the tensor cores cut a running sum off where float32 rounds, so its error grows with the products in it: 2.2e-6 at K = 1,024, 7.8e-6 at 2,816, 1.4e-5
+// at 4,096 (operands of one sign, 2-norm, float32 results).  Few tiles, whose K would otherwise be cut into slices of 512 values and more (0.8e-6, 0.9e-6, 2.2e-6), keep no longer
+// sums here: a buffer of tensor memory holds PAIR_PART K-steps, and the epilogue's warps add them up in registers, rounded, while the other is filled.  A step's
+// issue is what bounds such a product, 280 clocks, and a part adds 500: 512 tokens x [2048, 2048] 9.7 -> 11.0 us.
 #define GROUP_MAX_TILES 1024
 #define GROUP_MAX_SEGS 1024
 #define PAIR_STAGES 6
 #define PAIR_BN 256
+#define PAIR_PART 8                           // K-steps of a part of a sum
+#define PAIR_PARTS_BN 128                     // most tokens of a tile with parts: 64 sums a thread in registers
 #define PAIR_BOX 64                           // tokens a load of a grouped product brings: half a tile is one or two of them
 #define PAIR_STAGE_BYTES (2 * 128 * BK * 2)
 #define PAIR_THREADS 320
@@ -960,7 +966,7 @@ __device__ __forceinline__ void store_pair(const GemmParams& p, const float* v, 
     }
 }
 
-template <int EPI, bool GROUPED>
+template <int EPI, bool GROUPED, bool IN_PARTS>
 __global__ __launch_bounds__(PAIR_THREADS, 1) void gemm_pair_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p, int bn, int tok_tiles) {
     pdl_trigger();
@@ -1061,62 +1067,108 @@ __global__ __launch_bounds__(PAIR_THREADS, 1) void gemm_pair_kernel(
         if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
     } else if (warp == 1) {
         if (rank == 0) {
-            int n = 0;
-            for (int tile = pair; tile < total && ok; tile += pairs, ++n) {
-                const int buf = n & 1, width = tile_of(tile).bn;
-                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-                if (!mbar_wait_warp(acce + 8 * buf, ((n >> 1) & 1) ^ 1)) { ok = false; break; }
+            int n = 0;                                             // sums so far
+            auto sum_up = [&](int first, int end, uint32_t idesc) {
+                const int buf = n & 1;
+                if (!mbar_wait_warp(acce + 8 * buf, ((n >> 1) & 1) ^ 1)) { ok = false; return; }
                 tc_fence_after();
-                for (int kb = 0; kb < kb_total; ++kb) {
-                    if (!mbar_wait_warp(full + 8 * s, phase)) { ok = false; break; }
+                for (int kb = first; kb < end; ++kb) {
+                    if (!mbar_wait_warp(full + 8 * s, phase)) { ok = false; return; }
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem) + s * PAIR_STAGE_BYTES;
                     const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + 128 * BK * 2);
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k)
-                            umma_bf16_pair(tmem + buf * PAIR_BN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                            umma_bf16_pair(tmem + buf * PAIR_BN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > first || k > 0) ? 1u : 0u);
                         umma_commit_pair(empty + 8 * s);
-                        if (kb + 1 == kb_total) umma_commit_pair(accf + 8 * buf);
+                        if (kb + 1 == end) umma_commit_pair(accf + 8 * buf);
                     }
                     __syncwarp();
                     if (++s == PAIR_STAGES) { s = 0; phase ^= 1; }
                 }
+                ++n;
+            };
+            for (int tile = pair; tile < total && ok; tile += pairs) {
+                const int width = tile_of(tile).bn;
+                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+                if (!IN_PARTS) sum_up(0, kb_total, idesc);
+                else for (int first = 0; first < kb_total && ok; first += PAIR_PART) sum_up(first, min(first + PAIR_PART, kb_total), idesc);
             }
             if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
         }
     } else {
         const int quad = warp & 3, half = (warp - 2) >> 2;         // two warps a quadrant of lanes, every other 32 columns
-        int n = 0;
-        for (int tile = pair; tile < total; tile += pairs, ++n) {
-            const int buf = n & 1;
+        int n = 0;                                                 // sums so far
+        for (int tile = pair; tile < total && ok; tile += pairs) {
             const Tile t = tile_of(tile);
             const int row = t.w0 + rank * 128 + quad * 32 + lane;
             const bool row_on = row < p.a_rows;
-            if (!mbar_wait(accf + 8 * buf, (n >> 1) & 1)) { atomicOr(p.err, AIRUN_DEV_TIMEOUT); break; }
-            tc_fence_after();
-            const uint32_t lanes = tmem + buf * PAIR_BN + ((uint32_t)(quad * 32) << 16);
-            auto hand_back = [&] {
+            const int cols = min(t.bn, t.t_end - t.t0);
+            auto ready = [&](int buf) {
+                ok = mbar_wait(accf + 8 * buf, (n >> 1) & 1);
+                if (!ok) atomicOr(p.err, AIRUN_DEV_TIMEOUT);
+                tc_fence_after();
+                return ok;
+            };
+            auto hand_back = [&](int buf) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(acce_lead + 8 * buf) : "memory");
             };
-            const int cols = min(t.bn, t.t_end - t.t0);
-            if (32 * half >= cols) hand_back();                    // nothing of this tile is this warp's
+            if constexpr (IN_PARTS) {
+                float acc[PAIR_PARTS_BN / 64][32];                 // columns 32 half + 64 j and 31 more
+                for (int kb = 0; kb < kb_total; kb += PAIR_PART, ++n) {
+                    const int buf = n & 1;
+                    if (!ready(buf)) break;
+                    const uint32_t lanes = tmem + buf * PAIR_BN + ((uint32_t)(quad * 32) << 16) + 32 * half;
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < PAIR_PARTS_BN / 64; ++j) {
+                        if (32 * half + 64 * j >= cols) break;
+                        uint32_t r[32];
+                        tmem_ld32_async(lanes + 64 * j, r);
+                        tmem_wait32(r);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) acc[j][i] = kb == 0 ? __uint_as_float(r[i]) : acc[j][i] + __uint_as_float(r[i]);
+                    }
+                    hand_back(buf);
+                }
+                if (!ok) break;
+                // one body for all columns, the next ones moved up in the registers (unrolled, the activations' code would not stay in the instruction cache)
 #pragma unroll 1
-            for (int c = 32 * half; c < cols; c += 64) {
-                uint32_t r[32];
-                __syncwarp();
-                tmem_ld32_async(lanes + c, r);
-                tmem_wait32(r);
-                if (c + 64 >= cols) hand_back();
+                for (int c = 32 * half; c < cols; c += 64) {
 #pragma unroll
-                for (int h = 0; h < 32; h += 16) {
-                    float v[16];
+                    for (int h = 0; h < 32; h += 16) {
+                        if (EPI != EPI_SWIGLU && p.act) epilogue_act(acc[0] + h, p.act - 1);
+                        store_pair<EPI>(p, acc[0] + h, row, row_on, t.t0 + c + h, cols - c - h);
+                    }
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h + i]);
-                    if (EPI != EPI_SWIGLU && p.act) epilogue_act(v, p.act - 1);
-                    store_pair<EPI>(p, v, row, row_on, t.t0 + c + h, cols - c - h);
+                    for (int j = 0; j + 1 < PAIR_PARTS_BN / 64; ++j)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) acc[j][i] = acc[j + 1][i];
+                }
+            } else {
+                const int buf = n & 1;
+                if (!ready(buf)) break;
+                ++n;
+                const uint32_t lanes = tmem + buf * PAIR_BN + ((uint32_t)(quad * 32) << 16);
+                if (32 * half >= cols) hand_back(buf);             // nothing of this tile is this warp's
+#pragma unroll 1
+                for (int c = 32 * half; c < cols; c += 64) {
+                    uint32_t r[32];
+                    __syncwarp();
+                    tmem_ld32_async(lanes + c, r);
+                    tmem_wait32(r);
+                    if (c + 64 >= cols) hand_back(buf);
+#pragma unroll
+                    for (int h = 0; h < 32; h += 16) {
+                        float v[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h + i]);
+                        if (EPI != EPI_SWIGLU && p.act) epilogue_act(v, p.act - 1);
+                        store_pair<EPI>(p, v, row, row_on, t.t0 + c + h, cols - c - h);
+                    }
                 }
             }
         }
@@ -1244,13 +1296,13 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmPa
 
 #if !AIRUN_FOLD_NORM
 // How many pairs the GPU holds at once (0: unknown).
-template <int EPI, bool GROUPED>
+template <int EPI, bool GROUPED, bool IN_PARTS>
 int pair_capacity() {
     static int known[64];
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if ((n = __atomic_load_n(&known[dev], __ATOMIC_RELAXED)) > 0) return n;
-    auto kern = gemm_pair_kernel<EPI, GROUPED>;
+    auto kern = gemm_pair_kernel<EPI, GROUPED, IN_PARTS>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2);
@@ -1268,14 +1320,14 @@ int pair_capacity() {
     return n;
 }
 
-template <int EPI, bool GROUPED>
+template <int EPI, bool GROUPED, bool IN_PARTS = false>
 int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int bn, int tok_tiles, cudaStream_t stream) {
-    const int cap = pair_capacity<EPI, GROUPED>();
+    const int cap = pair_capacity<EPI, GROUPED, IN_PARTS>();
     if (cap <= 0) { cudaGetLastError(); return AIRUN_ERR_UNSUPPORTED; }
     const long long total = (long long)((p.a_rows + 255) / 256) * tok_tiles;
     if (total > 0x3fffffff) return AIRUN_ERR_ARG;
     const int pairs = total < cap ? (int)total : cap;
-    airun_launch_clusters(gemm_pair_kernel<EPI, GROUPED>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, stream, dim3(2), mw, mx, p, bn, tok_tiles);
+    airun_launch_clusters(gemm_pair_kernel<EPI, GROUPED, IN_PARTS>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, stream, dim3(2), mw, mx, p, bn, tok_tiles);
     return airun_launch_status();
 }
 #endif
@@ -1440,12 +1492,13 @@ static int gemm_launch(const void* x, const void* W, void* out, int M, int N, in
 
 #if !AIRUN_FOLD_NORM
 // out[M][N] = x[M][K] * W[N][K]^T, two SMs to a tile of 256 weight rows x bn tokens (bn a multiple of 32 up to 256).  epi 0, 1, 2 as above; act: 0, or
-// 1 + the mode of an activation (epi 0 and 1); limit > 0: the clamped gated unit (epi 2).
+// 1 + the mode of an activation (epi 0 and 1); limit > 0: the clamped gated unit (epi 2).  in_parts: no sum over more than PAIR_PART K-steps in tensor
+// memory (bn up to PAIR_PARTS_BN).
 AIRUN_EXPORT int airun_gemm_pair(const void* x, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldc, int epi,
-                                 int act, float limit, float slope, int bn, int* err, cudaStream_t stream) {
+                                 int act, float limit, float slope, int bn, int in_parts, int* err, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0 || !err) return M == 0 ? AIRUN_OK : AIRUN_ERR_ARG;
     if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)W & 15)) return AIRUN_ERR_ARG;
-    if (bn < 32 || bn > PAIR_BN || bn % 32 || act < 0 || act > 5 || (epi == EPI_SWIGLU && (N % 32 != 0 || act))) return AIRUN_ERR_ARG;
+    if (bn < 32 || bn > (in_parts ? PAIR_PARTS_BN : PAIR_BN) || bn % 32 || act < 0 || act > 5 || (epi == EPI_SWIGLU && (N % 32 != 0 || act))) return AIRUN_ERR_ARG;
     GemmParams p = {};
     p.a_rows = N;
     p.b_rows = M;
@@ -1461,9 +1514,11 @@ AIRUN_EXPORT int airun_gemm_pair(const void* x, const void* W, void* out, int M,
     if ((r = make_map(&mw, W, N, K, ldw, 128)) != AIRUN_OK) return r;
     if ((r = make_map(&mx, x, M, K, ldx, bn / 2)) != AIRUN_OK) return r;
     const int tiles = (M + bn - 1) / bn;
-    if (epi == EPI_F32) return launch_pair<EPI_F32, false>(mw, mx, p, bn, tiles, stream);
-    if (epi == EPI_BF16) return launch_pair<EPI_BF16, false>(mw, mx, p, bn, tiles, stream);
-    if (epi == EPI_SWIGLU) return launch_pair<EPI_SWIGLU, false>(mw, mx, p, bn, tiles, stream);
+#define LAUNCH_PAIR(EPI) (in_parts ? launch_pair<EPI, false, true>(mw, mx, p, bn, tiles, stream) : launch_pair<EPI, false>(mw, mx, p, bn, tiles, stream))
+    if (epi == EPI_F32) return LAUNCH_PAIR(EPI_F32);
+    if (epi == EPI_BF16) return LAUNCH_PAIR(EPI_BF16);
+    if (epi == EPI_SWIGLU) return LAUNCH_PAIR(EPI_SWIGLU);
+#undef LAUNCH_PAIR
     return AIRUN_ERR_UNSUPPORTED;
 }
 #endif

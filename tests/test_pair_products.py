@@ -23,18 +23,21 @@ def check(got, want, most, K, dtype):
 
 
 @gpu
+@pytest.mark.parametrize("in_parts", [False, True])
 @pytest.mark.parametrize("M,N,K,bn", SHAPES)
-def test_plain_activation_and_gated(M, N, K, bn):
+def test_plain_activation_and_gated(M, N, K, bn, in_parts):
+    """``in_parts``: one part of a few K-steps to several with a short last one, over several tiles."""
     from airun_b200.kernels import fast, ops
+    bn = min(bn, fast.PAIR_PARTS_BN) if in_parts else bn
     x, w = operands(M, N, K, M + N + K)
     want, most = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     for dtype, epi in ((torch.float32, fast.EPI_F32), (torch.bfloat16, fast.EPI_BF16)):
         out = torch.full((M, N + 8), 3.0, device="cuda", dtype=dtype)
-        fast.gemm_pair(x, w, out[:, :N], epi, err, bn=bn)
+        fast.gemm_pair(x, w, out[:, :N], epi, err, bn=bn, in_parts=in_parts)
         check(out[:, :N], want, most, K, dtype)
         assert bool((out[:, N:] == 3.0).all())
-        fast.gemm_pair(x, w, out[:, :N], epi, err, bn=bn, act=ops.ACT_SILU)
+        fast.gemm_pair(x, w, out[:, :N], epi, err, bn=bn, act=ops.ACT_SILU, in_parts=in_parts)
         check(out[:, :N], want * torch.sigmoid(want), 1.1 * most, K, dtype)
     if N % 32 == 0:
         g, u = want.view(M, N // 32, 2, 16).unbind(2)
@@ -46,7 +49,7 @@ def test_plain_activation_and_gated(M, N, K, bn):
             else:
                 y = g * torch.sigmoid(g) * u
             out = torch.full((M, N // 2 + 8), 3.0, device="cuda", dtype=torch.bfloat16)
-            fast.gemm_pair(x, w, out[:, :N // 2], fast.EPI_SWIGLU, err, bn=bn, glu=(limit, slope))
+            fast.gemm_pair(x, w, out[:, :N // 2], fast.EPI_SWIGLU, err, bn=bn, glu=(limit, slope), in_parts=in_parts)
             size = (g.abs() + 1.0) * s[:, :, 1] + (u.abs() + 1.0) * s[:, :, 0] * 1.2
             check(out[:, :N // 2], y.reshape(M, -1), size.reshape(M, -1), K, torch.bfloat16)
             assert bool((out[:, N // 2:] == 3.0).all())
@@ -73,6 +76,46 @@ def test_segments(cuts):
 
 
 @gpu
+@pytest.mark.parametrize("one_sign", [False, True])
+@pytest.mark.parametrize("M,N,K", [(65, 64, 1024), (100, 1024, 1024), (128, 5632, 1000), (129, 300, 2048), (200, 2048, 2048), (900, 512, 2048)])
+def test_sums_are_no_less_exact_where_pairs_replace_slices(M, N, K, one_sign):
+    """Float32 results of the two against 64 bits.  Both cut K where one long sum in tensor memory, whose cuts grow with it, would be further off."""
+    from types import SimpleNamespace
+    from airun_b200.kernels import fast
+    x, w = operands(M, N, K, 12)
+    if one_sign:
+        x, w = x.abs(), w.abs()
+    ctx = SimpleNamespace(err=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    sms, plan = fast.machine().sms, fast.plan_gemm(M, N, K)
+    if sms == fast.B200_SMS:
+        assert plan[2] > 1 and fast.pair_form(M, N, K) == fast.PAIRS_PARTS
+    want, pairs, slices = x.double() @ w.double().T, torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    assert fast.linear_bf16(ctx, x, w, pairs)
+    fast.gemm_tcgen05(x, w, slices, fast.EPI_F32, *plan, ctx.err)
+    assert ctx.err.item() == 0 and (pairs.double() - want).norm() <= 1.02 * (slices.double() - want).norm()
+
+
+@gpu
+@pytest.mark.parametrize("K", [200, 1000])
+def test_more_tiles_of_segments_than_pairs(K):
+    """The stages and the two sums run on over tiles of different widths: K shorter and longer than the six stages."""
+    from types import SimpleNamespace
+    from airun_b200.kernels import fast
+    E, N, cuts = 6, 4160, [0, 1, 34, 291, 891, 891, 1400]
+    M = cuts[-1]
+    x, _ = operands(M, 1, K, 13)
+    x = x.contiguous()
+    w = (torch.randn(E, N, K, device="cuda") * K ** -0.5).bfloat16()
+    ctx, out = SimpleNamespace(err=torch.zeros(1, dtype=torch.int32, device="cuda")), torch.empty(M, N, device="cuda")
+    assert 17 * sum(-(-(b - a) // 256) for a, b in zip(cuts, cuts[1:])) > fast.machine().sms // 2
+    assert fast.grouped_linear_bf16(ctx, x, w, out, torch.tensor(cuts, dtype=torch.int32, device="cuda"))
+    for e in range(E):
+        a = x[cuts[e]:cuts[e + 1]].double()
+        check(out[cuts[e]:cuts[e + 1]], a @ w[e].double().T, a.abs() @ w[e].double().abs().T, K, torch.float32)
+    assert ctx.err.item() == 0
+
+
+@gpu
 @pytest.mark.parametrize("swiglu", [False, True])
 def test_segments_that_end_behind_the_rows(swiglu):
     """A list that names more rows than there are: no row behind the last is stored, the others are as without it."""
@@ -94,10 +137,27 @@ def test_segments_that_end_behind_the_rows(swiglu):
 
 
 def test_plan():
-    """Whatever the sizes, the width is one the kernel takes, and no narrower tile would need as few rounds."""
-    from airun_b200.kernels.fast import plan_pair
+    """Whatever the sizes, the width is one the kernel takes."""
+    from airun_b200.kernels.fast import PAIR_PARTS_BN, plan_pair
     for M in (1, 31, 129, 250, 512, 900, 1536, 2048, 8192):
         for N, K in ((32, 8), (300, 72), (2048, 2048), (6144, 2048), (24576, 4096), (151936, 4096)):
-            bn = plan_pair(M, N, K)
-            assert bn % 32 == 0 and 32 <= bn <= 256
+            for parts in (False, True):
+                bn = plan_pair(M, N, K, in_parts=parts)
+                assert bn % 32 == 0 and 32 <= bn <= (PAIR_PARTS_BN if parts else 256)
     assert plan_pair(512, 4096, 2048) == 128 and plan_pair(900, 6144, 2048) == 160 and plan_pair(2048, 2048, 6144) == 256
+
+
+def test_where_pairs_run():
+    """The borders of the rule: tokens, K-steps, rounds of tiles.  Where plan_gemm cuts K, no pair forms a sum over all of it."""
+    from airun_b200.kernels.fast import PAIRS_NOT, PAIRS_PARTS, PAIRS_WHOLE, pair_form, plan_gemm
+    for M, N, K, want in [
+            (64, 1024, 1024, PAIRS_NOT), (65, 1024, 1024, PAIRS_PARTS), (65, 1024, 1025, PAIRS_NOT), (128, 1024, 1024, PAIRS_PARTS),
+            (128, 12288, 2048, PAIRS_WHOLE), (128, 12288, 2056, PAIRS_NOT), (128, 20000, 1024, PAIRS_WHOLE),
+            (128, 32768, 2048, PAIRS_WHOLE), (129, 300, 2048, PAIRS_PARTS), (129, 128, 4096, PAIRS_NOT), (384, 2048, 3072, PAIRS_PARTS), (512, 2048, 6144, PAIRS_NOT),
+            (512, 4096, 2048, PAIRS_WHOLE), (2048, 2048, 2048, PAIRS_WHOLE),
+            (2048, 6144, 2048, PAIRS_WHOLE)]:
+        assert pair_form(M, N, K) == want, (M, N, K)
+    for M in (65, 100, 128, 129, 200, 256, 400, 512, 700, 1024, 2048):
+        for N in (64, 300, 1024, 2048, 4096, 6144, 12288, 20000):
+            for K in (512, 1024, 1536, 2048, 2816, 4096, 6144, 12288):
+                assert (pair_form(M, N, K) == PAIRS_WHOLE) <= (plan_gemm(M, N, K)[2] == 1)

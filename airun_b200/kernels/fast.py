@@ -281,16 +281,18 @@ def pair_form(M: int, N: int, K: int, sms: int = B200_SMS) -> int:
     [5632, 1024] 8.3, 7.2; 128 x [2048, 2048] 7.2, 9.3; 256 x [2048, 2048] 9.6, 9.6; 512 x [300, 2048] 9.9, 7.8; 384 x [2048, 3072] 15.8, 13.2; 512 x
     [2048, 3072] 13.2, 13.6; 900 x [2048, 6144] 27.5, 25.9; 512 x [1024, 2816] 10.2, 11.5.
 
-    Elsewhere, up to 128 tokens: K is short, or the rows are many.  128 tokens x [12288, 2048] 17.1, 13.9; [32768, 2048] 30.4, 28.6; 128 x [24576, 4096] 43.0, 44.0.  Above: few tiles by the estimates of both, more of
+    Elsewhere, up to 128 tokens: K is short, or the tiles fill their rounds of pairs.  128 tokens x [12288, 2048] 17.1, 13.9; [32768, 2048] 30.4, 28.6; 100 x
+    [20000, 2048], 79 tiles for 74 pairs, 20.7, 22.3; 128 x [24576, 4096] 43.0, 44.0.  Above: few tiles by the estimates of both, more of
     them always.  (Alone, one nearly full round of 128 x 256 with a short K is as fast or faster on single SMs, 2,048 x [2048, 2048] 15.0, 15.6, 768 x [5632,
     1024] 9.9, 10.8; within calls it is not: Gamanex's prompt, with those on single SMs, 2,599 -> 2,624 us.)"""
     if M <= 64:
         return PAIRS_NOT
-    kb, rows, mt = (K + 63) // 64, (N + 255) // 256, (M + 127) // 128
+    kb, rows, pairs, mt = (K + 63) // 64, (N + 255) // 256, sms // 2, (M + 127) // 128
     if plan_gemm(M, N, K, Machine(sms))[2] > 1:
         return PAIRS_PARTS if (kb <= 16 if M <= 128 else _plan_pair(M, N, K, sms, True)[1] <= _few_tiles_us(mt, N, kb, sms)) else PAIRS_NOT
     if M <= 128:
-        return PAIRS_WHOLE if kb <= 16 or kb <= 32 and 2 * ((N + 127) // 128) > sms else PAIRS_NOT
+        full = rows <= pairs or 4 * rows >= 3 * pairs * ((rows + pairs - 1) // pairs)
+        return PAIRS_WHOLE if kb <= 16 or kb <= 32 and full and 2 * ((N + 127) // 128) > sms else PAIRS_NOT
     if N >= 256 and mt * rows >= sms * 96 // B200_SMS:
         return PAIRS_WHOLE
     return PAIRS_WHOLE if _plan_pair(M, N, K, sms)[1] <= _few_tiles_us(mt, N, kb, sms) else PAIRS_NOT

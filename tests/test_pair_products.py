@@ -152,7 +152,7 @@ def test_where_pairs_run():
     from airun_b200.kernels.fast import PAIRS_NOT, PAIRS_PARTS, PAIRS_WHOLE, pair_form, plan_gemm
     for M, N, K, want in [
             (64, 1024, 1024, PAIRS_NOT), (65, 1024, 1024, PAIRS_PARTS), (65, 1024, 1025, PAIRS_NOT), (128, 1024, 1024, PAIRS_PARTS),
-            (128, 12288, 2048, PAIRS_WHOLE), (128, 12288, 2056, PAIRS_NOT), (128, 20000, 1024, PAIRS_WHOLE),
+            (128, 12288, 2048, PAIRS_WHOLE), (128, 12288, 2056, PAIRS_NOT), (128, 20000, 2048, PAIRS_NOT), (128, 20000, 1024, PAIRS_WHOLE),
             (128, 32768, 2048, PAIRS_WHOLE), (129, 300, 2048, PAIRS_PARTS), (129, 128, 4096, PAIRS_NOT), (384, 2048, 3072, PAIRS_PARTS), (512, 2048, 6144, PAIRS_NOT),
             (512, 4096, 2048, PAIRS_WHOLE), (2048, 2048, 2048, PAIRS_WHOLE),
             (2048, 6144, 2048, PAIRS_WHOLE)]:

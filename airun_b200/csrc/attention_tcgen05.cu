@@ -759,11 +759,11 @@ __device__ __forceinline__ float w_sigmoid(float x) {
 }
 enum { W_KFULL = 0, W_KEMPTY = 2, W_VFULL = 4, W_VEMPTY = 6, W_SFULL = 8, W_PFULL = 10, W_FINAL = 12, W_PHALF = 13 };
 
-// SPLIT (W_SIGMOID): two CTAs (a cluster) to a tile, each with half of the tile's keys.  With no more tiles than SMs the time is that of the longest tile, of
+// SPLIT (W_SIGMOID): two CTAs (a cluster) to a tile, each with half of the tile's keys.  With one tile an SM and no more, the time is that of the longest tile, of
 // twice the average's keys under a causal mask.  Afterwards CTA x takes Q tile x: the peer stores its part of the sums into this CTA's memory (the stages of K),
 // and they are added up.  Tiles of up to SPLIT_MIN_KEYS tiles of keys stay whole: the second CTA leaves at once.  A 2,048-token prompt of Gamanex (16 heads over 8 KV
 // heads, six layers) 2,636 -> 2,576 us (2,612 with tiles of up to 8 whole).  The softmax kinds, whose steps are shorter and whose sums need a common
-// scale, gained nothing: 3,050 -> 3,085 us for Tagulix, which has them with a table and with a window.
+// scale, gained nothing: 3,050 -> 3,085 us for Tagulix, which has them with a table and with a window.  Where it is taken: halves_of_keys.
 constexpr int SPLIT_MIN_KEYS = 4;
 template <int KIND, bool SPLIT = false>
 __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
@@ -1450,6 +1450,17 @@ AIRUN_EXPORT int airun_attn_prefill_wide(const void* q, void* out, const void* p
 }
 
 #if HD == 128
+// Two CTAs share a tile's keys where tiles of two Q tiles (chosen from wide_min_ctas on, 128 of 148 SMs: kernels/fast.py) come to no more than one an SM, with the
+// spare ones that the launch is sized for, and a window leaves them enough keys: prompts of one portion, 2,048 to 2,175 tokens with 8 KV heads in
+// groups of two, to 2,303 with 4 in groups of four.  B200, us, whole and halves: 2,048 tokens of 16 heads over 8 83.6, 63.8, behind 2,000 others 161, 128;
+// 2,300 of 16 over 4 102.5, 80.4.  Outside: more tiles than SMs are slower in halves (2,048 of 32 heads over 8 97.7, 129; three portions of 700 35.5, 46.5).  Shorter
+// prompts run one Q tile a CTA, and halves of those gain where they are few (1,024 tokens of 8 heads over 8 35.5, 25.1; of 16 over 8 40.5, 40.9, of which
+// two Q tiles a CTA in halves would take 29.4): not taken yet.
+static bool halves_of_keys(int kind, long long n_tiles, int nkv, int tile_rows, int window) {
+    return kind == W_SIGMOID && tile_rows == 2 * QM && n_tiles * nkv <= airun_sm_count() && (window == 0 || window > 2 * SPLIT_MIN_KEYS * KN);
+}
+AIRUN_EXPORT int airun_attn_prefill_in_halves(int kind, int n_tiles, int nkv, int tile_rows, int window) { return halves_of_keys(kind, n_tiles, nkv, tile_rows, window); }
+
 // The wide kernel for the softmax attention with its options and for the attention without softmax (head and value size
 // 128); tiles of up to tile_rows / G tokens, tile_rows 128 or 256.  kind: W_OPTIONS, W_TABLE or W_SIGMOID.  tail >= 0: the
 // pages hold one row of 128 + tail elements for key and value.  out, gate: rows of out_stride and gate_stride elements,
@@ -1492,9 +1503,7 @@ AIRUN_EXPORT int airun_attn_prefill_kinds(int kind, const void* q, void* out, lo
     const int r = kv_map_for(&map, pool, (long long)num_pages * (tail >= 0 ? 1 : 2) * nkv * page_size, width);
     if (r != AIRUN_OK) return r;
     static unsigned long long configured[4];             // one bit per device
-    // two CTAs share a tile's keys while all tiles would run at once, one to an SM, and a window leaves them enough keys
-    const bool split = kind == W_SIGMOID && tile_rows == 2 * QM && (long long)n_tiles * nkv <= airun_sm_count() &&
-                       (window == 0 || window > 2 * SPLIT_MIN_KEYS * KN);
+    const bool split = halves_of_keys(kind, n_tiles, nkv, tile_rows, window);
     auto go = [&](auto kern, int i) -> int {
         if (first_on_device(configured[i])) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);

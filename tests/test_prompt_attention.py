@@ -109,10 +109,21 @@ def test_attention_without_softmax(nh, nkv, page, window, dist, offset, spans):
 
 
 @gpu
-@pytest.mark.parametrize("nh,nkv,page,window,spans", [(2, 1, 16, 0, [(900, 1143)]), (1, 1, 32, 0, [(1500, 1900), (3, 4)]), (4, 2, 32, 1100, [(1900, 2300)]),
-                                                      (16, 8, 16, 0, [(512, 640), (0, 640)])])
-def test_attention_without_softmax_in_halves(nh, nkv, page, window, spans):
-    """Few tiles of many keys, whose halves two CTAs take: tiles of one and of two query tiles, whole ones among them, a window."""
+@pytest.mark.parametrize("nh,nkv,page,window,spans,halves", [
+    (16, 8, 16, 0, [(0, 2048)], True), (16, 8, 16, 0, [(512, 2612)], True), (16, 8, 32, 1100, [(300, 2360)], True), (16, 4, 16, 0, [(0, 2290)], True),
+    (16, 4, 32, 0, [(100, 2148), (3, 4)], True), (16, 4, 16, 1200, [(77, 2300)], True), (16, 8, 16, 1024, [(0, 2048)], False),
+    (16, 8, 16, 0, [(0, 2176)], False), (2, 1, 16, 0, [(900, 1143)], False)])
+def test_attention_without_softmax_in_halves(nh, nkv, page, window, spans, halves):
+    """Tiles whose keys two CTAs take, and that it is so: whole tiles of few keys beside them, a last tile of few rows and of one query tile, windows that cut
+    the first half's keys, tokens in front; and the borders of the rule."""
+    from airun_b200.kernels import fast
+    from ctypes import c_int
+    ctx, T, G = batch_ctx(spans), sum(e - s for s, e in spans), nh // nkv
+    rows = fast._prompt_tile_rows(T, G, nkv, torch.device("cuda"))
+    n = fast._prompt_tiles(ctx, G, rows, T)[1]
+    if fast.machine().sms == fast.B200_SMS:
+        f = fast._fn("attention_tcgen05", "airun_attn_prefill_in_halves", [c_int] * 5, {"HD": 128})
+        assert bool(f(fast.PROMPT_KINDS["sigmoid"], n, nkv, rows, window)) == halves
     test_attention_without_softmax(nh, nkv, page, window, True, True, spans)
 
 

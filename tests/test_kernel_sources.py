@@ -48,13 +48,19 @@ def test_what_a_step_writes_is_not_read_as_unchanging():
 
 
 def test_kernels_wait_before_they_end_and_trigger_first():
-    """A kernel that is launched early and never waits would let the kernel behind it start over unfinished work."""
+    """A kernel that is launched early and never waits would let the kernel behind it start over unfinished work.  Every kernel is looked at, however it is launched
+    (by name, through a variable or a macro, in clusters), but for those launched without the attribute."""
+    seen = set()
     for name, text in SOURCES.items():
-        launched = set(re.findall(r"airun_launch(?:_cluster)?\(\(*(\w+?)(?:<|,)", text))
-        for k in launched - {"kern", "KERNEL"}:
-            at = re.search(r"__global__[^;{]*?\b%s\s*\(" % k, text)
-            if at is None:
+        plain = set(re.findall(r"\b(\w+)(?:<[^<>;()]*>)?\s*<<<", text))
+        for at in re.finditer(r"__global__\s*(?:__launch_bounds__\([^)]*\))?\s*void\s+(\w+)\s*\(", text):
+            if at.group(1) in plain:
                 continue
             end = text.find("__global__", at.end())
             body = text[at.end():end if end > 0 else len(text)]
-            assert "pdl_wait()" in body and "pdl_trigger()" in body and body.index("pdl_trigger()") < body.index("pdl_wait()"), (name, k)
+            assert "pdl_wait()" in body and "pdl_trigger()" in body and body.index("pdl_trigger()") < body.index("pdl_wait()"), (name, at.group(1))
+            seen.add(at.group(1))
+        assert len(re.findall("__global__", text)) == len(re.findall(r"__global__\s*(?:__launch_bounds__\([^)]*\))?\s*void\s+\w+\s*\(", text)), name
+        launched = set(re.findall(r"\bairun_launch\w*\(\(*(\w+?)(?:<|,)", text))
+        assert launched <= seen | {"kern", "KERNEL", "kernel"}, (name, launched - seen)
+    assert {"gemm_pair_kernel", "gemm_tcgen05_kernel", "gemm_rows_kernel", "delta_chunk_kernel"} <= seen

@@ -160,6 +160,48 @@ def _check_gemm_tc(dev, M, N, K, epi, swap, bn, ksplit) -> Tuple[float, float]:
     return _rel(out, want), tol
 
 
+def check_gemm_f32_parts(dev) -> Tuple[float, float]:
+    """Float32 operands in three bfloat16 parts (csrc/gemm_simt.cu): rows that do not fill a tile, a last K-step that is not whole; the bound of one
+    float32 sum over all of K's steps."""
+    from .kernels import ops
+    M, N, K = 130, 260, 1100
+    a, w = torch.randn(M, K), torch.randn(N, K)
+    out, err = torch.empty(M, N, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    ops.gemm_simt(a.to(dev), w.to(dev), out, err)
+    torch.cuda.synchronize()
+    if int(err.item()):
+        raise RuntimeError(f"device error word {int(err.item())}")
+    want, most = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
+    return float(((out.double().cpu() - want).abs() / most).max()), 2.0 ** -23 * 5 + (K // 50 + 3) * 2.0 ** -24
+
+
+def check_gemm_pair(dev) -> Tuple[float, float]:
+    """Pairs of SMs (csrc/gemm_tcgen05.cu): ragged tokens and rows, whole sums and sums in parts, gated units, and experts' rows."""
+    from .kernels import fast
+    M, N, K, worst = 130, 328, 1096, 0.0
+    a, err = torch.randn(M, K).to(torch.bfloat16), torch.zeros(1, dtype=torch.int32, device=dev)
+    w = (torch.randn(2, N, K) * 0.05).to(torch.bfloat16)
+    full, most = a.double() @ w[0].double().T, a.double().abs() @ w[0].double().abs().T
+    for parts in (False, True):
+        out = torch.empty(M, N, device=dev)
+        fast.gemm_pair(a.to(dev), w[0].to(dev), out, fast.EPI_F32, err, in_parts=parts)
+        worst = max(worst, float(((out.double().cpu() - full).abs() / most).max()) / (K * 2.0 ** -23))
+    g, u = full[:, :320].view(M, -1, 2, 16)[:, :, 0].reshape(M, -1), full[:, :320].view(M, -1, 2, 16)[:, :, 1].reshape(M, -1)
+    out = torch.empty(M, 160, dtype=torch.bfloat16, device=dev)
+    fast.gemm_pair(a.to(dev), w[0, :320].contiguous().to(dev), out, fast.EPI_SWIGLU, err)
+    want = g / (1 + torch.exp(-g)) * u
+    worst = max(worst, float((out.double().cpu() - want).abs().max()) / (0.01 * (1.0 + float(want.abs().max()))))
+    ctx, out = _Ctx(dev, [0], [0], 1, [1], [1]), torch.empty(M, N, device=dev)
+    if not fast.grouped_linear_bf16(ctx, a.to(dev), w.to(dev), out, torch.tensor([0, 33, M], dtype=torch.int32, device=dev)):
+        raise RuntimeError("the experts' product did not run")
+    want = torch.cat([a[:33].double() @ w[0].double().T, a[33:].double() @ w[1].double().T])
+    most = torch.cat([a[:33].double().abs() @ w[0].double().abs().T, a[33:].double().abs() @ w[1].double().abs().T])
+    worst = max(worst, float(((out.double().cpu() - want).abs() / most).max()) / (K * 2.0 ** -23))
+    if int(err.item()) or int(ctx.err.item()):
+        raise RuntimeError(f"device error word {int(err.item()) | int(ctx.err.item())}")
+    return worst, 1.0
+
+
 def check_gemm_tc_portion(dev):
     from .kernels import fast
     return _check_gemm_tc(dev, 300, 520, 264, fast.EPI_F32, False, 256, 1)
@@ -714,6 +756,8 @@ CHECKS: List[Tuple[str, Callable]] = [
     ("swiglu", check_swiglu),
     ("q/k norm + rotary + cache write", check_qkv_post),
     ("product, float32 FFMA", check_gemm_simt),
+    ("product, float32 in parts on tcgen05", check_gemm_f32_parts),
+    ("product, tcgen05 on pairs of SMs, plain, gated and of experts", check_gemm_pair),
     ("product, tcgen05 128x256 tiles", check_gemm_tc_portion),
     ("product, tcgen05 swapped + split-K", check_gemm_tc_decode),
     ("product, tcgen05 SwiGLU epilogue", check_gemm_tc_swiglu),

@@ -24,7 +24,7 @@
 // error bit, skips the rest of its work, frees its tensor memory and returns.
 // From 17 tokens on the K slices of a tile run as one thread-block cluster and add up through distributed
 // shared memory (see push_slices); no TMA load uses multicast.
-// Most products of more than 128 tokens and all of experts run on pairs of SMs: gemm_pair_kernel.
+// Most products of more than 128 tokens, shorter ones of 65 on, and all of experts run on pairs of SMs: gemm_pair_kernel (kernels/fast.py: pair_form).
 //
 // The reference's counterparts are its wmma prefill GEMM and its half-precision
 // matvec kernels (crates/airun-cuda/kernels/matmul.cu:518-636, :1498-1563); its
@@ -696,7 +696,7 @@ __global__ __launch_bounds__(GEMM_THREADS, 1) void gemm_tcgen05_kernel(
     }
 }
 
-// ------------------------------------------------------------------ persistent variant (prompt portions)
+// ------------------------------------------------------------------ persistent variant (wide products of 65 to 128 tokens, per-head products, the folded norm)
 // One CTA per SM walks the tiles of the product (m fastest, so CTAs running side by side share a
 // weight tile).  The stage ring runs on across tiles, and the accumulator is double-buffered in
 // tensor memory (2 x 256 columns): while the epilogue warps drain tile i, the MMA thread is already

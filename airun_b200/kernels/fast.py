@@ -168,8 +168,9 @@ def plan_gemm(M: int, N: int, K: int, mach: Optional[Machine] = None) -> Tuple[b
     into up to 8 slices that run as one thread-block cluster and add up through distributed shared
     memory: as many as keep the CTAs within SPLIT_CTAS (all clusters must be resident at once; 288
     CTAs in clusters of 6 were not and took half as long again) and a slice at 8 K-steps or more.  Above
-    128 tokens, tiles of 128 x 256 on the persistent kernel once there are 96 of them; fewer tiles
-    leave SMs idle, so the tile narrows to 128 x 128 or K is cut, whichever takes less time (_plan_few_tiles).
+    128 tokens, tiles of 128 x 256 on the persistent kernel once there are 96 of them (only with the norm folded in: plain products
+    of that size run on pairs); fewer tiles leave SMs idle, so the tile narrows to 128 x 128 or K is cut, whichever takes less time
+    (_plan_few_tiles).  ``pair_form`` asks this plan whether K would be cut.
     All rules come from sweeps over the
     Qwen3-1.7B and -8B shapes, 1 to 2048 tokens, timed inside CUDA graphs."""
     mach = mach or machine()
@@ -381,7 +382,7 @@ def linear_swiglu_bf16(ctx, x: torch.Tensor, w_gu: torch.Tensor, out: torch.Tens
     return True
 
 
-GROUPED_MAX_TILES = 1024
+GROUPED_MAX_TILES = 1024               # of 256 rows or fewer, on pairs of SMs
 # A product goes to csrc/gemm_rows.cu up to this many rows a segment on average and up to this many tokens, which is what one
 # segment can hold: a segment reads its matrix again for every 8 or 16 rows.  16 matrices of 3072 x 2048 as gated units, weights
 # not in the L2 cache, tcgen05 and rows, us: 8 tokens of 4 experts 44.1, 35.7; 16 of 8 44.5, 42.4; 32 of 4 44.4, 42.5.  All
@@ -401,7 +402,7 @@ def grouped_linear_bf16(ctx, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor
     M, K = x.shape
     E, N = w.shape[0], w.shape[1]
     if ("gemm" in DISABLED or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or M == 0 or K % 8 or not x.is_contiguous()
-            or not w.is_contiguous() or x.data_ptr() % 16 or w.data_ptr() % 16 or (M + 127) // 128 + E > GROUPED_MAX_TILES):
+            or not w.is_contiguous() or x.data_ptr() % 16 or w.data_ptr() % 16 or (M + 255) // 256 + E > GROUPED_MAX_TILES):
         return False
     if swiglu_group:
         if swiglu_group != 16 or N % 32 or out.dtype != torch.bfloat16 or tuple(out.shape) != (M, N // 2):

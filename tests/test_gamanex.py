@@ -275,7 +275,7 @@ def test_activations_gates_and_the_scaled_head():
 @pytest.mark.parametrize("M,N,K", [(1, 320, 256), (9, 4096, 2048), (40, 512, 1024), (100, 768, 512), (300, 1024, 256), (1500, 4096, 512)])
 def test_activation_in_the_products_epilogue(M, N, K):
     """f(x W^T) with f applied to the finished sums inside the tensor-core product, for every way the product is cut
-    (weights or tokens as the wide operand, K in slices, the persistent kernel), against float64."""
+    (weights or tokens as the wide operand, K in slices, pairs of SMs), against float64."""
     from airun_b200.kernels import fast, ops
     g = torch.Generator().manual_seed(M + N)
     x = P.to_bf16_and_back(torch.randn(M, K, generator=g))

@@ -116,6 +116,25 @@ def test_more_tiles_of_segments_than_pairs(K):
 
 
 @gpu
+def test_as_many_rows_as_the_list_of_tiles_holds():
+    """The largest number of rows for five matrices, and one more, which is another kernel's."""
+    from types import SimpleNamespace
+    from airun_b200.kernels import fast
+    E, N, K = 5, 32, 64
+    M = 256 * (fast.GROUPED_MAX_TILES - E)
+    g = torch.Generator(device="cuda").manual_seed(14)
+    x, w = torch.randn(M + 1, K, device="cuda", generator=g).bfloat16(), torch.randn(E, N, K, device="cuda", generator=g).bfloat16()
+    cuts = [0, 1, M // 3, M // 3 + 1, M - 300, M]
+    seg, ctx = torch.tensor(cuts, dtype=torch.int32, device="cuda"), SimpleNamespace(err=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    out = torch.full((M + 1, N), 7.0, device="cuda")
+    assert not fast.grouped_linear_bf16(ctx, x, w, out, seg) and fast.grouped_linear_bf16(ctx, x[:M], w, out[:M], seg)
+    for e in range(E):
+        a = x[cuts[e]:cuts[e + 1]].double()
+        check(out[cuts[e]:cuts[e + 1]], a @ w[e].double().T, a.abs() @ w[e].double().abs().T, K, torch.float32)
+    assert bool((out[M] == 7.0).all()) and ctx.err.item() == 0
+
+
+@gpu
 @pytest.mark.parametrize("swiglu", [False, True])
 def test_segments_that_end_behind_the_rows(swiglu):
     """A list that names more rows than there are: no row behind the last is stored, the others are as without it."""

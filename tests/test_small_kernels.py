@@ -130,7 +130,7 @@ def test_products_with_the_tokens_as_columns(M, bn, epi, ksplit):
 
 
 @gpu
-@pytest.mark.parametrize("how", ["rows", "rows grouped", "columns", "columns cluster", "persistent", "persistent grouped"])
+@pytest.mark.parametrize("how", ["rows", "rows grouped", "columns", "columns cluster", "persistent", "pairs", "pairs grouped"])
 @pytest.mark.parametrize("limit", [0.0, 7.0])
 def test_gated_units_of_gates_far_below_zero(how, limit):
     """silu(-88) is -5e-37 and is multiplied by up to 1e30: the quotient's divisor, e^88, lies beyond 2^126, where the fast
@@ -163,6 +163,8 @@ def test_gated_units_of_gates_far_below_zero(how, limit):
             assert fast.grouped_linear_bf16(ctx, xd, wd[None].contiguous(), out, seg, swiglu_group=16, **(dict(glu=glu) if limit else {}))
         finally:
             fast.GROUPED_ROWS_MAX = old
+    elif how == "pairs":
+        fast.gemm_pair(xd, wd, out, fast.EPI_SWIGLU, ctx.err, glu=glu, in_parts=limit > 0)
     elif limit:
         assert fast.linear_glu_clamped_bf16(ctx, xd, wd, out, 16, limit, 1.0)
     elif how == "rows":

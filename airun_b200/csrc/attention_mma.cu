@@ -22,8 +22,7 @@
 //    memory.  With more than one slice each CTA
 //    writes (max, sum, acc) to scratch and the last CTA of the token and head (a
 //    counter, no spinning) merges the slices in order.
-#include "common.cuh"
-#include <cuda.h>
+#include "tcgen05.cuh"
 #include <mutex>
 #include <unordered_map>
 #include <cstring>
@@ -41,7 +40,6 @@ static_assert(HD % 16 == 0 && HD >= 16 && HD <= 256, "head_dim must be a multipl
 
 namespace {
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ int swz(int row, int chunk) { return SWZ ? (chunk ^ (row & 7)) : chunk; }
 // byte offset of (row, chunk) inside a [rows][HD] bf16 tile
 __device__ __forceinline__ uint32_t tile_off(int row, int chunk) { return (uint32_t)(row * CHUNKS + swz(row, chunk)) * 16u; }
@@ -70,38 +68,6 @@ __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b
 // A 16-key K (or V) tile is HD/64 boxes of 16 rows x 128 bytes, landed with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t tile_off_tma(int row, int chunk) {
     return (uint32_t)((chunk >> 3) * 2048 + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {     // bounded: about two seconds
-    for (int i = 0; i < 64; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    unsigned long long t0, t1;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    for (;;) {
-        for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-        if (t1 - t0 > 2000000000ull) return false;
-    }
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -809,23 +775,6 @@ __global__ __launch_bounds__(32 * DW) void attn_decode_kernel(const AttnParams p
             }
         }
     }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)f;
-    });
-    return fn;
 }
 
 // Tensor map of one layer's pages seen as [rows][HD] bfloat16, boxes of 16 rows x 64 values.

@@ -3,9 +3,9 @@
 //
 // One CTA = 128 packed query rows (128/G tokens x the G heads of one KV head) of one request.
 // Keys and values come in tiles of 128 keys:
-//   warp 0   : one thread issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of the K and V
+//   warp 0   : one elected thread issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of the K and V
 //              tiles, 16 keys (one page or a part of one) per box, into two stages each;
-//   warp 1   : allocates tensor memory; one thread issues tcgen05.mma:
+//   warp 1   : allocates tensor memory; one elected thread issues tcgen05.mma:
 //                S_j = Q K_j^T   (M=128, N=128, K=HD)   into one of two S buffers in tensor memory,
 //                O  += P_j V_j   (M=128, N=HD,  K=128)  into the O buffer, P_j read from shared memory,
 //                                                        V_j as an MN-major operand straight from its tile;
@@ -24,8 +24,7 @@
 // Every mbarrier wait is bounded (about two seconds); on a time-out the kernel sets an error
 // bit, stops working, frees its tensor memory and returns.  A launch of few tiles runs as clusters (SPLIT below); no load is
 // multicast.
-#include "common.cuh"
-#include <cuda.h>
+#include "tcgen05.cuh"
 #include <mutex>
 #include <unordered_map>
 #include <utility>
@@ -43,61 +42,11 @@ static_assert(HD == 64 || HD == 128, "this kernel is built for head_dim 64 or 12
 #define TC_THREADS 320
 #define NEG_BIG (-1.0e30f)
 #define LOG2E 1.4426950408889634f
-#define WAIT_NS 2000000000ull
 
 namespace {
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < 64; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    unsigned long long t0, t1;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    for (;;) {
-        for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-        if (t1 - t0 > WAIT_NS) return false;
-    }
-}
-// The same for a converged warp, with one answer for all of its lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // the A operand in tensor memory (rows on the lanes, two 16-bit values per column)
 __device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -129,11 +78,6 @@ __device__ __forceinline__ void umma_bf16_ta_lh(uint32_t tmem_d, uint32_t tmem_a
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     uint32_t r[32];
     asm volatile(
@@ -1338,21 +1282,6 @@ __global__ __launch_bounds__(TC_THREADS, 1) void attn_prefill_wide_kernel(
 }
 
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)f;
-    });
-    return fn;
-}
 // One layer's pages seen as [rows][row_elems] bfloat16, boxes of 16 rows x 64 values.
 int kv_map_for(CUtensorMap* out, const void* pool, long long rows, int row_elems = HD) {
     static std::unordered_map<const void*, std::pair<std::pair<long long, int>, CUtensorMap>> cache;

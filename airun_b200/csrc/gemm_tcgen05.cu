@@ -893,8 +893,8 @@ __global__ __launch_bounds__(P_THREADS, 1) void gemm_tcgen05_persistent_kernel(
 // memory: 32 KB an SM and step for the same products.  The weights are the 256-row operand so that the tokens, whose number is any, set the tile's other
 // side in steps of 32.  Pairs walk the tiles (tokens fastest: pairs side by side share weights); the stage ring runs on across tiles, the accumulator is
 // double-buffered.
-//   warp 0   : one thread issues this CTA's TMA loads (no multicast); they count towards the leader's barrier;
-//   warp 1   : allocates tensor memory; in the leader one thread issues the products and commits to both CTAs' barriers;
+//   warp 0   : one elected thread issues this CTA's TMA loads (no multicast); they count towards the leader's barrier;
+//   warp 1   : allocates tensor memory; in the leader one elected thread issues the products and commits to both CTAs' barriers;
 //   warps 2-9: epilogue; a lane is a weight row, so a warp stores 32 neighbouring results of a token at once.
 // GROUPED: the tokens' rows are segments, each with a weight matrix of its own (the experts of a routed feed-forward whose rows have been sorted by
 // expert).  Where the segments lie is only known on the device, so every CTA first lists their tiles in shared memory.  A segment is cut into tiles of

@@ -1,4 +1,4 @@
-// The instructions around tcgen05.mma, TMA and mbarriers that csrc/gemm_simt.cu and csrc/gemm_tcgen05.cu share.
+// The instructions around tcgen05.mma, TMA and mbarriers that the kernels on them share.
 #pragma once
 #include "common.cuh"
 #include <cuda.h>
@@ -90,7 +90,7 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
 
 // 32 columns of this thread's row, asked for and not waited for; tmem_wait32 waits for every load asked for so far and
 // hands the registers on (they are operands of the wait, so nothing that reads them is moved ahead of it).
-__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -100,7 +100,7 @@ __device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_wait32(uint32_t* r) {
     asm volatile(
         "tcgen05.wait::ld.sync.aligned;"
         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),

@@ -320,9 +320,9 @@ __global__ __launch_bounds__(256, 2) void gemm_f32_kernel(
 // 0.6, 1.0 (0.5, 0.6); 1 % 0.5, 0.5 (0.4, 0.4); one 0.25, 0.25.  K = 4,096 dense 1.8, 5.7 (1.6, 2.5); 10 % 1.4, 1.9 (1.3, 0.8); 1 % 0.9, 0.7 (0.7, 0.5): of many steps
 // with a few terms of one sign each, adding up the steps is the larger part.  Six products and one sum had 0.55 for one product.
 //
-// What the parts cannot hold is found and formed by a plain loop of multiply-adds (f32_plain_results): results that are not finite (an infinite operand
-// has no parts, and small products can overflow with the other sign), results below 2^-100, whose small products end at 2^-149, and the rows and columns
-// of an operand below 2^-110, whose last bits end at 2^-133.
+// What the parts cannot hold is found and formed by multiply-adds (f32_plain_results): results that are not finite (an infinite operand
+// has no parts, and small products can overflow with the other sign), results below 2^-100, whose small products end at 2^-149, and small results of
+// rows and columns with an operand below 2^-110, whose last bits end at 2^-133.
 //
 // A tile is 128 weight rows by `bn` rows of A (16 .. 128), its K range cut into `ks` slices that run as one cluster and are added up in order
 // through distributed shared memory.
@@ -392,23 +392,46 @@ __device__ __forceinline__ uint32_t f32_least(uint32_t least, const float4& v) {
 // Not a number for a result that the parts may not hold (see above), else zero (added up, one check answers for many results).
 __device__ __forceinline__ float f32_doubt(float v) { return fabsf(v) < 7.888609e-31f && v != 0.0f ? __int_as_float(0x7fffffff) : v * 0.0f; }
 
-// The results of a tile in doubt, and those in marked rows and columns, each by itself: columns first, first + step, .. of the tile.
+// The results of a tile that are in doubt, and the small ones (below 2^-20, whose terms' last bits can count) of marked rows and columns, a warp each: columns
+// first, first + step, .. of the tile.  Columns whose row of A holds a NaN are NaN already.  (Rows of padding hold whatever was in their place, so this must not be
+// slow: 642 x [3072, 1024], 29 us, with 64 rows of one infinite value 452 us (6,671 with a thread each), of one NaN 39, of one value below 2^-110 38, of nothing else 452.)
 __device__ __noinline__ void f32_plain_results(const float* A, const float* W, float* C, int K, long long lda, long long ldw, long long ldc, int m0,
                                                int cols, int n0, int rows, const uint32_t* marks, int first, int step) {
-    for (int i = threadIdx.x; i < cols * rows; i += blockDim.x) {
-        const int col = i / rows, r = i % rows;
-        if (col % step != first) continue;
-        float* c = C + (size_t)(m0 + col) * ldc + n0 + r;
-        const float doubt = f32_doubt(__ldcg(c));
-        if (doubt == doubt && !(((marks[r >> 5] >> (r & 31)) | (marks[4 + (col >> 5)] >> (col & 31))) & 1u)) continue;
-        const float4 *a = reinterpret_cast<const float4*>(A + (size_t)(m0 + col) * lda), *w = reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * ldw);
-        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int k = 0; 4 * k < K; ++k) {                      // (rows of a multiple of four values, aligned)
-            const float4 x = a[k], y = w[k];
-            s.x = fmaf(x.x, y.x, s.x); s.y = fmaf(x.y, y.y, s.y); s.z = fmaf(x.z, y.z, s.z); s.w = fmaf(x.w, y.w, s.w);
+    __shared__ uint32_t nan_cols[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    if (threadIdx.x < 4) nan_cols[threadIdx.x] = 0;
+    __syncthreads();
+    if (marks[8]) {
+        for (int col = warp; col < cols; col += warps) {
+            if (col % step != first) continue;
+            const float4* a = reinterpret_cast<const float4*>(A + (size_t)(m0 + col) * lda);
+            bool nan = false;
+            for (int k = lane; 4 * k < K; k += 32) { const float4 x = a[k]; nan |= isnan(x.x) | isnan(x.y) | isnan(x.z) | isnan(x.w); }
+            if (__any_sync(0xffffffffu, nan) && lane == 0) atomicOr(&nan_cols[col >> 5], 1u << (col & 31));
         }
-        const float v = (s.x + s.y) + (s.z + s.w);
-        *c = v;
+    }
+    __syncthreads();
+    for (int base = 32 * warp; base < cols * rows; base += 32 * warps) {
+        const int i = base + lane, col = i / rows, r = i % rows;
+        bool form = false;
+        if (i < cols * rows && col % step == first && !((nan_cols[col >> 5] >> (col & 31)) & 1u)) {
+            const float v = __ldcg(C + (size_t)(m0 + col) * ldc + n0 + r), doubt = f32_doubt(v);
+            form = doubt != doubt || (fabsf(v) < 9.5367432e-7f && (((marks[r >> 5] >> (r & 31)) | (marks[4 + (col >> 5)] >> (col & 31))) & 1u));
+        }
+        for (uint32_t left = __ballot_sync(0xffffffffu, form); left; left &= left - 1) {
+            const int j = base + __ffs(left) - 1, jc = j / rows, jr = j % rows;
+            const float4 *a = reinterpret_cast<const float4*>(A + (size_t)(m0 + jc) * lda), *w = reinterpret_cast<const float4*>(W + (size_t)(n0 + jr) * ldw);
+            float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+            for (int k = lane; 4 * k < K; k += 32) {           // (rows of a multiple of four values, aligned)
+                const float4 x = a[k], y = w[k];
+                s.x = fmaf(x.x, y.x, s.x); s.y = fmaf(x.y, y.y, s.y); s.z = fmaf(x.z, y.z, s.z); s.w = fmaf(x.w, y.w, s.w);
+            }
+            float v = (s.x + s.y) + (s.z + s.w);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) C[(size_t)(m0 + jc) * ldc + n0 + jr] = v;
+        }
     }
 }
 

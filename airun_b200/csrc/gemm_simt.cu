@@ -329,7 +329,7 @@ __global__ __launch_bounds__(256, 2) void gemm_f32_kernel(
 //   warps 0-7  : read the sums from tensor memory (a quadrant of lanes each, every other 16 columns) and add them up; they store the tile;
 //   warps 8-15 : cut the 64 k-values of a step of every row of both operands.  The parts of W go to tensor memory, those of A to shared memory
 //                (128-byte swizzle): with both there, what the products, the cutting and the loads move through shared memory is the bound (390 KB a
-//                step of 128 x 112, 3,300 clocks for 1,540 of products).  They load nothing themselves: their fence would wait for loads under way;
+//                step of 128 x 112, 3,300 clocks for 1,540 of six products).  They load nothing themselves: their fence would wait for loads under way;
 //   warp 16    : issues the 32 tcgen05.mma of a step (in a warp that adds up, no product would run while it does), the small products first: meanwhile
 //                the leading sum of the step before is read;
 //   warp 17    : issues the TMA loads, two steps ahead.
